@@ -262,16 +262,7 @@ __global__ void __launch_bounds__(S1_THREADS) sparse_stage1_score_kernel(const S
     }
 }
 
-// ---- max-pool to 64-token blocks, top-k, bitmask.  grid (T, hkv), 256 threads, up to 4096 blocks.
-constexpr int PT_THREADS = 256, PT_PER = 16;
-
-__device__ __forceinline__ unsigned long long score_key(bf16 v, int idx) {
-    // order: value descending, lower index first  (0 is below every key)
-    unsigned short b = __bfloat16_as_ushort(v);
-    b = (b & 0x8000u) ? static_cast<unsigned short>(~b) : static_cast<unsigned short>(b | 0x8000u);
-    return (static_cast<unsigned long long>(b) << 32) | static_cast<unsigned int>(0x7fffffff - idx);
-}
-
+// ---- max-pool to 64-token blocks, top-k, bitmask.
 struct PoolArgs {
     const bf16* scores;  // [hkv][T][score_ld]
     int score_ld, T;
@@ -284,8 +275,9 @@ struct PoolArgs {
     int bm_words;
 };
 
-// Pooled score of block k for query token t (maxpooling_kernel of the reference) as a selection key.
-__device__ __forceinline__ unsigned long long pooled_key(const PoolArgs& a, const bf16* in, int k, int k_len, int q_block) {
+// Pooled score of block k for query token t (maxpooling_kernel of the reference) as 16 bits whose unsigned order is
+// the order of the values; 0 is below every score.
+__device__ __forceinline__ uint32_t pooled_key(const PoolArgs& a, const bf16* in, int k, int k_len, int q_block) {
     bf16 v;
     if (k < a.init_blocks) {
         v = __ushort_as_bfloat16(0x7f80);  // +inf
@@ -299,23 +291,27 @@ __device__ __forceinline__ unsigned long long pooled_key(const PoolArgs& a, cons
         for (int i = start + 1; i < end; ++i) mx = fmaxf(mx, __bfloat162float(in[i]));
         v = __float2bfloat16(mx);
     }
-    return score_key(v, k);
+    const unsigned short b = __bfloat16_as_ushort(v);
+    return (b & 0x8000u) ? static_cast<unsigned short>(~b) : static_cast<unsigned short>(b | 0x8000u);
 }
 
-// One CTA of 128 threads per (kv head, token) row for up to 128 * PB blocks; thread i owns the PB consecutive
-// blocks i * PB ...  The row's scores are staged in shared memory (coalesced).  Instead of extracting one
-// maximum per round, the k-th largest 16-bit score is found by a bitwise binary search with block-wide counts
-// (16 steps, one barrier each), every block above it is taken, and the remaining picks among the blocks equal
-// to it go to the lowest indices (exclusive scan of the per-thread counts in thread = index order): the same
-// set as "value descending, lower index first".  grid (T, hkv).
+// One CTA of 128 threads per (kv head, token) row for up to 128 * PB blocks.  The row's scores are staged in shared
+// memory (coalesced), pooled with neighbouring threads on neighbouring blocks, and dealt out again: thread i owns the
+// ceil(blocks / 128) consecutive blocks from i * that on, so that the work follows the blocks there ARE, whatever the
+// cache could hold.  Instead of extracting one maximum per round, the k-th largest 16-bit score is found by a bitwise
+// binary search with block-wide counts (16 steps, one barrier each), every block above it is taken, and the remaining
+// picks among the blocks equal to it go to the lowest indices (exclusive scan of the per-thread counts in thread =
+// index order): the same set as "value descending, lower index first".  Latency of those barriers bounds it: over
+// a 32768-token prompt in chunks of 2048 (two key heads, cache of 65536 rows) a launch takes 16.5 us on average where a
+// loop that extracted one maximum per pick took 374 us.  grid (T, hkv).
 template <int PB>
-__global__ void __launch_bounds__(128) sparse_pool_topk_block_kernel(const PoolArgs a) {
+__global__ void __launch_bounds__(128) sparse_pool_topk_kernel(const PoolArgs a) {
     grid_dependency_sync();
     constexpr int CAP = 128 * PB * 4 + 128;   // staged scores: four per block and the pooling halo
     __shared__ __align__(16) bf16 row_s[CAP];
     __shared__ uint32_t s_cnt[2][4];
-    __shared__ uint32_t s_tot[2][4];
-    __shared__ unsigned long long s_words[PB * 2];
+    __shared__ uint32_t s_tot[4];
+    __shared__ unsigned long long s_words[PB * 2 + 1];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int t = blockIdx.x, g = blockIdx.y;
     uint64_t* out = a.blockmask + (static_cast<size_t>(g) * a.T + t) * a.bm_words;
@@ -330,20 +326,33 @@ __global__ void __launch_bounds__(128) sparse_pool_topk_block_kernel(const PoolA
     }
     const int n1 = compressed_len(L, C1_STRIDE);
     const int k_len = (n1 + 127) / 128 * 128;
-    const int out_len = (L + BLOCK - 1) / BLOCK;
+    const int out_len = min((L + BLOCK - 1) / BLOCK, 128 * PB);
     const int q_block = (t + L) / BLOCK;
     const bf16* in = a.scores + (static_cast<size_t>(g) * a.T + t) * a.score_ld;
     for (int i = tid * 8; i < k_len && i < CAP; i += 1024) {
         *reinterpret_cast<uint4*>(row_s + i) = *reinterpret_cast<const uint4*>(in + i);
     }
-    if (tid < PB * 2) s_words[tid] = 0ull;
+    for (int w = tid; w < PB * 2 + 1; w += 128) s_words[w] = 0ull;
     __syncthreads();
-    uint32_t val[PB];  // orderable 16-bit score of block tid * PB + j, 0 = no such block
+    uint32_t val[PB];  // first the keys of blocks tid, tid + 128, ..., then of the thread's own consecutive ones; 0 = no such block
+#pragma unroll
+    for (int j = 0; j < PB; ++j) {
+        const int k = tid + j * 128;
+        val[j] = (k < out_len) ? pooled_key(a, row_s, k, k_len, q_block) : 0u;
+    }
+    __syncthreads();
+    uint16_t* keys_s = reinterpret_cast<uint16_t*>(row_s);
+#pragma unroll
+    for (int j = 0; j < PB; ++j) {
+        const int k = tid + j * 128;
+        if (k < out_len) keys_s[k] = static_cast<uint16_t>(val[j]);
+    }
+    __syncthreads();
+    const int per = (out_len + 127) / 128, k0 = tid * per;   // uniform count, at most PB
     uint32_t valid = 0;
 #pragma unroll
     for (int j = 0; j < PB; ++j) {
-        const int k = tid * PB + j;
-        val[j] = (k < out_len) ? static_cast<uint32_t>(pooled_key(a, row_s, k, k_len, q_block) >> 32) : 0u;
+        val[j] = (j < per && k0 + j < out_len) ? keys_s[k0 + j] : 0u;
         valid += val[j] != 0u;
     }
     // block-wide sum of a per-thread count; `slot` alternates so that one barrier per call is enough
@@ -380,10 +389,10 @@ __global__ void __launch_bounds__(128) sparse_pool_topk_block_kernel(const PoolA
         const uint32_t up = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += up;
     }
-    if (lane == 31) s_tot[0][wid] = incl;
+    if (lane == 31) s_tot[wid] = incl;
     __syncthreads();
     uint32_t rank = incl - eq;
-    for (int w = 0; w < wid; ++w) rank += s_tot[0][w];
+    for (int w = 0; w < wid; ++w) rank += s_tot[w];
     uint32_t bits = 0;
 #pragma unroll
     for (int j = 0; j < PB; ++j) {
@@ -392,80 +401,13 @@ __global__ void __launch_bounds__(128) sparse_pool_topk_block_kernel(const PoolA
         rank += is_eq;
         bits |= static_cast<uint32_t>(take) << j;
     }
-    if (bits) atomicOr(&s_words[(tid * PB) >> 6], static_cast<unsigned long long>(bits) << ((tid * PB) & 63));
+    if (bits) {   // up to 32 bits from bit k0 on: they may reach into the next word
+        const int w = k0 >> 6, sh = k0 & 63;
+        atomicOr(&s_words[w], static_cast<unsigned long long>(bits) << sh);
+        if (sh > 32) atomicOr(&s_words[w + 1], static_cast<unsigned long long>(bits) >> (64 - sh));
+    }
     __syncthreads();
     for (int w = tid; w < a.bm_words; w += 128) out[w] = (w < PB * 2) ? s_words[w] : 0ull;
-}
-
-__global__ void __launch_bounds__(PT_THREADS) sparse_pool_topk_kernel(const PoolArgs a) {
-    grid_dependency_sync();
-    __shared__ unsigned long long sh_best[PT_THREADS / 32];
-    __shared__ unsigned long long words[64];
-    const int t = blockIdx.x, g = blockIdx.y, tid = threadIdx.x;
-    uint64_t* out = a.blockmask + (static_cast<size_t>(g) * a.T + t) * a.bm_words;
-    const int L = *a.kv_len + a.kv_add;
-    if (!selection_active(L, a.sparse_switch, a.compress_lse)) {
-        for (int w = tid; w < a.bm_words; w += PT_THREADS) out[w] = ~0ull;
-        return;
-    }
-    if (a.n_valid != nullptr && t >= *a.n_valid) {
-        for (int w = tid; w < a.bm_words; w += PT_THREADS) out[w] = 0ull;
-        return;
-    }
-    const int n1 = compressed_len(L, C1_STRIDE);
-    const int k_len = (n1 + 127) / 128 * 128;
-    const int out_len = (L + BLOCK - 1) / BLOCK;
-    const int q_block = (t + L) / BLOCK;
-    const bf16* in = a.scores + (static_cast<size_t>(g) * a.T + t) * a.score_ld;
-    unsigned long long keys[PT_PER];
-#pragma unroll
-    for (int j = 0; j < PT_PER; ++j) {
-        const int k = j * PT_THREADS + tid;
-        keys[j] = 0ull;
-        if (k < out_len) {
-            bf16 v;
-            if (k < a.init_blocks) {
-                v = __ushort_as_bfloat16(0x7f80);  // +inf
-            } else if (q_block - a.local_blocks < k) {
-                v = __ushort_as_bfloat16(0xff80);  // -inf
-            } else {
-                int start = k * 4 - 1, end = start + 5;
-                start = max(start, 0);
-                end = min(end, k_len);
-                float mx = __bfloat162float(in[start]);
-                for (int i = start + 1; i < end; ++i) mx = fmaxf(mx, __bfloat162float(in[i]));
-                v = __float2bfloat16(mx);
-            }
-            keys[j] = score_key(v, k);
-        }
-    }
-    if (tid < 64) words[tid] = 0ull;
-    __syncthreads();
-    for (int round = 0; round < a.topk; ++round) {
-        unsigned long long best = 0ull;
-#pragma unroll
-        for (int j = 0; j < PT_PER; ++j) best = (keys[j] > best) ? keys[j] : best;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
-            best = (other > best) ? other : best;
-        }
-        if ((tid & 31) == 0) sh_best[tid >> 5] = best;
-        __syncthreads();
-        best = sh_best[0];
-#pragma unroll
-        for (int w = 1; w < PT_THREADS / 32; ++w) best = (sh_best[w] > best) ? sh_best[w] : best;
-        __syncthreads();
-        if (best == 0ull) break;  // fewer blocks than topk: all of them are selected
-        const int idx = 0x7fffffff - static_cast<int>(best & 0xffffffffu);
-        if (tid == 0) words[idx >> 6] |= 1ull << (idx & 63);
-#pragma unroll
-        for (int j = 0; j < PT_PER; ++j) {
-            if (keys[j] == best) keys[j] = 0ull;
-        }
-    }
-    __syncthreads();
-    for (int w = tid; w < a.bm_words; w += PT_THREADS) out[w] = (w < 64) ? words[w] : 0ull;
 }
 
 }  // namespace
@@ -511,12 +453,15 @@ void launch_sparse_select(const SparseBuffers& b, const SparseConfig& cfg, int l
     p.init_blocks = cfg.sink_blocks; p.local_blocks = cfg.window_blocks; p.topk = cfg.topk;
     p.blockmask = b.blockmask; p.bm_words = b.bm_words;
     CPM_REQUIRE(b.bm_words <= 64, "sparse selection: at most 4096 blocks (262144 tokens)");
-    const int max_blocks = b.score_ld / 4 + 1;  // score_ld >= budget / 16
+    const int max_blocks = b.score_ld / 4;  // score_ld >= budget / 16, four scores a block
+    // the smallest variant that holds the cache's blocks: registers and staging grow with it
     if (max_blocks <= 512) {
-        launch_kernel(sparse_pool_topk_block_kernel<4>, dim3(T, hkv), dim3(128), 0, s, p);
+        launch_kernel(sparse_pool_topk_kernel<4>, dim3(T, hkv), dim3(128), 0, s, p);
     } else if (max_blocks <= 1024) {
-        launch_kernel(sparse_pool_topk_block_kernel<8>, dim3(T, hkv), dim3(128), 0, s, p);
+        launch_kernel(sparse_pool_topk_kernel<8>, dim3(T, hkv), dim3(128), 0, s, p);
+    } else if (max_blocks <= 2048) {
+        launch_kernel(sparse_pool_topk_kernel<16>, dim3(T, hkv), dim3(128), 0, s, p);
     } else {
-        launch_kernel(sparse_pool_topk_kernel, dim3(T, hkv), dim3(PT_THREADS), 0, s, p);
+        launch_kernel(sparse_pool_topk_kernel<32>, dim3(T, hkv), dim3(128), 0, s, p);
     }
 }

@@ -55,6 +55,12 @@ SELECT_CASES = [
     (16, 4, 1, 1000, 64, 1, 3, True, None),   # fewer candidate blocks than top-k
     (9, 8, 2, 3000, 12, 1, 4, True, 40960),   # up to 1024 blocks: 32 keys per lane
     (9, 8, 2, 3000, 12, 1, 4, True, 69632),   # more than 1024 blocks: block-wide selection
+    # a thread owns ceil(blocks / 128) blocks: fewer blocks than threads, one block too many for an even share, ties across
+    # mask words (the walk's first blocks score alike), the largest cache, and a cache that is full to the last row
+    (5, 16, 1, 5000, 64, 1, 4, True, 65536),
+    (6, 8, 2, 8256, 30, 1, 2, True, 131072),
+    (3, 4, 1, 20000, 64, 1, 32, True, 262144),
+    (4, 8, 2, 16380, 7, 0, 1, False, 16384),
 ]
 
 
