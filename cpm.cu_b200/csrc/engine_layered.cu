@@ -532,7 +532,7 @@ void Engine::layered_mixture(int i, LayeredPlans& lp, cudaStream_t s) {
         launch_linear_f32(single ? x : static_cast<const float*>(moe_x_), L, w.gate_up, moe_gate_up_offset(sp, L, 1), gu, 2 * ff, 0, 2 * ff, L,
                           moe_.entries, moe_.n_entries, most, false, s);
         launch_silu_f32(gu, 2 * ff, act, ff, slots, ff, s);
-        launch_linear_f32(act, ff, w.down, moe_down_offset(sp, W, 1), y, L, 0, W, ff, moe_.entries, moe_.n_entries, most, true, s);
+        launch_linear_f32(act, ff, w.down, moe_down_offset(sp, W, 1), y, L, rows, W, ff, moe_.entries, moe_.n_entries, most, true, s);
         if (ffs > 0) {
             launch_linear_f32(x, L, w.gate_up + moe_gate_up_offset(sp, L, sp.experts), 0, gu, 2 * ffs, rows, 2 * ffs, L, nullptr, nullptr, 0, false, s);
             launch_silu_f32(gu, 2 * ffs, act, ffs, rows, ffs, s);

@@ -209,7 +209,7 @@ bool scan_step_fits(int dim, int vdim, bool time_mix);
 template <typename T>
 void launch_scan_step(const ScanStepArgs& a, cudaStream_t s);
 
-// Attention of any head width up to 512, one warp per (token, head); q [tq][hq][dk], caches [.][hkv][dk | dv], out rows
+// Attention of any head width up to 512; q [tq][hq][dk], caches [.][hkv][dk | dv], out rows
 // of hq * out_cols.  The bias, window and kv_len arguments are those of make_biased_attn_plan.
 struct PlainAttnArgs {
     const void *q, *k_cache, *v_cache;
@@ -227,7 +227,7 @@ template <typename T>
 void launch_plain_attention(const PlainAttnArgs& a, cudaStream_t s);
 
 // fp32 Y[M][ldy] = X[M][ldx] W[N][K]^T with bf16 W, row-major.  With `entries` the rows come in groups, one per blockIdx.z:
-// {expert, first x row, first y row, rows <= kF32Rows}; expert e's matrix is w + e * w_stride.  x_at_y: the
+// {expert, first x row, first y row, rows <= min(M, kF32Rows)}; expert e's matrix is w + e * w_stride.  x_at_y: the
 // rows of x are those of y (a product of what an earlier grouped product wrote).
 constexpr int kF32Rows = 64;
 void launch_linear_f32(const float* x, int ldx, const bf16* w, size_t w_stride, float* y, int ldy, int M, int N, int K,

@@ -1,5 +1,4 @@
-// Row-wise kernels, plain attention and the fp32 matrix product of layered models (layered.cuh).  Norms, the residual
-// sum, attention scores and weights are fp32 whatever T is.
+// Row-wise kernels of layered models (layered.cuh).  Norms and the residual sum are fp32 whatever T is.
 #include <algorithm>
 
 #include "row_ops.cuh"
@@ -228,124 +227,6 @@ __global__ void norm_rows_kernel(const float* __restrict__ x32, const int32_t* _
     }
 }
 
-// One warp per (token, head): lanes take keys for the scores and value columns for the output.
-constexpr int PA_WARPS = 4, PA_MAX_D = 512;
-
-template <typename T>
-__global__ void plain_attention_kernel(const PlainAttnArgs a) {
-    grid_dependency_sync();
-    __shared__ float sq[PA_WARPS][PA_MAX_D];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int item = blockIdx.x * PA_WARPS + warp;
-    if (item >= a.tq * a.hq) return;
-    const int t = item / a.hq, h = item - t * a.hq;
-    const int g = h / (a.hq / a.hkv);
-    const T* q = static_cast<const T*>(a.q) + static_cast<size_t>(item) * a.dk;
-    for (int c = lane; c < a.dk; c += 32) sq[warp][c] = to_float<T>(q[c]);
-    __syncwarp();
-    const int i = *a.kv_len + a.kv_len_add - a.tq + t;   // position of this token
-    const int lo = a.window > 0 ? max(i - a.window + 1, 0) : 0;
-    const float slope = a.bias_exp > 0.f ? exp2f(-a.bias_exp * static_cast<float>(h + 1) / static_cast<float>(a.hq)) : 0.f;
-    const T* kc = static_cast<const T*>(a.k_cache) + static_cast<size_t>(g) * a.dk;
-    const T* vc = static_cast<const T*>(a.v_cache) + static_cast<size_t>(g) * a.dv;
-    const size_t kld = static_cast<size_t>(a.hkv) * a.dk, vld = static_cast<size_t>(a.hkv) * a.dv;
-    float m = -INFINITY, l = 0.f, acc[PA_MAX_D / 32];
-#pragma unroll
-    for (int c = 0; c < PA_MAX_D / 32; ++c) acc[c] = 0.f;
-    for (int j0 = lo; j0 <= i; j0 += 32) {
-        const int j = j0 + lane;
-        float s = -INFINITY;
-        if (j <= i) {
-            const T* k = kc + static_cast<size_t>(j) * kld;
-            float d = 0.f, f[8];
-            for (int c = 0; c < a.dk; c += 8) {   // dk is padded to a multiple of 64
-                load_vec<8>(k + c, f);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) d += sq[warp][c + e] * f[e];
-            }
-            s = d * a.scale - slope * static_cast<float>(i - j);
-        }
-        float mx = s;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        const float m_new = fmaxf(m, mx);
-        const float alpha = expf(m - m_new);
-        const float p = expf(s - m_new);
-        l = l * alpha + warp_sum(p);
-        m = m_new;
-#pragma unroll
-        for (int c = 0; c < PA_MAX_D / 32; ++c) acc[c] *= alpha;
-        const int n = min(32, i - j0 + 1);
-        for (int jj = 0; jj < n; ++jj) {
-            const float pj = __shfl_sync(0xffffffffu, p, jj);
-            const T* v = vc + static_cast<size_t>(j0 + jj) * vld;
-#pragma unroll
-            for (int c = 0; c < PA_MAX_D / 32; ++c) {
-                if (c * 32 + lane < a.out_cols) acc[c] += pj * to_float<T>(v[c * 32 + lane]);
-            }
-        }
-    }
-    T* out = static_cast<T*>(a.out) + static_cast<size_t>(t) * a.out_ld + static_cast<size_t>(h) * a.out_cols;
-    if (a.sink != 0) l += expf(-m);
-    const float inv = l > 0.f ? a.out_scale / l : 0.f;
-#pragma unroll
-    for (int c = 0; c < PA_MAX_D / 32; ++c) {
-        if (c * 32 + lane < a.out_cols) out[c * 32 + lane] = from_float<T>(acc[c] * inv);
-    }
-}
-
-// 64 x 64 output tile, 16 x 16 threads with 4 x 4 outputs each.
-__global__ void __launch_bounds__(256)
-linear_f32_kernel(const float* __restrict__ x, int ldx, const bf16* __restrict__ w, size_t w_stride, float* __restrict__ y, int ldy,
-                  int M, int N, int K, const int4* __restrict__ entries, const int32_t* __restrict__ n_entries, int x_at_y) {
-    grid_dependency_sync();
-    constexpr int KT = 32;
-    __shared__ float sx[KT][kF32Rows + 4], sw[KT][64 + 4];
-    int x0 = blockIdx.y * kF32Rows, y0 = x0, rows = min(kF32Rows, M - x0);
-    if (entries != nullptr) {
-        if (static_cast<int>(blockIdx.z) >= *n_entries) return;
-        const int4 e = entries[blockIdx.z];
-        w += static_cast<size_t>(e.x) * w_stride;
-        x0 = x_at_y ? e.z : e.y; y0 = e.z; rows = e.w;
-    }
-    const int n0 = blockIdx.x * 64;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += KT) {   // K is a multiple of 64
-        for (int i = threadIdx.x; i < 64 * (KT / 4); i += 256) {
-            const int r = i / (KT / 4), c = (i - r * (KT / 4)) * 4;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (r < rows) v = *reinterpret_cast<const float4*>(x + static_cast<size_t>(x0 + r) * ldx + k0 + c);
-            sx[c][r] = v.x; sx[c + 1][r] = v.y; sx[c + 2][r] = v.z; sx[c + 3][r] = v.w;
-            bf16 b[4] = {};
-            if (n0 + r < N) *reinterpret_cast<uint2*>(b) = *reinterpret_cast<const uint2*>(w + static_cast<size_t>(n0 + r) * K + k0 + c);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) sw[c + e][r] = __bfloat162float(b[e]);
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < KT; ++k) {
-            const float4 xv = *reinterpret_cast<const float4*>(&sx[k][ty * 4]);
-            const float4 wv = *reinterpret_cast<const float4*>(&sw[k][tx * 4]);
-            const float xs[4] = {xv.x, xv.y, xv.z, xv.w}, ws[4] = {wv.x, wv.y, wv.z, wv.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(xs[i], ws[j], acc[i][j]);
-            }
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        if (ty * 4 + i >= rows) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (n0 + tx * 4 + j < N) y[static_cast<size_t>(y0 + ty * 4 + i) * ldy + n0 + tx * 4 + j] = acc[i][j];
-        }
-    }
-}
-
 __global__ void silu_f32_kernel(const float* __restrict__ gu, int ld_gu, float* __restrict__ act, int ld_act, int ff) {
     grid_dependency_sync();
     const float* g = gu + static_cast<size_t>(blockIdx.x) * ld_gu;
@@ -395,22 +276,6 @@ void launch_norm_rows(const float* x32, const int32_t* rows_idx, const bf16* w, 
     launch_kernel(norm_rows_kernel<T>, dim3(rows), dim3(256), 0, s, x32, rows_idx, w, y, width, ld, eps);
 }
 
-template <typename T>
-void launch_plain_attention(const PlainAttnArgs& a, cudaStream_t s) {
-    ProfileScope prof(KC_ATTENTION, s);
-    CPM_REQUIRE(a.dk % 64 == 0 && a.dk <= PA_MAX_D && a.out_cols <= PA_MAX_D && a.hq % a.hkv == 0, "attention: head width above 512");
-    launch_kernel(plain_attention_kernel<T>, dim3(ceil_div(a.tq * a.hq, PA_WARPS)), dim3(PA_WARPS * 32), 0, s, a);
-}
-
-void launch_linear_f32(const float* x, int ldx, const bf16* w, size_t w_stride, float* y, int ldy, int M, int N, int K,
-                       const int4* entries, const int32_t* n_entries, int max_entries, bool x_at_y, cudaStream_t s) {
-    ProfileScope prof(entries ? KC_MOE : KC_LINEAR, s);
-    CPM_REQUIRE(K % 64 == 0 && ldx % 4 == 0, "linear_f32: K must be a multiple of 64");
-    dim3 grid(ceil_div(N, 64), entries ? 1 : ceil_div(M, kF32Rows), entries ? max_entries : 1);
-    launch_kernel(linear_f32_kernel, grid, dim3(256), 0, s, x, ldx, w, w_stride, y, ldy, M, N, K, entries, n_entries,
-                  x_at_y ? 1 : 0);
-}
-
 void launch_silu_f32(const float* gu, int ld_gu, float* act, int ld_act, int rows, int ff, cudaStream_t s) {
     ProfileScope prof(KC_ROW, s);
     launch_kernel(silu_f32_kernel, dim3(rows), dim3(256), 0, s, gu, ld_gu, act, ld_act, ff);
@@ -420,7 +285,6 @@ void launch_silu_f32(const float* gu, int ld_gu, float* act, int ld_act, int row
     template void launch_embed_rows<T>(const int32_t*, const bf16*, int, float, float*, T*, int, int, const StateCheck&, cudaStream_t); \
     template void launch_qkv_norm_append<T>(const QkvNormArgs&, int, cudaStream_t);                                                 \
     template void launch_out_norm<T>(float*, T*, const T*, const MoeMix&, float, const bf16*, int, int, int, float, cudaStream_t);  \
-    template void launch_norm_rows<T>(const float*, const int32_t*, const bf16*, T*, int, int, int, float, cudaStream_t);           \
-    template void launch_plain_attention<T>(const PlainAttnArgs&, cudaStream_t);
+    template void launch_norm_rows<T>(const float*, const int32_t*, const bf16*, T*, int, int, int, float, cudaStream_t);
 CPM_INSTANTIATE(bf16)
 CPM_INSTANTIATE(float)
