@@ -247,12 +247,16 @@ class LLM(torch.nn.Module):
         out = torch.empty((len(want), self.config.vocab_size), dtype=self.dtype, device="cuda")
         for i in range(0, n, self.chunk_length):
             m = min(n - i, self.chunk_length)
-            rows = sorted({w - i for w in want if i <= w < i + m})
-            part = torch.empty((len(rows), self.config.vocab_size), dtype=self.dtype, device="cuda")
-            C.prefill_rows(m, history + i, ids[i:].data_ptr(), pos[i:].data_ptr(), rows, part.data_ptr())
-            for k, w in enumerate(want):
-                if i <= w < i + m:
-                    out[k] = part[rows.index(w - i)]
+            places = [k for k, w in enumerate(want) if i <= w < i + m]
+            rows = [want[k] - i for k in places]
+            if places == list(range(places[0], places[0] + len(places)) if places else []) and rows == sorted(set(rows)):
+                # in order and without repeats: they are written where they belong
+                C.prefill_rows(m, history + i, ids[i:].data_ptr(), pos[i:].data_ptr(), rows, out[places[0]:].data_ptr() if places else 0)
+                continue
+            own = sorted(set(rows))
+            part = torch.empty((len(own), self.config.vocab_size), dtype=self.dtype, device="cuda")
+            C.prefill_rows(m, history + i, ids[i:].data_ptr(), pos[i:].data_ptr(), own, part.data_ptr())
+            out[places] = part[[own.index(w) for w in rows]]
         return out
 
     def _pick(self, logits):

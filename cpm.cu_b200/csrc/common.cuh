@@ -285,6 +285,20 @@ void launch_add_scaled(bf16* x, const bf16* a, const bf16* b, float scale_b, int
                        cudaStream_t s);  // x = a + b*scale
 void launch_scale(bf16* out, const bf16* in, float scale, size_t n, cudaStream_t s);
 // x = (a + bias[col]) + b, each sum rounded to bf16 (bias may be null): the two halves of a quantised fc
+// out[i] = bf16(src[list.row[i]] * scale), rows of `dim` elements (a multiple of 8)
+struct RowList {
+    static constexpr int kMax = 64;
+    int n;
+    int32_t row[kMax];
+};
+void launch_gather_rows(bf16* out, const bf16* src, const RowList& list, int dim, float scale, cudaStream_t s);
+// The inputs of a decode pass (at most 64 tokens; mask may be null) into one set of buffers
+struct DecodeInputs {
+    int32_t *ids = nullptr, *pos = nullptr, *len = nullptr;
+    uint64_t* mask = nullptr;
+};
+void launch_stage_decode(const DecodeInputs& dst, const int32_t* ids, const int32_t* pos, const int32_t* len, const uint64_t* mask, int n,
+                         cudaStream_t s);
 void launch_add_bias_add(bf16* x, const bf16* a, const bf16* bias, const bf16* b, int rows, int dim, cudaStream_t s);
 size_t argmax_workspace_bytes(int rows, int vocab);
 void launch_argmax(const bf16* logits, int rows, int vocab, int ld, int32_t* out, void* workspace, cudaStream_t s);

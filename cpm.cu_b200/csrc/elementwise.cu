@@ -252,6 +252,32 @@ __global__ void scale_kernel(bf16* __restrict__ out, const bf16* __restrict__ in
     if (i < n) out[i] = __float2bfloat16(__bfloat162float(in[i]) * scale);
 }
 
+__global__ void gather_rows_kernel(bf16* __restrict__ out, const bf16* __restrict__ src, const RowList list, int dim, float scale) {
+    grid_dependency_sync();
+    const bf16* from = src + static_cast<size_t>(list.row[blockIdx.x]) * dim;
+    bf16* to = out + static_cast<size_t>(blockIdx.x) * dim;
+    for (int c = threadIdx.x * 8; c < dim; c += blockDim.x * 8) {
+        uint4 v = *reinterpret_cast<const uint4*>(from + c);
+        bf16* e = reinterpret_cast<bf16*>(&v);
+        if (scale != 1.f) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) e[i] = __float2bfloat16(__bfloat162float(e[i]) * scale);
+        }
+        *reinterpret_cast<uint4*>(to + c) = v;
+    }
+}
+
+__global__ void stage_decode_kernel(const DecodeInputs dst, const int32_t* __restrict__ ids, const int32_t* __restrict__ pos,
+                                    const int32_t* __restrict__ len, const uint64_t* __restrict__ mask, int n) {
+    grid_dependency_sync();
+    const int i = threadIdx.x;
+    if (i == 0) *dst.len = *len;
+    if (i >= n) return;
+    dst.ids[i] = ids[i];
+    dst.pos[i] = pos[i];
+    if (mask != nullptr) dst.mask[i] = mask[i];
+}
+
 // Row argmax over bf16 logits, lowest index wins ties.  Stage 1: each CTA scans one
 // 8192-entry chunk of a row with 16-byte loads; stage 2: one warp per row merges.
 constexpr int AM_CHUNK = 8192;
@@ -569,6 +595,16 @@ void launch_add_bias_add(bf16* x, const bf16* a, const bf16* bias, const bf16* b
 void launch_scale(bf16* out, const bf16* in, float scale, size_t n, cudaStream_t s) {
     if (n == 0) return;
     launch_kernel(scale_kernel, dim3(static_cast<unsigned>((n + 255) / 256)), dim3(256), 0, s, out, in, scale, n);
+}
+
+void launch_gather_rows(bf16* out, const bf16* src, const RowList& list, int dim, float scale, cudaStream_t s) {
+    if (list.n <= 0) return;
+    launch_kernel(gather_rows_kernel, dim3(list.n), dim3(256), 0, s, out, src, list, dim, scale);
+}
+
+void launch_stage_decode(const DecodeInputs& dst, const int32_t* ids, const int32_t* pos, const int32_t* len, const uint64_t* mask, int n,
+                         cudaStream_t s) {
+    launch_kernel(stage_decode_kernel, dim3(1), dim3(64), 0, s, dst, ids, pos, len, mask, n);
 }
 
 size_t argmax_workspace_bytes(int rows, int vocab) {

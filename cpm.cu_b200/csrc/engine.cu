@@ -645,9 +645,16 @@ void Engine::prefill_rows(int n, int history, const int32_t* ids, const int32_t*
         rt.profile = true;
     }
     target_forward(fp, c, ids, false, last_only ? static_cast<bf16*>(logits_out) : nullptr, mc_.vocab, s);
-    for (int i = 0; i < n_want && !last_only; ++i) {
-        lm_head_rows(norm_out_ + static_cast<size_t>(want[i]) * H, 1, 1, static_cast<bf16*>(logits_out) + static_cast<size_t>(i) * mc_.vocab,
-                     mc_.vocab, s);
+    for (int i = 0; i < n_want && !last_only; i += RowList::kMax) {
+        // the head streams its whole matrix per product: up to 64 chosen rows share one (64 rows of a 2048 x 32768 head:
+        // 64 x 28 us one by one, 35 us together)
+        RowList list;
+        list.n = std::min(RowList::kMax, n_want - i);
+        for (int k = 0; k < list.n; ++k) list.row[k] = want[i + k];
+        launch_gather_rows(lm_in_, norm_out_, list, H, mc_.scale_lmhead, s);
+        launch_linear(checked(make_linear_plan(lm_in_, list.n, lm_head_, list.n, mc_.vocab, H,
+                                               static_cast<bf16*>(logits_out) + static_cast<size_t>(i) * mc_.vocab, mc_.vocab, nullptr,
+                                               gemm_ws_, tickets_, rt.num_sms)), s);
     }
     if (prof_prefill) {
         // CUDA events around every launch of the pass: time per kernel class, and the GEMMs of the last layer
