@@ -241,7 +241,7 @@ class LLM(torch.nn.Module):
             raise ValueError(f"{history} cached + {n} new tokens exceed the {self.max_total_length} tokens the KV cache holds "
                              f"under the current memory limit")
         if n == 1 and history > 0:
-            return self._decode_one(tokens[0], history)[[0] * len(want)]
+            return self._decode_one(tokens[0], history).repeat(len(want), 1)
         ids = torch.tensor(tokens, dtype=torch.int32, device="cuda")
         pos = torch.arange(history, history + n, dtype=torch.int32, device="cuda")
         out = torch.empty((len(want), self.config.vocab_size), dtype=self.dtype, device="cuda")

@@ -72,6 +72,7 @@ enum KernelClass : int {
 struct Runtime {
     cudaStream_t stream = nullptr;
     int* d_error = nullptr;  // device error word, or-ed into by kernels
+    int* h_error = nullptr;  // pinned copy of it
     unsigned* d_accept_ticket = nullptr;  // CTAs of the acceptance kernel that have read the tree (zero between launches)
     int num_sms = 148;
     int device = 0;
@@ -284,7 +285,6 @@ void launch_silu_gate(const bf16* gate_up, bf16* out, int rows, int inter, cudaS
 void launch_add_scaled(bf16* x, const bf16* a, const bf16* b, float scale_b, int rows, int dim,
                        cudaStream_t s);  // x = a + b*scale
 void launch_scale(bf16* out, const bf16* in, float scale, size_t n, cudaStream_t s);
-// x = (a + bias[col]) + b, each sum rounded to bf16 (bias may be null): the two halves of a quantised fc
 // out[i] = bf16(src[list.row[i]] * scale), rows of `dim` elements (a multiple of 8)
 struct RowList {
     static constexpr int kMax = 64;
@@ -299,6 +299,7 @@ struct DecodeInputs {
 };
 void launch_stage_decode(const DecodeInputs& dst, const int32_t* ids, const int32_t* pos, const int32_t* len, const uint64_t* mask, int n,
                          cudaStream_t s);
+// x = (a + bias[col]) + b, each sum rounded to bf16 (bias may be null): the two halves of a quantised fc
 void launch_add_bias_add(bf16* x, const bf16* a, const bf16* bias, const bf16* b, int rows, int dim, cudaStream_t s);
 size_t argmax_workspace_bytes(int rows, int vocab);
 void launch_argmax(const bf16* logits, int rows, int vocab, int ld, int32_t* out, void* workspace, cudaStream_t s);

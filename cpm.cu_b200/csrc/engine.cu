@@ -89,11 +89,19 @@ Engine::Engine(const ModelConfig& mc) : mc_(mc) {
 Engine::~Engine() {
     if (step_graph_) cudaGraphExecDestroy(step_graph_);
     if (decode_graph_) cudaGraphExecDestroy(decode_graph_);
+    drop_decode_graphs();
     if (ev0_) cudaEventDestroy(ev0_);
     if (ev1_) cudaEventDestroy(ev1_);
     if (ev_mid_) cudaEventDestroy(ev_mid_);
     if (pool_.base) cudaFree(pool_.base);
     if (h_result_) cudaFreeHost(h_result_);
+}
+
+void Engine::drop_decode_graphs() {
+    for (auto& g : decode_graphs_) {
+        if (g.second.exec) cudaGraphExecDestroy(g.second.exec);
+    }
+    decode_graphs_.clear();
 }
 
 void Engine::attach_eagle(const EagleConfig& ec) {
@@ -214,6 +222,10 @@ void Engine::lay_out(Pool& p) {
     t_parent_ = take<int32_t>(p, 64);
     t_gt_ = take<int32_t>(p, 64);
     t_mask_ = take<uint64_t>(p, 64);
+    d_in_.ids = take<int32_t>(p, 64);
+    d_in_.pos = take<int32_t>(p, 64);
+    d_in_.len = take<int32_t>(p, 1);
+    d_in_.mask = take<uint64_t>(p, 64);
     accept_result_ = take<int32_t>(p, 32);
     argmax_ws_ = p.take(argmax_workspace_bytes(64, V));
     d_publish_ = take<int32_t>(p, 32);
@@ -691,7 +703,6 @@ void Engine::prefill_rows(int n, int history, const int32_t* ids, const int32_t*
         first_draft_ = true;
     }
     host_len_ = static_cast<long>(history) + n;
-    CUDA_CHECK(cudaStreamSynchronize(s));
     check_errors("prefill");
 }
 
@@ -708,17 +719,56 @@ void Engine::decode(int n, int padded_len, const int32_t* ids, const int32_t* po
         return;
     }
     (void)cuda_graph;
-    cudaStream_t s = runtime().stream;
+    Runtime& rt = runtime();
+    cudaStream_t s = rt.stream;
     RowCtx c;
     c.rows = n;
-    c.pos = pos;
-    c.kv_len = cache_length;  // the caller has already added n (reference cpmcu/llm.py:263-283)
     c.kv_append_off = -n;
     c.attn_kv_add = 0;
-    c.mask = mask;
     c.mask_k = mask ? n : 0;
-    target_forward(target_plans(n), c, ids, true, static_cast<bf16*>(logits_out), mc_.vocab, s);
-    CUDA_CHECK(cudaStreamSynchronize(s));
+    // A pass of a small model is a row of two- to six-microsecond kernels: launched one by one they wait for the host.  From
+    // the second pass of a shape on, it is replayed as a graph over the engine's own input and logits buffers; the caller's
+    // are copied in and out, so that nothing depends on where they lie.
+    DecodeGraph* graph = nullptr;
+    if (!rt.profile && bm_capture_ == nullptr) {
+        const int key = 2 * n + (mask != nullptr);
+        if (decode_graphs_.size() >= 16 && decode_graphs_.find(key) == decode_graphs_.end()) drop_decode_graphs();
+        graph = &decode_graphs_[key];
+        if (graph->passes++ == 0) graph = nullptr;
+    }
+    if (graph == nullptr) {
+        c.pos = pos;
+        c.kv_len = cache_length;  // the caller has already added n (reference cpmcu/llm.py:263-283)
+        c.mask = mask;
+        target_forward(target_plans(n), c, ids, true, static_cast<bf16*>(logits_out), mc_.vocab, s);
+    } else {
+        launch_stage_decode(d_in_, ids, pos, cache_length, mask, n, s);
+        if (graph->exec == nullptr) {
+            c.pos = d_in_.pos;
+            c.kv_len = d_in_.len;
+            c.mask = mask ? d_in_.mask : nullptr;
+            ForwardPlans& fp = target_plans(n);
+            const long before = rt.launches;
+            cudaGraph_t g = nullptr;
+            CUDA_CHECK(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
+            try {
+                target_forward(fp, c, d_in_.ids, true, logits_, mc_.vocab, s);
+            } catch (...) {
+                cudaStreamEndCapture(s, &g);
+                if (g) cudaGraphDestroy(g);
+                throw;
+            }
+            CUDA_CHECK(cudaStreamEndCapture(s, &g));
+            const cudaError_t made = cudaGraphInstantiate(&graph->exec, g, 0);
+            cudaGraphDestroy(g);
+            CUDA_CHECK(made);
+            graph->launches = rt.launches - before;
+            rt.launches = before;
+        }
+        CUDA_CHECK(cudaGraphLaunch(graph->exec, s));
+        rt.launches += graph->launches;
+        CUDA_CHECK(cudaMemcpyAsync(logits_out, logits_, static_cast<size_t>(n) * mc_.vocab * 2, cudaMemcpyDeviceToDevice, s));
+    }
     check_errors("decode");
 }
 
@@ -884,7 +934,6 @@ void Engine::draft(int32_t* tree_ids, int32_t* tree_pos, const int32_t* cache_le
     }
     draft_levels(tree_ids, tree_pos, cache_length, tree_mask, tree_parent, first_draft_, s);
     first_draft_ = false;
-    CUDA_CHECK(cudaStreamSynchronize(s));
     check_errors("draft");
 }
 

@@ -363,6 +363,15 @@ private:
     int catchup_rows_ = 0;
 
     std::map<int, std::unique_ptr<ForwardPlans>> plans_;
+    // captured decode passes of Llama-format models by 2 * tokens + (tree mask given), and the inputs they read
+    struct DecodeGraph {
+        long passes = 0;
+        cudaGraphExec_t exec = nullptr;
+        long launches = 0;
+    };
+    std::map<int, DecodeGraph> decode_graphs_;
+    DecodeInputs d_in_;
+    void drop_decode_graphs();
     LayerPlans eplan_level_, eplan_catchup_;
     LinearPlan fc_plan_level_, fc_plan_catchup_, dlm_plan_level_, dlm_plan_catchup_;
     LinearPlan fc2_plan_level_, fc2_plan_catchup_;  // W4A16 drafter: the hidden-state half of fc

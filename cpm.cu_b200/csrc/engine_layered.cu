@@ -529,7 +529,7 @@ void Engine::layered_mixture(int i, LayeredPlans& lp, cudaStream_t s) {
         float *gu = static_cast<float*>(moe_gu_), *act = static_cast<float*>(moe_act_), *y = static_cast<float*>(moe_y_);
         const int ff = pad64(sp.expert_ff), ffs = pad64(sp.shared_ff), slots = rows * sp.top;
         const int most = moe_max_entries(sp, rows, tile);
-        launch_linear_f32(single ? x : static_cast<const float*>(moe_x_), L, w.gate_up, moe_gate_up_offset(sp, L, 1), gu, 2 * ff, 0, 2 * ff, L,
+        launch_linear_f32(single ? x : static_cast<const float*>(moe_x_), L, w.gate_up, moe_gate_up_offset(sp, L, 1), gu, 2 * ff, rows, 2 * ff, L,
                           moe_.entries, moe_.n_entries, most, false, s);
         launch_silu_f32(gu, 2 * ff, act, ff, slots, ff, s);
         launch_linear_f32(act, ff, w.down, moe_down_offset(sp, W, 1), y, L, rows, W, ff, moe_.entries, moe_.n_entries, most, true, s);
@@ -775,7 +775,6 @@ void Engine::layered_prefill(int n, int history, const int32_t* ids, const int32
         else layered_logits<bf16>(want_, n_want, logits_out, s);
     }
     host_len_ = static_cast<long>(history) + n;
-    CUDA_CHECK(cudaStreamSynchronize(s));
     layered_check_errors("prefill");
 }
 
@@ -830,9 +829,8 @@ void Engine::layered_decode(int n, const int32_t* ids, const int32_t* cache_leng
         enqueue();
         CUDA_CHECK(cudaEventRecord(ev1_, s));
     }
-    CUDA_CHECK(cudaStreamSynchronize(s));
+    layered_check_errors("decode");
     float ms = 0.f;
     CUDA_CHECK(cudaEventElapsedTime(&ms, ev0_, ev1_));
     last_step_ms_ = ms;
-    layered_check_errors("decode");
 }

@@ -50,6 +50,7 @@ Runtime& runtime() {
         CUDA_CHECK(cudaStreamCreate(&rt.stream));
         CUDA_CHECK(cudaMalloc(&rt.d_error, sizeof(int)));
         CUDA_CHECK(cudaMemset(rt.d_error, 0, sizeof(int)));
+        CUDA_CHECK(cudaMallocHost(&rt.h_error, sizeof(int)));
         CUDA_CHECK(cudaMalloc(&rt.d_accept_ticket, sizeof(unsigned)));
         CUDA_CHECK(cudaMemset(rt.d_accept_ticket, 0, sizeof(unsigned)));
         ready = true;
@@ -59,9 +60,9 @@ Runtime& runtime() {
 
 int read_and_clear_error() {
     Runtime& rt = runtime();
-    int h = 0;
-    CUDA_CHECK(cudaMemcpyAsync(&h, rt.d_error, sizeof(int), cudaMemcpyDeviceToHost, rt.stream));
+    CUDA_CHECK(cudaMemcpyAsync(rt.h_error, rt.d_error, sizeof(int), cudaMemcpyDeviceToHost, rt.stream));
     CUDA_CHECK(cudaStreamSynchronize(rt.stream));
+    const int h = *rt.h_error;
     if (h != 0) {
         CUDA_CHECK(cudaMemsetAsync(rt.d_error, 0, sizeof(int), rt.stream));
         CUDA_CHECK(cudaStreamSynchronize(rt.stream));
