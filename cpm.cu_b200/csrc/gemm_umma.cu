@@ -540,6 +540,11 @@ LinearPlan make_linear_plan(const bf16* x, int x_rows, const bf16* w, int M, int
     p.mt = linear_pick_mt(M);
     p.y = y; p.ldy = ldy; p.bias = bias;
     p.workspace = workspace; p.tickets = tickets;
+    p.x = x; p.w = w;
+    if (M == 1) {   // launch_linear_one_row: neither maps nor a division of the tiles
+        p.grid = 1;
+        return p;
+    }
     const int n_tiles = ceil_div(N, BLOCK_N), m_tiles = ceil_div(M, p.mt), kblocks = K / BLOCK_K;
     const long long units = static_cast<long long>(n_tiles) * m_tiles * kblocks;
     long long grid = base_grid(n_tiles, m_tiles, kblocks, M, grid_limit);
@@ -606,6 +611,7 @@ static int swiglu_grid(int n_tiles, int m_tiles, int grid_limit) {
 // (launches smaller than the grid limit always qualify: they are a single wave either way).
 bool linear_swiglu_fits(int M, int inter, int grid_limit) {
     if (inter < 64 || inter % 64 != 0) return false;
+    if (M == 1) return true;   // no tiles
     const int n_tiles = inter / 64, m_tiles = ceil_div(M, linear_pick_mt(M));
     const long long tiles = static_cast<long long>(n_tiles) * m_tiles;
     if (tiles <= grid_limit) return true;
@@ -628,6 +634,11 @@ LinearPlan make_linear_swiglu_plan(const bf16* x, int x_rows, const bf16* w, int
     p.mt = linear_pick_mt(M);
     p.y = act; p.ldy = ld; p.bias = nullptr;
     p.swiglu = 1;
+    p.x = x; p.w = w;
+    if (M == 1) {
+        p.grid = 1;
+        return p;
+    }
     const long long tiles = static_cast<long long>(inter / 64) * ceil_div(M, p.mt);
     const int m_tiles = ceil_div(M, p.mt);
     p.grid = swiglu_grid(inter / 64, m_tiles, grid_limit);
@@ -647,6 +658,11 @@ void launch_linear(const LinearPlan& p, cudaStream_t stream) {
         return;
     }
     ProfileScope prof(KC_LINEAR, stream);
+    // one row needs no tensor core and was faster without at every size (one_row.cu has both sides' times)
+    if (p.M == 1) {
+        launch_linear_one_row(p, stream);
+        return;
+    }
     LinearArgs a;
     a.M = p.M; a.N = p.N; a.K = p.K;
     a.n_tiles = ceil_div(p.N, BLOCK_N);

@@ -282,6 +282,8 @@ struct MoeGemmPlan {
     int ldy = 0;
     const int4* entries = nullptr;
     const int32_t* n_entries = nullptr;
+    const bf16 *w = nullptr, *x = nullptr, *xs = nullptr;   // the operands themselves; xs: the shared expert's rows
+    int ldx = 0;
     int uniform = 0;                 // > 0: no router, this many matrices whose rows lie one block of `rows` after the other
 };
 // `n` products of the same shape in one launch: rows [i * rows, (i + 1) * rows) of x times matrix i [N][K], into the same rows
@@ -295,6 +297,7 @@ MoeGemmPlan make_moe_gate_up_plan(const LayerSpec& sp, const bf16* w, const bf16
 MoeGemmPlan make_moe_down_plan(const LayerSpec& sp, const bf16* w, const bf16* act, int act_rows, int ld_act, int width, bf16* y,
                                int ld_y, int rows, int tile, const MoeBuffers& b);
 void launch_moe_gemm(const MoeGemmPlan& p, cudaStream_t s);
+void launch_moe_one_row(const MoeGemmPlan& p, cudaStream_t s);   // rows == 1 (one_row.cu)
 // elements of the two weight buffers (tile-major), and where an expert's (index `experts`: the shared expert's) part begins
 size_t moe_gate_up_elems(const LayerSpec& sp, int K);
 size_t moe_down_elems(const LayerSpec& sp, int width);

@@ -1,0 +1,195 @@
+// Products of ONE token row with bf16 weights: y[N] = x[K] W[N,K]^T, alone (LinearPlan) or grouped by expert
+// (MoeGemmPlan), with the SwiGLU and clamped-gate epilogues of the tensor-core kernels.
+//
+// Bound: the weights' bytes from HBM, 2 FLOP each, so the tensor cores have nothing to do, and what the tile kernels need
+// before the first byte arrives (tensor memory, descriptors, barriers) and after the last one (tensor memory back to
+// registers, pieces of split tiles summed through a workspace) is most of a product of a few megabytes.  Here a CTA
+// owns R output rows over the whole of K: eight lanes read 128 consecutive bytes of one row (the tile-major
+// layout keeps the R rows of a k-block together), the eight warps take k-blocks in turn, and only sums of one CTA
+// meet.  A warp keeps eight 16-byte loads per lane in flight, the first of them before the wait for the predecessor.  About
+// 20 instructions per 16 bytes leave three quarters of the issue slots free at the HBM rate.
+// Back to back, weights from HBM, tensor-core tiles before / now: 2048 x 2048 6.9 / 3.6 us, 3072 x 2048 5.5 / 4.1,
+// 2048 x 8192 10.9 / 8.2, 11008 x 4096 gated 39.8 / 28.6, 73448 x 4096 88 / 84 (7.2 TB/s); 512 x 256 3.7 / 3.5.
+#include "common.cuh"
+#include "layered.cuh"
+#include "row_ops.cuh"
+
+namespace {
+
+constexpr int ONE_WARPS = 8;
+constexpr int TILE_ROWS = 128, BLOCK_COLS = 64;           // tile-major layout (linear_weight_elems)
+constexpr int BLOCK_ELEMS = TILE_ROWS * BLOCK_COLS;
+
+struct OneRowArgs {
+    const bf16 *w, *x, *xs;
+    bf16* y;
+    const bf16* bias;
+    int N, kblocks, ctas;            // one matrix
+    int N_s, kblocks_s, ctas_s;      // the shared expert's (or the grouped product's extra one); ctas_s = 0: none
+    long long stride, w_s;           // elements from one matrix to the next; the shared one's start
+    int ldx, ldy, xs_row, ys_row;
+    const int4* entries;             // router's choice: {expert, input row, output row, 1}
+    const int32_t* n_entries;
+    int uniform;                     // > 0: matrix i has row i of x and y
+    float gate_limit, gate_alpha;
+};
+
+__device__ __forceinline__ uint4 load_stream(const bf16* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ f32x2 widen(uint32_t two) { return pair(__uint_as_float(two << 16), __uint_as_float(two & 0xffff0000u)); }
+
+// PAIR: the rows are R / 2 gate rows and the R / 2 up rows of the same features (64 + 64 in a tile).  EARLY: the router's
+// choice may be read before the wait for the predecessor.
+template <int R, bool PAIR, bool EARLY>
+__global__ void __launch_bounds__(ONE_WARPS * 32, 4)
+one_row_kernel(const OneRowArgs a) {
+    constexpr int LOADS = R / 4;                       // per lane and k-block
+    constexpr int U = 8 / LOADS;                       // k-blocks per batch
+    __shared__ float part[ONE_WARPS][R];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (EARLY) grid_dep_trigger();
+
+    const bool shared = static_cast<int>(blockIdx.x) < a.ctas_s;
+    const int b = shared ? blockIdx.x : blockIdx.x - a.ctas_s;
+    const int g = shared ? 0 : b / a.ctas;
+    const int c = b - g * a.ctas;
+    int4 e = make_int4(g, g, g, 1);
+    bool there = true, waited = false;
+    if (!shared && a.uniform == 0) {
+        if (!EARLY) {
+            grid_dep_wait();
+            grid_dep_trigger();
+            waited = true;
+        }
+        there = g < __ldcg(a.n_entries);
+        if (there) e = __ldcg(a.entries + g);
+    }
+    const int N = shared ? a.N_s : a.N, kblocks = shared ? a.kblocks_s : a.kblocks;
+    const int first = c * (PAIR ? R / 2 : R);          // output
+    const int tile = first / (PAIR ? 64 : TILE_ROWS), r0 = first % (PAIR ? 64 : TILE_ROWS);
+    const bf16* w = a.w + (shared ? a.w_s : static_cast<long long>(e.x) * a.stride) + static_cast<size_t>(tile) * kblocks * BLOCK_ELEMS +
+                    (r0 + (lane >> 3)) * BLOCK_COLS + (lane & 7) * 8;
+
+    uint4 wv[U][LOADS];
+    auto load = [&](int kb0) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int kb = kb0 + u * ONE_WARPS;
+#pragma unroll
+            for (int i = 0; i < LOADS; ++i) {
+                const int row = PAIR && i >= LOADS / 2 ? 64 + (i - LOADS / 2) * 4 : i * 4;
+                wv[u][i] = there && kb < kblocks ? load_stream(w + static_cast<size_t>(kb) * BLOCK_ELEMS + row * BLOCK_COLS) : make_uint4(0u, 0u, 0u, 0u);
+            }
+        }
+    };
+    load(warp);
+    if (!waited) {
+        grid_dep_wait();
+        if (!EARLY) grid_dep_trigger();
+    }
+    if (!there) return;
+    const bf16* x = (shared ? a.xs + static_cast<size_t>(a.xs_row) * a.ldx
+                            : a.x + static_cast<size_t>(a.uniform > 0 || PAIR ? e.y : e.z) * a.ldx) + (lane & 7) * 8;
+    f32x2 acc[LOADS];
+#pragma unroll
+    for (int i = 0; i < LOADS; ++i) acc[i] = 0;
+    for (int kb0 = warp; kb0 < kblocks; kb0 += U * ONE_WARPS) {
+        uint4 xv[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int kb = kb0 + u * ONE_WARPS;
+            xv[u] = kb < kblocks ? *reinterpret_cast<const uint4*>(x + kb * BLOCK_COLS) : make_uint4(0u, 0u, 0u, 0u);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const f32x2 x0 = widen(xv[u].x), x1 = widen(xv[u].y), x2 = widen(xv[u].z), x3 = widen(xv[u].w);
+#pragma unroll
+            for (int i = 0; i < LOADS; ++i) {
+                acc[i] = fma2(widen(wv[u][i].x), x0, acc[i]);
+                acc[i] = fma2(widen(wv[u][i].y), x1, acc[i]);
+                acc[i] = fma2(widen(wv[u][i].z), x2, acc[i]);
+                acc[i] = fma2(widen(wv[u][i].w), x3, acc[i]);
+            }
+        }
+        if (kb0 + U * ONE_WARPS < kblocks) load(kb0 + U * ONE_WARPS);
+    }
+#pragma unroll
+    for (int i = 0; i < LOADS; ++i) {
+        const float2 p = unpair(acc[i]);
+        float v = p.x + p.y;
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if ((lane & 7) == 0) part[warp][i * 4 + (lane >> 3)] = v;
+    }
+    __syncthreads();
+    const int t = threadIdx.x;
+    if (t >= (PAIR ? R / 2 : R) || first + t >= N) return;
+    float sum = 0.f, up = 0.f;
+#pragma unroll
+    for (int k = 0; k < ONE_WARPS; ++k) {
+        sum += part[k][t];
+        if (PAIR) up += part[k][(R / 2 + t) % R];
+    }
+    if (PAIR) {
+        // both projections are rounded to bf16 before silu's product, as where they are stored in between
+        sum = a.gate_limit > 0.f ? clamped_gate(sum, up, a.gate_limit, a.gate_alpha)
+                                 : silu_mul(__bfloat162float(__float2bfloat16(sum)), __bfloat162float(__float2bfloat16(up)));
+    } else if (a.bias != nullptr) {
+        sum += __bfloat162float(a.bias[first + t]);
+    }
+    a.y[static_cast<size_t>(shared ? a.ys_row : e.z) * a.ldy + first + t] = __float2bfloat16(sum);
+}
+
+// Output rows per CTA: 16 while that leaves every SM two to three CTAs, else 8: more CTAs even out the SMs' shares and keep more
+// loads in flight, more rows make longer bursts and fewer sums.  Rows x K with 16 / 8 rows: 4096 x 4096 7.8 / 7.0 us,
+// 2048 x 8192 11.3 / 8.2, 8192 x 3072 9.2 / 10.2, 16384 x 2048 (gated) 11.9 / 12.5.  4 rows (2048 x 2048 4.0 us against 3.6) and
+// 32 (73448 x 4096 90 us against 84) were slower.
+int rows_per_cta(long long outputs) {
+    static const char* forced = tuning_env("CPMCU_ONE_ROW");   // bench only
+    if (forced) return atoi(forced);
+    return outputs / 16 < runtime().num_sms * 5 / 2 ? 8 : 16;
+}
+
+template <bool PAIR, bool EARLY>
+void launch(int R, const OneRowArgs& a, int grid, cudaStream_t s) {
+    switch (R) {
+        case 8: launch_kernel(one_row_kernel<8, PAIR, EARLY>, dim3(grid), dim3(ONE_WARPS * 32), 0, s, a); break;
+        default: launch_kernel(one_row_kernel<16, PAIR, EARLY>, dim3(grid), dim3(ONE_WARPS * 32), 0, s, a); break;
+    }
+}
+
+}  // namespace
+
+void launch_linear_one_row(const LinearPlan& p, cudaStream_t s) {
+    OneRowArgs a = {};
+    a.w = p.w; a.x = p.x; a.y = p.y; a.bias = p.bias;
+    a.N = p.N; a.kblocks = p.K / BLOCK_COLS;
+    a.ldx = p.K; a.ldy = p.ldy;
+    a.uniform = 1;
+    a.gate_limit = p.gate_limit; a.gate_alpha = p.gate_alpha;
+    const int R = rows_per_cta(p.swiglu ? 2LL * p.N : p.N);
+    a.ctas = ceil_div(p.N, p.swiglu ? R / 2 : R);
+    if (p.swiglu) launch<true, true>(R, a, a.ctas, s);
+    else launch<false, true>(R, a, a.ctas, s);
+}
+
+void launch_moe_one_row(const MoeGemmPlan& p, cudaStream_t s) {
+    OneRowArgs a = {};
+    a.w = p.w; a.x = p.x; a.xs = p.xs; a.y = p.y;
+    a.N = p.N; a.kblocks = p.kblocks; a.N_s = p.N_s; a.kblocks_s = p.kblocks_s;
+    a.stride = static_cast<long long>(p.n_tiles) * p.kblocks * BLOCK_ELEMS;
+    a.w_s = p.w_row_s * BLOCK_COLS;
+    a.ldx = p.ldx; a.ldy = p.ldy; a.xs_row = p.xs_row0; a.ys_row = p.ys_row0;
+    a.entries = p.entries; a.n_entries = p.n_entries; a.uniform = p.uniform;
+    const int per = p.swiglu ? 2 : 1;
+    const int R = rows_per_cta(static_cast<long long>(per) * (static_cast<long long>(p.max_entries) * p.N + (p.n_tiles_s > 0 ? p.N_s : 0)));
+    a.ctas = ceil_div(p.N, R / per);
+    a.ctas_s = p.n_tiles_s > 0 ? ceil_div(p.N_s, R / per) : 0;
+    const int grid = a.ctas_s + p.max_entries * a.ctas;
+    // the router's choice: gate/up waits for it and lets its successor start only then, so down may read it at once
+    if (p.swiglu) launch<true, false>(R, a, grid, s);
+    else launch<false, true>(R, a, grid, s);
+}
