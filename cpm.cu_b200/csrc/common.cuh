@@ -212,6 +212,7 @@ struct LinearPlan {
     int* tickets = nullptr;      // two counters per output tile (pieces counted, readers gone), zero between launches
     int debug = 0;               // timing experiments of -DCPMCU_TUNING builds (CPM_EXPERIMENT); unused otherwise
     int cluster = 0;             // > 0: CTAs per tile, pieces summed inside a thread-block cluster (bf16 path)
+    int pair = 0;                // 1: two CTAs per tile of 256 weight rows (gemm_pair.cu)
     int wave_tiles = 0;          // several token tiles: tiles computed whole, in waves of `grid` (the rest is cut along K)
     int tail_grid = 0;           // CTAs that share the tiles after wave_tiles (0 = all)
     int swiglu = 0;              // SwiGLU epilogue: w = [gate ; up], N = output features, y = silu(gate) * up

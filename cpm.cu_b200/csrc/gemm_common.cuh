@@ -151,8 +151,8 @@ struct PendingTile {
 
 // Sum tokens [t_begin, t_end) of a split tile over its pieces in CTA order (deterministic) and store them:
 // CH tokens per pass, the coalesced loads of up to four pieces (4 * CH per thread) in flight before the adds.
-template <int MT, int CH>
-__device__ __forceinline__ void sum_pieces(const LinearArgs& a, const PendingTile& p, int t_begin, int t_end, int row) {
+template <int MT, int CH, int CSZ>
+__device__ __forceinline__ void sum_pieces(const LinearArgs& a, const PendingTile& p, int t_begin, int t_end, int row, int rank) {
     const int g_last = p.g_first + p.nseg - 1;
 #pragma unroll 1
     for (int c0 = t_begin; c0 < t_end; c0 += CH) {
@@ -165,7 +165,7 @@ __device__ __forceinline__ void sum_pieces(const LinearArgs& a, const PendingTil
 #pragma unroll
             for (int s = 0; s < 4; ++s) {
                 const int gg = g0 + s;
-                const float* ws = a.workspace + (static_cast<size_t>(gg) * 2 + (gg == p.g_first ? 1 : 0)) * (MT * BLOCK_N) +
+                const float* ws = a.workspace + (static_cast<size_t>(gg * CSZ + rank) * 2 + (gg == p.g_first ? 1 : 0)) * (MT * BLOCK_N) +
                                   static_cast<size_t>(c0) * BLOCK_N + row;
 #pragma unroll
                 for (int c = 0; c < CH; ++c) v[s][c] = (gg <= g_last && c0 + c < t_end) ? __ldcg(ws + c * BLOCK_N) : 0.f;
@@ -203,12 +203,14 @@ constexpr long long kFixupBudgetClocks = 100000000LL;
 // counters for the next launch).  That path needs the whole grid resident (grid <= SMs, one CTA per
 // SM).  Pieces are always added in CTA order, so the result does not depend on timing.  CH = tokens
 // summed per pass.  chain2_off != 0: the MMA role accumulated alternate k-blocks into a second
-// accumulator that many columns further on; the two are added here.
-template <int MT, int CH>
+// accumulator that many columns further on; the two are added here.  CSZ = 2: CTA pairs share the tiles of `it` (256 features), g
+// and G count pairs, this CTA has the 128 features of its rank, with partials and counters of its own, and acc_empty is
+// the one of rank 0.
+template <int MT, int CH, int CSZ = 1>
 __device__ __forceinline__ void run_epilogue(const LinearArgs& a, SegIter it, uint32_t tmem_base, uint64_t* acc_full,
                                              uint64_t* acc_empty, volatile int* abort_flag, volatile int* s_last, int warp,
                                              int lane, int epi_tid, int g, int G, uint32_t chain2_off = 0,
-                                             int acc_stages = 2, float* swiglu_xch = nullptr) {
+                                             int acc_stages = 2, float* swiglu_xch = nullptr, int rank = 0) {
     const int q = warp & 3;                 // TMEM lane quarter this warp may read
     const int row = q * 32 + lane;          // output feature within the tile
     int acc = 0;
@@ -217,6 +219,10 @@ __device__ __forceinline__ void run_epilogue(const LinearArgs& a, SegIter it, ui
     PendingTile pend[2];
     int n_pend = 0;
     int xi = 0;  // SwiGLU exchange buffer of the next 16-token batch
+    auto free_acc = [&](int i) {
+        if constexpr (CSZ == 1) ptx::mbar_arrive(&acc_empty[i]);
+        else ptx::mbar_arrive_cluster(ptx::cluster_map(ptx::smem_u32(&acc_empty[i]), 0));
+    };
     // ---- split tiles: wait for the other pieces, sum this CTA's share of the tokens
     auto flush_pending = [&]() {
         for (int i = 0; i < n_pend; ++i) {
@@ -224,7 +230,7 @@ __device__ __forceinline__ void run_epilogue(const LinearArgs& a, SegIter it, ui
             if (epi_tid == 0) {
                 const long long t0 = clock64();
                 int ok = 1;
-                while (ld_acquire(&a.tickets[2 * p.tile]) < p.nseg) {
+                while (ld_acquire(&a.tickets[2 * (p.tile * CSZ + rank)]) < p.nseg) {
                     if (*abort_flag || clock64() - t0 > kFixupBudgetClocks) { ok = 0; *abort_flag = 1; break; }
                 }
                 *s_last = ok;
@@ -234,17 +240,17 @@ __device__ __forceinline__ void run_epilogue(const LinearArgs& a, SegIter it, ui
             ptx::named_bar_sync(1, 128);  // everyone has read s_last before it can change
             if (ready && !CPM_EXPERIMENT(a, 16)) {
                 const int piece = g - p.g_first;
-                sum_pieces<MT, CH>(a, p, (p.m_cnt * piece) / p.nseg, (p.m_cnt * (piece + 1)) / p.nseg, row);
+                sum_pieces<MT, CH, CSZ>(a, p, (p.m_cnt * piece) / p.nseg, (p.m_cnt * (piece + 1)) / p.nseg, row, rank);
             }
             if (ready) {
                 // the partials of this tile may be overwritten once every piece's reader has left
                 ptx::named_bar_sync(1, 128);
                 if (epi_tid == 0) {
-                    const int old = atomicAdd(&a.tickets[2 * p.tile + 1], 1);
+                    const int old = atomicAdd(&a.tickets[2 * (p.tile * CSZ + rank) + 1], 1);
                     if (old == p.nseg - 1) {
-                        a.tickets[2 * p.tile + 1] = 0;
+                        a.tickets[2 * (p.tile * CSZ + rank) + 1] = 0;
                         __threadfence();
-                        a.tickets[2 * p.tile] = 0;  // ready for the next launch
+                        a.tickets[2 * (p.tile * CSZ + rank)] = 0;  // ready for the next launch
                     }
                 }
             }
@@ -257,6 +263,7 @@ __device__ __forceinline__ void run_epilogue(const LinearArgs& a, SegIter it, ui
         if (n_pend > 0 && tile < a.wave_tiles) flush_pending();
         int m_tile, n_tile;
         tile_to_mn(a, tile, m_tile, n_tile);
+        n_tile = n_tile * CSZ + rank;
         const int m_base = m_tile * MT;
         if (a.swiglu != 0 && swiglu_xch != nullptr) {
             // Lanes 0-63 of the accumulator hold the gate projection of 64 features, lanes 64-127 the up projection
@@ -301,7 +308,7 @@ __device__ __forceinline__ void run_epilogue(const LinearArgs& a, SegIter it, ui
                 }
             }
             ptx::tc_fence_before();
-            ptx::mbar_arrive(&acc_empty[acc]);
+            free_acc(acc);
             if (++acc == acc_stages) { acc = 0; acc_phase ^= 1; }
             continue;
         }
@@ -311,7 +318,7 @@ __device__ __forceinline__ void run_epilogue(const LinearArgs& a, SegIter it, ui
         const bool complete = (kb0 == 0 && kb1 == a.kblocks);
         // partial slot: pieces that start mid-tile use slot 0 of this CTA, the
         // piece that starts a tile but does not finish it uses slot 1
-        float* my_ws = a.workspace + (static_cast<size_t>(g) * 2 + (kb0 == 0 ? 1 : 0)) * (MT * BLOCK_N);
+        float* my_ws = a.workspace + (static_cast<size_t>(g * CSZ + rank) * 2 + (kb0 == 0 ? 1 : 0)) * (MT * BLOCK_N);
         const float bias_v = (a.bias != nullptr && n < a.N) ? __bfloat162float(a.bias[n]) : 0.f;
 
         if (!ptx::mbar_wait_warp(&acc_full[acc], acc_phase, abort_flag)) break;  // also converges the warp
@@ -349,7 +356,7 @@ __device__ __forceinline__ void run_epilogue(const LinearArgs& a, SegIter it, ui
             }
         }
         ptx::tc_fence_before();
-        ptx::mbar_arrive(&acc_empty[acc]);
+        free_acc(acc);
         if (++acc == acc_stages) { acc = 0; acc_phase ^= 1; }
 
         if (!complete && !CPM_EXPERIMENT(a, 2 | 8)) {
@@ -364,13 +371,13 @@ __device__ __forceinline__ void run_epilogue(const LinearArgs& a, SegIter it, ui
             __threadfence();               // this thread's partials are visible before the count
             ptx::named_bar_sync(1, 128);
             if (spread) {
-                if (epi_tid == 0) atomicAdd(&a.tickets[2 * tile], 1);
+                if (epi_tid == 0) atomicAdd(&a.tickets[2 * (tile * CSZ + rank)], 1);
                 pend[n_pend++] = p;
             } else {
                 if (epi_tid == 0) {
-                    const int old = atomicAdd(&a.tickets[2 * tile], 1);
+                    const int old = atomicAdd(&a.tickets[2 * (tile * CSZ + rank)], 1);
                     const int last = (old == p.nseg - 1) ? 1 : 0;
-                    if (last) a.tickets[2 * tile] = 0;  // ready for the next launch
+                    if (last) a.tickets[2 * (tile * CSZ + rank)] = 0;  // ready for the next launch
                     *s_last = last;
                 }
                 ptx::named_bar_sync(1, 128);
@@ -378,7 +385,7 @@ __device__ __forceinline__ void run_epilogue(const LinearArgs& a, SegIter it, ui
                 ptx::named_bar_sync(1, 128);  // everyone has read s_last before it can change
                 if (is_last && !CPM_EXPERIMENT(a, 16)) {
                     __threadfence();
-                    sum_pieces<MT, CH>(a, p, 0, m_cnt, row);
+                    sum_pieces<MT, CH, CSZ>(a, p, 0, m_cnt, row, rank);
                 }
             }
         }

@@ -29,6 +29,7 @@
 
 #include "common.cuh"
 #include "gemm_common.cuh"
+#include "gemm_pair.cuh"
 #include "ptx.cuh"
 
 using namespace gemm;
@@ -494,6 +495,15 @@ static long long base_grid(int n_tiles, int m_tiles, int kblocks, int M, int gri
     return grid;
 }
 
+// Pairs of CTAs of a launch, 0 = single CTAs: several token tiles, an even number of 128-row weight tiles, and as many pairs
+// at once as the split of the last wave relies on (its pieces wait for one another).
+static int pair_count(int n_tiles, int m_tiles, int kblocks, int mt, int grid_limit) {
+    static const bool off = tuning_env("CPMCU_LINEAR_NO_PAIR") != nullptr;   // bench only
+    if (off || m_tiles < 2 || mt != 256 || n_tiles % 2 != 0 || grid_limit < 2) return 0;
+    const long long units = static_cast<long long>(n_tiles / 2) * m_tiles * kblocks;
+    return static_cast<int>(std::min<long long>({std::max<long long>(1, units / 4), grid_limit / 2, linear_pair_capacity()}));
+}
+
 // Host-side walk of the work distribution make_linear_plan + launch_linear give a launch (without the cluster
 // variant, which cuts every tile into equal pieces): for every CTA its segments as six ints
 // (cta, tile, token tile, feature tile, first k-block, end k-block), in the order the CTA runs them.  The same
@@ -547,6 +557,14 @@ LinearPlan make_linear_plan(const bf16* x, int x_rows, const bf16* w, int M, int
     }
     const int n_tiles = ceil_div(N, BLOCK_N), m_tiles = ceil_div(M, p.mt), kblocks = K / BLOCK_K;
     const long long units = static_cast<long long>(n_tiles) * m_tiles * kblocks;
+    if (const int pairs = pair_count(n_tiles, m_tiles, kblocks, p.mt, grid_limit)) {
+        p.pair = 1;
+        p.grid = 2 * pairs;
+        plan_waves(static_cast<long long>(n_tiles / 2) * m_tiles, kblocks, pairs, p.wave_tiles, p.tail_grid);
+        p.tm_w = make_weight_tmap(w, N, K);
+        p.tm_x = make_tmap_2d(x, K, x_rows, static_cast<uint64_t>(K) * 2, BLOCK_K, p.mt / 2);
+        return p;
+    }
     long long grid = base_grid(n_tiles, m_tiles, kblocks, M, grid_limit);
     {
         static const char* forced = tuning_env("CPMCU_LINEAR_GRID");  // bench only: sweep the grid size
@@ -642,6 +660,15 @@ LinearPlan make_linear_swiglu_plan(const bf16* x, int x_rows, const bf16* w, int
     const long long tiles = static_cast<long long>(inter / 64) * ceil_div(M, p.mt);
     const int m_tiles = ceil_div(M, p.mt);
     p.grid = swiglu_grid(inter / 64, m_tiles, grid_limit);
+    if (const int pairs = pair_count(inter / 64, m_tiles, K / BLOCK_K, p.mt, grid_limit)) {
+        p.pair = 1;
+        p.wave_tiles = static_cast<int>(tiles / 2);
+        p.tail_grid = 1;
+        p.grid = 2 * std::min(pairs, p.wave_tiles);
+        p.tm_w = make_weight_tmap(w, 2 * inter, K);
+        p.tm_x = make_tmap_2d(x, K, x_rows, static_cast<uint64_t>(K) * 2, BLOCK_K, p.mt / 2);
+        return p;
+    }
     // No tile is cut, nothing goes through the workspace.  Several token tiles: whole tiles in waves.  One token tile:
     // the grid divides the tiles, and every CTA takes consecutive ones (one contiguous run of gate rows and one of up
     // rows per CTA instead of two scattered 64-row slabs per tile).
@@ -675,10 +702,11 @@ void launch_linear(const LinearPlan& p, cudaStream_t stream) {
     a.band = raster_band(p.mt, p.K);
     if (p.swiglu) {   // N = output features; a tile covers 64 of them (gate + up rows)
         a.n_tiles = ceil_div(p.N, 64);
-        CPM_REQUIRE(p.cluster == 0 && (p.wave_tiles == a.n_tiles * a.m_tiles ||
-                                       (a.m_tiles == 1 && p.wave_tiles == 0 && a.n_tiles % p.grid == 0)),
+        CPM_REQUIRE(p.pair || (p.cluster == 0 && (p.wave_tiles == a.n_tiles * a.m_tiles ||
+                                       (a.m_tiles == 1 && p.wave_tiles == 0 && a.n_tiles % p.grid == 0))),
                     "linear: the SwiGLU epilogue needs whole tiles");
     }
+    if (p.pair) a.n_tiles /= 2;
     a.total_units = (static_cast<long long>(a.n_tiles) * a.m_tiles - a.wave_tiles) * a.kblocks;
     a.y = p.y; a.ldy = p.ldy; a.bias = p.bias;
     a.workspace = p.workspace; a.tickets = p.tickets;
@@ -710,6 +738,10 @@ void launch_linear(const LinearPlan& p, cudaStream_t stream) {
                             "mean %lld max %lld; epilogue done min %lld mean %lld max %lld\n",
                     p.grid, lo[0], sum[0] / p.grid, hi[0], lo[1], sum[1] / p.grid, hi[1]);
         }
+    }
+    if (p.pair) {
+        launch_linear_pair(p, a, stream);
+        return;
     }
     if (p.cluster != 0 && launch_cluster_any(p, a, stream)) return;
     switch (p.mt) {
