@@ -31,9 +31,10 @@ struct LinearArgs {
     int band = 16;   // token tiles per raster band (tile_to_mn)
 };
 
-// Shared memory the SwiGLU epilogue exchanges up-projection values through: two buffers of
-// [2 warps][16 tokens][32 lanes] floats.
-constexpr int SWIGLU_XCH_BYTES = 2 * 2 * 16 * 32 * 4;
+// Shared memory of the epilogue: per warp [16 tokens][32 features] floats, for the values the two halves of a SwiGLU tile
+// exchange and for bf16 results on their way to 16-byte stores.
+constexpr int EPI_WARP_BYTES = 16 * 32 * 4;
+constexpr int EPI_XCH_BYTES = 4 * EPI_WARP_BYTES;
 
 #ifdef CPMCU_GEMM_PROFILE
 constexpr bool kGemmProf = true;
@@ -143,6 +144,82 @@ __device__ __forceinline__ int ld_acquire(const int* p) {
     return v;
 }
 
+// Results of one warp: v[c] is feature n0 + lane of token row y_row + c, c < T.  An accumulator's lanes are features, so a direct
+// store writes two bytes per lane; through `buf` (EPI_WARP_BYTES of this warp's own) eight features are one 16-byte store:
+// 4096 x 2048 x 128 (rows x N x K, all epilogue) 22.8 us with two-byte stores, 12.4 this way.
+// `vec`: rows and widths allow that.
+template <int T>
+__device__ __forceinline__ void store_tokens(bf16* y, int ldy, int N, int y_row, int cnt, int n0, const float (&v)[T], uint8_t* buf, int lane, bool vec) {
+    if (vec) {
+        bf16* b = reinterpret_cast<bf16*>(buf);
+        __syncwarp();   // the buffer's earlier contents have been read
+#pragma unroll
+        for (int c = 0; c < T; ++c) b[c * 32 + lane] = __float2bfloat16(v[c]);
+        __syncwarp();
+        const int f = n0 + (lane & 3) * 8;
+#pragma unroll
+        for (int k = 0; k < T; k += 8) {
+            const int c = k + (lane >> 2);
+            const uint4 w = *reinterpret_cast<const uint4*>(buf + c * 64 + (lane & 3) * 16);
+            if (c < cnt && f < N) *reinterpret_cast<uint4*>(y + static_cast<size_t>(y_row + c) * ldy + f) = w;
+        }
+    } else if (n0 + lane < N) {
+#pragma unroll
+        for (int c = 0; c < T; ++c) {
+            if (c < cnt) y[static_cast<size_t>(y_row + c) * ldy + n0 + lane] = __float2bfloat16(v[c]);
+        }
+    }
+}
+__device__ __forceinline__ bool rows_take_16_bytes(const bf16* y, int ldy, int N) {
+    return ((reinterpret_cast<uintptr_t>(y) | (static_cast<uintptr_t>(ldy) * 2) | (static_cast<uintptr_t>(N) * 2)) & 15) == 0;
+}
+
+// SwiGLU of one accumulator tile: lanes 0-63 hold the gate projection of 64 features, lanes 64-127 the up projection of the same
+// ones.  Warps q and q + 2 hand each other half of the tokens of a batch, so all four compute, each on independent elements
+// whose exponentials and divisions overlap.  (With a branch per element and the gate warps idle, an element took 200 cycles: a
+// 256-token tile 29 us beside 17 us of MMAs at K = 4096; 4096 x 16384 x 4096 gated 816 us then, 545 now, K = 2048 x 8192 395
+// then, 154 now, and 60 rows x 16384 x 4096, where it is the tail of the launch, 47.9 then, 43.4 now.)  Both projections are
+// rounded to bf16 first as the unfused pair of kernels stores them; the clamped form takes them in fp32.  n0: first of this
+// warp's 32 features.
+template <int MT>
+__device__ __forceinline__ void swiglu_tile(uint32_t t_addr, int m_cnt, bf16* y, int ldy, int N, int y_row, int n0, float limit, float alpha,
+                                            float* xch, int q, int lane, bool vec) {
+    constexpr int HB = MT >= 32 ? 16 : 8;   // tokens per warp and batch
+    float* out = xch + q * (EPI_WARP_BYTES / 4);          // to the partner
+    float* in = xch + (q ^ 2) * (EPI_WARP_BYTES / 4);     // from the partner; then this warp's results
+    const int pair_bar = 2 + (q & 1);
+    const bool gates = q < 2;
+#pragma unroll 1
+    for (int c0 = 0; c0 < m_cnt; c0 += 2 * HB) {   // uniform across the CTA
+        uint32_t r[2 * HB];
+        ptx::tmem_ld16(t_addr + c0, r);
+        if constexpr (HB == 16) ptx::tmem_ld16(t_addr + c0 + 16, r + 16);
+        ptx::tmem_wait_ld();
+        // gate warps keep the first half of the tokens, up warps the second
+#pragma unroll
+        for (int c = 0; c < HB; ++c) out[c * 32 + lane] = __uint_as_float(gates ? r[HB + c] : r[c]);
+        ptx::named_bar_sync(pair_bar, 64);
+        float v[HB];
+        if (limit > 0.f) {
+#pragma unroll
+            for (int c = 0; c < HB; ++c) {
+                const float mine = __uint_as_float(gates ? r[c] : r[HB + c]), other = in[c * 32 + lane];
+                v[c] = clamped_gate(gates ? mine : other, gates ? other : mine, limit, alpha);
+            }
+        } else {
+#pragma unroll
+            for (int c = 0; c < HB; ++c) {
+                const float mine = __bfloat162float(__float2bfloat16(__uint_as_float(gates ? r[c] : r[HB + c])));
+                const float other = __bfloat162float(__float2bfloat16(in[c * 32 + lane]));
+                v[c] = silu_mul(gates ? mine : other, gates ? other : mine);
+            }
+        }
+        const int first = c0 + (gates ? 0 : HB);
+        store_tokens<HB>(y, ldy, N, y_row + first, m_cnt - first, n0, v, reinterpret_cast<uint8_t*>(in), lane, vec);
+        ptx::named_bar_sync(pair_bar, 64);   // the partner may write `in` again
+    }
+}
+
 // A split tile this CTA holds a piece of: summed after the CTA's last segment.
 struct PendingTile {
     int tile, g_first, nseg, m_base, m_cnt, n;
@@ -152,7 +229,7 @@ struct PendingTile {
 // Sum tokens [t_begin, t_end) of a split tile over its pieces in CTA order (deterministic) and store them:
 // CH tokens per pass, the coalesced loads of up to four pieces (4 * CH per thread) in flight before the adds.
 template <int MT, int CH, int CSZ>
-__device__ __forceinline__ void sum_pieces(const LinearArgs& a, const PendingTile& p, int t_begin, int t_end, int row, int rank) {
+__device__ __forceinline__ void sum_pieces(const LinearArgs& a, const PendingTile& p, int t_begin, int t_end, int row, int rank, uint8_t* buf, bool vec) {
     const int g_last = p.g_first + p.nseg - 1;
 #pragma unroll 1
     for (int c0 = t_begin; c0 < t_end; c0 += CH) {
@@ -176,13 +253,12 @@ __device__ __forceinline__ void sum_pieces(const LinearArgs& a, const PendingTil
                 for (int c = 0; c < CH; ++c) sum[c] += v[s][c];
             }
         }
-        if (p.n < a.N) {
 #pragma unroll
-            for (int c = 0; c < CH; ++c) {
-                if (c0 + c < t_end) {
-                    a.y[static_cast<size_t>(p.m_base + c0 + c) * a.ldy + p.n] = __float2bfloat16(sum[c] + p.bias);
-                }
-            }
+        for (int h = 0; h < CH; h += 16) {
+            float v[CH < 16 ? CH : 16];
+#pragma unroll
+            for (int c = 0; c < CH && c < 16; ++c) v[c] = sum[h + c] + p.bias;
+            store_tokens(a.y, a.ldy, a.N, p.m_base + c0 + h, t_end - c0 - h, p.n & ~31, v, buf, row & 31, vec);
         }
     }
 }
@@ -210,7 +286,7 @@ template <int MT, int CH, int CSZ = 1>
 __device__ __forceinline__ void run_epilogue(const LinearArgs& a, SegIter it, uint32_t tmem_base, uint64_t* acc_full,
                                              uint64_t* acc_empty, volatile int* abort_flag, volatile int* s_last, int warp,
                                              int lane, int epi_tid, int g, int G, uint32_t chain2_off = 0,
-                                             int acc_stages = 2, float* swiglu_xch = nullptr, int rank = 0) {
+                                             int acc_stages = 2, float* xch = nullptr, int rank = 0) {
     const int q = warp & 3;                 // TMEM lane quarter this warp may read
     const int row = q * 32 + lane;          // output feature within the tile
     int acc = 0;
@@ -218,7 +294,8 @@ __device__ __forceinline__ void run_epilogue(const LinearArgs& a, SegIter it, ui
     int tile, kb0, kb1;
     PendingTile pend[2];
     int n_pend = 0;
-    int xi = 0;  // SwiGLU exchange buffer of the next 16-token batch
+    uint8_t* buf = reinterpret_cast<uint8_t*>(xch) + q * EPI_WARP_BYTES;   // xch null: never used
+    const bool vec = xch != nullptr && rows_take_16_bytes(a.y, a.ldy, a.N);
     auto free_acc = [&](int i) {
         if constexpr (CSZ == 1) ptx::mbar_arrive(&acc_empty[i]);
         else ptx::mbar_arrive_cluster(ptx::cluster_map(ptx::smem_u32(&acc_empty[i]), 0));
@@ -240,7 +317,7 @@ __device__ __forceinline__ void run_epilogue(const LinearArgs& a, SegIter it, ui
             ptx::named_bar_sync(1, 128);  // everyone has read s_last before it can change
             if (ready && !CPM_EXPERIMENT(a, 16)) {
                 const int piece = g - p.g_first;
-                sum_pieces<MT, CH, CSZ>(a, p, (p.m_cnt * piece) / p.nseg, (p.m_cnt * (piece + 1)) / p.nseg, row, rank);
+                sum_pieces<MT, CH, CSZ>(a, p, (p.m_cnt * piece) / p.nseg, (p.m_cnt * (piece + 1)) / p.nseg, row, rank, buf, vec);
             }
             if (ready) {
                 // the partials of this tile may be overwritten once every piece's reader has left
@@ -265,48 +342,13 @@ __device__ __forceinline__ void run_epilogue(const LinearArgs& a, SegIter it, ui
         tile_to_mn(a, tile, m_tile, n_tile);
         n_tile = n_tile * CSZ + rank;
         const int m_base = m_tile * MT;
-        if (a.swiglu != 0 && swiglu_xch != nullptr) {
-            // Lanes 0-63 of the accumulator hold the gate projection of 64 features, lanes 64-127 the up projection
-            // of the same features.  Both are rounded to bf16 as the unfused pair of kernels stores them; the two
-            // warps of the gate half pass theirs through shared memory and the two warps of the up half (the ones
-            // that share no scheduler with the producer or the MMA warp) store silu(gate) * up.
+        if (a.swiglu != 0 && xch != nullptr) {
             int m_cnt = a.M - m_base;
             if (m_cnt > MT) m_cnt = MT;
-            const int n_out = n_tile * 64 + (row & 63);
             if (!ptx::mbar_wait_warp(&acc_full[acc], acc_phase, abort_flag)) break;
             ptx::tc_fence_after();
-            const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * MT;
-#pragma unroll 1
-            for (int c0 = 0; c0 < MT; c0 += 16) {
-                if (c0 >= m_cnt) break;  // uniform across the CTA
-                uint32_t r[16];
-                ptx::tmem_ld16(t_addr + c0, r);
-                ptx::tmem_wait_ld();
-                float* xb = swiglu_xch + (xi & 1) * (2 * 16 * 32);
-                ++xi;
-                if (q < 2) {
-#pragma unroll
-                    for (int c = 0; c < 16; ++c) {
-                        const float gv = __uint_as_float(r[c]);
-                        xb[(q * 16 + c) * 32 + lane] = a.gate_limit > 0.f ? gv : __bfloat162float(__float2bfloat16(gv));
-                    }
-                }
-                // the batch after the next one reuses this buffer: its writers pass the next batch's barrier only
-                // after this batch's readers have arrived there
-                ptx::named_bar_sync(1, 128);
-                if (q >= 2 && n_out < a.N) {
-#pragma unroll
-                    for (int c = 0; c < 16; ++c) {
-                        if (c0 + c < m_cnt) {
-                            const float uv = __uint_as_float(r[c]);
-                            const float gv = xb[((q - 2) * 16 + c) * 32 + lane];
-                            const float av = a.gate_limit > 0.f ? clamped_gate(gv, uv, a.gate_limit, a.gate_alpha)
-                                                                : silu_mul(gv, __bfloat162float(__float2bfloat16(uv)));
-                            a.y[static_cast<size_t>(m_base + c0 + c) * a.ldy + n_out] = __float2bfloat16(av);
-                        }
-                    }
-                }
-            }
+            swiglu_tile<MT>(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * MT, m_cnt, a.y, a.ldy, a.N, m_base,
+                            n_tile * 64 + (q & 1) * 32, a.gate_limit, a.gate_alpha, xch, q, lane, vec);
             ptx::tc_fence_before();
             free_acc(acc);
             if (++acc == acc_stages) { acc = 0; acc_phase ^= 1; }
@@ -339,15 +381,10 @@ __device__ __forceinline__ void run_epilogue(const LinearArgs& a, SegIter it, ui
             }
             ptx::tmem_wait_ld();
             if (complete) {
-                if (n < a.N) {
+                float v[16];
 #pragma unroll
-                    for (int c = 0; c < 16; ++c) {
-                        if (c0 + c < m_cnt) {
-                            a.y[static_cast<size_t>(m_base + c0 + c) * a.ldy + n] =
-                                __float2bfloat16(__uint_as_float(r[c]) + bias_v);
-                        }
-                    }
-                }
+                for (int c = 0; c < 16; ++c) v[c] = __uint_as_float(r[c]) + bias_v;
+                store_tokens(a.y, a.ldy, a.N, m_base + c0, m_cnt - c0, n & ~31, v, buf, lane, vec);
             } else if (!CPM_EXPERIMENT(a, 4)) {
 #pragma unroll
                 for (int c = 0; c < 16; ++c) {
@@ -385,7 +422,7 @@ __device__ __forceinline__ void run_epilogue(const LinearArgs& a, SegIter it, ui
                 ptx::named_bar_sync(1, 128);  // everyone has read s_last before it can change
                 if (is_last && !CPM_EXPERIMENT(a, 16)) {
                     __threadfence();
-                    sum_pieces<MT, CH, CSZ>(a, p, 0, m_cnt, row, rank);
+                    sum_pieces<MT, CH, CSZ>(a, p, 0, m_cnt, row, rank, buf, vec);
                 }
             }
         }

@@ -6,8 +6,8 @@
 // launches is the tensor pipe and, in a warm pass, the power cap: per MMA an SM reads 8 KB of operands from shared memory
 // instead of 12, and per k-block 32 KB come in instead of 48, so L2 and shared memory spend less of the power.
 // Loads carry no multicast; the barrier that counts both CTAs' copies is rank 0's.
-// Back to back on constant data, single CTAs / pairs: 4096 x 4096 x 16384 (rows x N x K) 357 / 283 us, 4096 x 4608 x 4096 113 / 107,
-// 2048 x 4096 x 16384 191 / 151; with K = 2048 the epilogue hides the difference (71.3 / 70.6 us for N = 3072).
+// Back to back on constant data, single CTAs / pairs, both with the former epilogue: 4096 x 4096 x 16384 (rows x N x K) 357 / 283 us,
+// 4096 x 4608 x 4096 113 / 107, 2048 x 4096 x 16384 191 / 151; with the present one (gemm_common.cuh) 274, 87 and 144.
 #include <algorithm>
 
 #include "common.cuh"
@@ -26,7 +26,7 @@ constexpr int STAGE_BYTES = W_BYTES + X_BYTES;
 constexpr int STAGES = 6;
 constexpr int TMEM_COLS = 2 * MT;
 constexpr int CTRL_BYTES = 256;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + CTRL_BYTES + SWIGLU_XCH_BYTES + 1024;
+constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + CTRL_BYTES + EPI_XCH_BYTES + 1024;
 constexpr int NUM_THREADS = 192;   // warp 0 TMA, warp 1 MMA (rank 0) + TMEM, warps 2-5 epilogue
 static_assert(SMEM_BYTES <= 232448, "shared memory budget");
 
@@ -41,7 +41,7 @@ linear_umma_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_c
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     volatile int* s_last = abort_flag + 1;
-    float* swiglu_xch = reinterpret_cast<float*>(smem + STAGES * STAGE_BYTES + CTRL_BYTES);
+    float* epi_xch = reinterpret_cast<float*>(smem + STAGES * STAGE_BYTES + CTRL_BYTES);
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -158,7 +158,7 @@ linear_umma_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_c
     } else {
         // ------------------------------------------------ epilogue (128 threads of each CTA, its own 128 features)
         run_epilogue<MT, 32, 2>(a, it, tmem_base, acc_full, acc_empty, abort_flag, s_last, warp, lane, threadIdx.x - 64, g, G, 0, 2,
-                                swiglu_xch, rank);
+                                epi_xch, rank);
     }
 
     ptx::tc_fence_before();

@@ -48,7 +48,7 @@ struct Cfg {
     static constexpr int STAGES = (MT <= 16) ? 10 : (MT <= 32) ? 9 : (MT <= 64) ? 8 : (MT <= 128) ? 6 : 4;
     static constexpr int TMEM_COLS = (2 * MT < 32) ? 32 : 2 * MT;
     static constexpr int CTRL_BYTES = 256;
-    static constexpr int XCH_BYTES = SWIGLU_XCH_BYTES;   // SwiGLU epilogue: gate values on their way to the up warps
+    static constexpr int XCH_BYTES = EPI_XCH_BYTES;   // values on their way between the epilogue warps and to memory
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + CTRL_BYTES + XCH_BYTES + 1024;
 };
 
@@ -67,7 +67,7 @@ linear_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     volatile int* s_last = abort_flag + 1;
-    float* swiglu_xch = (C::XCH_BYTES > 0) ? reinterpret_cast<float*>(smem + C::STAGES * C::STAGE_BYTES + C::CTRL_BYTES) : nullptr;
+    float* epi_xch = (C::XCH_BYTES > 0) ? reinterpret_cast<float*>(smem + C::STAGES * C::STAGE_BYTES + C::CTRL_BYTES) : nullptr;
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -202,7 +202,7 @@ linear_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     } else {
         // ------------------------------------------------ epilogue (128 threads)
         run_epilogue<MT, (MT < 32) ? MT : 32>(a, it, tmem_base, acc_full, acc_empty, abort_flag, s_last, warp, lane,
-                                              threadIdx.x - 64, g, G, 0, 2, swiglu_xch);
+                                              threadIdx.x - 64, g, G, 0, 2, epi_xch);
         if (kGemmProf && a.prof != nullptr && threadIdx.x == 64) a.prof[g * 4 + 1] = clock64() - pt_dep;  // epilogue done
     }
     if (kGemmProf && a.prof != nullptr && warp == 1 && lane == 0) a.prof[g * 4 + 0] = clock64() - pt_dep;  // last MMA issued

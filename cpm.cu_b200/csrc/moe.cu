@@ -384,7 +384,7 @@ struct Cfg {
     static constexpr int TMEM_COLS = (2 * MT < 32) ? 32 : 2 * MT;
     static constexpr int CTRL_BYTES = 256;
     static constexpr int ENTRY_BYTES = 16 * kMoeMaxEntries;
-    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + CTRL_BYTES + gemm::SWIGLU_XCH_BYTES + ENTRY_BYTES + 1024;
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + CTRL_BYTES + gemm::EPI_XCH_BYTES + ENTRY_BYTES + 1024;
     static_assert(SMEM_BYTES <= 232448, "shared memory budget");
 };
 
@@ -460,7 +460,7 @@ moe_gemm_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     float* xch = reinterpret_cast<float*>(smem + C::STAGES * C::STAGE_BYTES + C::CTRL_BYTES);
-    int4* entries = reinterpret_cast<int4*>(smem + C::STAGES * C::STAGE_BYTES + C::CTRL_BYTES + gemm::SWIGLU_XCH_BYTES);
+    int4* entries = reinterpret_cast<int4*>(smem + C::STAGES * C::STAGE_BYTES + C::CTRL_BYTES + gemm::EPI_XCH_BYTES);
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -595,47 +595,27 @@ moe_gemm_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
     } else {
         // ------------------------------------------------ epilogue (128 threads; lane = feature, column = row of the group)
         const int q = warp & 3;
-        const int row = q * 32 + lane;
-        int acc = 0, xi = 0;
+        int acc = 0;
         uint32_t acc_phase = 0;
         for (int t = blockIdx.x; t < total; t += gridDim.x) {
             const TileJob j = tile_job<SWIGLU>(a, entries, t);
-            const int n = SWIGLU ? j.n_tile * 64 + (row & 63) : j.n_tile * gemm::BLOCK_N + row;
             if (!ptx::mbar_wait_warp(&acc_full[acc], acc_phase, abort_flag)) break;
             ptx::tc_fence_after();
             const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * MT;
+            const bool vec = gemm::rows_take_16_bytes(a.y, a.ldy, j.N);
+            if constexpr (SWIGLU) {
+                gemm::swiglu_tile<MT>(t_addr, j.rows, a.y, a.ldy, j.N, j.y_row, j.n_tile * 64 + (q & 1) * 32, 0.f, 0.f, xch, q, lane, vec);
+            } else {
 #pragma unroll 1
-            for (int c0 = 0; c0 < MT; c0 += 16) {
-                if (c0 >= j.rows) break;   // uniform across the CTA
-                uint32_t r[16];
-                ptx::tmem_ld16(t_addr + c0, r);
-                ptx::tmem_wait_ld();
-                bf16* y = a.y + static_cast<size_t>(j.y_row + c0) * a.ldy + n;
-                if constexpr (SWIGLU) {
-                    // lanes 0-63 hold the gate projection, lanes 64-127 the up projection of the same 64 features; the gate
-                    // values pass through one of two shared-memory buffers to the warps of the up half, which store
-                    float* xb = xch + (xi & 1) * (2 * 16 * 32);
-                    ++xi;
-                    if (q < 2) {
+                for (int c0 = 0; c0 < j.rows; c0 += 16) {   // uniform across the CTA
+                    uint32_t r[16];
+                    ptx::tmem_ld16(t_addr + c0, r);
+                    ptx::tmem_wait_ld();
+                    float v[16];
 #pragma unroll
-                        for (int c = 0; c < 16; ++c) xb[(q * 16 + c) * 32 + lane] = __bfloat162float(__float2bfloat16(__uint_as_float(r[c])));
-                    }
-                    // a buffer is written again two batches later, past the next batch's barrier
-                    ptx::named_bar_sync(1, 128);
-                    if (q >= 2 && n < j.N) {
-#pragma unroll
-                        for (int c = 0; c < 16; ++c) {
-                            if (c0 + c < j.rows) {
-                                const float uv = __bfloat162float(__float2bfloat16(__uint_as_float(r[c])));
-                                y[static_cast<size_t>(c) * a.ldy] = __float2bfloat16(silu_mul(xb[((q - 2) * 16 + c) * 32 + lane], uv));
-                            }
-                        }
-                    }
-                } else if (n < j.N) {
-#pragma unroll
-                    for (int c = 0; c < 16; ++c) {
-                        if (c0 + c < j.rows) y[static_cast<size_t>(c) * a.ldy] = __float2bfloat16(__uint_as_float(r[c]));
-                    }
+                    for (int c = 0; c < 16; ++c) v[c] = __uint_as_float(r[c]);
+                    gemm::store_tokens(a.y, a.ldy, j.N, j.y_row + c0, j.rows - c0, j.n_tile * gemm::BLOCK_N + q * 32, v,
+                                       reinterpret_cast<uint8_t*>(xch) + q * gemm::EPI_WARP_BYTES, lane, vec);
                 }
             }
             ptx::tc_fence_before();
