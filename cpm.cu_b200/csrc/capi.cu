@@ -628,6 +628,7 @@ int cpmcu_sparse_select(const void* q, int q_ld, int tq, int hq, int hkv, const 
         b.blockmask = static_cast<uint64_t*>(bm.p);
         b.bm_words = bm_words;
         b.max_tokens = tq;
+        b.budget = budget;
         SparseConfig cfg;
         cfg.enabled = true;
         cfg.sink_blocks = sink_window_size;

@@ -266,6 +266,7 @@ void Engine::lay_out(Pool& p) {
         sp_.c1 = take<bf16>(p, sp_.c1_layer_stride * mc_.layers + static_cast<size_t>(16) * kvd);
         sp_.c2 = mc_.sparse.compress_lse ? take<bf16>(p, sp_.c2_layer_stride * mc_.layers + static_cast<size_t>(16) * kvd) : nullptr;
         sp_.done = take<int32_t>(p, 2);
+        sp_.budget = budget_;
         sp_.score_ld = (budget_ / 16 + 127) / 128 * 128;
         sp_.max_tokens = static_cast<int>(R);
         sp_.scores = take<bf16>(p, static_cast<size_t>(mc_.hkv) * R * sp_.score_ld + 8);

@@ -65,7 +65,8 @@ __global__ void sparse_commit_kernel(const int32_t* __restrict__ kv_len, int kv_
     done[1] = compressed_len(L, C2_STRIDE);
 }
 
-// ---- stage 1.  Scores are a small GEMM (tokens x heads against a few thousand compressed keys, 0.6 GFLOP
+// ---- stage 1 of decode-sized launches, and of prefill chunks with fewer than 16 query heads per key head (the others:
+// sparse_stage1.cu).  A 60-token pass is a small GEMM (tokens x heads against a few thousand compressed keys, 0.6 GFLOP
 // per layer at 32k context) that is latency- and L2-bound, not tensor-bound: warp-level mma (wmma, 16 x 16 x 16
 // bf16) with the 16 heads of a KV group as the M = 16 fragment is enough and keeps the kernel short.
 //   lse kernel    grid (ceil(T / 8), hkv, key chunks of 128): per (token, head, chunk) the max and exp-sum of
@@ -439,7 +440,11 @@ void launch_sparse_select(const SparseBuffers& b, const SparseConfig& cfg, int l
     a.lse = b.lse;
     a.lse_chunks = b.score_ld / 128;
     const int lse_z = cfg.compress_lse ? ceil_div(a.lse_chunks, 4) : a.lse_chunks;
-    if (T <= 64) {
+    // 16 heads x 8 tokens fill a tensor-core tile; fewer heads per key head, and decode-sized launches (whose latency is that
+    // of their longest CTA), stay with warp-level fragments dealt over chunks of keys
+    if (T > 64 && grp == S1_MAXGRP) {
+        launch_sparse_stage1_prefill(b, cfg, layer, q, q_ld, T, hkv, kv_len, kv_add, n_valid, s);
+    } else if (T <= 64) {
         launch_kernel(sparse_stage1_lse_kernel<2>, dim3(ceil_div(T, 2), hkv, lse_z), dim3(S1_THREADS), 0, s, a);
         launch_kernel(sparse_stage1_score_kernel<2>, dim3(ceil_div(T, 2), hkv, b.score_ld / 128), dim3(S1_THREADS), 0, s, a);
     } else {

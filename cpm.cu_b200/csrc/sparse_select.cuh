@@ -24,12 +24,17 @@ struct SparseBuffers {
     uint64_t* blockmask = nullptr;  // [hkv][max_tokens][bm_words]
     int bm_words = 0;
     int max_tokens = 0;
+    int budget = 0;              // rows of the K/V cache
 };
 
 // Bring the compressed caches of all layers up to the L = *kv_len + kv_add accepted rows
 // (max_new = upper bound on entries added since the previous call).
 void launch_sparse_compress(const SparseBuffers& b, bf16* const* caches, int layers, int kv_dim, const int32_t* kv_len,
                             int kv_add, int max_new, cudaStream_t s);
+
+// Stage-1 scores alone, prefill-sized launches with 16 query heads per key head (sparse_stage1.cu).
+void launch_sparse_stage1_prefill(const SparseBuffers& b, const SparseConfig& cfg, int layer, const bf16* q, int q_ld, int T, int hkv,
+                                  const int32_t* kv_len, int kv_add, const int32_t* n_valid, cudaStream_t s);
 
 // Stage-1 scores of `T` query rows against the layer's compressed keys, then max-pool / top-k /
 // bitmask into b.blockmask ([hkv][T][bm_words], all ones while selection is not active).

@@ -36,14 +36,14 @@
 #include <type_traits>
 #include <vector>
 
+#include "attn_common.cuh"
 #include "common.cuh"
 #include "ptx.cuh"
 
+using namespace attn;
+
 namespace {
 
-constexpr int ROWS = 128;       // query rows per tile (UMMA M)
-constexpr int KEYS = 128;       // keys per tile
-constexpr int HALF_BYTES = ROWS * 128;        // 64 columns of a tile: 128 rows x 128 B
 // DK, DV: columns of a query / key row and of a value row of one head in memory, 64 or 128
 template <int DK, int DV>
 struct AttnCfg {
@@ -93,12 +93,6 @@ constexpr bool kAttnProf = true;
 constexpr bool kAttnProf = false;
 #endif
 __device__ __forceinline__ long long prof_clock() { return kAttnProf ? clock64() : 0; }
-
-__device__ __forceinline__ float fast_exp2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 
 // Software pipeline over 128-key tiles.  The control warp keeps the tensor pipe one tile
 // ahead: S(i+1) = Q K(i+1)^T is already in TMEM (two S stages) while the softmax warps work
