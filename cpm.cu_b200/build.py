@@ -15,7 +15,7 @@ CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "cpmcu")
 OBJ_DIR = os.path.join(HERE, "build")
 LIB = os.path.join(OUT_DIR, "libcpmcu_b200.so")
-SOURCES = ["runtime.cu", "gemm_umma.cu", "gemm_pair.cu", "gemm_w4_umma.cu", "elementwise.cu", "tree_attn.cu", "draft_tree.cu", "accept.cu",
+SOURCES = ["runtime.cu", "gemm_umma.cu", "gemm_pair.cu", "gemm_w4_umma.cu", "elementwise.cu", "tree_attn.cu", "pair_attn.cu", "draft_tree.cu", "accept.cu",
            "marlin_unpack.cu", "sparse_select.cu", "sparse_stage1.cu", "layered_ops.cu", "plain_ops.cu", "one_row.cu", "tanh_rows.cu", "recurrence.cu", "moe.cu", "engine.cu", "engine_layered.cu", "capi.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "--threads", "2"]

@@ -326,6 +326,7 @@ struct AttnPlan {
     int sink = 0;                     // 1: one more score of 0, without a value, in every softmax
     float out_scale = 1.f;            // factor of the output
     int splits = 1;
+    bool pair = false;                // two query tiles per CTA (pair_attn.cu)
     const int32_t* kv_len = nullptr;  // device scalar
     int kv_len_add = 0;               // keys visible = *kv_len + kv_len_add
     const int32_t* n_valid = nullptr; // device scalar: valid query rows (null = tq)

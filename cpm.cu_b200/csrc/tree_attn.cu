@@ -62,30 +62,6 @@ constexpr int TMEM_O = 256;
 constexpr int SOFTMAX_THREADS = 256;  // two threads per query row: warps 0-3 keys 0-63 of a tile, warps 4-7 keys 64-127
 constexpr int NTHREADS = SOFTMAX_THREADS + 32;  // + one control warp (TMA and MMA issue)
 
-struct AttnArgs {
-    int tq, hq, hkv, grp, tok_per_tile, num_mtiles;
-    int heavy_first;  // causal prefill: token tiles are handed out last-to-first, longest key range first
-    const int32_t* kv_len;
-    int kv_len_add;
-    const int32_t* n_valid;
-    const uint64_t* mask;
-    int mask_k;
-    int window;
-    int exact_window;    // > 0: per-token sliding window (tokens); BIASED instantiations only
-    float bias_exp;      // > 0: distance bias with slopes 2^(-bias_exp * (h + 1) / hq); BIASED instantiations only
-    int sink;            // 1: exp(0) is added to every row's sum
-    float out_scale;     // factor of the output
-    int out_cols;        // value columns that are stored per head (the rest of DV is padding)
-    const uint64_t* blockmask;  // [hkv][tq][bm_words] bits over 64-key blocks, or null
-    int bm_words, block_window;
-    float scale_log2;
-    bf16* out;
-    int out_ld;
-    float* ws_o;
-    float* ws_ml;
-    int* error;
-    long long* prof;  // bench only (-DCPMCU_ATTN_PROFILE): clock counters of CTA 0, or null
-};
 
 #ifdef CPMCU_ATTN_PROFILE
 constexpr bool kAttnProf = true;
@@ -682,8 +658,13 @@ AttnPlan make_biased_attn_plan(const bf16* q, int q_ld_tokens, const bf16* k_cac
     p.scale = scale;
     p.tm_q = make_tmap_3d(q, dk, hq, tq, static_cast<uint64_t>(dk) * 2, static_cast<uint64_t>(q_ld_tokens) * 2, 64, grp,
                           ROWS / grp);
-    p.tm_k = make_tmap_2d(k_cache, static_cast<uint64_t>(hkv) * dk, budget, static_cast<uint64_t>(hkv) * dk * 2, 64, KEYS);
-    p.tm_v = make_tmap_2d(v_cache, static_cast<uint64_t>(hkv) * dv, budget, static_cast<uint64_t>(hkv) * dv * 2, 64, KEYS);
+    // Two tiles per CTA (pair_attn.cu) once such CTAs number one and a half times the SMs: causal tiles differ in length, and fewer
+    // CTAs cannot even that out.  Query rows x heads / key heads, one tile / two tiles per CTA: 1024 x 32/2 (128 CTAs of two)
+    // 21.1 / 25.2 us, 2048 x 32/2 (256) 60 / 48, 4096 x 16/4 (256) 97 / 76, 4096 x 32/2 (512) 191 / 152.
+    p.pair = splits == 1 && 2LL * ceil_div(ceil_div(tq, ROWS / grp), 2) * hkv >= 3LL * runtime().num_sms;
+    const int box = p.pair ? 64 : KEYS;
+    p.tm_k = make_tmap_2d(k_cache, static_cast<uint64_t>(hkv) * dk, budget, static_cast<uint64_t>(hkv) * dk * 2, 64, box);
+    p.tm_v = make_tmap_2d(v_cache, static_cast<uint64_t>(hkv) * dv, budget, static_cast<uint64_t>(hkv) * dv * 2, 64, box);
     return p;
 }
 
@@ -760,6 +741,10 @@ void launch_tree_attention(const AttnPlan& p, cudaStream_t s) {
         }
     }
     CPM_REQUIRE(p.splits == 1 || (p.ws_o != nullptr && p.ws_ml != nullptr), "attention: split-KV needs a workspace");
+    if (p.pair) {
+        launch_pair_attention(p, a, s);
+        return;
+    }
     if (!p.biased) launch_attn<128, 128, false>(p, a, s);
     else if (p.d == 128 && p.dv == 128) launch_attn<128, 128, true>(p, a, s);
     else if (p.d == 128) launch_attn<128, 64, true>(p, a, s);
