@@ -6,6 +6,9 @@
 //   src/model/norm.cuh:8-99, embedding.cuh:7-52, rotary.cuh:7-34,
 //   attn.cuh:14-40 (copy_to_kvcache / permute), activation.cuh:7-18,
 //   elementwise.cuh:8-87.
+#include <algorithm>
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace {
@@ -146,63 +149,90 @@ __global__ void embedding_gather_kernel(const int32_t* __restrict__ ids, const b
     }
 }
 
+// VEC consecutive elements of a head's lower half and of its upper half, and their rotation.
+template <int VEC>
+struct RopeItem {
+    using Raw = typename std::conditional<VEC == 8, uint4, uint32_t>::type;
+    Raw lo, hi;
+    __device__ __forceinline__ void load(const bf16* p, int half) {
+        lo = *reinterpret_cast<const Raw*>(p);
+        hi = *reinterpret_cast<const Raw*>(p + half);
+    }
+    __device__ __forceinline__ void rotate(const float* cs, const float* sn) {
+        bf16* l = reinterpret_cast<bf16*>(&lo);
+        bf16* u = reinterpret_cast<bf16*>(&hi);
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) {
+            const float a = __bfloat162float(l[e]), b = __bfloat162float(u[e]);
+            l[e] = __float2bfloat16(a * cs[e] - b * sn[e]);
+            u[e] = __float2bfloat16(a * sn[e] + b * cs[e]);
+        }
+    }
+    __device__ __forceinline__ void store(bf16* p, int half) const {
+        *reinterpret_cast<Raw*>(p) = lo;
+        *reinterpret_cast<Raw*>(p + half) = hi;
+    }
+};
+
 // One CTA per token row.  q heads rotate in place; k heads rotate into the
 // cache; v heads are copied into the cache.  The d/2 sines and cosines of the row's
-// position are computed once per CTA; each thread then rotates element pairs
-// (c, c+1) and (c + d/2, c + d/2 + 1) with 4-byte accesses.
+// position are computed once per CTA.  Latency of one memory round trip after the other bounds a decode pass's launch, so a
+// thread's first elements and its values are requested before the position is known, and VEC = 8 (16-byte accesses, head
+// widths that are multiples of 16) leaves one trip for up to 64 heads of 128; with 4-byte accesses and five trips
+// a 60-row launch of 34 heads took 3.9 us in the step and one of 4096 rows 22 us.
+template <int VEC>
 __global__ void rope_append_kernel(bf16* __restrict__ qkv, int hq, int hkv, int d, const float* __restrict__ inv_freq,
                                    const int32_t* __restrict__ pos, const int32_t* __restrict__ pos_base, int pos_off,
                                    int pos_step, bf16* __restrict__ k_cache, bf16* __restrict__ v_cache,
                                    const int32_t* __restrict__ kv_len, int kv_off,
                                    const int32_t* __restrict__ n_valid, int cache_rows, int* __restrict__ error) {
-    grid_dependency_sync();
-    __shared__ float s_cos[128], s_sin[128];
+    grid_dep_trigger();
+    __shared__ __align__(16) float s_cos[128], s_sin[128];
     const int r = blockIdx.x;
     const int half = d >> 1;
     const int ld = (hq + 2 * hkv) * d;
     bf16* row = qkv + static_cast<size_t>(r) * ld;
+    const int per_head = half / VEC, items = (hq + hkv) * per_head;
+    const int kv_dim = hkv * d;
+    const bf16* vsrc = row + (hq + hkv) * d;
+    const float freq = threadIdx.x < half ? inv_freq[threadIdx.x] : 0.f;   // a constant of the model
+    grid_dep_wait();
     const int p = (pos != nullptr) ? pos[r] : (*pos_base + pos_off + r * pos_step);
-    bool store_kv = (n_valid == nullptr) || (r < *n_valid);
+    const int n_rows = (n_valid == nullptr) ? 0x7fffffff : *n_valid;
     const long long kv_row = static_cast<long long>(*kv_len) + kv_off + r;
+    int i = threadIdx.x;
+    RopeItem<VEC> item;
+    auto at = [&](int k) { const int h = k / per_head; return h * d + (k - h * per_head) * VEC; };
+    if (i < items) item.load(row + at(i), half);
+    uint4 v0 = make_uint4(0u, 0u, 0u, 0u);
+    const int vi = threadIdx.x * 8;
+    if (vi < kv_dim) v0 = *reinterpret_cast<const uint4*>(vsrc + vi);
+    bool store_kv = r < n_rows;
     if (store_kv && kv_row >= cache_rows) {  // host-side length checks come first; this only keeps memory intact
         store_kv = false;
         if (threadIdx.x == 0) atomicOr(error, ERR_KV_OVERFLOW);
     }
-    const int kv_dim = hkv * d;
+    store_kv = store_kv && kv_row >= 0;
     if (threadIdx.x < half) {
         float sn, cs;
-        sincosf(p * inv_freq[threadIdx.x], &sn, &cs);
+        sincosf(p * freq, &sn, &cs);
         s_cos[threadIdx.x] = cs;
         s_sin[threadIdx.x] = sn;
     }
     __syncthreads();
-    const int pairs = half >> 1;  // bf16x2 pairs per half head
-    for (int i = threadIdx.x; i < (hq + hkv) * pairs; i += blockDim.x) {
-        const int h = i / pairs, c = (i - h * pairs) * 2;
-        bf16* hp = row + h * d;
-        const __nv_bfloat162 lo = *reinterpret_cast<const __nv_bfloat162*>(hp + c);
-        const __nv_bfloat162 hi = *reinterpret_cast<const __nv_bfloat162*>(hp + c + half);
-        const float a0 = __bfloat162float(lo.x), a1 = __bfloat162float(lo.y);
-        const float b0 = __bfloat162float(hi.x), b1 = __bfloat162float(hi.y);
-        __nv_bfloat162 o_lo, o_hi;
-        o_lo.x = __float2bfloat16(a0 * s_cos[c] - b0 * s_sin[c]);
-        o_lo.y = __float2bfloat16(a1 * s_cos[c + 1] - b1 * s_sin[c + 1]);
-        o_hi.x = __float2bfloat16(a0 * s_sin[c] + b0 * s_cos[c]);
-        o_hi.y = __float2bfloat16(a1 * s_sin[c + 1] + b1 * s_cos[c + 1]);
-        if (h < hq) {
-            *reinterpret_cast<__nv_bfloat162*>(hp + c) = o_lo;
-            *reinterpret_cast<__nv_bfloat162*>(hp + c + half) = o_hi;
-        } else if (store_kv && kv_row >= 0) {
-            bf16* kd = k_cache + kv_row * kv_dim + (h - hq) * d;
-            *reinterpret_cast<__nv_bfloat162*>(kd + c) = o_lo;
-            *reinterpret_cast<__nv_bfloat162*>(kd + c + half) = o_hi;
-        }
+    while (i < items) {
+        const int h = i / per_head, c = (i - h * per_head) * VEC;
+        item.rotate(s_cos + c, s_sin + c);
+        if (h < hq) item.store(row + h * d + c, half);
+        else if (store_kv) item.store(k_cache + kv_row * kv_dim + (h - hq) * d + c, half);
+        i += blockDim.x;
+        if (i < items) item.load(row + at(i), half);
     }
-    if (store_kv && kv_row >= 0) {
-        const bf16* vsrc = row + (hq + hkv) * d;
+    if (store_kv) {
         bf16* vdst = v_cache + kv_row * kv_dim;
-        for (int i = threadIdx.x * 8; i < kv_dim; i += blockDim.x * 8) {
-            *reinterpret_cast<uint4*>(vdst + i) = *reinterpret_cast<const uint4*>(vsrc + i);
+        if (vi < kv_dim) *reinterpret_cast<uint4*>(vdst + vi) = v0;
+        for (int k = vi + blockDim.x * 8; k < kv_dim; k += blockDim.x * 8) {
+            *reinterpret_cast<uint4*>(vdst + k) = *reinterpret_cast<const uint4*>(vsrc + k);
         }
     }
 }
@@ -464,8 +494,16 @@ void launch_rope_append(bf16* qkv, int rows, int hq, int hkv, int d, const float
     if (rows <= 0) return;
     CPM_REQUIRE(pos != nullptr || pos_base != nullptr, "rope: no positions given");
     CPM_REQUIRE(d % 4 == 0 && d <= 256, "rope: head_dim must be a multiple of 4 and at most 256");
-    launch_kernel(rope_append_kernel, dim3(rows), dim3(256), 0, s, qkv, hq, hkv, d, inv_freq, pos, pos_base, pos_off,
-                  pos_step, k_cache, v_cache, kv_len, kv_off, n_valid, cache_rows, runtime().d_error);
+    auto run = [&](auto kernel, int vec) {
+        // a thread per item where that fits a CTA; at least the head's angles
+        const int items = (hq + hkv) * (d / 2 / vec);
+        const int threads = std::min(512, std::max(ceil_div(items, 32) * 32, ceil_div(d / 2, 32) * 32));
+        launch_kernel(kernel, dim3(rows), dim3(threads), 0, s, qkv, hq, hkv, d, inv_freq, pos, pos_base, pos_off, pos_step, k_cache, v_cache,
+                      kv_len, kv_off, n_valid, cache_rows, runtime().d_error);
+    };
+    const uintptr_t all = reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(k_cache);
+    if (d % 16 == 0 && (all & 15) == 0) run(rope_append_kernel<8>, 8);
+    else run(rope_append_kernel<2>, 2);
 }
 
 void launch_silu_gate(const bf16* gate_up, bf16* out, int rows, int inter, cudaStream_t s, bool interleaved) {
