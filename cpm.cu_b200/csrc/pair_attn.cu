@@ -13,9 +13,12 @@
 //                iteration before they are needed
 //   softmax      two threads per row, 64 keys each; the row maximum is exchanged through shared memory, once per iteration
 // Keys come in blocks of 64: thread half ch of iteration i works on block 2 i + ch.  Block-sparse mode lists the union of the
-// two tiles' blocks, so an iteration's two blocks need not be neighbours.
+// two tiles' blocks, so an iteration's two blocks need not be neighbours.  A tile's P V takes only the blocks some row of that tile
+// sees: a probability of zero does not hide an infinity or a NaN among the values, so no row meets values that the one-tile
+// kernel would not have shown it.
 // Tensor memory: S_A [0,128) S_B [128,256) O_A [256,384) O_B [384,512).
 #include <algorithm>
+#include <type_traits>
 
 #include "attn_common.cuh"
 
@@ -40,7 +43,8 @@ struct PairCfg {
     static constexpr int SMEM_P = SMEM_V + V_TILE;               // 2 tiles
     static constexpr int SMEM_LIST = SMEM_P + 2 * P_TILE;        // block numbers, 16 bits each
     static constexpr int SMEM_UNION = SMEM_LIST + MAX_BLOCKS * 2;    // 64 words of 64 blocks, then 65 prefix counts
-    static constexpr int SMEM_XCH = SMEM_UNION + 64 * 8 + 320;   // [2 tiles][2 buffers][2 halves][128] floats
+    static constexpr int SMEM_SEEN = SMEM_UNION + 64 * 8 + 320;  // [2 tiles] the words of that tile alone
+    static constexpr int SMEM_XCH = SMEM_SEEN + 2 * 64 * 8;      // [2 tiles][2 buffers][2 halves][128] floats
     static constexpr int SMEM_CTRL = SMEM_XCH + 8 * ROWS * 4;
     static constexpr int SMEM_TOTAL = SMEM_CTRL + 256 + 1024;
     static_assert(SMEM_TOTAL <= 232448, "shared memory budget");
@@ -68,6 +72,8 @@ pair_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     uint16_t* list = reinterpret_cast<uint16_t*>(smem + C::SMEM_LIST);
     unsigned long long* uni = reinterpret_cast<unsigned long long*>(smem + C::SMEM_UNION);
     int* uni_at = reinterpret_cast<int*>(uni + 64);
+    unsigned long long* seen = reinterpret_cast<unsigned long long*>(smem + C::SMEM_SEEN);
+    int* run = uni_at + 65;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     grid_dep_trigger();
@@ -125,23 +131,35 @@ pair_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     if (BIASED && a.exact_window > 0) key_lo = max(causal_base + t0 - a.exact_window + 1, 0);
     const int blk_lo = key_lo / BLK;
     const int blk_hi = (key_hi + BLK - 1) / BLK;
+    // blocks [lo, hi) that rows of one of the two tiles may see
+    auto tile_blocks = [&](int tile, int& lo, int& hi) {
+        const int first = t0 + tile * a.tok_per_tile, end = min(first + a.tok_per_tile, tq_eff);
+        lo = (BIASED && a.exact_window > 0 ? max(causal_base + first - a.exact_window + 1, 0) : tile_lo(first)) / BLK;
+        hi = end > first ? (max(min(kv_total, causal_base + end), 0) + BLK - 1) / BLK : 0;
+    };
     int n_blk = max(blk_hi - blk_lo, 0);
 
     const bool sparse = (a.blockmask != nullptr);
     if (sparse) {
-        if (tid < 64) {
+        if (tid == 0) { run[0] = 0; run[1] = MAX_BLOCKS; }
+        if (tid < 128) {   // 64 words of each tile
+            const int tile = tid >> 6, word = tid & 63;
+            const int first = t0 + tile * a.tok_per_tile, end = min(first + a.tok_per_tile, t_end);
             unsigned long long m = 0ull;
-            if (tid < a.bm_words) {
-                const uint64_t* r = a.blockmask + (static_cast<size_t>(h) * a.tq + t0) * a.bm_words + tid;
-                for (int t = t0; t < t_end; ++t, r += a.bm_words) m |= *r;
+            if (word < a.bm_words) {
+                const uint64_t* r = a.blockmask + (static_cast<size_t>(h) * a.tq + first) * a.bm_words + word;
+                for (int t = first; t < end; ++t, r += a.bm_words) m |= *r;
             }
-            // the trailing window of the pair's first token reaches furthest back
-            const int left = max((t0 + causal_base + 63) / 64 - a.block_window, 0);
-            const int b0 = tid * 64;
+            // the trailing window of the tile's first token reaches furthest back
+            const int left = max((first + causal_base + 63) / 64 - a.block_window, 0);
+            const int b0 = word * 64;
             auto from = [&](int b) -> unsigned long long { return b <= b0 ? ~0ull : b >= b0 + 64 ? 0ull : ~0ull << (b - b0); };
-            m = (m | from(left)) & from(blk_lo) & ~from(min(blk_hi, MAX_BLOCKS));
-            uni[tid] = n_blk > 0 ? m : 0ull;
+            int lo, hi;
+            tile_blocks(tile, lo, hi);
+            seen[tid] = (m | from(left)) & from(lo) & ~from(min(hi, MAX_BLOCKS));
         }
+        __syncthreads();
+        if (tid < 64) uni[tid] = seen[tid] | seen[64 + tid];
         __syncthreads();
         if (warp == 0) {   // exclusive prefix counts of the 64 words, two per lane
             const int c0 = __popcll(uni[2 * lane]), c1 = __popcll(uni[2 * lane + 1]);
@@ -156,15 +174,27 @@ pair_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             if (lane == 31) uni_at[64] = sum;
         }
         __syncthreads();
+        n_blk = uni_at[64];
         if (tid < 512) {   // eight blocks per thread
             const int word = tid >> 3, bit0 = (tid & 7) * 8;
-            const unsigned long long m = uni[word];
+            const unsigned long long m = uni[word], shared = seen[word] & seen[64 + word];
             int at = uni_at[word] + __popcll(m & ((1ull << bit0) - 1ull));
+            int lo = 0, hi = n_blk;
             for (int k = bit0; k < bit0 + 8; ++k) {
-                if ((m >> k) & 1ull) list[at++] = static_cast<uint16_t>(word * 64 + k);
+                if (!((m >> k) & 1ull)) continue;
+                if (!((shared >> k) & 1ull)) {
+                    if (2 * at < n_blk) lo = at + 1;
+                    else hi = min(hi, at);
+                }
+                list[at++] = static_cast<uint16_t>(word * 64 + k);
+            }
+            lo = __reduce_max_sync(0xffffffffu, lo);
+            hi = __reduce_min_sync(0xffffffffu, hi);
+            if (lane == 0) {
+                if (lo > 0) atomicMax(run, lo);
+                if (hi < n_blk) atomicMin(run + 1, hi);
             }
         }
-        n_blk = uni_at[64];
         __syncthreads();
     }
     const int n_it = (n_blk + 1) / 2;
@@ -173,34 +203,49 @@ pair_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     if (warp == SOFT_WARPS) {
         // ================================================= MMA issue
         if (lane == 0 && n_it > 0) {
+            int lo_a, hi_a, lo_b, hi_b;
+            tile_blocks(0, lo_a, hi_a);
+            tile_blocks(1, lo_b, hi_b);
+            auto tile_sees = [&](int tile, int b) -> bool {
+                return sparse ? (seen[64 * tile + (b >> 6)] >> (b & 63)) & 1ull : b >= (tile ? lo_b : lo_a) && b < (tile ? hi_b : hi_a);
+            };
+            // iterations [whole_lo, whole_hi) have two blocks that both tiles see: the longest stretch in the middle of the list
+            const int whole_lo = ((sparse ? run[0] : max(lo_b - blk_lo, 0)) + 1) / 2, whole_hi = (sparse ? min(run[1], n_blk) : max(min(hi_a, hi_b) - blk_lo, 0)) / 2;
             constexpr uint32_t idesc_s = ptx::umma_idesc_bf16(ROWS, KEYS, 0, 0);
             constexpr uint32_t idesc_o = ptx::umma_idesc_bf16(ROWS, DV, 0, 1);
             const uint32_t q_addr = ptx::smem_u32(smem + C::SMEM_Q), k_addr = ptx::smem_u32(smem + C::SMEM_K),
                            v_addr = ptx::smem_u32(smem + C::SMEM_V), p_addr = ptx::smem_u32(smem + C::SMEM_P);
+            // descriptors of the first 16 columns or rows; one further on is its distance in 16-byte units away
+            const uint64_t q_desc = ptx::umma_desc_sw128(q_addr, 16, 1024), k_desc = ptx::umma_desc_sw128(k_addr, 16, 1024),
+                           p_desc = ptx::umma_desc_sw128(p_addr, 16, 1024), v_desc = ptx::umma_desc_sw128(v_addr, HALF_BYTES, 1024);
             auto issue_s = [&](int tile) {
-                const uint32_t qa = q_addr + tile * C::Q_TILE;
 #pragma unroll
-                for (int dh = 0; dh < DK / 64; ++dh) {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const uint64_t da = ptx::umma_desc_sw128(qa + dh * HALF_BYTES + j * 32, 16, 1024);
-                        const uint64_t db = ptx::umma_desc_sw128(k_addr + dh * HALF_BYTES + j * 32, 16, 1024);
-                        ptx::umma_ss(tmem_base + tile * KEYS, da, db, idesc_s, (dh | j) ? 1u : 0u);
-                    }
+                for (int j = 0; j < DK / 16; ++j) {
+                    const int off = (j >> 2) * HALF_BYTES + (j & 3) * 32;
+                    ptx::umma_ss(tmem_base + tile * KEYS, q_desc + (tile * C::Q_TILE + off) / 16, k_desc + off / 16, idesc_s, j ? 1u : 0u);
                 }
                 ptx::umma_commit(&s_bar[tile]);
             };
-            auto issue_pv = [&](int tile, int i) {
-                const uint32_t pa = p_addr + tile * C::P_TILE;
+            // bit 2 tile + j: some row of the tile sees block j of iteration i
+            auto blocks_of = [&](int i) -> uint32_t {
+                uint32_t f = 0;
+                for (int j = 0; j < 2; ++j) {
+                    if (2 * i + j >= n_blk) break;
+                    const int b = block_of(2 * i + j);
+                    for (int tile = 0; tile < 2; ++tile) f |= static_cast<uint32_t>(tile_sees(tile, b)) << (2 * tile + j);
+                }
+                return f;
+            };
+            uint32_t begun = 0;   // tiles whose O holds something
+            // O += P V of a tile, for all 128 keys or for one block of 64
+            auto issue_pv = [&](int tile, int kk0, int steps, uint32_t acc) {
 #pragma unroll
-                for (int kk = 0; kk < KEYS / 16; ++kk) {
+                for (int kk = kk0; kk < kk0 + steps; ++kk) {
                     // A: P, K-major: 64-key half (kk / 4), 32 B per 16-key step inside it;  B: V, N-major: 16 key rows of 128 B per
                     // step, 64-wide halves of the value columns HALF_BYTES apart
-                    const uint64_t da = ptx::umma_desc_sw128(pa + (kk >> 2) * HALF_BYTES + (kk & 3) * 32, 16, 1024);
-                    const uint64_t db = ptx::umma_desc_sw128(v_addr + kk * 16 * 128, HALF_BYTES, 1024);
-                    ptx::umma_ss(tmem_base + PAIR_TMEM_O + tile * 128, da, db, idesc_o, (i > 0 || kk > 0) ? 1u : 0u);
+                    ptx::umma_ss(tmem_base + PAIR_TMEM_O + tile * 128, p_desc + (tile * C::P_TILE + (kk >> 2) * HALF_BYTES + (kk & 3) * 32) / 16,
+                                 v_desc + kk * 16 * 128 / 16, idesc_o, kk > kk0 ? 1u : acc);
                 }
-                ptx::umma_commit(&o_bar[tile]);
             };
             bool w = ptx::mbar_wait(q_bar, 0, abort_flag) && ptx::mbar_wait(k_full, 0, abort_flag);
             if (w) {
@@ -209,7 +254,7 @@ pair_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                 issue_s(1);
                 ptx::umma_commit(k_empty);
             }
-            for (int i = 0; w && i < n_it; ++i) {
+            auto iterate = [&](int i, auto whole) {   // whole: both tiles see both blocks
                 if (i + 1 < n_it) {
                     w = ptx::mbar_wait(k_full, (i + 1) & 1, abort_flag);
                     for (int tile = 0; w && tile < 2; ++tile) {
@@ -218,18 +263,31 @@ pair_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                         ptx::tc_fence_after();
                         issue_s(tile);
                     }
-                    if (!w) break;
+                    if (!w) return;
                     ptx::umma_commit(k_empty);
                 }
+                const uint32_t blocks = decltype(whole)::value ? 15u : blocks_of(i);
                 w = ptx::mbar_wait(v_full, i & 1, abort_flag);
                 for (int tile = 0; w && tile < 2; ++tile) {
                     w = ptx::mbar_wait(&p_ready[tile], i & 1, abort_flag);
                     if (!w) break;
                     ptx::tc_fence_after();
-                    issue_pv(tile, i);
+                    const uint32_t own = (blocks >> (2 * tile)) & 3u, old = (begun >> tile) & 1u;
+                    if (decltype(whole)::value) {
+                        issue_pv(tile, 0, KEYS / 16, old);
+                    } else {
+                        if (own & 1u) issue_pv(tile, 0, BLK / 16, old);
+                        if (own & 2u) issue_pv(tile, BLK / 16, BLK / 16, old | (own & 1u));
+                    }
+                    begun |= own != 0u ? 1u << tile : 0u;
+                    ptx::umma_commit(&o_bar[tile]);
                 }
                 if (w) ptx::umma_commit(v_empty);
-            }
+            };
+            int i = 0;
+            for (; w && i < min(whole_lo, n_it); ++i) iterate(i, std::false_type{});
+            for (; w && i < whole_hi; ++i) iterate(i, std::true_type{});
+            for (; w && i < n_it; ++i) iterate(i, std::false_type{});
         }
     } else if (warp == SOFT_WARPS + 1) {
         // ================================================= TMA producer
@@ -419,6 +477,7 @@ pair_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         if (ok) {
             const bool store = row_in && (t < a.tq);
             const float inv = (l_row > 0.f) ? (BIASED ? a.out_scale : 1.f) / l_row : 0.f;
+            const bool none = l_row == 0.f;   // a row that sees no key: its tile's O may never have been written
             bf16* dst = a.out + static_cast<size_t>(store ? t : 0) * a.out_ld + qh * (BIASED ? a.out_cols : DV) + ch * (DV / 2);
             const int cols = BIASED ? a.out_cols - ch * (DV / 2) : DV / 2;   // real columns of this thread's half
             const bool whole = !BIASED || (a.out_cols % 8 == 0 && a.out_ld % 8 == 0);
@@ -428,7 +487,8 @@ pair_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                 if (n_it > 0) {  // uniform across the CTA
                     ptx::tmem_ld32(tmem_o + c0, r);
                     ptx::tmem_wait_ld();
-                } else {
+                }
+                if (n_it == 0 || none) {
 #pragma unroll
                     for (int c = 0; c < 32; ++c) r[c] = 0;
                 }

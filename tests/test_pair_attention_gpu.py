@@ -96,3 +96,129 @@ def test_layered(mix, tq, before):
     q, k, v = qkv(mix, tq, before + tq, seed=tq)
     ref = T.attention(q, k, v, mix["scale"], T.mask_size(mix), before)
     assert (run_attention(mix, q, k, v, 1, False) - ref).abs().max() < 0.03
+
+
+# A row's output depends on no value beyond the 128-key tiles that some row of its query tile sees (the tiles of the one-tile
+# kernel): a NaN there stays there, also where the other tile of the pair sees it.
+def reached(vis, tok, at):
+    """vis [T, n] bool -> [T] bool: some row of the query tile of `tok` tokens sees a key of the 128-key tile of key `at`."""
+    block = vis[:, at // 128 * 128:at // 128 * 128 + 128].any(1)
+    rows = torch.zeros((len(block) + tok - 1) // tok * tok, dtype=torch.bool, device=block.device)
+    rows[:len(block)] = block
+    return rows.view(-1, tok).any(1).repeat_interleave(tok)[:len(block)]
+
+
+@pytest.mark.parametrize("tq,hq,hkv,L,window", [(1792, 32, 2, 120, 0), (1769, 32, 2, 0, 0), (3545, 16, 1, 56, 512), (7200, 8, 4, 96, 0)])
+def test_values_of_the_other_tile(tq, hq, hkv, L, window):
+    import cpmcu.C as C
+    kv_total, tok = L + tq, 128 * hkv // hq
+    q, k, v, budget = operands(tq, hq, hkv, kv_total, tq + L)
+    at, t = torch.arange(kv_total, device="cuda"), torch.arange(tq, device="cuda")
+    vis = at[None] < L + t[:, None] + 1
+    if window:
+        first = t // tok * tok   # the window's first key is the same for all rows of a query tile
+        vis &= at[None] >= (((L + first // 64 * 64 + 127) // 128 - window // 128).clamp(min=0) * 128)[:, None]
+    kv_len = torch.tensor([kv_total], dtype=torch.int32, device="cuda")
+
+    def run(v):
+        out = torch.full((tq, hq * 128), float("nan"), dtype=torch.bfloat16, device="cuda")
+        C.call("cpmcu_tree_attention", ptr(q), q.shape[1], ptr(k), ptr(v), budget, tq, hq, hkv, ptr(kv_len), 0, None, None, 0, window, 1, ptr(out), hq * 128)
+        return out
+
+    clean = run(v)
+    for p in (128, 130, 640, kv_total // 2 // 128 * 128, kv_total - 1):
+        bad = v.clone()
+        bad[p] = float("nan")
+        far = ~reached(vis, tok, p)
+        out = run(bad)
+        assert torch.equal(out[far], clean[far]), p
+        assert bool(torch.isnan(out[vis[:, p]].float()).all())
+
+
+def test_values_of_the_other_tiles_blocks():
+    import cpmcu.C as C
+    tq, hq, hkv, L, window = 1792, 32, 2, 3000, 2
+    kv_total, tok = L + tq, 8
+    q, k, v, budget = operands(tq, hq, hkv, kv_total, 5)
+    nblk = (kv_total + 63) // 64
+    # tiles of eight tokens choose different blocks: tile i the blocks 2 (i % 20) and 2 (i % 20) + 1
+    t = torch.arange(tq, device="cuda")
+    blocks = torch.arange(nblk, device="cuda")
+    bits = (blocks[None] // 2) == (t[:, None] // tok % 20)
+    words = (nblk + 63) // 64
+    m = torch.zeros(tq, words, dtype=torch.int64, device="cuda")
+    for b in range(nblk):
+        m[:, b // 64] |= bits[:, b].long() << (b % 64)
+    bm = m[None].repeat(hkv, 1, 1).contiguous()
+    seen = bits | (blocks[None] >= ((t + L + 63) // 64 - window)[:, None])
+    vis = seen.repeat_interleave(64, dim=1)[:, :kv_total] & (torch.arange(kv_total, device="cuda")[None] < L + t[:, None] + 1)
+    kv_len = torch.tensor([kv_total], dtype=torch.int32, device="cuda")
+
+    def run(v):
+        out = torch.full((tq, hq * 128), float("nan"), dtype=torch.bfloat16, device="cuda")
+        C.call("cpmcu_sparse_attention", ptr(q), q.shape[1], ptr(k), ptr(v), budget, tq, hq, hkv, ptr(kv_len), 0, None, 0, ptr(bm), words, window, 1, ptr(out),
+               hq * 128)
+        return out
+
+    clean = run(v)
+    for p in (0, 200, 128 * 7 + 70, 128 * 19, L + 100):
+        bad = v.clone()
+        bad[p] = float("nan")
+        far = ~reached(vis, tok, p)
+        out = run(bad)
+        assert torch.equal(out[far], clean[far]), p
+        assert bool(torch.isnan(out[vis[:, p]].float()).all())
+
+
+def test_exact_windows_and_values_of_others():
+    """Sliding windows that begin at an odd block, rows of the cache nobody sees at its end."""
+    import ctypes as ct
+
+    import cpmcu.C as C
+    from test_tipetar_gpu import padded, spec_of
+    mix = attn(16, 4, 128, 128, 300)
+    tq, before = 3570, 64 + 900
+    keys, tok = tq + before, 32
+    q, k, v = qkv(mix, tq, keys, seed=2)
+    budget = (keys + 127) // 128 * 128 + 256
+    kc, vc = (torch.zeros(budget, 4, 128, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    kc[:keys], vc[:keys] = k.to(torch.bfloat16), v.to(torch.bfloat16)
+    qc = padded(q.cuda(), 128, torch.bfloat16)
+    sp = spec_of(mix)
+
+    def run(v):
+        out = torch.zeros(tq, 16 * 128, dtype=torch.bfloat16, device="cuda")
+        C.call("cpmcu_layer_attention", ct.byref(sp), qc.data_ptr(), kc.data_ptr(), v.data_ptr(), budget, tq, keys, 1, 0, out.data_ptr())
+        return out
+
+    clean = run(vc)
+    at, t = torch.arange(budget, device="cuda"), torch.arange(tq, device="cuda")
+    vis = (at[None] <= before + t[:, None]) & (at[None] > before + t[:, None] - 300)
+    for p in (700, 767, 1024, 1500, keys - 1, (keys + 127) // 128 * 128, budget - 1):
+        bad = vc.clone()
+        bad[p] = float("nan")
+        far = ~reached(vis, tok, p)
+        out = run(bad)
+        assert torch.equal(out[far], clean[far]), p
+
+
+# A tree mask reaches this kernel only through the C entry, with key heads enough: 64 tokens, 56 key heads.
+def test_tree_mask():
+    import cpmcu.C as C
+    tq, hq, hkv, L = 64, 16 * 56, 56, 700
+    kv_total = L + tq
+    q, k, v, budget = operands(tq, hq, hkv, kv_total, 9)
+    parent = np.random.default_rng(4).integers(0, np.maximum(np.arange(tq), 1))
+    bits = np.zeros((tq, tq), dtype=bool)
+    for i in range(tq):
+        bits[i] = bits[parent[i]] if i else False
+        bits[i, i] = True
+    mask = (bits.astype(np.uint64) << np.arange(64, dtype=np.uint64)).sum(-1, dtype=np.uint64)
+    vis = torch.ones(tq, kv_total, dtype=torch.bool, device="cuda")
+    vis[:, L:] = torch.from_numpy(bits).cuda()
+    out = torch.full((tq, hq * 128), float("nan"), dtype=torch.bfloat16, device="cuda")
+    kv_len = torch.tensor([kv_total], dtype=torch.int32, device="cuda")
+    m = torch.from_numpy(mask.view(np.int64)).cuda()
+    C.call("cpmcu_tree_attention", ptr(q), q.shape[1], ptr(k), ptr(v), budget, tq, hq, hkv, ptr(kv_len), 0, None, ptr(m), tq, 0, 1, ptr(out), hq * 128)
+    ref = reference(*views(q, k, v, tq, hq, hkv, kv_total), vis)
+    assert float((out.float().view(tq, hq, 128) - ref).abs().max()) < 3e-2
