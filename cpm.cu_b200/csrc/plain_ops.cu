@@ -69,6 +69,7 @@ __global__ void __launch_bounds__(256) plain_attention_kernel(const PlainAttnArg
     const int step = nks * PA_TILE;
     // `n` rows of `cols` columns into shared memory rows of `st`, zeros up to `step` rows; four requests in flight per thread
     auto stage = [&](const T* src, size_t ld, int cols, float* dst, int st, int n) {
+        float odd[4] = {0.f, 0.f, 0.f, 0.f};   // NaN once an element is not finite
         for (int i0 = threadIdx.x * 8; i0 < step * cols; i0 += threads * 32) {
             float f[4][8];
 #pragma unroll
@@ -85,15 +86,17 @@ __global__ void __launch_bounds__(256) plain_attention_kernel(const PlainAttnArg
                 float4* d = reinterpret_cast<float4*>(dst + j * st + c);
                 d[0] = make_float4(f[u][0], f[u][1], f[u][2], f[u][3]);
                 d[1] = make_float4(f[u][4], f[u][5], f[u][6], f[u][7]);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) odd[u] = fmaf(f[u][e], 0.f, odd[u]);
             }
         }
+        return (odd[0] + odd[1]) + (odd[2] + odd[3]) != 0.f;
     };
     for (int j0 = lo + rank * step; j0 < hi; j0 += sh.cluster * step) {
         const int n = min(step, hi - j0);
         __syncthreads();   // the last tiles have been read
         stage(kc + static_cast<size_t>(j0) * kld, kld, a.dk, sk, kst, n);
-        stage(vc + static_cast<size_t>(j0) * vld, vld, a.dv, sv, vst, n);
-        __syncthreads();
+        const int not_finite = __syncthreads_or(stage(vc + static_cast<size_t>(j0) * vld, vld, a.dv, sv, vst, n));
         if (ks >= nks || ks * PA_TILE >= n) continue;   // warp-uniform
         const int j = j0 + ks * PA_TILE + lane;
         const float* k = sk + (ks * PA_TILE + lane) * kst;
@@ -130,6 +133,24 @@ __global__ void __launch_bounds__(256) plain_attention_kernel(const PlainAttnArg
         }
         __syncwarp();
         const float* v = sv + ks * PA_TILE * vst + lane;
+        if (not_finite) {
+            // A probability of zero does not hide an infinity or a NaN: values are added only to the rows that see their key.
+            const int t0 = j0 + ks * PA_TILE;
+#pragma unroll 1
+            for (int jj = 0; jj < PA_TILE; ++jj) {
+#pragma unroll
+                for (int x = 0; x < R; ++x) {
+                    if (t0 + jj < low[x] || t0 + jj > pos[x]) continue;
+                    const float p = p_s[x * 32 + jj];
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) {
+                        if (c * 32 < a.dv) acc[x][c] += p * v[jj * vst + c * 32];
+                    }
+                }
+            }
+            __syncwarp();
+            continue;
+        }
 #pragma unroll 2
         for (int jj = 0; jj < PA_TILE; jj += 4) {
             float4 p[R];

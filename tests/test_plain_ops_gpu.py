@@ -21,6 +21,28 @@ def test_attention_divisions(mix, tq, keys):
     assert (run_attention(mix, q, k, v, 0, False) - ref).abs().max() < 0.03
 
 
+# A row's output does not depend on values it may not see, infinities and NaN among them: those of later tokens, those before
+# its window.  Query rows of one launch share key tiles; with 1 or 11 rows the keys are dealt to warps and CTAs.
+@pytest.mark.parametrize("mix", [attn(3, 1, 72, 72, None), attn(12, 4, 64, 40, 50), attn(8, 1, 128, 128, 33), attn(4, 2, 300, 500, 200, scale=0.05)],
+                         ids=["g3", "window", "narrow", "wide"])
+@pytest.mark.parametrize("tq,keys", [(1, 700), (11, 700), (130, 600), (300, 300)])
+def test_values_that_a_row_may_not_see(mix, tq, keys):
+    q, k, v = qkv(mix, tq, keys, seed=tq)
+    window = T.mask_size(mix) or keys + 1
+    i = torch.arange(keys - tq, keys)
+    for fp32 in (True, False):
+        clean = run_attention(mix, q, k, v, 0, fp32)
+        for p, value in ((keys - 1, float("nan")), (keys - 1 - tq // 2, float("inf")), (keys - 40, float("nan")), (keys - 2 - window, float("-inf"))):
+            if not 0 <= p < keys:
+                continue
+            bad = v.clone()
+            bad[p] = value
+            out = run_attention(mix, q, k, bad, 0, fp32)
+            sees = (i >= p) & (i - p < window)
+            assert torch.equal(out[~sees], clean[~sees]), (p, value)
+            assert not bool(torch.isfinite(out[sees]).any())
+
+
 @pytest.mark.parametrize("name", ["mixed", "odd"])
 def test_products_of_every_row_count(name):
     import cpmcu.C as C
