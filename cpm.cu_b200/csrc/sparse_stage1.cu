@@ -5,6 +5,10 @@
 // 128: first the keys of the log-sum-exp (running maximum and sum per row), then the scored keys, whose exponentials are
 // normalised and summed over the 16 heads: lanes of a warp, 15 shuffles per 16 keys leave lane l with key l.  The exponentials bound
 // it (16384 per chunk on the MUFU pipe, 1024 cycles; the MMAs take 512); two CTAs per SM hide one another's latencies.
+// The blocks of peaked heads are told apart by scores below 2^-126, which ex2.approx.ftz makes equal: a chunk with a sum below 2^-98
+// (above, what 16 flushed terms would add is below the last place) is gone through again with exp2f, as in sparse_select.cu,
+// from its scores in tensor memory.  Beside the row's largest term of the log-sum-exp, which is one, what is flushed there is below the
+// last place as well.
 // A 32768-token prompt in chunks of 2048, 32 query heads, 44 us a launch on average; as warp-level fragments in two kernels with
 // partial sums through memory 146 + 64 us.
 #include "attn_common.cuh"
@@ -130,15 +134,18 @@ sparse_stage1_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
             ptx::tmem_ld32(tmem_s + st * KEYS, sc);
             ptx::tmem_ld32(tmem_s + st * KEYS + 32, sc + 32);
             ptx::tmem_wait_ld();
+            return true;
+        };
+        auto release = [&](int i) {
             ptx::tc_fence_before();
             __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&s_free[st]);
-            return true;
+            if (lane == 0) ptx::mbar_arrive(&s_free[i & 1]);
         };
         float m = -INFINITY, sum = 0.f;
         for (int i = 0; ok && i < chunks_l; ++i) {
             ok = fetch(i);
             if (!ok) break;
+            release(i);
             const int left = nl - i * KEYS - ch * 64;   // keys of this thread that exist
             if (left < 64) {
 #pragma unroll
@@ -177,12 +184,8 @@ sparse_stage1_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
             if (!ok) break;
             const int key0 = (i - chunks_l) * KEYS;
             const int left = n1 - key0 - ch * 64;
-#pragma unroll
-            for (int c0 = 0; c0 < 64; c0 += 16) {
-                float v[16];
-#pragma unroll
-                for (int c = 0; c < 16; ++c) v[c] = c0 + c < left ? fast_exp2((__uint_as_float(sc[c0 + c]) - m_row) * sl2) * inv : 0.f;
-                // sum over the 16 lanes of a token: each step a lane keeps half of its columns and hands over the rest
+            // sum over the 16 lanes of a token: each step a lane keeps half of its columns and hands over the rest
+            auto store_sums = [&](float (&v)[16], int c0) {
 #pragma unroll
                 for (int h = 8; h > 0; h >>= 1) {
                     const bool upper = (lane & h) != 0;
@@ -193,7 +196,29 @@ sparse_stage1_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                     }
                 }
                 if (t < t_end) dst[key0 + c0] = __float2bfloat16(v[0]);
+            };
+            bool small = false;
+#pragma unroll
+            for (int c0 = 0; c0 < 64; c0 += 16) {
+                float v[16];
+#pragma unroll
+                for (int c = 0; c < 16; ++c) v[c] = c0 + c < left ? fast_exp2((__uint_as_float(sc[c0 + c]) - m_row) * sl2) * inv : 0.f;
+                store_sums(v, c0);
+                small = small || (v[0] < 0x1p-98f && c0 + (lane & 15) < left);
             }
+            if (__any_sync(0xffffffffu, small)) {
+#pragma unroll 1
+                for (int c0 = 0; c0 < 64; c0 += 16) {
+                    uint32_t r[16];
+                    float v[16];
+                    ptx::tmem_ld16(tmem_s + (i & 1) * KEYS + c0, r);
+                    ptx::tmem_wait_ld();
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) v[c] = c0 + c < left ? exp2f((__uint_as_float(r[c]) - m_row) * sl2) * inv : 0.f;
+                    store_sums(v, c0);
+                }
+            }
+            release(i);
         }
     }
 
