@@ -441,8 +441,11 @@ void launch_sparse_select(const SparseBuffers& b, const SparseConfig& cfg, int l
     a.lse_chunks = b.score_ld / 128;
     const int lse_z = cfg.compress_lse ? ceil_div(a.lse_chunks, 4) : a.lse_chunks;
     // 16 heads x 8 tokens fill a tensor-core tile; fewer heads per key head, and decode-sized launches (whose latency is that
-    // of their longest CTA), stay with warp-level fragments dealt over chunks of keys
-    if (T > 64 && grp == S1_MAXGRP) {
+    // of their longest CTA), stay with warp-level fragments dealt over chunks of keys.  So do fewer than a dozen CTAs that could have
+    // to walk more than 131072 rows' keys, where the fragments have few of them for the log-sum-exp: one key head, 65 / 80 / 96
+    // tokens behind 190000, tiles 205 / 205 / 206 us (with the compression before), fragments 199 / 194 / 215; behind 250000
+    // 268 / 268 / 270 and 220 / 249 / 271; behind 130000 144 / 144 / 144 and 215 / 159 / 178.
+    if (T > 64 && grp == S1_MAXGRP && (ceil_div(T, 8) * hkv >= 12 || b.budget <= 131072 || !cfg.compress_lse)) {
         launch_sparse_stage1_prefill(b, cfg, layer, q, q_ld, T, hkv, kv_len, kv_add, n_valid, s);
     } else if (T <= 64) {
         launch_kernel(sparse_stage1_lse_kernel<2>, dim3(ceil_div(T, 2), hkv, lse_z), dim3(S1_THREADS), 0, s, a);

@@ -11,7 +11,9 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("T,hq,hkv,L,top,sink,window,lse,budget", [
     (65, 16, 1, 5000, 64, 1, 4, True, None), (100, 32, 2, 3000, 16, 1, 8, False, None), (131, 32, 2, 2064, 8, 2, 2, True, 65536),
-    (72, 16, 1, 8256, 30, 1, 2, True, 131072), (67, 16, 1, 2048, 7, 0, 1, False, None), (80, 48, 3, 16300, 64, 1, 32, True, 16384 + 128)])
+    (72, 16, 1, 8256, 30, 1, 2, True, 131072), (67, 16, 1, 2048, 7, 0, 1, False, None), (80, 48, 3, 16300, 64, 1, 32, True, 16384 + 128),
+    # caches beyond 131072 rows: few CTAs go to the decode-sized kernels where the log-sum-exp has keys of its own
+    (95, 16, 1, 9000, 32, 1, 8, True, 196608), (95, 16, 1, 9000, 32, 1, 8, False, 196608), (96, 16, 1, 9000, 32, 1, 8, True, 196608)])
 def test_block_selection(T, hq, hkv, L, top, sink, window, lse, budget):
     check_selection(T, hq, hkv, L, top, sink, window, lse, budget)
 
