@@ -149,7 +149,7 @@ one_row_kernel(const OneRowArgs a) {
 // 32 (73448 x 4096 90 us against 84) were slower.
 int rows_per_cta(long long outputs) {
     static const char* forced = tuning_env("CPMCU_ONE_ROW");   // bench only
-    if (forced) return atoi(forced);
+    if (forced) return atoi(forced) == 8 ? 8 : 16;
     return outputs / 16 < runtime().num_sms * 5 / 2 ? 8 : 16;
 }
 
