@@ -496,42 +496,65 @@ static long long base_grid(int n_tiles, int m_tiles, int kblocks, int M, int gri
 }
 
 // Pairs of CTAs of a launch, 0 = single CTAs: several token tiles, an even number of 128-row weight tiles, and as many pairs
-// at once as the split of the last wave relies on (its pieces wait for one another).
-static int pair_count(int n_tiles, int m_tiles, int kblocks, int mt, int grid_limit) {
+// at once as the split of the last wave relies on (its pieces wait for one another): at most the `capacity` the device runs.
+static int pair_count(int n_tiles, int m_tiles, int kblocks, int mt, int grid_limit, int capacity) {
     static const bool off = tuning_env("CPMCU_LINEAR_NO_PAIR") != nullptr;   // bench only
     if (off || m_tiles < 2 || mt != 256 || n_tiles % 2 != 0 || grid_limit < 2) return 0;
     const long long units = static_cast<long long>(n_tiles / 2) * m_tiles * kblocks;
-    return static_cast<int>(std::min<long long>({std::max<long long>(1, units / 4), grid_limit / 2, linear_pair_capacity()}));
+    return static_cast<int>(std::min<long long>({std::max<long long>(1, units / 4), grid_limit / 2, capacity}));
+}
+// make_linear_plan asks the device only where pairs come into question
+static int pair_count(int n_tiles, int m_tiles, int kblocks, int mt, int grid_limit) {
+    const int wanted = pair_count(n_tiles, m_tiles, kblocks, mt, grid_limit, grid_limit);
+    return wanted > 0 ? std::min(wanted, linear_pair_capacity()) : 0;
 }
 
-// Host-side walk of the work distribution make_linear_plan + launch_linear give a launch (without the cluster
-// variant, which cuts every tile into equal pieces): for every CTA its segments as six ints
-// (cta, tile, token tile, feature tile, first k-block, end k-block), in the order the CTA runs them.  The same
-// iterator and raster functions the kernels use, compiled for the host.  Returns the number of segments, or -1 when
-// `cap` segments do not hold them.
+// How a launch of more than one row is divided (without the cluster variant, which cuts every tile into equal pieces).
+struct LinearSplit {
+    int pairs = 0;            // > 0: pairs of CTAs on tiles of 256 weight rows
+    int workers = 0;          // pairs or CTAs
+    int wave_tiles = 0, tail_grid = 0;
+};
+static LinearSplit split_linear(int M, int N, int K, int mt, int grid_limit, int pairs) {
+    const int n_tiles = ceil_div(N, BLOCK_N), m_tiles = ceil_div(M, mt), kblocks = K / BLOCK_K;
+    LinearSplit s;
+    s.pairs = pairs;
+    s.workers = pairs > 0 ? pairs : static_cast<int>(base_grid(n_tiles, m_tiles, kblocks, M, grid_limit));
+    if (m_tiles > 1) plan_waves(static_cast<long long>(pairs > 0 ? n_tiles / 2 : n_tiles) * m_tiles, kblocks, s.workers, s.wave_tiles, s.tail_grid);
+    return s;
+}
+
+// Host-side walk of the work distribution make_linear_plan + launch_linear give a launch of more than one row (one row has no
+// tiles) on a device that runs grid_limit / 2 pairs of CTAs at once: for every CTA its segments as six ints (cta, tile, token
+// tile, feature tile, first k-block, end k-block), in the order the CTA runs them; the two CTAs of a pair have consecutive
+// numbers, tiles, feature tiles and counters.  The same iterator and raster functions the kernels use, compiled for the
+// host.  Returns the number of segments, or -1 when `cap` segments do not hold them.
 int linear_schedule_dump(int M, int N, int K, int grid_limit, int32_t* out, int cap) {
+    CPM_REQUIRE(M > 1, "linear schedule: one row is not divided into tiles");
     LinearArgs a = {};
     const int mt = linear_pick_mt(M);
     a.M = M; a.N = N; a.K = K;
     a.n_tiles = ceil_div(N, BLOCK_N);
     a.m_tiles = ceil_div(M, mt);
     a.kblocks = K / BLOCK_K;
-    const int grid = static_cast<int>(base_grid(a.n_tiles, a.m_tiles, a.kblocks, M, grid_limit));
-    a.wave_tiles = 0;
-    a.tail_grid = 0;
-    if (a.m_tiles > 1) plan_waves(static_cast<long long>(a.n_tiles) * a.m_tiles, a.kblocks, grid, a.wave_tiles, a.tail_grid);
+    const LinearSplit split = split_linear(M, N, K, mt, grid_limit, pair_count(a.n_tiles, a.m_tiles, a.kblocks, mt, grid_limit, grid_limit / 2));
+    const int size = split.pairs > 0 ? 2 : 1;   // CTAs that share a tile
+    a.n_tiles /= size;
+    a.wave_tiles = split.wave_tiles;
+    a.tail_grid = split.tail_grid;
     a.total_units = (static_cast<long long>(a.n_tiles) * a.m_tiles - a.wave_tiles) * a.kblocks;
     a.band = raster_band(mt, K);
     int n = 0;
-    for (int g = 0; g < grid; ++g) {
-        SegIter it = make_seg_iter(a, g, grid);
+    for (int cta = 0; cta < split.workers * size; ++cta) {
+        const int rank = cta % size;
+        SegIter it = make_seg_iter(a, cta / size, split.workers);
         int tile, kb0, kb1;
         while (it.next(tile, kb0, kb1)) {
             if (n >= cap) return -1;
             int m_tile, n_tile;
             tile_to_mn(a, tile, m_tile, n_tile);
             int32_t* o = out + static_cast<size_t>(n) * 6;
-            o[0] = g; o[1] = tile; o[2] = m_tile; o[3] = n_tile; o[4] = kb0; o[5] = kb1;
+            o[0] = cta; o[1] = tile * size + rank; o[2] = m_tile; o[3] = n_tile * size + rank; o[4] = kb0; o[5] = kb1;
             ++n;
         }
     }
@@ -557,15 +580,17 @@ LinearPlan make_linear_plan(const bf16* x, int x_rows, const bf16* w, int M, int
     }
     const int n_tiles = ceil_div(N, BLOCK_N), m_tiles = ceil_div(M, p.mt), kblocks = K / BLOCK_K;
     const long long units = static_cast<long long>(n_tiles) * m_tiles * kblocks;
-    if (const int pairs = pair_count(n_tiles, m_tiles, kblocks, p.mt, grid_limit)) {
+    const LinearSplit split = split_linear(M, N, K, p.mt, grid_limit, pair_count(n_tiles, m_tiles, kblocks, p.mt, grid_limit));
+    p.wave_tiles = split.wave_tiles;
+    p.tail_grid = split.tail_grid;
+    if (split.pairs > 0) {
         p.pair = 1;
-        p.grid = 2 * pairs;
-        plan_waves(static_cast<long long>(n_tiles / 2) * m_tiles, kblocks, pairs, p.wave_tiles, p.tail_grid);
+        p.grid = 2 * split.pairs;
         p.tm_w = make_weight_tmap(w, N, K);
         p.tm_x = make_tmap_2d(x, K, x_rows, static_cast<uint64_t>(K) * 2, BLOCK_K, p.mt / 2);
         return p;
     }
-    long long grid = base_grid(n_tiles, m_tiles, kblocks, M, grid_limit);
+    long long grid = split.workers;
     {
         static const char* forced = tuning_env("CPMCU_LINEAR_GRID");  // bench only: sweep the grid size
         if (forced && atoi(forced) >= 1 && atoi(forced) <= grid_limit && atoi(forced) <= units) grid = atoi(forced);
@@ -584,7 +609,8 @@ LinearPlan make_linear_plan(const bf16* x, int x_rows, const bf16* w, int M, int
     p.grid = static_cast<int>(grid);
     if (m_tiles > 1) {
         static const bool flat = tuning_env("CPMCU_LINEAR_NO_WAVES") != nullptr;   // bench only: plain stream-K
-        if (!flat) plan_waves(static_cast<long long>(n_tiles) * m_tiles, kblocks, p.grid, p.wave_tiles, p.tail_grid);
+        if (flat) p.wave_tiles = p.tail_grid = 0;
+        else if (p.grid != split.workers) plan_waves(static_cast<long long>(n_tiles) * m_tiles, kblocks, p.grid, p.wave_tiles, p.tail_grid);
     }
     // CS CTAs per tile with equal k ranges: sum the pieces inside a cluster when the device runs all clusters at once
     p.cluster = 0;
