@@ -219,7 +219,8 @@ struct LinearPlan {
     float gate_limit = 0.f, gate_alpha = 0.f;   // gate_limit > 0: clamped_gate instead of silu_mul
     // W4A16: when wq is set the weights are 4-bit blocks in the streaming layout (see gemm_w4_umma.cu)
     const void* wq = nullptr;
-    // one token row, bf16 weights: the operands themselves (one_row.cu)
+    // one token row, bf16 weights, without tiles: the operands themselves (one_row.cu)
+    int one_row = 0;
     const bf16 *x = nullptr, *w = nullptr;
 };
 
@@ -246,6 +247,7 @@ LinearPlan make_linear_swiglu_plan(const bf16* x, int x_rows, const bf16* w, int
                                    int grid_limit);
 void launch_linear(const LinearPlan& plan, cudaStream_t stream);
 void launch_linear_one_row(const LinearPlan& plan, cudaStream_t stream);   // M == 1, bf16 weights
+bool linear_one_row_fits(int N, int K, int sms);   // whether that is the faster way for one row of N outputs
 // Same contract with 4-bit weights, w = (q - 8) * scale, K % 256 == 0 and N % 128 == 0.  `wq` holds one
 // contiguous 16896-byte block per (128-feature tile, 256-k unit), tile-major: [4 k-blocks][2 halves]
 // [128 rows][16 B] of nibbles (a 32-bit word holds k0 k2 k4 k6 k1 k3 k5 k7 from bit 0) then

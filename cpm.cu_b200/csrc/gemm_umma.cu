@@ -509,7 +509,7 @@ static int pair_count(int n_tiles, int m_tiles, int kblocks, int mt, int grid_li
     return wanted > 0 ? std::min(wanted, linear_pair_capacity()) : 0;
 }
 
-// How a launch of more than one row is divided (without the cluster variant, which cuts every tile into equal pieces).
+// How a launch on tiles is divided (without the cluster variant, which cuts every tile into equal pieces).
 struct LinearSplit {
     int pairs = 0;            // > 0: pairs of CTAs on tiles of 256 weight rows
     int workers = 0;          // pairs or CTAs
@@ -524,13 +524,13 @@ static LinearSplit split_linear(int M, int N, int K, int mt, int grid_limit, int
     return s;
 }
 
-// Host-side walk of the work distribution make_linear_plan + launch_linear give a launch of more than one row (one row has no
-// tiles) on a device that runs grid_limit / 2 pairs of CTAs at once: for every CTA its segments as six ints (cta, tile, token
+// Host-side walk of the work distribution make_linear_plan + launch_linear give a launch on tiles (one row
+// mostly has none) on a device that runs grid_limit / 2 pairs of CTAs at once: for every CTA its segments as six ints (cta, tile, token
 // tile, feature tile, first k-block, end k-block), in the order the CTA runs them; the two CTAs of a pair have consecutive
 // numbers, tiles, feature tiles and counters.  The same iterator and raster functions the kernels use, compiled for the
 // host.  Returns the number of segments, or -1 when `cap` segments do not hold them.
 int linear_schedule_dump(int M, int N, int K, int grid_limit, int32_t* out, int cap) {
-    CPM_REQUIRE(M > 1, "linear schedule: one row is not divided into tiles");
+    CPM_REQUIRE(M > 1 || !linear_one_row_fits(N, K, grid_limit), "linear schedule: this row is not divided into tiles");
     LinearArgs a = {};
     const int mt = linear_pick_mt(M);
     a.M = M; a.N = N; a.K = K;
@@ -573,8 +573,9 @@ LinearPlan make_linear_plan(const bf16* x, int x_rows, const bf16* w, int M, int
     p.mt = linear_pick_mt(M);
     p.y = y; p.ldy = ldy; p.bias = bias;
     p.workspace = workspace; p.tickets = tickets;
-    p.x = x; p.w = w;
-    if (M == 1) {   // launch_linear_one_row: neither maps nor a division of the tiles
+    if (M == 1 && linear_one_row_fits(N, K, runtime().num_sms)) {   // neither maps nor a division of the tiles
+        p.one_row = 1;
+        p.x = x; p.w = w;
         p.grid = 1;
         return p;
     }
@@ -678,8 +679,9 @@ LinearPlan make_linear_swiglu_plan(const bf16* x, int x_rows, const bf16* w, int
     p.mt = linear_pick_mt(M);
     p.y = act; p.ldy = ld; p.bias = nullptr;
     p.swiglu = 1;
-    p.x = x; p.w = w;
     if (M == 1) {
+        p.one_row = 1;
+        p.x = x; p.w = w;
         p.grid = 1;
         return p;
     }
@@ -711,8 +713,7 @@ void launch_linear(const LinearPlan& p, cudaStream_t stream) {
         return;
     }
     ProfileScope prof(KC_LINEAR, stream);
-    // one row needs no tensor core and was faster without at every size (one_row.cu has both sides' times)
-    if (p.M == 1) {
+    if (p.one_row) {
         launch_linear_one_row(p, stream);
         return;
     }

@@ -143,15 +143,31 @@ one_row_kernel(const OneRowArgs a) {
     a.y[static_cast<size_t>(shared ? a.ys_row : e.z) * a.ldy + first + t] = __float2bfloat16(sum);
 }
 
-// Output rows per CTA: 16 while that leaves every SM two to three CTAs, else 8: more CTAs even out the SMs' shares and keep more
-// loads in flight, more rows make longer bursts and fewer sums.  Rows x K with 16 / 8 rows: 4096 x 4096 7.8 / 7.0 us,
-// 2048 x 8192 11.3 / 8.2, 8192 x 3072 9.2 / 10.2, 16384 x 2048 (gated) 11.9 / 12.5.  4 rows (2048 x 2048 4.0 us against 3.6) and
-// 32 (73448 x 4096 90 us against 84) were slower.
-int rows_per_cta(long long outputs) {
+// Output rows per CTA: 16 make longer bursts and fewer sums, 8 even out the SMs' shares.  The GPU holds four CTAs per SM: 8 rows while
+// CTAs of 8 all fit at once, and where those of 16 would leave a second wave less than half full and a CTA has enough to
+// read for that to matter.  Rows x K with 8 / 16 rows, us: 4096 x 8192 11.7 / 13.2, 4608 x 13824 20.1 / 21.6; 4864 x 8192 16.4 / 15.0,
+// 9216 x 5120 16.4 / 15.3; 9728 x 8192 26.3 / 30.6, 12288 x 13824 50.0 / 53.7, 12288 x 2048 9.8 / 10.1, 12288 x 1024 7.1 / 6.2;
+// 16384 x 5120 27.2 / 25.8, 32768 (gated) x 1024 16.7 / 12.0.  4 rows (2048 x 2048 4.0 us against 3.6) and 32 (73448 x 4096 90 us against
+// 84) were slower.
+int rows_per_cta(long long outputs, int kblocks) {
     static const char* forced = tuning_env("CPMCU_ONE_ROW");   // bench only
     if (forced) return atoi(forced) == 8 ? 8 : 16;
-    return outputs / 16 < runtime().num_sms * 5 / 2 ? 8 : 16;
+    const long long resident = 4LL * runtime().num_sms;
+    const bool short_wave = outputs > 16 * resident && outputs <= 24 * resident && kblocks >= 32;
+    return outputs <= 8 * resident || short_wave ? 8 : 16;
 }
+
+}  // namespace
+
+// Everywhere but where long rows meet SMs that are dealt three CTAs of 16 rows beside SMs with two: there nothing evens out the SMs'
+// shares and the tiles, which cut K, keep up.  N x K, here / tiles, us: 5120 x 13824 26.5 / 24.4, 5632 x 13824 27.7 / 25.8; 4864 x 13824
+// 23.7 / 24.2, 5888 x 13824 28.2 / 33.3, 5120 x 8192 16.7 / 19.2, 5632 x 8192 17.3 / 18.9 (11000 is where the lines cross).
+bool linear_one_row_fits(int N, int K, int sms) {
+    const int ctas = ceil_div(N, 16), extra = ctas - 2 * sms;
+    return K < 11000 || extra * 10 < sms || extra * 20 > 9 * sms;
+}
+
+namespace {
 
 template <bool PAIR, bool EARLY>
 void launch(int R, const OneRowArgs& a, int grid, cudaStream_t s) {
@@ -170,7 +186,7 @@ void launch_linear_one_row(const LinearPlan& p, cudaStream_t s) {
     a.ldx = p.K; a.ldy = p.ldy;
     a.uniform = 1;
     a.gate_limit = p.gate_limit; a.gate_alpha = p.gate_alpha;
-    const int R = rows_per_cta(p.swiglu ? 2LL * p.N : p.N);
+    const int R = rows_per_cta(p.swiglu ? 2LL * p.N : p.N, a.kblocks);
     a.ctas = ceil_div(p.N, p.swiglu ? R / 2 : R);
     if (p.swiglu) launch<true, true>(R, a, a.ctas, s);
     else launch<false, true>(R, a, a.ctas, s);
@@ -185,7 +201,7 @@ void launch_moe_one_row(const MoeGemmPlan& p, cudaStream_t s) {
     a.ldx = p.ldx; a.ldy = p.ldy; a.xs_row = p.xs_row0; a.ys_row = p.ys_row0;
     a.entries = p.entries; a.n_entries = p.n_entries; a.uniform = p.uniform;
     const int per = p.swiglu ? 2 : 1;
-    const int R = rows_per_cta(static_cast<long long>(per) * (static_cast<long long>(p.max_entries) * p.N + (p.n_tiles_s > 0 ? p.N_s : 0)));
+    const int R = rows_per_cta(static_cast<long long>(per) * (static_cast<long long>(p.max_entries) * p.N + (p.n_tiles_s > 0 ? p.N_s : 0)), p.kblocks);
     a.ctas = ceil_div(p.N, R / per);
     a.ctas_s = p.n_tiles_s > 0 ? ceil_div(p.N_s, R / per) : 0;
     const int grid = a.ctas_s + p.max_entries * a.ctas;

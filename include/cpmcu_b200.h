@@ -250,8 +250,8 @@ int cpmcu_linear_w4a16(const void* x, const void* qweight, const void* scales, v
  * (the iterator and raster code of the kernels compiled for the host; a launch that uses the cluster variant cuts
  * every tile into equal pieces instead).  out: HOST int32[cap][6] = (cta, tile, token tile, feature tile, first
  * k-block, end k-block) per segment, in each CTA's execution order; where pairs of CTAs share a tile of 256 features,
- * each has its 128 of them, and the two have consecutive numbers.  M > 1 (one row is not divided into tiles).  Returns
- * the segment count, -1 on error or when cap is too small. */
+ * each has its 128 of them, and the two have consecutive numbers.  Returns the segment count, -1 on error, when
+ * cap is too small or when there are no tiles (most products of one row). */
 int cpmcu_debug_linear_schedule(int M, int N, int K, int grid_limit, int32_t* out, int cap);
 
 /* Times `iters` back-to-back launches of the linear kernel on the library's

@@ -35,7 +35,7 @@ def schedule(M, N, K, limit):
 
 SHAPES = [
     # decode-sized (one token tile): plain stream-K
-    (60, 4608, 4096, 148), (10, 73448, 4096, 148), (60, 1000, 2048, 3), (2, 256, 256, 148), (33, 300, 128, 148),
+    (60, 4608, 4096, 148), (10, 73448, 4096, 148), (60, 1000, 2048, 3), (2, 256, 256, 148), (1, 5120, 13824, 148), (33, 300, 128, 148),
     # prefill-sized: whole tiles in waves, the rest cut along K; on pairs of CTAs where the weight tiles come in twos
     (4096, 4608, 4096, 148), (4096, 4096, 4096, 148), (4096, 32768, 4096, 148), (4096, 4096, 16384, 148),
     (2048, 4096, 16384, 148), (4100, 1280, 256, 148), (700, 1024, 512, 7), (520, 384, 2048, 5), (257, 640, 1024, 11),

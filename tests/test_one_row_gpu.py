@@ -42,6 +42,12 @@ def test_product(N, K):
         check(y, x, w, bias)
 
 
+# where the tiles keep up (three CTAs on some SMs, two on others, long rows), and just beside that
+@pytest.mark.parametrize("N,K", [(5120, 13824), (5376, 11008), (5632, 11072), (4900, 11008), (5888, 11008), (5376, 10944), (9472, 256), (9473, 256), (4736, 128), (4737, 128)])
+def test_product_of_few_and_many_ctas(N, K):
+    test_product(N, K)
+
+
 @pytest.mark.parametrize("inter", [64, 192, 1472, 2944, 3008])
 @pytest.mark.parametrize("K", [64, 576, 1024])
 def test_gated_product(inter, K):
