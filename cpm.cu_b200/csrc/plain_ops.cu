@@ -476,9 +476,10 @@ void launch_linear_f32(const float* x, int ldx, const bf16* w, size_t w_stride, 
     CPM_REQUIRE(K % 64 == 0 && ldx % 4 == 0, "linear_f32: K must be a multiple of 64");
     const int z = entries ? max_entries : 1, most = entries ? std::min(M, kF32Rows) : M;
     // Up to eight rows a warp per two features reads every weight once; beyond, while few features make few warps, so do a
-    // warp's eight rows of several.  K = 1024, few / tile, us: 8 rows x 1024 8.8 / 11.9, 8 x 32768 46 / 66, 32 x 1024 9.1 /
-    // 12.4, 32 x 4096 33 / 38, 64 x 1024 17 / 12.5, 16 x 32768 92 / 66.
-    if (most <= 8 || (most <= 32 && ceil_div(most, 8) * N <= 16384)) {
+    // warp's eight rows of several.  K = 1024, few / tile, us, weights from HBM: 8 rows x 4096 9.4 / 30.4, 24 x 4096 25.5 / 30.7,
+    // 32 x 4096 33.5 / 30.7, 8 x 8192 17.8 / 29.9, 16 x 8192 31.5 / 30.0, 8 x 32768 48.8 / 66.6, 12 x 32768 75.9 / 66.8 (the tile waits
+    // for each step's weights); a model that fits L2: 16 x 2048 9.3 / 12.9, 32 x 1024 9.3 / 12.9, 32 x 2048 17.4 / 13.3, 64 x 1024 17.3 / 13.0.
+    if (most <= 8 || (most <= 32 && ceil_div(most, 8) * N < 16384)) {
         auto kernel = most == 1 ? linear_f32_few_kernel<1> : most == 2 ? linear_f32_few_kernel<2> : most <= 4 ? linear_f32_few_kernel<4> : linear_f32_few_kernel<8>;
         launch_kernel(kernel, dim3(ceil_div(N, 16), ceil_div(most, 8), z), dim3(256), 0, s, x, ldx, w, w_stride, y, ldy, M, N, K, entries, n_entries, x_at_y ? 1 : 0);
         return;
