@@ -236,7 +236,7 @@ class LLM(torch.nn.Module):
         """Append `tokens` (a list of ids) behind the `history` tokens the cache holds; history 0 starts a new sequence.
         Returns the logits [len(want), vocab] of the places `want` among these tokens.  A single token behind others is
         a decoding step, everything else a prefill in chunks."""
-        n = len(tokens)
+        n, want = len(tokens), list(want)
         if history + n > self.max_total_length:
             raise ValueError(f"{history} cached + {n} new tokens exceed the {self.max_total_length} tokens the KV cache holds "
                              f"under the current memory limit")
