@@ -436,6 +436,18 @@ int cpmcu_debug_linear_schedule(int M, int N, int K, int grid_limit, int32_t* ou
     return rc < 0 ? rc : n;
 }
 
+int cpmcu_debug_decode_graphs(const int32_t* shapes, int n, int32_t* acts) {
+    return guarded([&] {
+        CPM_REQUIRE(shapes != nullptr && acts != nullptr && n >= 0, "debug_decode_graphs: bad arguments");
+        GraphSlots slots;
+        for (int i = 0; i < n; ++i) {
+            int evict;
+            acts[i] = slots.pass(shapes[i], evict);
+        }
+        return 0;
+    });
+}
+
 int cpmcu_linear_swiglu_bf16(const void* x, const void* w, void* out, int rows, int inter, int K, int grid_limit) {
     return guarded([&] {
         Runtime& rt = runtime();

@@ -89,19 +89,12 @@ Engine::Engine(const ModelConfig& mc) : mc_(mc) {
 Engine::~Engine() {
     if (step_graph_) cudaGraphExecDestroy(step_graph_);
     if (decode_graph_) cudaGraphExecDestroy(decode_graph_);
-    drop_decode_graphs();
+    for (auto& g : decode_graphs_) cudaGraphExecDestroy(g.second.exec);
     if (ev0_) cudaEventDestroy(ev0_);
     if (ev1_) cudaEventDestroy(ev1_);
     if (ev_mid_) cudaEventDestroy(ev_mid_);
     if (pool_.base) cudaFree(pool_.base);
     if (h_result_) cudaFreeHost(h_result_);
-}
-
-void Engine::drop_decode_graphs() {
-    for (auto& g : decode_graphs_) {
-        if (g.second.exec) cudaGraphExecDestroy(g.second.exec);
-    }
-    decode_graphs_.clear();
 }
 
 void Engine::attach_eagle(const EagleConfig& ec) {
@@ -730,47 +723,80 @@ void Engine::decode(int n, int padded_len, const int32_t* ids, const int32_t* po
     // A pass of a small model is a row of two- to six-microsecond kernels: launched one by one they wait for the host.  From
     // the second pass of a shape on, it is replayed as a graph over the engine's own input and logits buffers; the caller's
     // are copied in and out, so that nothing depends on where they lie.
-    DecodeGraph* graph = nullptr;
+    const int key = 2 * n + (mask != nullptr);
+    GraphSlots::Act act = GraphSlots::PLAIN;
     if (!rt.profile && bm_capture_ == nullptr) {
-        const int key = 2 * n + (mask != nullptr);
-        if (decode_graphs_.size() >= 16 && decode_graphs_.find(key) == decode_graphs_.end()) drop_decode_graphs();
-        graph = &decode_graphs_[key];
-        if (graph->passes++ == 0) graph = nullptr;
+        int evict;
+        act = graph_slots_.pass(key, evict);
+        if (evict >= 0) drop_decode_graph(evict);
+        if (act == GraphSlots::CAPTURE) {
+            c.pos = d_in_.pos;
+            c.kv_len = d_in_.len;
+            c.mask = mask ? d_in_.mask : nullptr;
+            if (!capture_decode(key, c, s)) act = GraphSlots::PLAIN;
+        }
     }
-    if (graph == nullptr) {
+    if (act == GraphSlots::PLAIN) {
         c.pos = pos;
         c.kv_len = cache_length;  // the caller has already added n (reference cpmcu/llm.py:263-283)
         c.mask = mask;
         target_forward(target_plans(n), c, ids, true, static_cast<bf16*>(logits_out), mc_.vocab, s);
     } else {
         launch_stage_decode(d_in_, ids, pos, cache_length, mask, n, s);
-        if (graph->exec == nullptr) {
-            c.pos = d_in_.pos;
-            c.kv_len = d_in_.len;
-            c.mask = mask ? d_in_.mask : nullptr;
-            ForwardPlans& fp = target_plans(n);
-            const long before = rt.launches;
-            cudaGraph_t g = nullptr;
-            CUDA_CHECK(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
-            try {
-                target_forward(fp, c, d_in_.ids, true, logits_, mc_.vocab, s);
-            } catch (...) {
-                cudaStreamEndCapture(s, &g);
-                if (g) cudaGraphDestroy(g);
-                throw;
-            }
-            CUDA_CHECK(cudaStreamEndCapture(s, &g));
-            const cudaError_t made = cudaGraphInstantiate(&graph->exec, g, 0);
-            cudaGraphDestroy(g);
-            CUDA_CHECK(made);
-            graph->launches = rt.launches - before;
-            rt.launches = before;
-        }
-        CUDA_CHECK(cudaGraphLaunch(graph->exec, s));
-        rt.launches += graph->launches;
+        const DecodeGraph& graph = decode_graphs_.at(key);
+        CUDA_CHECK(cudaGraphLaunch(graph.exec, s));
+        rt.launches += graph.launches;
         CUDA_CHECK(cudaMemcpyAsync(logits_out, logits_, static_cast<size_t>(n) * mc_.vocab * 2, cudaMemcpyDeviceToDevice, s));
     }
     check_errors("decode");
+}
+
+void Engine::drop_decode_graph(int key) {
+    auto it = decode_graphs_.find(key);
+    if (it == decode_graphs_.end()) return;
+    cudaGraphExecDestroy(it->second.exec);
+    decode_graphs_.erase(it);
+}
+
+// Captures the pass of `c` over d_in_ and logits_.  A graph needs device memory beside the pool (0.7 MB for 32 layers), and a pool that
+// fills the GPU leaves none: then the shape runs launch by launch for good (false).
+bool Engine::capture_decode(int key, const RowCtx& c, cudaStream_t s) {
+    Runtime& rt = runtime();
+    const long before = rt.launches;
+    DecodeGraph graph;
+    cudaGraph_t g = nullptr;
+    try {
+        ForwardPlans& fp = target_plans(c.rows);
+        CUDA_CHECK(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
+        try {
+            target_forward(fp, c, d_in_.ids, true, logits_, mc_.vocab, s);
+        } catch (...) {
+            cudaStreamEndCapture(s, &g);
+            if (g) cudaGraphDestroy(g);
+            throw;
+        }
+        CUDA_CHECK(cudaStreamEndCapture(s, &g));
+    } catch (...) {
+        graph_slots_.bar(key);
+        rt.launches = before;
+        throw;
+    }
+    graph.launches = rt.launches - before;
+    rt.launches = before;
+    cudaError_t made = cudaGraphInstantiate(&graph.exec, g, 0);
+    cudaGraphDestroy(g);
+    if (made == cudaSuccess) {
+        made = cudaGraphUpload(graph.exec, s);   // its memory is there before a pass depends on it
+        if (made != cudaSuccess) cudaGraphExecDestroy(graph.exec);
+    }
+    if (made != cudaSuccess) {
+        graph_slots_.bar(key);
+        if (made != cudaErrorMemoryAllocation) CUDA_CHECK(made);
+        cudaGetLastError();   // dealt with here
+        return false;
+    }
+    decode_graphs_[key] = graph;
+    return true;
 }
 
 // ------------------------------------------------------------------ draft

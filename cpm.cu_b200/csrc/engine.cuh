@@ -15,6 +15,7 @@
 
 #include "common.cuh"
 #include "draft_tree.cuh"
+#include "graph_slots.h"
 #include "layered.cuh"
 #include "sparse_select.cuh"
 
@@ -365,13 +366,14 @@ private:
     std::map<int, std::unique_ptr<ForwardPlans>> plans_;
     // captured decode passes of Llama-format models by 2 * tokens + (tree mask given), and the inputs they read
     struct DecodeGraph {
-        long passes = 0;
         cudaGraphExec_t exec = nullptr;
         long launches = 0;
     };
+    GraphSlots graph_slots_;
     std::map<int, DecodeGraph> decode_graphs_;
     DecodeInputs d_in_;
-    void drop_decode_graphs();
+    void drop_decode_graph(int key);
+    bool capture_decode(int key, const RowCtx& c, cudaStream_t s);
     LayerPlans eplan_level_, eplan_catchup_;
     LinearPlan fc_plan_level_, fc_plan_catchup_, dlm_plan_level_, dlm_plan_catchup_;
     LinearPlan fc2_plan_level_, fc2_plan_catchup_;  // W4A16 drafter: the hidden-state half of fc

@@ -159,7 +159,9 @@ int cpmcu_prefill_rows(int input_length, int history_length, const int32_t* inpu
  * input_length (reference cpmcu/llm.py:263-283); mask_2d may be NULL (causal).
  * `output` is [input_length, vocab] in the model dtype.  padded_length is accepted for
  * compatibility; cuda_graph matters for layered models only, whose one-token step it captures and
- * replays while the three device pointers stay the same. */
+ * replays while the three device pointers stay the same.  Llama-format models replay a pass of a shape
+ * (tokens, with or without mask) they have seen before whatever the flag says, for up to 16 shapes and
+ * over buffers of their own. */
 int cpmcu_decode(int input_length, int padded_length, const int32_t* input, const int32_t* position_ids,
                  const int32_t* cache_length, const uint64_t* mask_2d, void* output, int cuda_graph);
 
@@ -253,6 +255,10 @@ int cpmcu_linear_w4a16(const void* x, const void* qweight, const void* scales, v
  * each has its 128 of them, and the two have consecutive numbers.  Returns the segment count, -1 on error, when
  * cap is too small or when there are no tiles (most products of one row). */
 int cpmcu_debug_linear_schedule(int M, int N, int K, int grid_limit, int32_t* out, int cap);
+
+/* Host only, no GPU needed: what cpmcu_decode does with each pass of a sequence of shapes (HOST int32[n]; any numbers
+ * that tell shapes apart) on a Llama-format model: acts (HOST int32[n]) = 0 launched kernel by kernel, 1 captured first, 2 replayed. */
+int cpmcu_debug_decode_graphs(const int32_t* shapes, int n, int32_t* acts);
 
 /* Times `iters` back-to-back launches of the linear kernel on the library's
  * stream with CUDA events, cycling through `copies` separate weight buffers so
