@@ -8,8 +8,8 @@
 // layout keeps the R rows of a k-block together), the eight warps take k-blocks in turn, and only sums of one CTA
 // meet.  A warp keeps eight 16-byte loads per lane in flight, the first of them before the wait for the predecessor.  About
 // 20 instructions per 16 bytes leave three quarters of the issue slots free at the HBM rate.
-// Back to back, weights from HBM, tensor-core tiles before / now: 2048 x 2048 6.9 / 3.6 us, 3072 x 2048 5.5 / 4.1,
-// 2048 x 8192 10.9 / 8.2, 11008 x 4096 gated 39.8 / 28.6, 73448 x 4096 88 / 84 (7.2 TB/s); 512 x 256 3.7 / 3.5.
+// Back to back, weights from HBM, tensor-core tiles / this: 2048 x 2048 7.0 / 3.5 us, 2048 x 8192 11.0 / 8.1, 4096 x 16384 22.8 / 21.2,
+// 11008 x 4096 gated 39.8 / 28.8, 73448 x 4096 88 / 84 (7.2 TB/s); 512 x 256 3.7 / 3.5.
 #include "common.cuh"
 #include "layered.cuh"
 #include "row_ops.cuh"

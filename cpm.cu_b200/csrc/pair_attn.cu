@@ -4,8 +4,12 @@
 // What bounds it.  A 128-row query tile against 128 keys costs 1024 cycles of tensor pipe (S = Q K^T and P V, 128 x 128 x 128 each)
 // and 1024 cycles of exponentials (16384 on the MUFU pipe).  With one tile per CTA the two follow one another with their latencies
 // between them (2750 cycles per tile) and every tile fetches its own keys.  Here two tiles A and B share one fetch of the keys
-// and the SM's pipes, 2200 cycles per tile, of which the longest single part is the exponentials of both.  4096 causal rows, 32
-// query heads on 2 key heads: 191 -> 152 us; 2048 rows behind 14336: 665 -> 522 (990 TFLOP/s).
+// and the SM's pipes: about 4600 cycles for both, in which either pipe is busy for 2048.  The rest is the softmax's own chain: of a
+// softmax thread's cycles by role clocks 1450 are exponentials and their stores, 800 waits for scores, 700 maxima, 300 the exchange of
+// maxima, 260 waits for P V, 230 loads of scores; what is left are instructions between them.  576 threads leave 96 registers,
+// and beside 64 scores a thread keeps 44 to 116 bytes of addresses and bounds in local memory.
+// One tile / two tiles per CTA, 32 query heads on 2 key heads: 4096 causal rows 192 / 154 us, 2048 behind 30000 1330 / 1077
+// (970 TFLOP/s); block-sparse, 2048 behind 30000, 5 % and 40 % of the blocks per token: 969 / 776 and 1564 / 1276.
 //   S            one buffer per tile in tensor memory; it is free as soon as the softmax holds the scores in registers, so S(i+1) is
 //                computed while the softmax of iteration i runs
 //   P            bf16 in shared memory, one buffer per tile; PV(i) runs under the next softmax

@@ -658,9 +658,11 @@ AttnPlan make_biased_attn_plan(const bf16* q, int q_ld_tokens, const bf16* k_cac
     p.scale = scale;
     p.tm_q = make_tmap_3d(q, dk, hq, tq, static_cast<uint64_t>(dk) * 2, static_cast<uint64_t>(q_ld_tokens) * 2, 64, grp,
                           ROWS / grp);
-    // Two tiles per CTA (pair_attn.cu) once such CTAs number one and a half times the SMs: causal tiles differ in length, and fewer
-    // CTAs cannot even that out.  Query rows x heads / key heads, one tile / two tiles per CTA: 1024 x 32/2 (128 CTAs of two)
-    // 21.1 / 25.2 us, 2048 x 32/2 (256) 60 / 48, 4096 x 16/4 (256) 97 / 76, 4096 x 32/2 (512) 191 / 152.
+    // Two tiles per CTA (pair_attn.cu) once such CTAs number one and a half times the SMs: the tiles of a prompt's first chunk differ
+    // in length, and fewer CTAs cannot even that out.  Query rows x heads / key heads, one tile / two tiles per CTA: 1024 x 32/2
+    // (128 CTAs of two) 21.1 / 25.2 us, 2048 x 32/2 (256) 60 / 49, 4096 x 16/4 (256) 99 / 79, 4096 x 32/2 (512) 192 / 154.  Behind
+    // a long prefix tiles are alike and fewer CTAs would do (700 x 32/2, 4096 keys in all: 86 / 77); how long the prefix will be is
+    // not known here, and the line is the first chunk's.
     p.pair = splits == 1 && 2LL * ceil_div(ceil_div(tq, ROWS / grp), 2) * hkv >= 3LL * runtime().num_sms;
     const int box = p.pair ? 64 : KEYS;
     p.tm_k = make_tmap_2d(k_cache, static_cast<uint64_t>(hkv) * dk, budget, static_cast<uint64_t>(hkv) * dk * 2, 64, box);
