@@ -415,14 +415,15 @@ struct TileJob {
     int x_row, y_row, rows;
 };
 
-template <bool SWIGLU>
-__device__ __forceinline__ TileJob tile_job(const GemmArgs& a, const int4* entries, int t) {
+// CSZ 2: jobs of a pair of CTAs, a.n_tiles and a.n_tiles_s count pairs of feature tiles, of which `rank` takes one.
+template <bool SWIGLU, int CSZ = 1>
+__device__ __forceinline__ TileJob tile_job(const GemmArgs& a, const int4* entries, int t, int rank = 0) {
     TileJob j;
     const int ts = a.groups_s * a.n_tiles_s;
     if (t < ts) {
         const int g = t / a.n_tiles_s;
         j.shared = true;
-        j.n_tile = t - g * a.n_tiles_s;
+        j.n_tile = (t - g * a.n_tiles_s) * CSZ + rank;
         j.kblocks = a.kblocks_s;
         j.N = a.N_s;
         j.w_row = static_cast<int>(a.w_row_s) + j.n_tile * a.kblocks_s * gemm::BLOCK_N;
@@ -433,15 +434,51 @@ __device__ __forceinline__ TileJob tile_job(const GemmArgs& a, const int4* entri
         const int g = (t - ts) / a.n_tiles;
         const int4 e = entries[g];
         j.shared = false;
-        j.n_tile = (t - ts) - g * a.n_tiles;
+        j.n_tile = ((t - ts) - g * a.n_tiles) * CSZ + rank;
         j.kblocks = a.kblocks;
         j.N = a.N;
-        j.w_row = (e.x * a.n_tiles + j.n_tile) * a.kblocks * gemm::BLOCK_N;
+        j.w_row = (e.x * CSZ * a.n_tiles + j.n_tile) * a.kblocks * gemm::BLOCK_N;
         j.x_row = SWIGLU ? e.y : e.z;   // the down product reads the rows gate/up wrote
         j.y_row = e.z;
         j.rows = e.w;
     }
     return j;
+}
+
+// The row groups of the launch into shared memory, by all threads; returns how many there are.
+__device__ __forceinline__ int read_groups(const GemmArgs& a, int4* entries) {
+    if (a.uniform > 0) {
+        const int per = (a.rows + a.tile - 1) / a.tile, n = a.uniform * per;
+        for (int i = threadIdx.x; i < n; i += NUM_THREADS) {
+            const int m = i / per, r = (i - m * per) * a.tile;
+            entries[i] = make_int4(m, m * a.rows + r, m * a.rows + r, min(a.tile, a.rows - r));
+        }
+        return n;
+    }
+    const int n = min(__ldcg(a.n_entries), kMoeMaxEntries);
+    for (int i = threadIdx.x; i < n; i += NUM_THREADS) entries[i] = __ldcg(a.entries + i);
+    return n;
+}
+
+// A finished tile out of tensor memory, by the four epilogue warps (lane = feature, column = row of the group).
+template <int MT, bool SWIGLU>
+__device__ __forceinline__ void store_job(const GemmArgs& a, const TileJob& j, uint32_t t_addr, float* xch, int q, int lane) {
+    const bool vec = gemm::rows_take_16_bytes(a.y, a.ldy, j.N);
+    if constexpr (SWIGLU) {
+        gemm::swiglu_tile<MT>(t_addr, j.rows, a.y, a.ldy, j.N, j.y_row, j.n_tile * 64 + (q & 1) * 32, 0.f, 0.f, xch, q, lane, vec);
+    } else {
+#pragma unroll 1
+        for (int c0 = 0; c0 < j.rows; c0 += 16) {   // uniform across the CTA
+            uint32_t r[16];
+            ptx::tmem_ld16(t_addr + c0, r);
+            ptx::tmem_wait_ld();
+            float v[16];
+#pragma unroll
+            for (int c = 0; c < 16; ++c) v[c] = __uint_as_float(r[c]);
+            gemm::store_tokens(a.y, a.ldy, j.N, j.y_row + c0, j.rows - c0, j.n_tile * gemm::BLOCK_N + q * 32, v,
+                               reinterpret_cast<uint8_t*>(xch) + q * gemm::EPI_WARP_BYTES, lane, vec);
+        }
+    }
 }
 
 template <int MT, bool SWIGLU>
@@ -485,20 +522,7 @@ moe_gemm_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
         ptx::tmem_alloc(tmem_slot, C::TMEM_COLS);
         ptx::tmem_relinquish();
     }
-    auto read_groups = [&]() -> int {
-        if (a.uniform > 0) {
-            const int per = (a.rows + a.tile - 1) / a.tile, n = a.uniform * per;
-            for (int i = threadIdx.x; i < n; i += NUM_THREADS) {
-                const int m = i / per, r = (i - m * per) * a.tile;
-                entries[i] = make_int4(m, m * a.rows + r, m * a.rows + r, min(a.tile, a.rows - r));
-            }
-            return n;
-        }
-        const int n = min(__ldcg(a.n_entries), kMoeMaxEntries);
-        for (int i = threadIdx.x; i < n; i += NUM_THREADS) entries[i] = __ldcg(a.entries + i);
-        return n;
-    };
-    int n_entries = kGroupsEarly ? read_groups() : 0;
+    int n_entries = kGroupsEarly ? read_groups(a, entries) : 0;
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();
@@ -520,7 +544,7 @@ moe_gemm_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
     grid_dep_wait();
     if (!kGroupsEarly) {
         grid_dep_trigger();
-        n_entries = read_groups();
+        n_entries = read_groups(a, entries);
         __syncthreads();
     }
     const int total = shared_tiles + n_entries * a.n_tiles;
@@ -602,22 +626,7 @@ moe_gemm_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
             if (!ptx::mbar_wait_warp(&acc_full[acc], acc_phase, abort_flag)) break;
             ptx::tc_fence_after();
             const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * MT;
-            const bool vec = gemm::rows_take_16_bytes(a.y, a.ldy, j.N);
-            if constexpr (SWIGLU) {
-                gemm::swiglu_tile<MT>(t_addr, j.rows, a.y, a.ldy, j.N, j.y_row, j.n_tile * 64 + (q & 1) * 32, 0.f, 0.f, xch, q, lane, vec);
-            } else {
-#pragma unroll 1
-                for (int c0 = 0; c0 < j.rows; c0 += 16) {   // uniform across the CTA
-                    uint32_t r[16];
-                    ptx::tmem_ld16(t_addr + c0, r);
-                    ptx::tmem_wait_ld();
-                    float v[16];
-#pragma unroll
-                    for (int c = 0; c < 16; ++c) v[c] = __uint_as_float(r[c]);
-                    gemm::store_tokens(a.y, a.ldy, j.N, j.y_row + c0, j.rows - c0, j.n_tile * gemm::BLOCK_N + q * 32, v,
-                                       reinterpret_cast<uint8_t*>(xch) + q * gemm::EPI_WARP_BYTES, lane, vec);
-                }
-            }
+            store_job<MT, SWIGLU>(a, j, t_addr, xch, q, lane);
             ptx::tc_fence_before();
             ptx::mbar_arrive(&acc_empty[acc]);
             if (++acc == 2) { acc = 0; acc_phase ^= 1; }
@@ -631,6 +640,191 @@ moe_gemm_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
         ptx::tmem_dealloc(tmem_base, C::TMEM_COLS);
     }
     if (threadIdx.x == 0 && *abort_flag) atomicOr(a.error, ERR_GEMM_TIMEOUT);
+}
+
+// The same on pairs of CTAs (gemm_pair.cu): a cluster of two takes two neighbouring feature tiles of one row group, each CTA fetches its
+// own weights and half of the group's rows, and one tcgen05.mma.cta_group::2 multiplies both.  What bounds the single CTAs
+// is their operands' way into shared memory: 48 KB per 512 cycles of MMAs at 256 rows, 94 bytes a cycle and SM; a pair's CTAs take 32 KB
+// each.  Launches over 4096 tokens, single / pairs: gate/up of 60 experts of 1024, top 6, width 2048, with a shared one of 2048
+// 260 / 214 us, down 136 / 106; four 2048 x 2048 products and one of 64 117 / 98.  777 tokens, 30 experts of 2048, top 4, width 4096 (groups of 128
+// rows) 273 / 258 and 142 / 135: there the weights' bytes are the larger part.
+template <int MT>
+struct PairCfg {
+    static constexpr int STAGE_BYTES = W_TILE_BYTES + MT / 2 * BLOCK_K * 2;
+    static constexpr int STAGES = MT <= 128 ? 8 : 6;
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + Cfg<MT>::CTRL_BYTES + gemm::EPI_XCH_BYTES + Cfg<MT>::ENTRY_BYTES + 1024;
+    static_assert(SMEM_BYTES <= 232448, "shared memory budget");
+};
+
+template <int MT, bool SWIGLU>
+__global__ void __launch_bounds__(NUM_THREADS, 1)
+moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
+                     const __grid_constant__ CUtensorMap tm_xs, const GemmArgs a) {
+    using C = PairCfg<MT>;
+    constexpr int XBOX = 64, XBOX_BYTES = XBOX * BLOCK_K * 2;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + C::STAGES * C::STAGE_BYTES);   // rank 0's count both CTAs' copies
+    uint64_t* empty = full + C::STAGES;
+    uint64_t* acc_full = empty + C::STAGES;
+    uint64_t* acc_empty = acc_full + 2;                                                // rank 0's
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    float* xch = reinterpret_cast<float*>(smem + C::STAGES * C::STAGE_BYTES + Cfg<MT>::CTRL_BYTES);
+    int4* entries = reinterpret_cast<int4*>(smem + C::STAGES * C::STAGE_BYTES + Cfg<MT>::CTRL_BYTES + gemm::EPI_XCH_BYTES);
+
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const int rank = static_cast<int>(ptx::cluster_ctarank());
+    const int G = gridDim.x / 2, g = blockIdx.x / 2;
+    constexpr bool kGroupsEarly = !SWIGLU;
+    if (kGroupsEarly) grid_dep_trigger();
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < C::STAGES; ++s) {
+            ptx::mbar_init(&full[s], 1);
+            ptx::mbar_init(&empty[s], 1);
+        }
+        for (int s = 0; s < 2; ++s) {
+            ptx::mbar_init(&acc_full[s], 1);
+            ptx::mbar_init(&acc_empty[s], 2 * 128);
+        }
+        *abort_flag = 0;
+        ptx::mbar_fence_init();
+        ptx::prefetch_tensormap(&tm_w);
+        ptx::prefetch_tensormap(&tm_x);
+        ptx::prefetch_tensormap(&tm_xs);
+    }
+    if (warp == 1) ptx::tmem_alloc_pair(tmem_slot, 2 * MT);
+    int n_entries = kGroupsEarly ? read_groups(a, entries) : 0;
+    ptx::tc_fence_before();
+    __syncthreads();
+    ptx::cluster_sync();   // both CTAs' barriers are there before either copies or arrives
+    ptx::tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    const int shared_tiles = a.groups_s * a.n_tiles_s;
+    // columns of the product (a group that is not full costs only its rows) and the boxes of rows that each CTA fetches
+    auto columns = [](const TileJob& j) { return min(MT, (j.rows + 15) & ~15); };
+    auto boxes_of = [&](const TileJob& j) { return (columns(j) / 2 + XBOX - 1) / XBOX; };
+    auto load_w = [&](int s, const TileJob& j, int kb) {
+        if (rank == 0) ptx::mbar_arrive_expect_tx(&full[s], 2 * (W_TILE_BYTES + boxes_of(j) * XBOX_BYTES));
+        ptx::tma_load_2d_pair(smem + s * C::STAGE_BYTES, &tm_w, ptx::cluster_map(ptx::smem_u32(&full[s]), 0), 0, j.w_row + kb * gemm::BLOCK_N);
+    };
+    // weights of the first k-blocks, as far as the tiles are known, before the wait for the predecessor
+    int pre = 0;
+    if (threadIdx.x == 0) {
+        const int known = shared_tiles + n_entries * a.n_tiles;
+        for (int t = g; t < known && pre < C::STAGES; t += G) {
+            const TileJob j = tile_job<SWIGLU, 2>(a, entries, t, rank);
+            for (int kb = 0; kb < j.kblocks && pre < C::STAGES; ++kb, ++pre) load_w(pre, j, kb);
+        }
+    }
+    grid_dep_wait();
+    if (!kGroupsEarly) {
+        grid_dep_trigger();
+        n_entries = read_groups(a, entries);
+        __syncthreads();
+    }
+    const int total = shared_tiles + n_entries * a.n_tiles;
+
+    if (warp == 0) {
+        // ------------------------------------------------ TMA producer (both CTAs)
+        if (lane == 0) {
+            int stage = 0;
+            uint32_t phase = 0;
+            int issued = 0;
+            bool ok = true;
+            for (int t = g; ok && t < total; t += G) {
+                const TileJob j = tile_job<SWIGLU, 2>(a, entries, t, rank);
+                const int boxes = boxes_of(j), x_row = j.x_row + rank * (columns(j) / 2);
+                for (int kb = 0; kb < j.kblocks; ++kb, ++issued) {
+                    if (issued >= pre) {
+                        if (!ptx::mbar_wait(&empty[stage], phase ^ 1, abort_flag)) { ok = false; break; }
+                        load_w(stage, j, kb);
+                    }
+                    const uint32_t bar = ptx::cluster_map(ptx::smem_u32(&full[stage]), 0);
+                    for (int b = 0; b < boxes; ++b) {
+                        ptx::tma_load_2d_pair(smem + stage * C::STAGE_BYTES + W_TILE_BYTES + b * XBOX_BYTES, j.shared ? &tm_xs : &tm_x, bar,
+                                              kb * BLOCK_K, x_row + b * XBOX);
+                    }
+                    if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
+                }
+            }
+            if (!ok) {
+                // give copies already in flight time to land before the CTA retires
+                const long long t0 = clock64();
+                while (clock64() - t0 < 2000000LL) {}
+            }
+        }
+    } else if (warp == 1) {
+        // ------------------------------------------------ MMA issuer (rank 0)
+        if (lane == 0 && rank == 0) {
+            int stage = 0;
+            uint32_t phase = 0;
+            int acc = 0;
+            uint32_t acc_phase = 0;
+            bool ok = true;
+            for (int t = g; ok && t < total; t += G) {
+                const TileJob j = tile_job<SWIGLU, 2>(a, entries, t, rank);
+                const uint32_t idesc = ptx::umma_idesc_bf16(2 * gemm::BLOCK_N, columns(j), 0, 0);
+                if (!ptx::mbar_wait(&acc_empty[acc], acc_phase ^ 1, abort_flag)) break;
+                ptx::tc_fence_after();
+                const uint32_t d_tmem = tmem_base + acc * MT;
+                for (int kb = 0; kb < j.kblocks; ++kb) {
+                    if (!ptx::mbar_wait(&full[stage], phase, abort_flag)) { ok = false; break; }
+                    ptx::tc_fence_after();
+                    const uint32_t wa = ptx::smem_u32(smem + stage * C::STAGE_BYTES);
+                    const uint32_t xa = wa + W_TILE_BYTES;
+#pragma unroll
+                    for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
+                        const uint64_t da = ptx::umma_desc_sw128(wa + k * UMMA_K * 2, 16, 1024);
+                        const uint64_t db = ptx::umma_desc_sw128(xa + k * UMMA_K * 2, 16, 1024);
+                        ptx::umma_ss_pair(d_tmem, da, db, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                    }
+                    ptx::umma_commit_pair(&empty[stage]);
+                    if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
+                }
+                if (!ok) break;
+                ptx::umma_commit_pair(&acc_full[acc]);
+                acc ^= 1;
+                if (acc == 0) acc_phase ^= 1;
+            }
+        }
+    } else {
+        // ------------------------------------------------ epilogue (128 threads of each CTA, its own 128 features)
+        const int q = warp & 3;
+        const uint32_t freed = ptx::cluster_map(ptx::smem_u32(acc_empty), 0);
+        int acc = 0;
+        uint32_t acc_phase = 0;
+        for (int t = g; t < total; t += G) {
+            const TileJob j = tile_job<SWIGLU, 2>(a, entries, t, rank);
+            if (!ptx::mbar_wait_warp(&acc_full[acc], acc_phase, abort_flag)) break;
+            ptx::tc_fence_after();
+            store_job<MT, SWIGLU>(a, j, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * MT, xch, q, lane);
+            ptx::tc_fence_before();
+            ptx::mbar_arrive_cluster(freed + acc * 8);
+            if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+        }
+    }
+
+    ptx::tc_fence_before();
+    __syncthreads();
+    __syncwarp();
+    ptx::cluster_sync();   // neither CTA leaves while the other may still read its memory or arrive at its barriers
+    if (warp == 1) {
+        ptx::tc_fence_after();
+        ptx::tmem_dealloc_pair(tmem_base, 2 * MT);
+    }
+    if (threadIdx.x == 0 && *abort_flag) atomicOr(a.error, ERR_GEMM_TIMEOUT);
+}
+
+template <int MT, bool SWIGLU>
+void launch_pair(const MoeGemmPlan& p, const GemmArgs& a, int grid, cudaStream_t s) {
+    static bool configured = false;
+    if (!configured) {
+        CUDA_CHECK(cudaFuncSetAttribute(moe_gemm_pair_kernel<MT, SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<MT>::SMEM_BYTES));
+        configured = true;
+    }
+    launch_kernel_cluster(moe_gemm_pair_kernel<MT, SWIGLU>, dim3(grid), dim3(NUM_THREADS), PairCfg<MT>::SMEM_BYTES, s, 2, p.tm_w, p.tm_x, p.tm_xs, a);
 }
 
 template <int MT, bool SWIGLU>
@@ -792,6 +986,19 @@ void launch_moe_gemm(const MoeGemmPlan& p, cudaStream_t s) {
     a.error = runtime().d_error;
     const long long most = static_cast<long long>(a.groups_s) * a.n_tiles_s + static_cast<long long>(p.max_entries) * p.n_tiles;
     const int grid = static_cast<int>(std::max<long long>(1, std::min<long long>(most, runtime().num_sms)));
+    // Groups of 64 rows and fewer leave a pair as much weight to fetch as two CTAs, and halves of 32 rows to multiply them with.
+    if (p.tile >= 128 && p.n_tiles % 2 == 0) {
+        a.n_tiles /= 2;
+        a.n_tiles_s = ceil_div(a.n_tiles_s, 2);   // the shared matrix is the last one: an odd tile's partner reads zeros beyond the map
+        const int pairs = 2 * static_cast<int>(std::max<long long>(1, std::min<long long>(most / 2, runtime().num_sms / 2)));
+        switch (p.tile * 2 + p.swiglu) {
+            case 128 * 2: launch_pair<128, false>(p, a, pairs, s); break;
+            case 128 * 2 + 1: launch_pair<128, true>(p, a, pairs, s); break;
+            case 256 * 2: launch_pair<256, false>(p, a, pairs, s); break;
+            default: launch_pair<256, true>(p, a, pairs, s); break;
+        }
+        return;
+    }
     switch (p.tile * 2 + p.swiglu) {
         case 16 * 2: launch_gemm<16, false>(p, a, grid, s); break;
         case 16 * 2 + 1: launch_gemm<16, true>(p, a, grid, s); break;
