@@ -8,16 +8,25 @@
 // softmax thread's cycles by role clocks 1450 are exponentials and their stores, 800 waits for scores, 700 maxima, 300 the exchange of
 // maxima, 260 waits for P V, 230 loads of scores; what is left are instructions between them.  576 threads leave 96 registers,
 // and beside 64 scores a thread keeps 44 to 116 bytes of addresses and bounds in local memory.
-// One tile / two tiles per CTA, 32 query heads on 2 key heads: 4096 causal rows 192 / 154 us, 2048 behind 30000 1330 / 1077
-// (970 TFLOP/s); block-sparse, 2048 behind 30000, 5 % and 40 % of the blocks per token: 969 / 776 and 1564 / 1276.
+// One tile / two tiles per CTA, 32 query heads on 2 key heads: 4096 causal rows 192 / 149 us, 2048 behind 30000 1330 / 1048
+// (1.0 PFLOP/s).
+// Probabilities in tensor memory (in the scores' place, tiles taking turns), which spares shared memory a third of its traffic, took the
+// same 154 us as P in shared memory then did, and an issuing warp per tile 171: neither the memory nor the order of issue is the bound.
 //   S            one buffer per tile in tensor memory; it is free as soon as the softmax holds the scores in registers, so S(i+1) is
 //                computed while the softmax of iteration i runs
 //   P            bf16 in shared memory, one buffer per tile; PV(i) runs under the next softmax
 //   K, V         one stage each: K(i+2) is fetched from the end of S(i+1) on, V(i+1) from the end of PV(i) on, both most of an
 //                iteration before they are needed
-//   softmax      two threads per row, 64 keys each; the row maximum is exchanged through shared memory, once per iteration
+//   softmax      two threads per row, 64 keys each; the row maximum is exchanged through shared memory, once per iteration, by the two
+//                warps of 32 rows alone
 // Keys come in blocks of 64: thread half ch of iteration i works on block 2 i + ch.  Block-sparse mode lists the union of the
-// two tiles' blocks, so an iteration's two blocks need not be neighbours.  A tile's P V takes only the blocks some row of that tile
+// two tiles' blocks, so an iteration's two blocks need not be neighbours.  The union of sixteen tokens is nearly all blocks where each
+// sees an eighth of them, but a warp's 32 rows are two tokens (of 16 heads) and mostly see nothing: such a warp leaves out scores, maxima and
+// exponentials and only keeps zeros in its part of P.  Which tokens of the pair see a listed block is one word in shared memory,
+// filled once; read from the block mask in every iteration, the bits' latency stood before the wait for the scores.  Block-sparse, 2048 rows
+// behind 30000 keys, 5, 13, 40 and 100 % of the blocks per token, before / now: 771 / 603, 1162 / 914, 1276 / 1159, 1111 / 1031 us;
+// behind 9000, 13 %: 396 / 325.  Pairs of more than 32 tokens keep the mask's rows.
+// A tile's P V takes only the blocks some row of that tile
 // sees: a probability of zero does not hide an infinity or a NaN among the values, so no row meets values that the one-tile
 // kernel would not have shown it.
 // Tensor memory: S_A [0,128) S_B [128,256) O_A [256,384) O_B [384,512).
@@ -37,6 +46,9 @@ constexpr int SOFT_WARPS = 2 * TILE_THREADS / 32;
 constexpr int PAIR_THREADS = (SOFT_WARPS + 2) * 32;   // + MMA issuer, TMA producer
 constexpr int PAIR_TMEM_COLS = 512, PAIR_TMEM_O = 256;
 constexpr int MAX_BLOCKS = 4096;              // 262144 keys (block-sparse mode)
+// How a thread learns which blocks its token sees: all, from the token's row of the block mask, or from a word per listed block with
+// a bit per token of the pair (at most 32 tokens)
+enum { DENSE = 0, BY_ROW = 1, BY_WORD = 2 };
 
 template <int DK, int DV>
 struct PairCfg {
@@ -49,12 +61,13 @@ struct PairCfg {
     static constexpr int SMEM_UNION = SMEM_LIST + MAX_BLOCKS * 2;    // 64 words of 64 blocks, then 65 prefix counts
     static constexpr int SMEM_SEEN = SMEM_UNION + 64 * 8 + 320;  // [2 tiles] the words of that tile alone
     static constexpr int SMEM_XCH = SMEM_SEEN + 2 * 64 * 8;      // [2 tiles][2 buffers][2 halves][128] floats
-    static constexpr int SMEM_CTRL = SMEM_XCH + 8 * ROWS * 4;
+    static constexpr int SMEM_WORD = SMEM_XCH + 8 * ROWS * 4;    // BY_WORD: [MAX_BLOCKS] words
+    static constexpr int SMEM_CTRL = SMEM_WORD + MAX_BLOCKS * 4;
     static constexpr int SMEM_TOTAL = SMEM_CTRL + 256 + 1024;
     static_assert(SMEM_TOTAL <= 232448, "shared memory budget");
 };
 
-template <int DK, int DV, bool BIASED>
+template <int DK, int DV, bool BIASED, int SPARSE>
 __global__ void __launch_bounds__(PAIR_THREADS, 1)
 pair_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const AttnArgs a) {
@@ -78,6 +91,7 @@ pair_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     int* uni_at = reinterpret_cast<int*>(uni + 64);
     unsigned long long* seen = reinterpret_cast<unsigned long long*>(smem + C::SMEM_SEEN);
     int* run = uni_at + 65;
+    uint32_t* words = reinterpret_cast<uint32_t*>(smem + C::SMEM_WORD);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     grid_dep_trigger();
@@ -143,7 +157,7 @@ pair_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     };
     int n_blk = max(blk_hi - blk_lo, 0);
 
-    const bool sparse = (a.blockmask != nullptr);
+    constexpr bool sparse = SPARSE != DENSE;
     if (sparse) {
         if (tid == 0) { run[0] = 0; run[1] = MAX_BLOCKS; }
         if (tid < 128) {   // 64 words of each tile
@@ -200,6 +214,19 @@ pair_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             }
         }
         __syncthreads();
+        if (SPARSE == BY_WORD) {
+            for (int j = tid; j < n_blk; j += PAIR_THREADS) {
+                const int b = list[j];
+                uint32_t w = 0;
+                const uint64_t* r = a.blockmask + (static_cast<size_t>(h) * a.tq + t0) * a.bm_words + (b >> 6);
+                for (int t = t0; t < t_end; ++t, r += a.bm_words) {
+                    const bool sees = b >= (t + causal_base + 63) / 64 - a.block_window || ((b >> 6) < a.bm_words && ((*r >> (b & 63)) & 1ull));
+                    w |= static_cast<uint32_t>(sees) << (t - t0);
+                }
+                words[j] = w;
+            }
+            __syncthreads();
+        }
     }
     const int n_it = (n_blk + 1) / 2;
     auto block_of = [&](int j) -> int { return sparse ? list[min(j, n_blk - 1)] : blk_lo + j; };
@@ -351,76 +378,91 @@ pair_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         const float slope2 =   // log2(e) * slope of this row's head
             biased ? 1.4426950408889634f * exp2f(-a.bias_exp * static_cast<float>(qh + 1) / static_cast<float>(a.hq)) : 0.f;
         const float sl2 = biased ? 1.f : a.scale_log2;   // biased scores are brought to log2 units as they are read
-        const int win_left = sparse ? (t + causal_base + 63) / 64 - a.block_window : 0;
-        const uint64_t* bm_row = (sparse && row_valid) ? a.blockmask + (static_cast<size_t>(h) * a.tq + t) * a.bm_words : nullptr;
+        const int win_left = SPARSE == BY_ROW ? (t + causal_base + 63) / 64 - a.block_window : 0;
+        const uint64_t* bm_row = (SPARSE == BY_ROW && row_valid) ? a.blockmask + (static_cast<size_t>(h) * a.tq + t) * a.bm_words : nullptr;
         const uint32_t lane_sel = static_cast<uint32_t>((warp & 3) * 32) << 16;
         const uint32_t tmem_s = tmem_base + lane_sel + tile * KEYS + ch * 64;
         const uint32_t tmem_o = tmem_base + lane_sel + PAIR_TMEM_O + tile * 128 + ch * (DV / 2);
         float* xch = reinterpret_cast<float*>(smem + C::SMEM_XCH) + tile * 4 * ROWS;
         uint8_t* p_half = smem + C::SMEM_P + tile * C::P_TILE + ch * HALF_BYTES + row * 128;
-        const int bar_id = 1 + tile;
+        const int bar_id = 1 + tile * 4 + (warp & 3);   // the two warps of these 32 rows
         float m_run = -INFINITY;  // running max of raw scores (same in both threads of a row)
         float l_run = 0.f;        // this thread's share of the running sum
+        // BY_WORD: the tokens of this warp's 32 rows
+        const int tok0 = tile * a.tok_per_tile + (warp & 3) * 32 / a.grp;
+        const uint32_t warp_tokens = SPARSE == BY_WORD ? ((a.grp < 32 ? (1u << (32 / a.grp)) - 1u : 1u) << tok0) : 0u;
+        bool zeros = false;   // BY_WORD: this thread's part of P holds zeros
         bool ok = true;
         for (int i = 0; i < n_it; ++i) {
             const int j = 2 * i + ch;
             const int b = block_of(j);
             const int key0 = b * BLK;
             bool blk_ok = j < n_blk;
-            if (sparse) {
+            bool any = true;   // some row of this warp sees the block; where none does, neither scores nor exponentials are needed
+            if (SPARSE == BY_WORD) {
+                const uint32_t w = words[min(j, n_blk - 1)];
+                blk_ok = blk_ok && ((w >> (t - t0)) & 1u);
+                any = j < n_blk && (w & warp_tokens) != 0u;
+            }
+            if (SPARSE == BY_ROW) {
                 blk_ok = blk_ok && (b >= win_left || (bm_row != nullptr && (b >> 6) < a.bm_words && ((bm_row[b >> 6] >> (b & 63)) & 1ull)));
             }
             ok = ok && ptx::mbar_wait_warp(&s_bar[tile], i & 1, abort_flag);
             if (!ok) {
-                for (int k = i; k < n_it; ++k) ptx::named_bar_sync(bar_id, TILE_THREADS);   // every warp arrives equally often
+                for (int k = i; k < n_it; ++k) ptx::named_bar_sync(bar_id, 64);   // every warp arrives equally often
                 break;
             }
             ptx::tc_fence_after();
             uint32_t sc[64];
-            ptx::tmem_ld32(tmem_s, sc);
-            ptx::tmem_ld32(tmem_s + 32, sc + 32);
-            ptx::tmem_wait_ld();
+            if (any) {
+                ptx::tmem_ld32(tmem_s, sc);
+                ptx::tmem_ld32(tmem_s + 32, sc + 32);
+                ptx::tmem_wait_ld();
+            }
             ptx::tc_fence_before();
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&s_free[tile]);
-            if (biased) {
-                const float b0 = slope2 * static_cast<float>(key0 - (causal_base + t));   // <= 0 where the key is visible
+            float m_half = -INFINITY;
+            if (any) {
+                if (biased) {
+                    const float b0 = slope2 * static_cast<float>(key0 - (causal_base + t));   // <= 0 where the key is visible
 #pragma unroll
-                for (int c = 0; c < 64; ++c) {
-                    sc[c] = __float_as_uint(fmaf(__uint_as_float(sc[c]), a.scale_log2, fmaf(slope2, static_cast<float>(c), b0)));
+                    for (int c = 0; c < 64; ++c) {
+                        sc[c] = __float_as_uint(fmaf(__uint_as_float(sc[c]), a.scale_log2, fmaf(slope2, static_cast<float>(c), b0)));
+                    }
                 }
-            }
-            // visibility of this thread's 64 keys as one word: causal bound, window bound, tree-mask bits, block selection
-            uint64_t vb = ~0ull;
-            if (!blk_ok || limit <= key0 || row_lo >= key0 + 64) {
-                vb = 0ull;
-            } else {
-                if (limit < key0 + 64) vb &= (1ull << (limit - key0)) - 1ull;
-                if (row_lo > key0) vb &= ~((1ull << (row_lo - key0)) - 1ull);
-                const int mo = mbeg - key0;  // first column the tree mask applies to (mbeg is huge when there is none)
-                if (mo < 64) {
-                    const uint64_t tm = (mo >= 0) ? ((mo > 0 ? (mword << mo) : mword) | ((1ull << mo) - 1ull))
-                                                  : ((-mo < 64) ? (mword >> (-mo)) : 0ull);
-                    vb &= tm;
+                // visibility of this thread's 64 keys as one word: causal bound, window bound, tree-mask bits, block selection
+                uint64_t vb = ~0ull;
+                if (!blk_ok || limit <= key0 || row_lo >= key0 + 64) {
+                    vb = 0ull;
+                } else {
+                    if (limit < key0 + 64) vb &= (1ull << (limit - key0)) - 1ull;
+                    if (row_lo > key0) vb &= ~((1ull << (row_lo - key0)) - 1ull);
+                    const int mo = mbeg - key0;  // first column the tree mask applies to (mbeg is huge when there is none)
+                    if (mo < 64) {
+                        const uint64_t tm = (mo >= 0) ? ((mo > 0 ? (mword << mo) : mword) | ((1ull << mo) - 1ull))
+                                                      : ((-mo < 64) ? (mword >> (-mo)) : 0ull);
+                        vb &= tm;
+                    }
                 }
-            }
-            if (vb != ~0ull) {
+                if (vb != ~0ull) {
 #pragma unroll
-                for (int c = 0; c < 64; ++c) {
-                    if (!((vb >> c) & 1ull)) sc[c] = 0xff800000u;  // -inf
+                    for (int c = 0; c < 64; ++c) {
+                        if (!((vb >> c) & 1ull)) sc[c] = 0xff800000u;  // -inf
+                    }
                 }
-            }
-            float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+                float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-            for (int c = 0; c < 64; c += 8) {
+                for (int c = 0; c < 64; c += 8) {
 #pragma unroll
-                for (int e = 0; e < 4; ++e) mx[e] = fmaxf(mx[e], fmaxf(__uint_as_float(sc[c + e]), __uint_as_float(sc[c + 4 + e])));
+                    for (int e = 0; e < 4; ++e) mx[e] = fmaxf(mx[e], fmaxf(__uint_as_float(sc[c + e]), __uint_as_float(sc[c + 4 + e])));
+                }
+                m_half = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
             }
-            const float m_half = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
             // the buffer of iteration i is written again in i + 2, past the barrier of i + 1
             float* xb = xch + (i & 1) * 2 * ROWS;
             xb[ch * ROWS + row] = m_half;
-            ptx::named_bar_sync(bar_id, TILE_THREADS);
+            ptx::named_bar_sync(bar_id, 64);
             const float m_tile = fmaxf(m_half, xb[(ch ^ 1) * ROWS + row]);
             // lazy running maximum, as in tree_attn_kernel: it moves only for a new one more than 2^8 above it
             float m_new = m_run;
@@ -444,25 +486,34 @@ pair_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                 ptx::tmem_wait_st();
             }
             m_run = m_new;
-            // P = 2^((s - m) * scale) in bf16 into the swizzled A-operand tile; row sums in fp32
-            const float m_off = m_use * sl2;
-            float ls[4] = {0.f, 0.f, 0.f, 0.f};
+            if (any) {
+                // P = 2^((s - m) * scale) in bf16 into the swizzled A-operand tile; row sums in fp32
+                const float m_off = m_use * sl2;
+                float ls[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-            for (int c8 = 0; c8 < 8; ++c8) {
-                uint4 pk;
-                uint32_t* w = reinterpret_cast<uint32_t*>(&pk);
+                for (int c8 = 0; c8 < 8; ++c8) {
+                    uint4 pk;
+                    uint32_t* w = reinterpret_cast<uint32_t*>(&pk);
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float p0 = fast_exp2(fmaf(__uint_as_float(sc[c8 * 8 + 2 * e]), sl2, -m_off));
-                    const float p1 = fast_exp2(fmaf(__uint_as_float(sc[c8 * 8 + 2 * e + 1]), sl2, -m_off));
-                    ls[(2 * e) & 3] += p0;
-                    ls[(2 * e + 1) & 3] += p1;
-                    const __nv_bfloat162 b2 = __floats2bfloat162_rn(p0, p1);
-                    w[e] = *reinterpret_cast<const uint32_t*>(&b2);
+                    for (int e = 0; e < 4; ++e) {
+                        const float p0 = fast_exp2(fmaf(__uint_as_float(sc[c8 * 8 + 2 * e]), sl2, -m_off));
+                        const float p1 = fast_exp2(fmaf(__uint_as_float(sc[c8 * 8 + 2 * e + 1]), sl2, -m_off));
+                        ls[(2 * e) & 3] += p0;
+                        ls[(2 * e + 1) & 3] += p1;
+                        const __nv_bfloat162 b2 = __floats2bfloat162_rn(p0, p1);
+                        w[e] = *reinterpret_cast<const uint32_t*>(&b2);
+                    }
+                    *reinterpret_cast<uint4*>(p_half + ((c8 ^ (row & 7)) << 4)) = pk;
                 }
-                *reinterpret_cast<uint4*>(p_half + ((c8 ^ (row & 7)) << 4)) = pk;
+                l_run = l_run * alpha + ((ls[0] + ls[1]) + (ls[2] + ls[3]));
+            } else {
+                l_run *= alpha;
+                if (!zeros) {
+#pragma unroll
+                    for (int c8 = 0; c8 < 8; ++c8) *reinterpret_cast<uint4*>(p_half + ((c8 ^ (row & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
+                }
             }
-            l_run = l_run * alpha + ((ls[0] + ls[1]) + (ls[2] + ls[3]));
+            if (SPARSE == BY_WORD) zeros = !any;
             ptx::fence_proxy_async_smem();  // P stores -> visible to the tensor core's async proxy
             ptx::tc_fence_before();
             __syncwarp();
@@ -475,7 +526,7 @@ pair_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         // ---- write-out.  TMEM reads are warp-collective, so every thread runs them and only the stores depend on the row.
         float* xb = xch + (n_it & 1) * 2 * ROWS;   // the last maxima went through the other buffer
         xb[ch * ROWS + row] = l_run;
-        ptx::named_bar_sync(bar_id, TILE_THREADS);
+        ptx::named_bar_sync(bar_id, 64);
         float l_row = l_run + xb[(ch ^ 1) * ROWS + row];
         if (BIASED && a.sink != 0 && m_run != -INFINITY) l_row += exp2f(-m_run * sl2);
         if (ok) {
@@ -530,21 +581,24 @@ pair_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     if (tid == 0 && *abort_flag) atomicOr(a.error, ERR_ATTN_TIMEOUT);
 }
 
-template <int DK, int DV, bool BIASED>
+template <int DK, int DV, bool BIASED, int SPARSE = DENSE>
 void launch(const AttnPlan& p, const AttnArgs& a, cudaStream_t s) {
     static bool configured = false;
     if (!configured) {
-        CUDA_CHECK(cudaFuncSetAttribute(pair_attn_kernel<DK, DV, BIASED>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<DK, DV>::SMEM_TOTAL));
+        CUDA_CHECK(cudaFuncSetAttribute(pair_attn_kernel<DK, DV, BIASED, SPARSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<DK, DV>::SMEM_TOTAL));
         configured = true;
     }
-    launch_kernel(pair_attn_kernel<DK, DV, BIASED>, dim3(ceil_div(a.num_mtiles, 2) * p.hkv), dim3(PAIR_THREADS), PairCfg<DK, DV>::SMEM_TOTAL, s,
+    launch_kernel(pair_attn_kernel<DK, DV, BIASED, SPARSE>, dim3(ceil_div(a.num_mtiles, 2) * p.hkv), dim3(PAIR_THREADS), PairCfg<DK, DV>::SMEM_TOTAL, s,
                   p.tm_q, p.tm_k, p.tm_v, a);
 }
 
 }  // namespace
 
 void launch_pair_attention(const AttnPlan& p, const AttnArgs& a, cudaStream_t s) {
-    if (!p.biased) launch<128, 128, false>(p, a, s);
+    CPM_REQUIRE(!p.biased || p.blockmask == nullptr, "attention: a block mask needs an unbiased plan");
+    if (!p.biased && p.blockmask == nullptr) launch<128, 128, false>(p, a, s);
+    else if (!p.biased && 2 * a.tok_per_tile <= 32) launch<128, 128, false, BY_WORD>(p, a, s);
+    else if (!p.biased) launch<128, 128, false, BY_ROW>(p, a, s);
     else if (p.d == 128 && p.dv == 128) launch<128, 128, true>(p, a, s);
     else if (p.d == 128) launch<128, 64, true>(p, a, s);
     else if (p.dv == 128) launch<64, 128, true>(p, a, s);
