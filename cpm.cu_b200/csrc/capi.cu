@@ -425,6 +425,28 @@ int cpmcu_linear_bf16(const void* x, const void* w, const void* bias, void* y, i
     });
 }
 
+int cpmcu_qkv_rope_row(const void* x, const void* w, int K, int hq, int hkv, const float* inv_freq, const int32_t* pos, const int32_t* kv_len,
+                       int kv_off, const int32_t* n_valid, int cache_rows, void* q, void* k_cache, void* v_cache) {
+    return guarded([&] {
+        Runtime& rt = runtime();
+        const int N = (hq + 2 * hkv) * 128;
+        DeviceBuf wt(linear_weight_elems(N, K) * sizeof(bf16));
+        retile_weight_rows(w, N, K, static_cast<bf16*>(wt.p), K, 0, 0, 0, rt.stream);
+        LinearPlan p = make_linear_plan(static_cast<const bf16*>(x), 1, static_cast<const bf16*>(wt.p), 1, N, K, static_cast<bf16*>(q), N, nullptr,
+                                        nullptr, nullptr, rt.num_sms);
+        CPM_REQUIRE(p.one_row, "qkv_rope_row: a row of this size is computed as tiles");
+        RopeRow r;
+        r.hq = hq; r.hkv = hkv;
+        r.inv_freq = inv_freq; r.pos = pos;
+        r.k_cache = static_cast<bf16*>(k_cache); r.v_cache = static_cast<bf16*>(v_cache);
+        r.kv_len = kv_len; r.kv_off = kv_off; r.n_valid = n_valid; r.cache_rows = cache_rows;
+        r.error = rt.d_error;
+        launch_linear_one_row(p, rt.stream, &r);
+        sync_and_check("qkv_rope_row");
+        return 0;
+    });
+}
+
 int cpmcu_debug_linear_schedule(int M, int N, int K, int grid_limit, int32_t* out, int cap) {
     int n = -1;
     const int rc = guarded([&] {

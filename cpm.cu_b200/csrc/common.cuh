@@ -246,7 +246,21 @@ bool linear_swiglu_fits(int M, int inter, int grid_limit);
 LinearPlan make_linear_swiglu_plan(const bf16* x, int x_rows, const bf16* w, int M, int inter, int K, bf16* act, int ld,
                                    int grid_limit);
 void launch_linear(const LinearPlan& plan, cudaStream_t stream);
-void launch_linear_one_row(const LinearPlan& plan, cudaStream_t stream);   // M == 1, bf16 weights
+// Where the query, key and value of one row go (head width 128): what launch_rope_append does for it
+struct RopeRow {
+    int hq = 0, hkv = 0;
+    const float* inv_freq = nullptr;
+    const int32_t *pos = nullptr, *pos_base = nullptr;   // *pos, or *pos_base + pos_off
+    int pos_off = 0;
+    bf16 *k_cache = nullptr, *v_cache = nullptr;
+    const int32_t* kv_len = nullptr;
+    int kv_off = 0;
+    const int32_t* n_valid = nullptr;
+    int cache_rows = 0;
+    int* error = nullptr;
+};
+// M == 1, bf16 weights; with `rope` the product is q, k and v, which are rotated and appended
+void launch_linear_one_row(const LinearPlan& plan, cudaStream_t stream, const RopeRow* rope = nullptr);
 bool linear_one_row_fits(int N, int K, int sms);   // whether that is the faster way for one row of N outputs
 // Same contract with 4-bit weights, w = (q - 8) * scale, K % 256 == 0 and N % 128 == 0.  `wq` holds one
 // contiguous 16896-byte block per (128-feature tile, 256-k unit), tile-major: [4 k-blocks][2 halves]

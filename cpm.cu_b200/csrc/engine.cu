@@ -536,9 +536,22 @@ void Engine::layer_forward(LayerPlans& lp, const LayerWeights& w, const KVLayer&
         if (pending) launch_add_scaled(x, x, pending, pending_scale, rows, H, s);
         // (only the draft layer runs without a first norm; its q/k/v plan reads x directly: build_draft_plans)
     }
-    launch_linear(lp.qkv, s);
-    launch_rope_append(qkv_, rows, mc_.hq, mc_.hkv, mc_.head_dim, inv_freq_, c.pos, c.pos_base, c.pos_off, c.pos_step,
-                       kv.k, kv.v, c.kv_len, c.kv_append_off, c.n_valid, budget_, s);
+    if (lp.qkv.one_row) {   // a single row is rotated and appended where its product ends
+        RopeRow r;
+        r.hq = mc_.hq; r.hkv = mc_.hkv;
+        r.inv_freq = inv_freq_;
+        r.pos = c.pos; r.pos_base = c.pos_base; r.pos_off = c.pos_off;
+        r.k_cache = kv.k; r.v_cache = kv.v;
+        r.kv_len = c.kv_len; r.kv_off = c.kv_append_off; r.n_valid = c.n_valid;
+        r.cache_rows = budget_;
+        r.error = runtime().d_error;
+        ProfileScope prof(KC_LINEAR, s);
+        launch_linear_one_row(lp.qkv, s, &r);
+    } else {
+        launch_linear(lp.qkv, s);
+        launch_rope_append(qkv_, rows, mc_.hq, mc_.hkv, mc_.head_dim, inv_freq_, c.pos, c.pos_base, c.pos_off, c.pos_step,
+                           kv.k, kv.v, c.kv_len, c.kv_append_off, c.n_valid, budget_, s);
+    }
     lp.attn.kv_len = c.kv_len;
     lp.attn.kv_len_add = c.attn_kv_add;
     lp.attn.n_valid = c.n_valid;

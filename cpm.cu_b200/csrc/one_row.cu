@@ -32,6 +32,7 @@ struct OneRowArgs {
     const int32_t* n_entries;
     int uniform;                     // > 0: matrix i has row i of x and y
     float gate_limit, gate_alpha;
+    RopeRow rope;                    // ROPE
 };
 
 // A plain load that the compiler keeps in its place, not a read-only one: with ld.global.nc a product's first loads did not run beside its
@@ -43,11 +44,15 @@ __device__ __forceinline__ uint4 load_stream(const bf16* p) {
 }
 __device__ __forceinline__ f32x2 widen(uint32_t two) { return pair(__uint_as_float(two << 16), __uint_as_float(two & 0xffff0000u)); }
 
-// PAIR: the rows are R / 2 gate rows and the R / 2 up rows of the same features (64 + 64 in a tile).  EARLY: the router's
-// choice may be read before the wait for the predecessor.
-template <int R, bool PAIR, bool EARLY>
+// PLAIN, GATED: the rows are R / 2 gate rows and the R / 2 up rows of the same features (64 + 64 in a tile), ROPE: a tile is a head of 128, the
+// rows are R / 2 of its lower half and their partners of the upper half; queries are rotated, keys rotated and values copied into the cache.
+enum Epilogue { PLAIN, GATED, ROPE };
+// Rotation and append as a launch of their own cost 1.7 us a layer (8 layers of 2048: 418 us a pass, 410 with them here).
+// EARLY: the router's choice may be read before the wait for the predecessor.
+template <int R, Epilogue EPI, bool EARLY>
 __global__ void __launch_bounds__(ONE_WARPS * 32, 4)
 one_row_kernel(const OneRowArgs a) {
+    constexpr bool PAIR = EPI != PLAIN;
     constexpr int LOADS = R / 4;                       // per lane and k-block
     constexpr int U = 8 / LOADS;                       // k-blocks per batch
     __shared__ float part[ONE_WARPS][R];
@@ -93,6 +98,12 @@ one_row_kernel(const OneRowArgs a) {
         if (!EARLY) grid_dep_trigger();
     }
     if (!there) return;
+    int pos = 0, kv_len = 0, valid = 1;
+    if (EPI == ROPE && threadIdx.x < R / 2) {   // here before the sums are
+        pos = a.rope.pos != nullptr ? *a.rope.pos : *a.rope.pos_base + a.rope.pos_off;
+        kv_len = *a.rope.kv_len;
+        if (a.rope.n_valid != nullptr) valid = *a.rope.n_valid;
+    }
     const bf16* x = (shared ? a.xs + static_cast<size_t>(a.xs_row) * a.ldx
                             : a.x + static_cast<size_t>(a.uniform > 0 || PAIR ? e.y : e.z) * a.ldx) + (lane & 7) * 8;
     f32x2 acc[LOADS];
@@ -128,12 +139,38 @@ one_row_kernel(const OneRowArgs a) {
     }
     __syncthreads();
     const int t = threadIdx.x;
-    if (t >= (PAIR ? R / 2 : R) || first + t >= N) return;
+    if (t >= (PAIR ? R / 2 : R) || first + t >= (EPI == ROPE ? N / 2 : N)) return;
     float sum = 0.f, up = 0.f;
 #pragma unroll
     for (int k = 0; k < ONE_WARPS; ++k) {
         sum += part[k][t];
         if (PAIR) up += part[k][(R / 2 + t) % R];
+    }
+    if (EPI == ROPE) {
+        // rounded to bf16 before the rotation, as where the product is stored in between
+        const int f = r0 + t;
+        const long long kv_row = static_cast<long long>(kv_len) + a.rope.kv_off;
+        float lo = __bfloat162float(__float2bfloat16(sum)), hi = __bfloat162float(__float2bfloat16(up));
+        if (tile < a.rope.hq + a.rope.hkv) {
+            float sn, cs;
+            sincosf(pos * a.rope.inv_freq[f], &sn, &cs);
+            const float x0 = lo, x1 = hi;
+            lo = x0 * cs - x1 * sn;
+            hi = x0 * sn + x1 * cs;
+        }
+        bf16* dst = a.y + tile * 128 + f;
+        if (tile >= a.rope.hq) {
+            if (valid < 1 || kv_row < 0) return;
+            if (kv_row >= a.rope.cache_rows) {   // host-side length checks come first; this only keeps memory intact
+                atomicOr(a.rope.error, ERR_KV_OVERFLOW);
+                return;
+            }
+            const int kv_dim = a.rope.hkv * 128, h = tile - a.rope.hq;
+            dst = (h < a.rope.hkv ? a.rope.k_cache + h * 128 : a.rope.v_cache + (h - a.rope.hkv) * 128) + kv_row * kv_dim + f;
+        }
+        dst[0] = __float2bfloat16(lo);
+        dst[64] = __float2bfloat16(hi);
+        return;
     }
     if (PAIR) {
         // both projections are rounded to bf16 before silu's product, as where they are stored in between
@@ -171,17 +208,17 @@ bool linear_one_row_fits(int N, int K, int sms) {
 
 namespace {
 
-template <bool PAIR, bool EARLY>
+template <Epilogue EPI, bool EARLY>
 void launch(int R, const OneRowArgs& a, int grid, cudaStream_t s) {
     switch (R) {
-        case 8: launch_kernel(one_row_kernel<8, PAIR, EARLY>, dim3(grid), dim3(ONE_WARPS * 32), 0, s, a); break;
-        default: launch_kernel(one_row_kernel<16, PAIR, EARLY>, dim3(grid), dim3(ONE_WARPS * 32), 0, s, a); break;
+        case 8: launch_kernel(one_row_kernel<8, EPI, EARLY>, dim3(grid), dim3(ONE_WARPS * 32), 0, s, a); break;
+        default: launch_kernel(one_row_kernel<16, EPI, EARLY>, dim3(grid), dim3(ONE_WARPS * 32), 0, s, a); break;
     }
 }
 
 }  // namespace
 
-void launch_linear_one_row(const LinearPlan& p, cudaStream_t s) {
+void launch_linear_one_row(const LinearPlan& p, cudaStream_t s, const RopeRow* rope) {
     OneRowArgs a = {};
     a.w = p.w; a.x = p.x; a.y = p.y; a.bias = p.bias;
     a.N = p.N; a.kblocks = p.K / BLOCK_COLS;
@@ -190,8 +227,15 @@ void launch_linear_one_row(const LinearPlan& p, cudaStream_t s) {
     a.gate_limit = p.gate_limit; a.gate_alpha = p.gate_alpha;
     const int R = rows_per_cta(p.swiglu ? 2LL * p.N : p.N, a.kblocks);
     a.ctas = ceil_div(p.N, p.swiglu ? R / 2 : R);
-    if (p.swiglu) launch<true, true>(R, a, a.ctas, s);
-    else launch<false, true>(R, a, a.ctas, s);
+    if (rope != nullptr) {
+        CPM_REQUIRE(!p.swiglu && p.N == (rope->hq + 2 * rope->hkv) * 128, "one row: a rotated product is that of queries, keys and values of heads of 128");
+        a.rope = *rope;
+        launch<ROPE, true>(R, a, a.ctas, s);
+    } else if (p.swiglu) {
+        launch<GATED, true>(R, a, a.ctas, s);
+    } else {
+        launch<PLAIN, true>(R, a, a.ctas, s);
+    }
 }
 
 void launch_moe_one_row(const MoeGemmPlan& p, cudaStream_t s) {
@@ -208,6 +252,6 @@ void launch_moe_one_row(const MoeGemmPlan& p, cudaStream_t s) {
     a.ctas_s = p.n_tiles_s > 0 ? ceil_div(p.N_s, R / per) : 0;
     const int grid = a.ctas_s + p.max_entries * a.ctas;
     // the router's choice: gate/up waits for it and lets its successor start only then, so down may read it at once
-    if (p.swiglu) launch<true, false>(R, a, grid, s);
-    else launch<false, true>(R, a, grid, s);
+    if (p.swiglu) launch<GATED, false>(R, a, grid, s);
+    else launch<PLAIN, true>(R, a, grid, s);
 }

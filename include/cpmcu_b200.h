@@ -312,6 +312,11 @@ int cpmcu_rms_norm(void* x, const void* delta, float delta_scale, const void* we
 int cpmcu_rope_append(void* qkv, int rows, int hq, int hkv, const float* inv_freq, const int32_t* pos,
                       void* k_cache, void* v_cache, const int32_t* kv_len, int kv_off);
 
+/* One token row: the q, k, v product (w [(hq+2hkv)*128, K] row-major) and what cpmcu_rope_append does with it, in one launch; q
+ * [hq*128], the caches hold cache_rows rows, n_valid (device, may be null) 0 = no cache row is written. */
+int cpmcu_qkv_rope_row(const void* x, const void* w, int K, int hq, int hkv, const float* inv_freq, const int32_t* pos, const int32_t* kv_len,
+                       int kv_off, const int32_t* n_valid, int cache_rows, void* q, void* k_cache, void* v_cache);
+
 /* reference: gated_silu_interleaved, src/model/activation.cuh:7-18. */
 int cpmcu_silu_gate(const void* gate_up, void* out, int rows, int inter);
 
