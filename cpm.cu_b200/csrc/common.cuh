@@ -259,8 +259,14 @@ struct RopeRow {
     int cache_rows = 0;
     int* error = nullptr;
 };
-// M == 1, bf16 weights; with `rope` the product is q, k and v, which are rotated and appended
-void launch_linear_one_row(const LinearPlan& plan, cudaStream_t stream, const RopeRow* rope = nullptr);
+// The token side input of one row: y = gelu_tanh(product) * table[*ids][col0 ..]
+struct SideRow {
+    const int32_t* ids = nullptr;
+    const bf16* table = nullptr;
+    int table_ld = 0, col0 = 0, vocab = 0;
+};
+// M == 1, bf16 weights; with `rope` the product is q, k and v, which are rotated and appended; with `side` the side input's gate
+void launch_linear_one_row(const LinearPlan& plan, cudaStream_t stream, const RopeRow* rope = nullptr, const SideRow* side = nullptr);
 bool linear_one_row_fits(int N, int K, int sms);   // whether that is the faster way for one row of N outputs
 // Same contract with 4-bit weights, w = (q - 8) * scale, K % 256 == 0 and N % 128 == 0.  `wq` holds one
 // contiguous 16896-byte block per (128-feature tile, 256-k unit), tile-major: [4 k-blocks][2 halves]

@@ -679,28 +679,30 @@ bool Engine::layered_tanh_layer(int i, LayeredPlans& lp, const int32_t* ids, con
     const bool next = i + 1 < layers && mc_.side_dim > 0 && (rows == 1 || mc_.specs[i + 1].rec != REC_TIME_MIX);
     const DynTanh next_norm = next ? lw_[i + 1].tanh1 : DynTanh();
     const TokenShift next_shift = next ? token_shift(i + 1, rows, kv_len, kv_off) : TokenShift();
-    const bool side_step = rows == 1 && mc_.side_dim > 0 && mc_.side_dim <= 4096;
     if (sp.ff > 0) {
         launch_tanh_residual<T>(x32_, delta, w.tanh1b, w.tanh2, x, rows, L, s);
         layered_dense<T>(i, lp, s);
     }
     const DynTanh& last = sp.ff > 0 ? w.tanh2b : w.tanh1b;
-    if (side_step) {
-        SideStepArgs a;
-        a.x32 = x32_; a.delta = ldelta_;
-        a.post = last;
-        a.gate = w.side_gate; a.proj = w.side_proj; a.norm = w.side_norm;
-        a.ids = ids; a.table = side_embed_; a.table_ld = layers * mc_.side_dim; a.col0 = i * mc_.side_dim;
-        a.dim = mc_.side_dim; a.vocab = mc_.vocab;
-        a.next = next_norm; a.h = lx_; a.shift = next_shift;
-        a.width = W; a.ld = L; a.eps = mc_.eps;
-        launch_side_step<T>(a, s);
-        return next;
-    }
     launch_tanh_residual<T>(x32_, delta, last, DynTanh(), x, rows, L, s);
     if (mc_.side_dim == 0) return false;
-    run_product<T>(l.side_gate, rows, s);
-    launch_side_gate<T>(static_cast<const T*>(lside_), pad64(mc_.side_dim), ids, side_embed_, layers * mc_.side_dim, i * mc_.side_dim, mc_.side_dim,
+    bool gated = false;
+    if constexpr (sizeof(T) == 2) {
+        // A single row: residual sum, two products and the sum with norm and mixes are four launches of 1.3 to 3 us that start beside one
+        // another's ends.  One cluster of 16 CTAs with four dependent phases took 15.5 us a layer of width 3072 (24 tokens of
+        // nine layers 31.2 -> 29.8 ms; four layers of 4096 14.0 -> 13.2 ms over 40 tokens, of 2048 8.9 -> 8.6, of 512 7.2 and 7.3).
+        if (rows == 1 && l.side_gate.plan.one_row) {   // gated where the product ends
+            LinearPlan gate = l.side_gate.plan;
+            gate.y = static_cast<bf16*>(lsg_);
+            SideRow side;
+            side.ids = ids; side.table = side_embed_; side.table_ld = layers * mc_.side_dim; side.col0 = i * mc_.side_dim; side.vocab = mc_.vocab;
+            ProfileScope prof(KC_LINEAR, s);
+            launch_linear_one_row(gate, s, nullptr, &side);
+            gated = true;
+        }
+    }
+    if (!gated) run_product<T>(l.side_gate, rows, s);
+    if (!gated) launch_side_gate<T>(static_cast<const T*>(lside_), pad64(mc_.side_dim), ids, side_embed_, layers * mc_.side_dim, i * mc_.side_dim, mc_.side_dim,
                         mc_.vocab, static_cast<T*>(lsg_), rows, s);
     run_product<T>(l.side_proj, rows, s);
     launch_side_add<T>(x32_, delta, w.side_norm, next_norm, x, next_shift, rows, W, L, mc_.eps, s);

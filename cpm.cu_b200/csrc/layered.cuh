@@ -136,24 +136,6 @@ void launch_side_gate(const T* z, int ld, const int32_t* ids, const bf16* table,
 template <typename T>
 void launch_side_add(float* x32, const T* y, const bf16* w, const DynTanh& next, T* h, const TokenShift& shift, int rows, int width, int ld,
                      float eps, cudaStream_t s);
-// A single row from a sublayer's output to the next layer's input in one launch: x32 += post(delta), then the token side input
-// (gate product, launch_side_gate, projection, launch_side_add).  The two matrices are tile-major for bf16, row-major for fp32.
-struct SideStepArgs {
-    float* x32 = nullptr;
-    const void* delta = nullptr;
-    DynTanh post;
-    const bf16 *gate = nullptr, *proj = nullptr, *norm = nullptr;
-    const int32_t* ids = nullptr;
-    const bf16* table = nullptr;
-    int table_ld = 0, col0 = 0, dim = 0, vocab = 0;
-    DynTanh next;
-    void* h = nullptr;
-    TokenShift shift;
-    int width = 0, ld = 0;
-    float eps = 0.f;
-};
-template <typename T>
-void launch_side_step(const SideStepArgs& a, cudaStream_t s);
 // dst [cols][rows] = src [rows][cols], host or device memory
 void upload_transposed(const void* src, int rows, int cols, bf16* dst, cudaStream_t s);
 // Decays of a time-mix layer: out[r][c] = exp(-exp(sum_k w2[k][c] tanh(x[r][k]) + w0[c])), c < channels; x: `rank` columns of

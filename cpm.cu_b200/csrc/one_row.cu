@@ -33,6 +33,7 @@ struct OneRowArgs {
     int uniform;                     // > 0: matrix i has row i of x and y
     float gate_limit, gate_alpha;
     RopeRow rope;                    // ROPE
+    SideRow side;                    // SIDE
 };
 
 // A plain load that the compiler keeps in its place, not a read-only one: with ld.global.nc a product's first loads did not run beside its
@@ -46,13 +47,14 @@ __device__ __forceinline__ f32x2 widen(uint32_t two) { return pair(__uint_as_flo
 
 // PLAIN, GATED: the rows are R / 2 gate rows and the R / 2 up rows of the same features (64 + 64 in a tile), ROPE: a tile is a head of 128, the
 // rows are R / 2 of its lower half and their partners of the upper half; queries are rotated, keys rotated and values copied into the cache.
-enum Epilogue { PLAIN, GATED, ROPE };
+// SIDE: the output is gated into the token's side input.
+enum Epilogue { PLAIN, GATED, ROPE, SIDE };
 // Rotation and append as a launch of their own cost 1.7 us a layer (8 layers of 2048: 418 us a pass, 410 with them here).
 // EARLY: the router's choice may be read before the wait for the predecessor.
 template <int R, Epilogue EPI, bool EARLY>
 __global__ void __launch_bounds__(ONE_WARPS * 32, 4)
 one_row_kernel(const OneRowArgs a) {
-    constexpr bool PAIR = EPI != PLAIN;
+    constexpr bool PAIR = EPI == GATED || EPI == ROPE;
     constexpr int LOADS = R / 4;                       // per lane and k-block
     constexpr int U = 8 / LOADS;                       // k-blocks per batch
     __shared__ float part[ONE_WARPS][R];
@@ -106,6 +108,12 @@ one_row_kernel(const OneRowArgs a) {
     }
     const bf16* x = (shared ? a.xs + static_cast<size_t>(a.xs_row) * a.ldx
                             : a.x + static_cast<size_t>(a.uniform > 0 || PAIR ? e.y : e.z) * a.ldx) + (lane & 7) * 8;
+    float side = 0.f;
+    if (EPI == SIDE && threadIdx.x < R && first + static_cast<int>(threadIdx.x) < N) {
+        int id = *a.side.ids;
+        if (id < 0 || id >= a.side.vocab) id = 0;   // reported by the embedding
+        side = __bfloat162float(a.side.table[static_cast<size_t>(id) * a.side.table_ld + a.side.col0 + first + threadIdx.x]);
+    }
     f32x2 acc[LOADS];
 #pragma unroll
     for (int i = 0; i < LOADS; ++i) acc[i] = 0;
@@ -176,6 +184,8 @@ one_row_kernel(const OneRowArgs a) {
         // both projections are rounded to bf16 before silu's product, as where they are stored in between
         sum = a.gate_limit > 0.f ? clamped_gate(sum, up, a.gate_limit, a.gate_alpha)
                                  : silu_mul(__bfloat162float(__float2bfloat16(sum)), __bfloat162float(__float2bfloat16(up)));
+    } else if (EPI == SIDE) {
+        sum = gelu_tanh(__bfloat162float(__float2bfloat16(sum))) * side;
     } else if (a.bias != nullptr) {
         sum += __bfloat162float(a.bias[first + t]);
     }
@@ -218,7 +228,7 @@ void launch(int R, const OneRowArgs& a, int grid, cudaStream_t s) {
 
 }  // namespace
 
-void launch_linear_one_row(const LinearPlan& p, cudaStream_t s, const RopeRow* rope) {
+void launch_linear_one_row(const LinearPlan& p, cudaStream_t s, const RopeRow* rope, const SideRow* side) {
     OneRowArgs a = {};
     a.w = p.w; a.x = p.x; a.y = p.y; a.bias = p.bias;
     a.N = p.N; a.kblocks = p.K / BLOCK_COLS;
@@ -231,6 +241,10 @@ void launch_linear_one_row(const LinearPlan& p, cudaStream_t s, const RopeRow* r
         CPM_REQUIRE(!p.swiglu && p.N == (rope->hq + 2 * rope->hkv) * 128, "one row: a rotated product is that of queries, keys and values of heads of 128");
         a.rope = *rope;
         launch<ROPE, true>(R, a, a.ctas, s);
+    } else if (side != nullptr) {
+        CPM_REQUIRE(!p.swiglu && p.bias == nullptr, "one row: a side input's gate is a plain product");
+        a.side = *side;
+        launch<SIDE, true>(R, a, a.ctas, s);
     } else if (p.swiglu) {
         launch<GATED, true>(R, a, a.ctas, s);
     } else {

@@ -69,6 +69,9 @@ __device__ __forceinline__ float2 block_sum2(float a, float b, float* sh) {
 // asks for the cache line at p ahead of its use (weights, before the wait for the previous kernel)
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
+__device__ __forceinline__ float gelu_tanh(float z) {
+    return 0.5f * z * (1.f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
+}
 __device__ __forceinline__ float silu_f32(float v) { return v / (1.f + expf(-v)); }
 // of a value that is known to bf16 precision only: the approximate exponential and division are far finer than that
 __device__ __forceinline__ float silu_fast(float v) { return __fdividef(v, 1.f + __expf(-v)); }

@@ -112,10 +112,6 @@ __global__ void clamped_gate_kernel(const T* __restrict__ gu, int ld_gu, T* __re
     }
 }
 
-__device__ __forceinline__ float gelu_tanh(float z) {
-    return 0.5f * z * (1.f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
-}
-
 template <typename T>
 __global__ void side_gate_kernel(const T* __restrict__ z, int ld, const int32_t* __restrict__ ids, const bf16* __restrict__ table, int table_ld,
                                  int col0, int dim, int vocab, T* __restrict__ g) {
@@ -167,164 +163,6 @@ side_add_kernel(float* __restrict__ x32, const T* __restrict__ y, const bf16* __
             store_vec<8>(t.prev + c, h);
         }
     }
-}
-
-// ---------------------------------------------------------------- one row through the token side input
-constexpr int SIDE_CTAS = 16, SIDE_THREADS = 512;   // at most; a cluster of 16 is above the portable size
-
-// element (row, k) of a matrix with K columns: tile-major (linear_weight_elems) or row-major
-template <typename T>
-__device__ __forceinline__ size_t weight_at(int row, int k, int K) {
-    if constexpr (sizeof(T) == 2) {
-        return (static_cast<size_t>(row >> 7) * (K >> 6) + (k >> 6)) * (128 * 64) + static_cast<size_t>(row & 127) * 64 + (k & 63);
-    } else {
-        return static_cast<size_t>(row) * K + k;
-    }
-}
-
-// One cluster of SIDE_CTAS CTAs.  Every CTA takes the residual sum of the whole row; it computes its share of the gate's rows,
-// which go to all CTAs, then its share of the projection's rows = columns of the stream.
-template <typename T>
-__global__ void __launch_bounds__(SIDE_THREADS)
-side_step_kernel(const SideStepArgs a) {
-    extern __shared__ __align__(16) float sm[];
-    __shared__ float sh[64];
-    __shared__ float s_sum[SIDE_CTAS];
-    const int dim_p = (a.dim + 63) / 64 * 64;
-    float* xs = sm;                // [ld] the stream
-    float* sg = xs + a.ld;         // [dim_p] gated side input
-    float* ys = sg + dim_p;        // this CTA's columns of the projection
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int rank = static_cast<int>(ptx::cluster_ctarank());
-    const int ctas = gridDim.x;
-    const int whole = (a.ld / 8 + ctas - 1) / ctas * 8, col0 = min(rank * whole, a.ld), share = min(whole, a.ld - col0);
-    const int per = (a.dim + ctas - 1) / ctas, g0 = rank * per, g1 = min(g0 + per, a.dim);
-    grid_dep_trigger();
-    {
-        const int kb = a.ld / 64, lines = max(g1 - g0, 0) * kb;
-        for (int i = tid; i < lines; i += SIDE_THREADS) prefetch_l2(a.gate + weight_at<T>(g0 + i / kb, (i % kb) * 64, a.ld));
-        const int pb = dim_p / 64, plines = max(min(share, a.width - col0), 0) * pb;
-        for (int i = tid; i < plines; i += SIDE_THREADS) prefetch_l2(a.proj + weight_at<T>(col0 + i / pb, (i % pb) * 64, dim_p));
-        for (int c = tid * 64; c < a.ld; c += SIDE_THREADS * 64) {
-            prefetch_l2(a.post.w + c);
-            prefetch_l2(a.post.b + c);
-        }
-    }
-    for (int k = tid; k < dim_p; k += SIDE_THREADS) sg[k] = 0.f;
-    // what this thread's columns need at the end (all weights, and the mixer input of the step before, which the host has waited for)
-    const int mine = col0 + tid * 8;
-    const bool has = tid * 8 < share;
-    uint4 w_norm, w_next, b_next, w_mu[kMixes];
-    float prev[8];
-    w_norm = w_next = b_next = make_uint4(0, 0, 0, 0);
-#pragma unroll
-    for (int m = 0; m < kMixes; ++m) w_mu[m] = make_uint4(0, 0, 0, 0);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) prev[e] = 0.f;
-    if (has) {
-        w_norm = *reinterpret_cast<const uint4*>(a.norm + mine);
-        if (a.next.w != nullptr) {
-            w_next = *reinterpret_cast<const uint4*>(a.next.w + mine);
-            b_next = *reinterpret_cast<const uint4*>(a.next.b + mine);
-        }
-        if (a.shift.mu != nullptr) {
-#pragma unroll
-            for (int m = 0; m < kMixes; ++m) w_mu[m] = *reinterpret_cast<const uint4*>(a.shift.mu + static_cast<size_t>(m) * a.ld + mine);
-            load_vec<8>(a.shift.prev + mine, prev);
-        }
-    }
-    grid_dep_wait();
-    for (int c = tid * 8; c < a.ld; c += SIDE_THREADS * 8) {
-        float x[8], d[8], y[8];
-        load_vec<8>(a.x32 + c, x);
-        load_vec<8>(static_cast<const T*>(a.delta) + c, d);
-        tanh_norm8(d, a.post, c, y);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) x[e] += y[e];
-        store_vec<8>(xs + c, x);
-    }
-    int id = a.ids[0];
-    if (id < 0 || id >= a.vocab) id = 0;   // reported by the embedding
-    const bf16* side = a.table + static_cast<size_t>(id) * a.table_ld + a.col0;
-    ptx::cluster_sync();   // xs here; sg zeroed in every CTA
-    for (int row = g0 + warp; row < g1; row += SIDE_THREADS / 32) {
-        float z = 0.f;
-#pragma unroll 8
-        for (int k = lane * 8; k < a.ld; k += 256) {
-            float w[8], x[8];
-            load_vec<8>(a.gate + weight_at<T>(row, k, a.ld), w);
-            load_vec<8>(xs + k, x);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) z = fmaf(w[e], to_float<T>(from_float<T>(x[e])), z);
-        }
-        z = to_float<T>(from_float<T>(warp_sum(z)));
-        const float g = to_float<T>(from_float<T>(gelu_tanh(z) * __bfloat162float(side[row])));
-        if (lane < ctas) ptx::st_cluster_f32(ptx::cluster_map(ptx::smem_u32(sg + row), lane), g);
-    }
-    ptx::cluster_sync();
-    int lpr = 8;           // lanes per row of the projection
-    while (lpr < 32 && lpr * 8 < dim_p) lpr *= 2;
-    const int sub = lane / lpr, sl = lane % lpr, rpw = 32 / lpr;
-    float ss = 0.f;
-    constexpr int B = 8;   // rows in flight per group of lanes
-    for (int r0 = warp * rpw * B; r0 < share; r0 += SIDE_THREADS / 32 * rpw * B) {   // uniform within a warp
-        float y[B] = {};
-        for (int k = sl * 8; k < dim_p; k += lpr * 8) {
-            float g[8];
-            load_vec<8>(sg + k, g);
-            uint4 w[B];
-#pragma unroll
-            for (int n = 0; n < B; ++n) {
-                const int r = r0 + n * rpw + sub;
-                w[n] = make_uint4(0, 0, 0, 0);
-                if (r < share && col0 + r < a.width) w[n] = __ldg(reinterpret_cast<const uint4*>(a.proj + weight_at<T>(col0 + r, k, dim_p)));
-            }
-#pragma unroll
-            for (int n = 0; n < B; ++n) {
-                const bf16* e8 = reinterpret_cast<const bf16*>(&w[n]);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) y[n] = fmaf(__bfloat162float(e8[e]), g[e], y[n]);
-            }
-        }
-#pragma unroll
-        for (int n = 0; n < B; ++n) {
-            for (int o = lpr / 2; o > 0; o >>= 1) y[n] += __shfl_xor_sync(0xffffffffu, y[n], o);
-            y[n] = to_float<T>(from_float<T>(y[n]));
-            const int r = r0 + n * rpw + sub;
-            if (sl == 0 && r < share) {
-                ys[r] = y[n];
-                ss += y[n] * y[n];
-            }
-        }
-    }
-    ss = block_sum2(ss, 0.f, sh).x;
-    if (tid < ctas) ptx::st_cluster_f32(ptx::cluster_map(ptx::smem_u32(s_sum + rank), tid), ss);
-    ptx::cluster_sync();
-    float sum = 0.f;
-    for (int i = 0; i < ctas; ++i) sum += s_sum[i];
-    const float rs = rsqrtf(sum / a.width + a.eps);
-    if (!has) return;   // share <= 8 * SIDE_THREADS
-    auto bf8 = [](const uint4& u, int e) { return __bfloat162float(reinterpret_cast<const bf16*>(&u)[e]); };
-    float x[8], y[8], h[8];
-    load_vec<8>(xs + mine, x);
-    load_vec<8>(ys + tid * 8, y);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) x[e] += y[e] * rs * bf8(w_norm, e);
-    store_vec<8>(a.x32 + mine, x);
-    if (a.next.w == nullptr) return;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) h[e] = tanh_norm(x[e], a.next.alpha, bf8(w_next, e), bf8(b_next, e));
-    store_vec<8>(static_cast<T*>(a.h) + mine, h);
-    if (a.shift.mu == nullptr) return;
-    const bool first = *a.shift.kv_len + a.shift.kv_off == 0;
-#pragma unroll
-    for (int m = 0; m < kMixes; ++m) {
-        float f[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) f[e] = h[e] + ((first ? 0.f : prev[e]) - h[e]) * bf8(w_mu[m], e);
-        store_vec<8>(static_cast<T*>(a.shift.out) + m * a.shift.stride + mine, f);
-    }
-    store_vec<8>(a.shift.prev + mine, h);
 }
 
 // ROWS tokens x 256 channels per CTA, two neighbouring channels per thread.
@@ -520,23 +358,6 @@ void launch_side_add(float* x32, const T* y, const bf16* w, const DynTanh& next,
     if (vecs <= 512) launch_kernel(side_add_kernel<T, 1>, dim3(rows), dim3(threads), 0, s, x32, y, w, next, h, shift, width, ld, eps);
     else launch_kernel(side_add_kernel<T, 4>, dim3(rows), dim3(threads), 0, s, x32, y, w, next, h, shift, width, ld, eps);
 }
-
-template <typename T>
-void launch_side_step(const SideStepArgs& a, cudaStream_t s) {
-    ProfileScope prof(KC_ROW, s);
-    CPM_REQUIRE(a.ld % 64 == 0 && a.ld <= 16384 && a.dim >= 1 && a.dim <= 4096, "side_step: unsupported sizes");
-    static int ctas = 0;
-    if (ctas == 0) {
-        constexpr int kSmem = 96 * 1024;
-        CUDA_CHECK(cudaFuncSetAttribute(side_step_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-        CUDA_CHECK(cudaFuncSetAttribute(side_step_kernel<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        ctas = max_active_clusters(side_step_kernel<T>, dim3(SIDE_THREADS), kSmem, SIDE_CTAS) >= 1 ? SIDE_CTAS : 8;
-    }
-    const size_t smem = sizeof(float) * (a.ld + pad64(a.dim) + a.ld / 8);
-    launch_kernel_cluster(side_step_kernel<T>, dim3(ctas), dim3(SIDE_THREADS), smem, s, ctas, a);
-}
-template void launch_side_step<bf16>(const SideStepArgs&, cudaStream_t);
-template void launch_side_step<float>(const SideStepArgs&, cudaStream_t);
 
 template <typename T>
 void launch_decay(const T* x, int ld_x, const bf16* w2, const bf16* w0, int rank, int channels, float* out, int ld_out, int rows, cudaStream_t s) {
