@@ -48,6 +48,7 @@ _SIGNATURES = {
     "cpmcu_load_model": (_c_int, [_c_char_p, _c_void_p]),
     "cpmcu_prefill": (_c_int, [_c_int, _c_int, _c_void_p, _c_void_p, _c_void_p]),
     "cpmcu_prefill_rows": (_c_int, [_c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p]),
+    "cpmcu_decode_token": (_c_int, [_c_int, _c_int, _c_void_p, _c_void_p, _c_int]),
     "cpmcu_decode": (_c_int, [_c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int]),
     "cpmcu_draft": (_c_int, [_c_void_p] * 5),
     "cpmcu_verify_and_fix": (_c_int, [_c_int] + [_c_void_p] * 6),
@@ -248,6 +249,10 @@ def prefill_rows(input_length, history_length, input, position_ids, want, output
 def decode(input_length, padded_length, input, position_ids, cache_length, mask_2d, output, cuda_graph):
     call("cpmcu_decode", input_length, padded_length, input, position_ids, cache_length, mask_2d or None, output,
          int(cuda_graph))
+
+
+def decode_token(token, position, work, output, cuda_graph):
+    call("cpmcu_decode_token", token, position, work, output, int(cuda_graph))
 
 
 def draft(tree_draft_ids, tree_position_ids, cache_length, attn_mask, tree_parent):

@@ -220,17 +220,10 @@ class LLM(torch.nn.Module):
         return self.logits[:n].clone()
 
     def _decode_one(self, token, position):
-        """Logits [1, vocab] after `token`, which becomes row `position` of the cache.  The next call overwrites them."""
-        if not hasattr(self, "_step_host"):
-            # token id, position and cache length of a step travel in one copy from pinned memory
-            self._step_host = torch.zeros(3, dtype=torch.int32, pin_memory=True)
-            self._step_dev = torch.zeros(3, dtype=torch.int32, device="cuda")
-            self._step_np = self._step_host.numpy()
-        self._step_np[:] = (token, position, position + 1)
-        self._step_dev.copy_(self._step_host, non_blocking=True)
-        at = self._step_dev.data_ptr()
-        C.decode(1, (position + 128) // 128 * 128, at, at + 4, at + 8, 0, self.logits.data_ptr(), self.cuda_graph)
-        return self.logits[:1]
+        """Logits [1, vocab] after `token`, which becomes row `position` of the cache."""
+        out = torch.empty((1, self.config.vocab_size), dtype=self.dtype, device="cuda")
+        C.decode_token(int(token), position, self.logits.data_ptr(), out.data_ptr(), self.cuda_graph)
+        return out
 
     def extend(self, tokens, history, want):
         """Append `tokens` (a list of ids) behind the `history` tokens the cache holds; history 0 starts a new sequence.
@@ -241,7 +234,8 @@ class LLM(torch.nn.Module):
             raise ValueError(f"{history} cached + {n} new tokens exceed the {self.max_total_length} tokens the KV cache holds "
                              f"under the current memory limit")
         if n == 1 and history > 0:
-            return self._decode_one(tokens[0], history).repeat(len(want), 1)
+            out = self._decode_one(tokens[0], history)
+            return out if len(want) == 1 else out.repeat(len(want), 1)
         ids = torch.tensor(tokens, dtype=torch.int32, device="cuda")
         pos = torch.arange(history, history + n, dtype=torch.int32, device="cuda")
         out = torch.empty((len(want), self.config.vocab_size), dtype=self.dtype, device="cuda")

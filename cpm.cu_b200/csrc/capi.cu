@@ -314,6 +314,13 @@ int cpmcu_decode(int input_length, int padded_length, const int32_t* input, cons
     });
 }
 
+int cpmcu_decode_token(int token, int position, void* work, void* output, int cuda_graph) {
+    return guarded([&] {
+        engine().decode_token(token, position, work, output, cuda_graph != 0);
+        return 0;
+    });
+}
+
 int cpmcu_draft(int32_t* tree_draft_ids, int32_t* tree_position_ids, const int32_t* cache_length,
                 uint64_t* attn_mask, int32_t* tree_parent) {
     return guarded([&] {

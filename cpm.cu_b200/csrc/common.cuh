@@ -325,6 +325,8 @@ struct DecodeInputs {
 };
 void launch_stage_decode(const DecodeInputs& dst, const int32_t* ids, const int32_t* pos, const int32_t* len, const uint64_t* mask, int n,
                          cudaStream_t s);
+// One token by value: its id, its position, and the cache length that counts it
+void launch_stage_token(const DecodeInputs& dst, int token, int position, cudaStream_t s);
 // x = (a + bias[col]) + b, each sum rounded to bf16 (bias may be null): the two halves of a quantised fc
 void launch_add_bias_add(bf16* x, const bf16* a, const bf16* bias, const bf16* b, int rows, int dim, cudaStream_t s);
 size_t argmax_workspace_bytes(int rows, int vocab);

@@ -308,6 +308,13 @@ __global__ void stage_decode_kernel(const DecodeInputs dst, const int32_t* __res
     if (mask != nullptr) dst.mask[i] = mask[i];
 }
 
+__global__ void stage_token_kernel(const DecodeInputs dst, int token, int position) {
+    grid_dependency_sync();
+    *dst.ids = token;
+    if (dst.pos != nullptr) *dst.pos = position;
+    *dst.len = position + 1;
+}
+
 // Row argmax over bf16 logits, lowest index wins ties.  Stage 1: each CTA scans one
 // 8192-entry chunk of a row with 16-byte loads; stage 2: one warp per row merges.
 constexpr int AM_CHUNK = 8192;
@@ -643,6 +650,10 @@ void launch_gather_rows(bf16* out, const bf16* src, const RowList& list, int dim
 void launch_stage_decode(const DecodeInputs& dst, const int32_t* ids, const int32_t* pos, const int32_t* len, const uint64_t* mask, int n,
                          cudaStream_t s) {
     launch_kernel(stage_decode_kernel, dim3(1), dim3(64), 0, s, dst, ids, pos, len, mask, n);
+}
+
+void launch_stage_token(const DecodeInputs& dst, int token, int position, cudaStream_t s) {
+    launch_kernel(stage_token_kernel, dim3(1), dim3(1), 0, s, dst, token, position);
 }
 
 size_t argmax_workspace_bytes(int rows, int vocab) {

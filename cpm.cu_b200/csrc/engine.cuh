@@ -155,6 +155,8 @@ public:
     void prefill_rows(int n, int history, const int32_t* ids, const int32_t* pos, const int32_t* want, int n_want, void* logits_out);
     void decode(int n, int padded_len, const int32_t* ids, const int32_t* pos, const int32_t* cache_length,
                 const uint64_t* mask, void* logits_out, bool cuda_graph);
+    // one token by value behind `position` cached ones; logits_out [vocab] may be any buffer, `work` [vocab] is the same one in every call
+    void decode_token(int token, int position, void* work, void* logits_out, bool cuda_graph);
     void draft(int32_t* tree_ids, int32_t* tree_pos, const int32_t* cache_length, uint64_t* tree_mask,
                int32_t* tree_parent);
     int verify_and_fix(int T, int32_t* pred, const int32_t* gt, const int32_t* pos, const int32_t* cache_length,
@@ -242,7 +244,8 @@ private:
     template <typename T>
     void layered_logits(const int32_t* rows_idx, int n, void* out, cudaStream_t s);
     void layered_prefill(int n, int history, const int32_t* ids, const int32_t* want, int n_want, void* logits_out);
-    void layered_decode(int n, const int32_t* ids, const int32_t* cache_length, void* logits_out, bool cuda_graph);
+    void decode_rows(int n, const int32_t* ids, const int32_t* pos, const int32_t* cache_length, const uint64_t* mask, void* logits_out);
+    void layered_decode(int n, const int32_t* ids, const int32_t* cache_length, void* logits_out, bool cuda_graph, void* copy = nullptr);
     int layered_attn_splits(const LayerSpec& sp, int rows) const;
     size_t elem_bytes() const { return mc_.fp32 ? 4 : 2; }
     int ld() const { return pad64(mc_.hidden); }

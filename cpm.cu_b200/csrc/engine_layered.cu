@@ -190,6 +190,8 @@ void Engine::lay_out_layered(Pool& p) {
     ldelta_ = p.take(R * L * es);
     lnorm_ = p.take(R * L * es);
     want_ = take<int32_t>(p, R);
+    d_in_.ids = take<int32_t>(p, 1);
+    d_in_.len = take<int32_t>(p, 1);
     lmix_ = p.take(mix * es);
     lrec_ = p.take(rec * es);
     ldecay_ = take<float>(p, R * channels);
@@ -782,7 +784,8 @@ void Engine::layered_prefill(int n, int history, const int32_t* ids, const int32
 
 // cache_length (device) already counts the n new tokens.  With cuda_graph a one-token step is captured on its second
 // call with the same buffers and replayed from then on.
-void Engine::layered_decode(int n, const int32_t* ids, const int32_t* cache_length, void* logits_out, bool cuda_graph) {
+// copy: where the logits [n, vocab] are wanted as well.
+void Engine::layered_decode(int n, const int32_t* ids, const int32_t* cache_length, void* logits_out, bool cuda_graph, void* copy) {
     CPM_REQUIRE(not_loaded_.empty(), "weights missing, for instance " + *not_loaded_.begin());
     Runtime& rt = runtime();
     cudaStream_t s = rt.stream;
@@ -831,6 +834,7 @@ void Engine::layered_decode(int n, const int32_t* ids, const int32_t* cache_leng
         enqueue();
         CUDA_CHECK(cudaEventRecord(ev1_, s));
     }
+    if (copy != nullptr) CUDA_CHECK(cudaMemcpyAsync(copy, logits_out, static_cast<size_t>(n) * mc_.vocab * elem_bytes(), cudaMemcpyDeviceToDevice, s));
     layered_check_errors("decode");
     float ms = 0.f;
     CUDA_CHECK(cudaEventElapsedTime(&ms, ev0_, ev1_));

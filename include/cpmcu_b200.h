@@ -165,6 +165,10 @@ int cpmcu_prefill_rows(int input_length, int history_length, const int32_t* inpu
 int cpmcu_decode(int input_length, int padded_length, const int32_t* input, const int32_t* position_ids,
                  const int32_t* cache_length, const uint64_t* mask_2d, void* output, int cuda_graph);
 
+/* cpmcu_decode of one token that the host has: `token` becomes cache row `position`, its logits [vocab] go to `output` (device, any
+ * buffer).  work: device buffer of the same size, the same one in every call (layered models capture the step over it). */
+int cpmcu_decode_token(int token, int position, void* work, void* output, int cuda_graph);
+
 /* reference: draft, src/entry.cu:498.  Reads tree_draft_ids[0] (root) and
  * *cache_length; writes tree_draft_ids[1:], positions, masks, parents. */
 int cpmcu_draft(int32_t* tree_draft_ids, int32_t* tree_position_ids, const int32_t* cache_length,
