@@ -35,15 +35,6 @@ __device__ __forceinline__ int key_index(unsigned long long k) {
     return static_cast<int>(0xFFFFFFFFu - static_cast<uint32_t>(k & 0xFFFFFFFFull));
 }
 
-// Warp-wide maximum of 64-bit keys as two 32-bit hardware reductions (value half, then the index half
-// among the lanes that hold the winning value).
-__device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v) {
-    const uint32_t hi = static_cast<uint32_t>(v >> 32), lo = static_cast<uint32_t>(v);
-    const uint32_t H = __reduce_max_sync(0xffffffffu, hi);
-    const uint32_t L = __reduce_max_sync(0xffffffffu, hi == H ? lo : 0u);
-    return (static_cast<unsigned long long>(H) << 32) | L;
-}
-
 __device__ __forceinline__ bf16 bf16_from_orderable(uint32_t o) {
     const uint16_t b = (o & 0x8000u) ? static_cast<uint16_t>(o & 0x7FFFu) : static_cast<uint16_t>(~o);
     return __ushort_as_bfloat16(b);
@@ -67,6 +58,44 @@ __device__ uint32_t warp_select(uint32_t* keys, int n, int k, int lane) {
     return mine;
 }
 
+// The k best of a row some of whose segments may hide entries, by one warp: lane n gets place n.  Whatever a segment hides has the
+// threshold's lp (tau) and no more (k candidates of one segment above it would have raised it), so the candidates above it (got, in order)
+// stay, and the places behind them go to the lowest indices at it: from a segment's own logits where it may hide some, and each such
+// segment has one at least, else from its candidates.  k passes over the row by one warp took 4.3 ms a level at 73448 entries, which two
+// levels of a 64-token request met; ten rows with their best entries in one segment 9.7 ms, now 44 us (37 without any).
+__device__ __noinline__ void entries_at_threshold(const bf16* x, int vocab, const float4* rst, const unsigned long long* mycand, int nseg, int k, uint32_t got,
+                                                  uint32_t tau, float mx, float ls, int lane, int& my_idx, bf16& my_lp) {
+    auto lp_of = [&](bf16 v) { return __float2bfloat16(__bfloat162float(v) - mx - ls); };
+    int have = __popc(__ballot_sync(0xffffffffu, lane < k && (got >> 16) > tau));
+    if (lane < have) my_idx = key_index(mycand[0xFFFF - (got & 0xFFFFu)]);
+    for (int sg = 0; sg < nseg && have < k; ++sg) {
+        const uint32_t xk = __float_as_uint(rst[sg].z);
+        if (xk != 0u && bf16_orderable(lp_of(bf16_from_orderable(xk))) >= tau) {
+            const int end = min((sg + 1) * SEG, vocab);
+            for (int at = sg * SEG; at < end && have < k; at += 256) {
+                bf16 v[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) v[j] = at + j * 32 + lane < end ? x[at + j * 32 + lane] : __float2bfloat16(0.f);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    uint32_t hit = __ballot_sync(0xffffffffu, at + j * 32 + lane < end && bf16_orderable(lp_of(v[j])) == tau);
+                    for (; hit != 0u && have < k; hit &= hit - 1u, ++have) {
+                        if (lane == have) my_idx = at + j * 32 + __ffs(hit) - 1;
+                    }
+                }
+            }
+        } else {
+            const unsigned long long c = lane < k ? mycand[sg * k + lane] : 0ull;   // in index order
+            uint32_t hit = __ballot_sync(0xffffffffu, c != 0ull && bf16_orderable(lp_of(bf16_from_orderable(static_cast<uint32_t>(c >> 32)))) == tau);
+            for (; hit != 0u && have < k; hit &= hit - 1u, ++have) {
+                const int idx = __shfl_sync(0xffffffffu, key_index(c), __ffs(hit) - 1);
+                if (lane == have) my_idx = idx;
+            }
+        }
+    }
+    if (lane < have) my_lp = lp_of(x[my_idx]);
+}
+
 // One launch per draft level: log-softmax statistics, top-k and frontier expansion.
 //
 // Every CTA owns one (row, 2048-entry vocabulary segment): it reduces the segment's (max, sum of exp) and extracts
@@ -80,8 +109,8 @@ __device__ uint32_t warp_select(uint32_t* keys, int n, int k, int lane) {
 // logits to one lp, and among equal lp the reference prefers the LOWER index, which a segment's logit order does not
 // know.  An element outside a segment's k best logits can only belong to the row's answer if that segment's own k-th
 // candidate still reaches the answer's threshold lp (all k of its candidates compete in the top bucket); the last
-// CTA detects that and re-selects such a row exactly from the full logit row.  With 36 segments and k = 10 this needs
-// ten of a row's best entries inside one segment; the small vocabularies of the tests take the path routinely.
+// CTA detects that and looks for such a row's entries at the threshold in those segments' logits.  With 36 segments and k = 10 this
+// needs ten of a row's best entries inside one segment; the small vocabularies of the tests take the path routinely.
 __global__ void draft_level_kernel(DraftTreeState st, const bf16* __restrict__ logits, int ld, int vocab, int nseg,
                                    float4* __restrict__ stats, unsigned long long* __restrict__ cand,
                                    unsigned* __restrict__ ticket, int level, const int32_t* __restrict__ last_row_ptr,
@@ -256,24 +285,7 @@ __global__ void draft_level_kernel(DraftTreeState st, const bf16* __restrict__ l
             bf16 my_lp = __float2bfloat16(0.f);
             int my_idx = 0;
             if (__any_sync(0xffffffffu, saturated)) {
-                // k rounds of "largest key below the previous pick" over the whole logit row
-                const bf16* x = logits + static_cast<size_t>(r + row0) * ld;
-                unsigned long long prev = ~0ull, mine64 = 0ull;
-                for (int round = 0; round < k; ++round) {
-                    unsigned long long best = 0ull;
-                    for (int i = lane; i < vocab; i += 32) {
-                        const bf16 lp = __float2bfloat16(__bfloat162float(x[i]) - mx - ls);
-                        const unsigned long long key = make_key(lp, i);
-                        if (key < prev && key > best) best = key;
-                    }
-                    best = warp_max_u64(best);
-                    if (lane == round) mine64 = best;
-                    prev = best;
-                }
-                if (mine64) {
-                    my_idx = key_index(mine64);
-                    my_lp = __float2bfloat16(__bfloat162float(x[my_idx]) - mx - ls);
-                }
+                entries_at_threshold(logits + static_cast<size_t>(r + row0) * ld, vocab, rst, mycand, nseg, k, got, tau, mx, ls, lane, my_idx, my_lp);
             } else if (got) {
                 const unsigned long long c = mycand[0xFFFF - (got & 0xFFFFu)];
                 my_idx = key_index(c);
