@@ -299,7 +299,6 @@ moe_route_kernel(const RouteArgs a) {
 constexpr int RT_PRE = 32;   // 128-column pieces of the weights held in registers
 __global__ void __launch_bounds__(RT_WARPS * 32)
 moe_route_one_kernel(const RouteArgs a) {
-    grid_dep_trigger();
     extern __shared__ float sm[];
     __shared__ int s_last;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -312,6 +311,7 @@ moe_route_one_kernel(const RouteArgs a) {
         wv[j] = c < a.ld ? __ldg(reinterpret_cast<const uint2*>(w + c)) : make_uint2(0u, 0u);
     }
     grid_dep_wait();
+    grid_dep_trigger();   // not before the row exists: the shared expert's product starts on it (one_row.cu)
     float acc = 0.f;
     auto add = [&](const uint2& wp, const float4& x) {
         const bf16* b = reinterpret_cast<const bf16*>(&wp);
