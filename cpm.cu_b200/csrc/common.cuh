@@ -266,7 +266,8 @@ struct SideRow {
     int table_ld = 0, col0 = 0, vocab = 0;
 };
 // M == 1, bf16 weights; with `rope` the product is q, k and v, which are rotated and appended; with `side` the side input's gate
-void launch_linear_one_row(const LinearPlan& plan, cudaStream_t stream, const RopeRow* rope = nullptr, const SideRow* side = nullptr);
+// hold: the next launch starts only after this one's wait (a plain product)
+void launch_linear_one_row(const LinearPlan& plan, cudaStream_t stream, const RopeRow* rope = nullptr, const SideRow* side = nullptr, bool hold = false);
 bool linear_one_row_fits(int N, int K, int sms);   // whether that is the faster way for one row of N outputs
 // Same contract with 4-bit weights, w = (q - 8) * scale, K % 256 == 0 and N % 128 == 0.  `wq` holds one
 // contiguous 16896-byte block per (128-feature tile, 256-k unit), tile-major: [4 k-blocks][2 halves]
@@ -378,4 +379,7 @@ bool biased_attn_fits(int hq, int hkv, int dk, int dv);
 AttnPlan make_biased_attn_plan(const bf16* q, int q_ld_tokens, const bf16* k_cache, const bf16* v_cache, int budget, int tq,
                                int hq, int hkv, int dk, int dv, int out_cols, int splits, float scale, int exact_window,
                                float bias_exp, bf16* out, int out_ld, float* ws_o, float* ws_ml);
-void launch_tree_attention(const AttnPlan& plan, cudaStream_t s);
+// One key split after the other, and the merge of several: in one call, or with other work between.  The merge alone runs beside its predecessor,
+// which starts it after its own wait, i.e. behind the splits.
+enum AttnPart { ATTN_ALL, ATTN_SPLITS, ATTN_MERGE };
+void launch_tree_attention(const AttnPlan& p, cudaStream_t s, AttnPart part = ATTN_ALL);

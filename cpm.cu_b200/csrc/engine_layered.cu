@@ -557,12 +557,11 @@ void Engine::run_product(const LayeredProduct& p, int rows, cudaStream_t s) {
 }
 
 template <typename T>
-void Engine::layered_attention(int i, LayeredPlans& lp, const int32_t* kv_len, int kv_off, cudaStream_t s) {
+void Engine::layered_queries(int i, LayeredPlans& lp, const int32_t* kv_len, int kv_off, bool beside, cudaStream_t s) {
     const LayerSpec& sp = mc_.specs[i];
     const LayeredWeights& w = lw_[i];
     LayeredPlans::Layer& l = lp.layers[i];
     const int rows = lp.rows;
-    run_product<T>(l.qkv, rows, s);
     QkvNormArgs a;
     a.qkv = lqkv_; a.ld = l.qkv.N;
     a.heads = sp.heads; a.kv_heads = sp.kv_heads;
@@ -573,12 +572,21 @@ void Engine::layered_attention(int i, LayeredPlans& lp, const int32_t* kv_len, i
     a.k_cache = sp.kv_from >= 0 ? nullptr : w.k;
     a.v_cache = sp.kv_from >= 0 ? nullptr : w.v;
     a.kv_len = kv_len; a.kv_off = kv_off; a.cache_rows = budget_; a.error = runtime().d_error;
+    a.beside = beside ? 1 : 0;
     launch_qkv_norm_append<T>(a, rows, s);
+}
+
+template <typename T>
+void Engine::layered_attention(int i, LayeredPlans& lp, const int32_t* kv_len, int kv_off, AttnPart part, cudaStream_t s) {
+    const LayerSpec& sp = mc_.specs[i];
+    const LayeredWeights& w = lw_[i];
+    LayeredPlans::Layer& l = lp.layers[i];
+    const int rows = lp.rows;
     if (l.tensor_attn) {
         l.attn.kv_len = kv_len;
         l.attn.kv_len_add = kv_off + rows;
-        launch_tree_attention(l.attn, s);
-    } else {
+        launch_tree_attention(l.attn, s, part);
+    } else if (part != ATTN_MERGE) {
         PlainAttnArgs pa;
         pa.q = lq_; pa.k_cache = w.k; pa.v_cache = w.v; pa.out = lattn_;
         pa.tq = rows; pa.hq = sp.heads; pa.hkv = sp.kv_heads;
@@ -591,17 +599,30 @@ void Engine::layered_attention(int i, LayeredPlans& lp, const int32_t* kv_len, i
 }
 
 template <typename T>
-void Engine::layered_recurrence(int i, LayeredPlans& lp, const int32_t* kv_len, int kv_off, cudaStream_t s) {
+bool Engine::layered_rec_products(int i, LayeredPlans& lp, bool hold, cudaStream_t s) {
+    LayeredPlans::Layer& l = lp.layers[i];
+    if (sizeof(T) == 2 && mc_.specs[i].rec == REC_TIME_MIX) {
+        launch_moe_gemm(l.mixes, s, hold);
+        return hold;
+    }
+    for (const LayeredProduct& p : l.rec) {
+        hold = hold && p.plan.one_row;
+        if (hold) {
+            ProfileScope prof(KC_LINEAR, s);
+            launch_linear_one_row(p.plan, s, nullptr, nullptr, true);
+        } else {
+            run_product<T>(p, lp.rows, s);
+        }
+    }
+    return hold;
+}
+
+template <typename T>
+void Engine::layered_recurrence(int i, LayeredPlans& lp, const int32_t* kv_len, int kv_off, bool hold, cudaStream_t s) {
     const LayerSpec& sp = mc_.specs[i];
     const LayeredWeights& w = lw_[i];
-    LayeredPlans::Layer& l = lp.layers[i];
     const int rows = lp.rows, nk = sp.rec_heads * sp.rec_dim, nv = sp.rec_heads * sp.rec_vdim, ldr = rec_ld(sp);
     const T* proj = static_cast<const T*>(lrec_);
-    if (sizeof(T) == 2 && sp.rec == REC_TIME_MIX) {
-        launch_moe_gemm(l.mixes, s);
-    } else {
-        for (const LayeredProduct& p : l.rec) run_product<T>(p, rows, s);
-    }
     ScanArgs a;
     a.heads = sp.rec_heads; a.dim = sp.rec_dim; a.vdim = sp.rec_vdim; a.rows = rows;
     a.ld_r = a.ld_k = a.ld_v = ldr;
@@ -634,6 +655,7 @@ void Engine::layered_recurrence(int i, LayeredPlans& lp, const int32_t* kv_len, 
         st.eps = mc_.eps; st.scale = sp.rec_scale;
         st.out = out;
         st.ticket = state_len_ + 1;
+        st.hold = hold ? 1 : 0;
         launch_scan_step<T>(st, s);
         return;
     }
@@ -674,8 +696,30 @@ bool Engine::layered_tanh_layer(int i, LayeredPlans& lp, const int32_t* ids, con
     LayeredPlans::Layer& l = lp.layers[i];
     const int rows = lp.rows, L = ld(), W = mc_.hidden, layers = static_cast<int>(lw_.size());
     T *x = static_cast<T*>(lx_), *delta = static_cast<T*>(ldelta_);
-    if (sp.heads > 0) layered_attention<T>(i, lp, kv_len, kv_off, s);
-    if (sp.rec != REC_NONE) layered_recurrence<T>(i, lp, kv_len, kv_off, s);
+    const bool both = sp.heads > 0 && sp.rec != REC_NONE;
+    if (both && sizeof(T) == 2 && rows == 1 && scan_step_fits(sp.rec_dim, sp.rec_vdim, sp.rec == REC_TIME_MIX)) {
+        // Two chains of one token's row: its queries and keys are normalised beside the recurrence's product, the splits of its attention are
+        // merged beside the recurrence's step.  Each of the two pairs is one launch that starts its successor after its own wait and a
+        // successor that waits at its end.  1405 + 24 tokens of nine layers of 3072, six of them of this kind: 29.6 ms one after the other, 28.95
+        // so; with the product beside the norms instead it starts its weights later and took 29.1.
+        const bool merge = l.tensor_attn && l.attn.splits > 1;
+        run_product<T>(l.qkv, rows, s);
+        const bool held = layered_rec_products<T>(i, lp, true, s);
+        layered_queries<T>(i, lp, kv_len, kv_off, held, s);
+        layered_attention<T>(i, lp, kv_len, kv_off, ATTN_SPLITS, s);
+        layered_recurrence<T>(i, lp, kv_len, kv_off, merge, s);
+        layered_attention<T>(i, lp, kv_len, kv_off, ATTN_MERGE, s);
+    } else {
+        if (sp.heads > 0) {
+            run_product<T>(l.qkv, rows, s);
+            layered_queries<T>(i, lp, kv_len, kv_off, false, s);
+            layered_attention<T>(i, lp, kv_len, kv_off, ATTN_ALL, s);
+        }
+        if (sp.rec != REC_NONE) {
+            layered_rec_products<T>(i, lp, false, s);
+            layered_recurrence<T>(i, lp, kv_len, kv_off, false, s);
+        }
+    }
     run_product<T>(l.o, rows, s);
     // a row's mixes need the row before it, which only a single row has at hand at a layer's end
     const bool next = i + 1 < layers && mc_.side_dim > 0 && (rows == 1 || mc_.specs[i + 1].rec != REC_TIME_MIX);
@@ -730,7 +774,9 @@ void Engine::layered_forward(int rows, const int32_t* ids, const int32_t* kv_len
             if (!ready) launch_tanh_norm<T>(x32_, nullptr, w.tanh1, static_cast<T*>(lx_), token_shift(li, rows, kv_len, kv_off), rows, L, s);
             ready = layered_tanh_layer<T>(li, lp, ids, kv_len, kv_off, s);
         } else {
-            layered_attention<T>(static_cast<int>(i), lp, kv_len, kv_off, s);
+            run_product<T>(lp.layers[i].qkv, rows, s);
+            layered_queries<T>(static_cast<int>(i), lp, kv_len, kv_off, false, s);
+            layered_attention<T>(static_cast<int>(i), lp, kv_len, kv_off, ATTN_ALL, s);
             run_product<T>(lp.layers[i].o, rows, s);
             launch_out_norm<T>(x32_, static_cast<T*>(lx_), static_cast<const T*>(ldelta_), MoeMix(), mc_.scale_residual, w.norm1, rows, W, L, mc_.eps, s);
             if (sp.experts + sp.identity > 0) layered_mixture<T>(static_cast<int>(i), lp, s);

@@ -82,6 +82,7 @@ struct QkvNormArgs {
     const int32_t* kv_len;
     int kv_off, cache_rows;
     int* error;
+    int beside = 0;          // the predecessor leaves qkv alone and has started this launch after its own wait: run beside it
 };
 template <typename T>
 void launch_qkv_norm_append(const QkvNormArgs& a, int rows, cudaStream_t s);
@@ -186,6 +187,7 @@ struct ScanStepArgs {
     float eps = 0.f, scale = 1.f;
     void* out = nullptr;           // T [heads * vdim]
     int32_t* ticket = nullptr;     // zero between launches
+    int hold = 0;                  // the next launch starts only after this one's wait
 };
 bool scan_step_fits(int dim, int vdim, bool time_mix);
 template <typename T>
@@ -278,8 +280,8 @@ MoeGemmPlan make_moe_gate_up_plan(const LayerSpec& sp, const bf16* w, const bf16
 // down: y[row][width]; act rows of ld_act columns
 MoeGemmPlan make_moe_down_plan(const LayerSpec& sp, const bf16* w, const bf16* act, int act_rows, int ld_act, int width, bf16* y,
                                int ld_y, int rows, int tile, const MoeBuffers& b);
-void launch_moe_gemm(const MoeGemmPlan& p, cudaStream_t s);
-void launch_moe_one_row(const MoeGemmPlan& p, cudaStream_t s);   // rows == 1 (one_row.cu)
+void launch_moe_gemm(const MoeGemmPlan& p, cudaStream_t s, bool hold = false);   // hold: one row, no router; as launch_linear_one_row's
+void launch_moe_one_row(const MoeGemmPlan& p, cudaStream_t s, bool hold = false);   // rows == 1 (one_row.cu)
 // elements of the two weight buffers (tile-major), and where an expert's (index `experts`: the shared expert's) part begins
 size_t moe_gate_up_elems(const LayerSpec& sp, int K);
 size_t moe_down_elems(const LayerSpec& sp, int width);

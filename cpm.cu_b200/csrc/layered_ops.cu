@@ -33,21 +33,37 @@ __global__ void embed_rows_kernel(const int32_t* __restrict__ ids, const bf16* _
 }
 
 // One CTA per token row.
-template <typename T, int VEC>
+template <int VEC, bool FRESH, typename T>
+__device__ __forceinline__ void load_row(const T* p, float* f) {
+    if constexpr (FRESH && VEC == 8 && sizeof(T) == 2) {
+        const uint4 v = __ldcg(reinterpret_cast<const uint4*>(p));
+        load_vec<8>(reinterpret_cast<const T*>(&v), f);
+    } else if constexpr (FRESH && sizeof(T) == 2) {
+        static_assert(VEC == 1, "pieces of 16 bytes or single elements");
+        f[0] = __bfloat162float(__ushort_as_bfloat16(__ldcg(reinterpret_cast<const unsigned short*>(p))));
+    } else {
+        load_vec<VEC>(p, f);
+    }
+}
+
+// BESIDE: the launch before the predecessor wrote the row, which is read past the first-level cache; the wait for the predecessor comes at the end,
+// so that whatever waits for this launch has waited for both.
+template <typename T, int VEC, bool BESIDE>
 __global__ void qkv_norm_append_kernel(const QkvNormArgs a) {
-    grid_dependency_sync();
+    grid_dep_trigger();
+    if (!BESIDE) grid_dep_wait();
     __shared__ float sh[64];
     __shared__ float2 turn[256];   // cos, sin of the row's angles
     const int r = blockIdx.x;
     const int nq = a.heads * a.dim, nk = a.kv_heads * a.dim, nv = a.kv_heads * a.vdim;
     const T* row = static_cast<const T*>(a.qkv) + static_cast<size_t>(r) * a.ld;
     const bool own_kv = a.k_cache != nullptr;
-    const long long kv_row = own_kv ? static_cast<long long>(*a.kv_len) + a.kv_off + r : 0;
+    const long long kv_row = own_kv ? static_cast<long long>(__ldcg(a.kv_len)) + a.kv_off + r : 0;
     const bool store_kv = own_kv && kv_row >= 0 && kv_row < a.cache_rows;
     if (own_kv && !store_kv && threadIdx.x == 0) atomicOr(a.error, ERR_KV_OVERFLOW);
     const int half = a.rot_dims / 2;
     if (half > 0) {
-        const float pos = static_cast<float>(*a.kv_len + a.kv_off + r);
+        const float pos = static_cast<float>(__ldcg(a.kv_len) + a.kv_off + r);
         for (int i = threadIdx.x; i < half; i += blockDim.x) {
             float sn, cs;
             sincosf(pos * a.inv_freq[i], &sn, &cs);
@@ -59,13 +75,13 @@ __global__ void qkv_norm_append_kernel(const QkvNormArgs a) {
     if (a.wq != nullptr) {
         float sq = 0.f, sk = 0.f, f[VEC];
         for (int c = threadIdx.x * VEC; c < nq; c += blockDim.x * VEC) {
-            load_vec<VEC>(row + c, f);
+            load_row<VEC, BESIDE>(row + c, f);
 #pragma unroll
             for (int e = 0; e < VEC; ++e) sq += f[e] * f[e];
         }
         if (own_kv) {
             for (int c = threadIdx.x * VEC; c < nk; c += blockDim.x * VEC) {
-                load_vec<VEC>(row + nq + c, f);
+                load_row<VEC, BESIDE>(row + nq + c, f);
 #pragma unroll
                 for (int e = 0; e < VEC; ++e) sk += f[e] * f[e];
             }
@@ -80,7 +96,7 @@ __global__ void qkv_norm_append_kernel(const QkvNormArgs a) {
             const int h = i / per, c = (i - h * per) * VEC;
             float f[VEC];
             if (c < d) {
-                load_vec<VEC>(src + h * d + c, f);
+                load_row<VEC, BESIDE>(src + h * d + c, f);
                 if (w != nullptr) {
                     float g[VEC];
                     load_vec<VEC>(w + h * d + c, g);
@@ -91,7 +107,7 @@ __global__ void qkv_norm_append_kernel(const QkvNormArgs a) {
                     const bool upper = c >= rot;
                     const int other = upper ? c - rot : c + rot, i0 = upper ? c - rot : c;
                     float p[VEC];
-                    load_vec<VEC>(src + h * d + other, p);
+                    load_row<VEC, BESIDE>(src + h * d + other, p);
                     if (w != nullptr) {
                         float g[VEC];
                         load_vec<VEC>(w + h * d + other, g);
@@ -120,6 +136,7 @@ __global__ void qkv_norm_append_kernel(const QkvNormArgs a) {
               static_cast<T*>(a.v_cache) + static_cast<size_t>(kv_row) * a.kv_heads * a.vdim_p, false, 0);
         (void)nv;
     }
+    if (BESIDE) grid_dep_wait();
 }
 
 template <typename T, int VPT, bool MIX>
@@ -248,8 +265,14 @@ void launch_qkv_norm_append(const QkvNormArgs& a, int rows, cudaStream_t s) {
     ProfileScope prof(KC_ROW, s);
     CPM_REQUIRE(a.rot_dims % 2 == 0 && a.rot_dims <= a.dim && a.rot_dims <= 512, "layered model: bad number of rotated dimensions");
     const bool v8 = a.dim % 8 == 0 && a.vdim % 8 == 0 && a.ld % 8 == 0 && (a.rot_dims / 2) % 8 == 0;
-    if (v8) launch_kernel(qkv_norm_append_kernel<T, 8>, dim3(rows), dim3(256), 0, s, a);
-    else launch_kernel(qkv_norm_append_kernel<T, 1>, dim3(rows), dim3(256), 0, s, a);
+    auto run = [&](auto kernel) { launch_kernel(kernel, dim3(rows), dim3(256), 0, s, a); };
+    if constexpr (sizeof(T) == 2) {
+        if (a.beside != 0) {
+            if (v8) run(qkv_norm_append_kernel<T, 8, true>); else run(qkv_norm_append_kernel<T, 1, true>);
+            return;
+        }
+    }
+    if (v8) run(qkv_norm_append_kernel<T, 8, false>); else run(qkv_norm_append_kernel<T, 1, false>);
 }
 
 template <typename T>

@@ -967,10 +967,10 @@ MoeGemmPlan make_moe_down_plan(const LayerSpec& sp, const bf16* w, const bf16* a
     return p;
 }
 
-void launch_moe_gemm(const MoeGemmPlan& p, cudaStream_t s) {
+void launch_moe_gemm(const MoeGemmPlan& p, cudaStream_t s, bool hold) {
     ProfileScope prof(p.uniform > 0 ? KC_LINEAR : KC_MOE, s);
     if (p.rows == 1) {   // 4 of 30 experts of width 4096, ff 2048, and a shared one: 45.8 + 28.9 us as tiles, see one_row.cu
-        launch_moe_one_row(p, s);
+        launch_moe_one_row(p, s, hold);
         return;
     }
     GemmArgs a;

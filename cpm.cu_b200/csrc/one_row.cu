@@ -55,7 +55,8 @@ enum Epilogue { PLAIN, GATED, ROPE, SIDE };
 // only when the row it reads exists (its own wait is over), so the shared matrix's CTAs compute and store beside it, with no wait.  The other
 // CTAs of the launch wait, and so this launch still ends after the router.  The router is 8 us of latency on five CTAs: 32 tokens of six layers
 // of 4096 with a shared expert of 4096 took 24.7 ms, now 22.5.
-template <int R, Epilogue EPI, bool EARLY>
+// HOLD: the successor starts only after this launch's wait; it may then run beside this launch on what was there before it.
+template <int R, Epilogue EPI, bool EARLY, bool HOLD>
 __global__ void __launch_bounds__(ONE_WARPS * 32, 4)
 one_row_kernel(const OneRowArgs a) {
     constexpr bool PAIR = EPI == GATED || EPI == ROPE;
@@ -63,7 +64,7 @@ one_row_kernel(const OneRowArgs a) {
     constexpr int U = 8 / LOADS;                       // k-blocks per batch
     __shared__ float part[ONE_WARPS][R];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (EARLY) grid_dep_trigger();
+    if (EARLY && !HOLD) grid_dep_trigger();
 
     const bool shared = static_cast<int>(blockIdx.x) < a.ctas_s;
     const int b = shared ? blockIdx.x : blockIdx.x - a.ctas_s;
@@ -102,7 +103,7 @@ one_row_kernel(const OneRowArgs a) {
     const bool ahead = !EARLY && shared && a.ahead != 0;
     if (!waited) {
         if (!ahead) grid_dep_wait();
-        if (!EARLY) grid_dep_trigger();
+        if (!EARLY || HOLD) grid_dep_trigger();
     }
     if (!there) return;
     int pos = 0, kv_len = 0, valid = 1;
@@ -225,17 +226,17 @@ bool linear_one_row_fits(int N, int K, int sms) {
 
 namespace {
 
-template <Epilogue EPI, bool EARLY>
+template <Epilogue EPI, bool EARLY, bool HOLD = false>
 void launch(int R, const OneRowArgs& a, int grid, cudaStream_t s) {
     switch (R) {
-        case 8: launch_kernel(one_row_kernel<8, EPI, EARLY>, dim3(grid), dim3(ONE_WARPS * 32), 0, s, a); break;
-        default: launch_kernel(one_row_kernel<16, EPI, EARLY>, dim3(grid), dim3(ONE_WARPS * 32), 0, s, a); break;
+        case 8: launch_kernel(one_row_kernel<8, EPI, EARLY, HOLD>, dim3(grid), dim3(ONE_WARPS * 32), 0, s, a); break;
+        default: launch_kernel(one_row_kernel<16, EPI, EARLY, HOLD>, dim3(grid), dim3(ONE_WARPS * 32), 0, s, a); break;
     }
 }
 
 }  // namespace
 
-void launch_linear_one_row(const LinearPlan& p, cudaStream_t s, const RopeRow* rope, const SideRow* side) {
+void launch_linear_one_row(const LinearPlan& p, cudaStream_t s, const RopeRow* rope, const SideRow* side, bool hold) {
     OneRowArgs a = {};
     a.w = p.w; a.x = p.x; a.y = p.y; a.bias = p.bias;
     a.N = p.N; a.kblocks = p.K / BLOCK_COLS;
@@ -254,12 +255,14 @@ void launch_linear_one_row(const LinearPlan& p, cudaStream_t s, const RopeRow* r
         launch<SIDE, true>(R, a, a.ctas, s);
     } else if (p.swiglu) {
         launch<GATED, true>(R, a, a.ctas, s);
+    } else if (hold) {
+        launch<PLAIN, true, true>(R, a, a.ctas, s);
     } else {
         launch<PLAIN, true>(R, a, a.ctas, s);
     }
 }
 
-void launch_moe_one_row(const MoeGemmPlan& p, cudaStream_t s) {
+void launch_moe_one_row(const MoeGemmPlan& p, cudaStream_t s, bool hold) {
     OneRowArgs a = {};
     a.w = p.w; a.x = p.x; a.xs = p.xs; a.y = p.y;
     a.N = p.N; a.kblocks = p.kblocks; a.N_s = p.N_s; a.kblocks_s = p.kblocks_s;
@@ -274,6 +277,8 @@ void launch_moe_one_row(const MoeGemmPlan& p, cudaStream_t s) {
     const int grid = a.ctas_s + p.max_entries * a.ctas;
     a.ahead = p.max_entries > 0;   // some CTA waits for the router
     // the router's choice: gate/up waits for it and lets its successor start only then, so down may read it at once
-    if (p.swiglu) launch<GATED, false>(R, a, grid, s);
+    CPM_REQUIRE(!hold || p.uniform > 0, "one row: the router's products have an order of their own");
+    if (hold) launch<PLAIN, true, true>(R, a, grid, s);
+    else if (p.swiglu) launch<GATED, false>(R, a, grid, s);
     else launch<PLAIN, true>(R, a, grid, s);
 }

@@ -386,7 +386,7 @@ scan_step_kernel(const StepParams p) {
     const int h = blockIdx.x, v0 = blockIdx.y * p.cols, vcols = min(p.cols, a.vdim - v0);
     const int cg = p.cols / 4, groups = STEP_THREADS / cg;
     const int c4 = (tid % cg) * 4, g = tid / cg;
-    grid_dep_trigger();
+    if (p.a.hold == 0) grid_dep_trigger();
     // the state was last written by the step before, which the host has waited for: it is fetched before this kernel's turn
     float* state = a.state + static_cast<size_t>(h) * p.kp * p.vp + v0 + c4;
     float4 S[STEP_LOADS];
@@ -408,6 +408,7 @@ scan_step_kernel(const StepParams p) {
         }
     }
     grid_dep_wait();
+    if (p.a.hold != 0) grid_dep_trigger();
     if (*a.kv_len + a.kv_off == 0) {
 #pragma unroll
         for (int n = 0; n < STEP_LOADS; ++n) S[n] = make_float4(0.f, 0.f, 0.f, 0.f);

@@ -550,8 +550,9 @@ tree_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 template <int DV>
 __global__ void attn_combine_kernel(const float* __restrict__ ws_o, const float* __restrict__ ws_ml, int nsplit,
                                     int rows, int hq, float scale_log2, bf16* __restrict__ out, int out_ld, int out_cols,
-                                    int sink, float out_scale) {
-    grid_dependency_sync();
+                                    int sink, float out_scale, int beside) {
+    grid_dep_trigger();
+    if (beside == 0) grid_dep_wait();   // else at the end (ATTN_MERGE): the partial results are there, their producer is two launches back
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (row >= rows) return;
@@ -570,7 +571,7 @@ __global__ void attn_combine_kernel(const float* __restrict__ ws_o, const float*
     }
     float m_s = -INFINITY, l_s = 0.f;
     if (lane < nsplit) {
-        const float2 ml = *reinterpret_cast<const float2*>(ws_ml + (static_cast<size_t>(lane) * rows + row) * 2);
+        const float2 ml = __ldcg(reinterpret_cast<const float2*>(ws_ml + (static_cast<size_t>(lane) * rows + row) * 2));
         m_s = ml.x;
         l_s = ml.y;
     }
@@ -620,6 +621,7 @@ __global__ void attn_combine_kernel(const float* __restrict__ ws_o, const float*
             if (lane * CPL + c < out_cols) dst[c] = e[c];
         }
     }
+    if (beside != 0) grid_dep_wait();
 }
 
 }  // namespace
@@ -672,24 +674,28 @@ AttnPlan make_biased_attn_plan(const bf16* q, int q_ld_tokens, const bf16* k_cac
 
 namespace {
 template <int DK, int DV, bool BIASED>
-void launch_attn(const AttnPlan& p, const AttnArgs& a, cudaStream_t s) {
+void launch_attn(const AttnPlan& p, const AttnArgs& a, AttnPart part, cudaStream_t s) {
     static bool configured = false;
     if (!configured) {
         CUDA_CHECK(cudaFuncSetAttribute(tree_attn_kernel<DK, DV, BIASED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         AttnCfg<DK, DV>::SMEM_TOTAL));
         configured = true;
     }
-    launch_kernel(tree_attn_kernel<DK, DV, BIASED>, dim3(a.num_mtiles * p.hkv, p.splits), dim3(NTHREADS), AttnCfg<DK, DV>::SMEM_TOTAL,
-                  s, p.tm_q, p.tm_k, p.tm_v, a);
-    if (p.splits > 1) {
+    if (part != ATTN_MERGE) {
+        launch_kernel(tree_attn_kernel<DK, DV, BIASED>, dim3(a.num_mtiles * p.hkv, p.splits), dim3(NTHREADS), AttnCfg<DK, DV>::SMEM_TOTAL,
+                      s, p.tm_q, p.tm_k, p.tm_v, a);
+    }
+    if (p.splits > 1 && part != ATTN_SPLITS) {
         const int rows = p.tq * p.hq;
         launch_kernel(attn_combine_kernel<DV>, dim3(ceil_div(rows, 4)), dim3(128), 0, s, p.ws_o, p.ws_ml, p.splits, rows, p.hq,
-                      BIASED && p.bias_exp > 0.f ? 1.f : a.scale_log2, p.out, p.out_ld, p.out_cols, p.sink, p.out_scale);
+                      BIASED && p.bias_exp > 0.f ? 1.f : a.scale_log2, p.out, p.out_ld, p.out_cols, p.sink, p.out_scale,
+                      part == ATTN_MERGE ? 1 : 0);
     }
 }
 }  // namespace
 
-void launch_tree_attention(const AttnPlan& p, cudaStream_t s) {
+void launch_tree_attention(const AttnPlan& p, cudaStream_t s, AttnPart part) {
+    if (part == ATTN_MERGE && p.splits == 1) return;
     ProfileScope prof(KC_ATTENTION, s);
     AttnArgs a;
     a.tq = p.tq; a.hq = p.hq; a.hkv = p.hkv;
@@ -747,9 +753,9 @@ void launch_tree_attention(const AttnPlan& p, cudaStream_t s) {
         launch_pair_attention(p, a, s);
         return;
     }
-    if (!p.biased) launch_attn<128, 128, false>(p, a, s);
-    else if (p.d == 128 && p.dv == 128) launch_attn<128, 128, true>(p, a, s);
-    else if (p.d == 128) launch_attn<128, 64, true>(p, a, s);
-    else if (p.dv == 128) launch_attn<64, 128, true>(p, a, s);
-    else launch_attn<64, 64, true>(p, a, s);
+    if (!p.biased) launch_attn<128, 128, false>(p, a, part, s);
+    else if (p.d == 128 && p.dv == 128) launch_attn<128, 128, true>(p, a, part, s);
+    else if (p.d == 128) launch_attn<128, 64, true>(p, a, part, s);
+    else if (p.dv == 128) launch_attn<64, 128, true>(p, a, part, s);
+    else launch_attn<64, 64, true>(p, a, part, s);
 }
