@@ -1122,6 +1122,7 @@ int cpmcu_layer_mixture(const cpmcu_layer_spec* spec, float* x32, void* xh, cons
         mix.y = y.p; mix.expert = m.b.expert; mix.weight = m.b.weight; mix.rank = m.b.rank; mix.offset = m.b.offset; mix.id_weight = m.b.id_weight;
         mix.top = sp.top; mix.experts = sp.experts;
         mix.shared_row0 = sp.shared_ff > 0 ? rows * sp.top : -1;
+        mix.early = single ? 1 : 0;
         launch_out_norm<bf16>(x32, static_cast<bf16*>(xh), nullptr, mix, mult, static_cast<const bf16*>(w), rows, width, ld, eps, s);
         sync_and_check("layer_mixture");
         return 0;

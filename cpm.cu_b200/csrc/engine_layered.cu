@@ -547,6 +547,7 @@ void Engine::layered_mixture(int i, LayeredPlans& lp, cudaStream_t s) {
     mix.expert = moe_.expert; mix.weight = moe_.weight; mix.rank = moe_.rank; mix.offset = moe_.offset; mix.id_weight = moe_.id_weight;
     mix.top = sp.top; mix.experts = sp.experts;
     mix.shared_row0 = sp.shared_ff > 0 ? rows * sp.top : -1;
+    mix.early = single && sizeof(T) == 2 ? 1 : 0;
     launch_out_norm<T>(x32_, static_cast<T*>(lx_), nullptr, mix, mc_.scale_residual, w.norm2, rows, W, L, mc_.eps, s);
 }
 

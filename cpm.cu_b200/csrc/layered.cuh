@@ -98,6 +98,7 @@ struct MoeMix {
     const float* id_weight = nullptr;// [rows]: weight of the input itself (identity experts)
     int top = 0, experts = 0;
     int shared_row0 = -1;            // >= 0: y rows from here are the shared expert's
+    int early = 0;                   // the router had finished before this launch could start (one bf16 row: gate/up and down hold it back)
 };
 template <typename T>
 void launch_out_norm(float* x32, T* xh, const T* delta, const MoeMix& mix, float mult, const bf16* w, int rows, int width, int ld,

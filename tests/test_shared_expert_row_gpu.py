@@ -1,7 +1,8 @@
-"""One token: the shared expert's gate/up product runs beside the router (one_row.cu).  More of its CTAs than the GPU holds at once, fewer, and a
-choice without any expert, against the plain mixture with the tolerances of the other mixtures; then whole passes, where the row, the activations
-and the cache lines of the layer before must not be seen: the same tokens twice give the same bits, and the logits agree with the plain
-model's as in the checks of whole models."""
+"""One token: the shared expert's gate/up product runs beside the router (one_row.cu), and the sum over the experts asks for the router's choice
+before its wait (layered_ops.cu).  More CTAs than the GPU holds at once, fewer, a choice without any expert, more experts than the sum
+has in flight, and a wide row, against the plain mixture with the tolerances of the other mixtures; then whole passes, where the row, the
+activations and the cache lines of the layer before must not be seen: the same tokens twice give the same bits, and the logits agree
+with the plain model's as in the checks of whole models."""
 import pytest
 import torch
 
@@ -13,7 +14,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("width,mlp", [(1024, moe(3, 2, 128, identity=1, shared=5200)), (512, moe(2, 1, 64, identity=6, shared=4800)),
-                                       (64, moe(1, 1, 64, identity=7, shared=64)), (4096, moe(2, 2, 8, shared=16))])
+                                       (64, moe(1, 1, 64, identity=7, shared=64)), (4096, moe(2, 2, 8, shared=16)),
+                                       (256, moe(40, 11, 64, identity=3, shared=64)), (4200, moe(3, 2, 16, identity=2, shared=16))])
 def test_mixture_of_one_row(width, mlp):
     mixture(width, mlp, 1)
 
