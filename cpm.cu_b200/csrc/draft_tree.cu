@@ -62,9 +62,10 @@ __device__ uint32_t warp_select(uint32_t* keys, int n, int k, int lane) {
 // threshold's lp (tau) and no more (k candidates of one segment above it would have raised it), so the candidates above it (got, in order)
 // stay, and the places behind them go to the lowest indices at it: from a segment's own logits where it may hide some, and each such
 // segment has one at least, else from its candidates.  k passes over the row by one warp took 4.3 ms a level at 73448 entries, which two
-// levels of a 64-token request met; ten rows with their best entries in one segment 9.7 ms, now 44 us (37 without any).
-__device__ __noinline__ void entries_at_threshold(const bf16* x, int vocab, const float4* rst, const unsigned long long* mycand, int nseg, int k, uint32_t got,
-                                                  uint32_t tau, float mx, float ls, int lane, int& my_idx, bf16& my_lp) {
+// levels of a 64-token request met; ten rows with their best entries in one segment 9.7 ms, now 55 us (45 without any).
+__device__ __noinline__ int2 entries_at_threshold(const bf16* x, int vocab, const float4* rst, const unsigned long long* mycand, int nseg, int k, uint32_t got,
+                                                  uint32_t tau, float mx, float ls, int lane) {
+    int my_idx = 0;
     auto lp_of = [&](bf16 v) { return __float2bfloat16(__bfloat162float(v) - mx - ls); };
     int have = __popc(__ballot_sync(0xffffffffu, lane < k && (got >> 16) > tau));
     if (lane < have) my_idx = key_index(mycand[0xFFFF - (got & 0xFFFFu)]);
@@ -72,12 +73,12 @@ __device__ __noinline__ void entries_at_threshold(const bf16* x, int vocab, cons
         const uint32_t xk = __float_as_uint(rst[sg].z);
         if (xk != 0u && bf16_orderable(lp_of(bf16_from_orderable(xk))) >= tau) {
             const int end = min((sg + 1) * SEG, vocab);
-            for (int at = sg * SEG; at < end && have < k; at += 256) {
-                bf16 v[8];
+            for (int at = sg * SEG; at < end && have < k; at += 128) {
+                bf16 v[4];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) v[j] = at + j * 32 + lane < end ? x[at + j * 32 + lane] : __float2bfloat16(0.f);
+                for (int j = 0; j < 4; ++j) v[j] = at + j * 32 + lane < end ? x[at + j * 32 + lane] : __float2bfloat16(0.f);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
+                for (int j = 0; j < 4; ++j) {
                     uint32_t hit = __ballot_sync(0xffffffffu, at + j * 32 + lane < end && bf16_orderable(lp_of(v[j])) == tau);
                     for (; hit != 0u && have < k; hit &= hit - 1u, ++have) {
                         if (lane == have) my_idx = at + j * 32 + __ffs(hit) - 1;
@@ -93,7 +94,7 @@ __device__ __noinline__ void entries_at_threshold(const bf16* x, int vocab, cons
             }
         }
     }
-    if (lane < have) my_lp = lp_of(x[my_idx]);
+    return make_int2(my_idx, lane < have ? static_cast<int>(__bfloat16_as_ushort(lp_of(x[my_idx]))) : 0);
 }
 
 // One launch per draft level: log-softmax statistics, top-k and frontier expansion.
@@ -111,7 +112,8 @@ __device__ __noinline__ void entries_at_threshold(const bf16* x, int vocab, cons
 // candidate still reaches the answer's threshold lp (all k of its candidates compete in the top bucket); the last
 // CTA detects that and looks for such a row's entries at the threshold in those segments' logits.  With 36 segments and k = 10 this
 // needs ten of a row's best entries inside one segment; the small vocabularies of the tests take the path routinely.
-__global__ void draft_level_kernel(DraftTreeState st, const bf16* __restrict__ logits, int ld, int vocab, int nseg,
+// Three CTAs per SM: the full vocabulary's 360 are one wave (with two per SM the six levels of a step took 1.432 ms with their passes, now 1.411).
+__global__ void __launch_bounds__(SCAN_THREADS, 3) draft_level_kernel(DraftTreeState st, const bf16* __restrict__ logits, int ld, int vocab, int nseg,
                                    float4* __restrict__ stats, unsigned long long* __restrict__ cand,
                                    unsigned* __restrict__ ticket, int level, const int32_t* __restrict__ last_row_ptr,
                                    int group_rows) {
@@ -285,7 +287,9 @@ __global__ void draft_level_kernel(DraftTreeState st, const bf16* __restrict__ l
             bf16 my_lp = __float2bfloat16(0.f);
             int my_idx = 0;
             if (__any_sync(0xffffffffu, saturated)) {
-                entries_at_threshold(logits + static_cast<size_t>(r + row0) * ld, vocab, rst, mycand, nseg, k, got, tau, mx, ls, lane, my_idx, my_lp);
+                const int2 at = entries_at_threshold(logits + static_cast<size_t>(r + row0) * ld, vocab, rst, mycand, nseg, k, got, tau, mx, ls, lane);
+                my_idx = at.x;
+                my_lp = __ushort_as_bfloat16(static_cast<unsigned short>(at.y));
             } else if (got) {
                 const unsigned long long c = mycand[0xFFFF - (got & 0xFFFFu)];
                 my_idx = key_index(c);
