@@ -252,6 +252,8 @@ def decode(input_length, padded_length, input, position_ids, cache_length, mask_
 
 
 def decode_token(token, position, work, output, cuda_graph):
+    if not -2**31 <= token < 2**31:   # ctypes would keep the low 32 bits without a word
+        raise OverflowError(f"token id {token} does not fit 32 bits")
     call("cpmcu_decode_token", token, position, work, output, int(cuda_graph))
 
 

@@ -734,6 +734,7 @@ void Engine::decode(int n, int padded_len, const int32_t* ids, const int32_t* po
 void Engine::decode_token(int token, int position, void* work, void* logits_out, bool cuda_graph) {
     CPM_REQUIRE(storage_ready_, "decode before init_storage");
     CPM_REQUIRE(position >= 0 && position < budget_, "decode: cache length + tokens exceeds the KV budget");
+    CPM_REQUIRE(token >= 0 && token < mc_.vocab, "decode: token id outside the vocabulary");
     require_room(1, "decode");
     launch_stage_token(d_in_, token, position, runtime().stream);
     if (layered()) layered_decode(1, d_in_.ids, d_in_.len, work, cuda_graph, logits_out);

@@ -166,7 +166,8 @@ int cpmcu_decode(int input_length, int padded_length, const int32_t* input, cons
                  const int32_t* cache_length, const uint64_t* mask_2d, void* output, int cuda_graph);
 
 /* cpmcu_decode of one token that the host has: `token` becomes cache row `position`, its logits [vocab] go to `output` (device, any
- * buffer).  work: device buffer of the same size, the same one in every call (layered models capture the step over it). */
+ * buffer).  work: device buffer of the same size, the same one in every call (layered models capture the step over it).  An id outside the
+ * vocabulary or a position outside the cache is refused before anything is launched. */
 int cpmcu_decode_token(int token, int position, void* work, void* output, int cuda_graph);
 
 /* reference: draft, src/entry.cu:498.  Reads tree_draft_ids[0] (root) and
