@@ -105,11 +105,18 @@ __global__ void rms_norm_kernel(bf16* __restrict__ x, int ldx, const bf16* __res
     }
 }
 
-__global__ void embedding_kernel(const int32_t* __restrict__ ids, const bf16* __restrict__ table,
-                                 bf16* __restrict__ out, int ld_out, int dim, float scale) {
+// The id of a row; outside the vocabulary: token 0, reported.
+__device__ __forceinline__ size_t known_token(int id, int vocab, int* error) {
+    if (id >= 0 && id < vocab) return id;
+    if (threadIdx.x == 0) atomicOr(error, ERR_BAD_TOKEN);
+    return 0;
+}
+
+__global__ void embedding_kernel(const int32_t* __restrict__ ids, const bf16* __restrict__ table, int vocab,
+                                 bf16* __restrict__ out, int ld_out, int dim, float scale, int* __restrict__ error) {
     grid_dependency_sync();
     const int row = blockIdx.x;
-    const size_t src = static_cast<size_t>(ids[row]) * dim;
+    const size_t src = known_token(ids[row], vocab, error) * dim;
     const size_t dst = static_cast<size_t>(row) * ld_out;
     for (int i = threadIdx.x * 8; i < dim; i += blockDim.x * 8) {
         uint4 v = *reinterpret_cast<const uint4*>(table + src + i);
@@ -124,10 +131,10 @@ __global__ void embedding_kernel(const int32_t* __restrict__ ids, const bf16* __
 
 // Embedding rows (blockIdx.y == 0) and, in the same launch, gathered hidden rows
 // hid_out[r] = h_rows[src[r]] (blockIdx.y == 1): the two halves of the draft layer's input.
-__global__ void embedding_gather_kernel(const int32_t* __restrict__ ids, const bf16* __restrict__ table,
+__global__ void embedding_gather_kernel(const int32_t* __restrict__ ids, const bf16* __restrict__ table, int vocab,
                                         bf16* __restrict__ out, int ld_out, int dim, float scale,
                                         const bf16* __restrict__ h_rows, int h_ld, const int32_t* __restrict__ src,
-                                        bf16* __restrict__ hid_out, int hid_ld) {
+                                        bf16* __restrict__ hid_out, int hid_ld, int* __restrict__ error) {
     grid_dependency_sync();
     const int row = blockIdx.x;
     if (blockIdx.y == 1) {
@@ -136,7 +143,7 @@ __global__ void embedding_gather_kernel(const int32_t* __restrict__ ids, const b
         for (int c = threadIdx.x; c < dim / 8; c += blockDim.x) d4[c] = s4[c];
         return;
     }
-    const size_t from = static_cast<size_t>(ids[row]) * dim;
+    const size_t from = known_token(ids[row], vocab, error) * dim;
     const size_t dst = static_cast<size_t>(row) * ld_out;
     for (int i = threadIdx.x * 8; i < dim; i += blockDim.x * 8) {
         uint4 v = *reinterpret_cast<const uint4*>(table + from + i);
@@ -478,21 +485,21 @@ void launch_add_rms_norm(bf16* x, const bf16* delta, float delta_scale, const bf
     }
 }
 
-void launch_embedding(const int32_t* ids, const bf16* table, bf16* out, int ld_out, int rows, int dim, float scale,
+void launch_embedding(const int32_t* ids, const bf16* table, int vocab, bf16* out, int ld_out, int rows, int dim, float scale,
                       cudaStream_t s) {
     if (rows <= 0) return;
     CPM_REQUIRE(dim % 8 == 0 && ld_out % 8 == 0, "embedding: dim must be a multiple of 8");
-    launch_kernel(embedding_kernel, dim3(rows), dim3(128), 0, s, ids, table, out, ld_out, dim, scale);
+    launch_kernel(embedding_kernel, dim3(rows), dim3(128), 0, s, ids, table, vocab, out, ld_out, dim, scale, runtime().d_error);
 }
 
-void launch_embedding_gather(const int32_t* ids, const bf16* table, bf16* out, int ld_out, int rows, int dim, float scale,
+void launch_embedding_gather(const int32_t* ids, const bf16* table, int vocab, bf16* out, int ld_out, int rows, int dim, float scale,
                              const bf16* h_rows, int h_ld, const int32_t* src, bf16* hid_out, int hid_ld,
                              cudaStream_t s) {
     if (rows <= 0) return;
     CPM_REQUIRE(dim % 8 == 0 && ld_out % 8 == 0 && h_ld % 8 == 0 && hid_ld % 8 == 0,
                 "embedding: dim and row strides must be multiples of 8");
-    launch_kernel(embedding_gather_kernel, dim3(rows, 2), dim3(128), 0, s, ids, table, out, ld_out, dim, scale, h_rows, h_ld,
-                  src, hid_out, hid_ld);
+    launch_kernel(embedding_gather_kernel, dim3(rows, 2), dim3(128), 0, s, ids, table, vocab, out, ld_out, dim, scale, h_rows, h_ld,
+                  src, hid_out, hid_ld, runtime().d_error);
 }
 
 void launch_rope_append(bf16* qkv, int rows, int hq, int hkv, int d, const float* inv_freq, const int32_t* pos,

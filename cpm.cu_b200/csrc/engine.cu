@@ -605,7 +605,7 @@ void Engine::lm_head_rows(const bf16* x, int x_rows, int rows, bf16* logits_out,
 void Engine::target_forward(ForwardPlans& fp, const RowCtx& c, const int32_t* ids, bool all_logits,
                             bf16* logits_out, int logits_ld, cudaStream_t s) {
     const int H = mc_.hidden, rows = c.rows;
-    launch_embedding(ids, embed_, x_, H, rows, H, mc_.scale_embed, s);
+    launch_embedding(ids, embed_, mc_.vocab, x_, H, rows, H, mc_.scale_embed, s);
     sparse_prepare(c, s);
     const bf16* pending = nullptr;
     for (int l = 0; l < mc_.layers; ++l) {
@@ -644,7 +644,7 @@ void Engine::prefill_rows(int n, int history, const int32_t* ids, const int32_t*
     const int H = mc_.hidden;
     if (has_eagle_ && history > 0) {
         // deferred draft prefill of the previous chunk; its last "next token" is this chunk's first token
-        launch_embedding(ids, embed_, prev_embed_ + static_cast<size_t>(num_prev_ - 1) * H, H, 1, H, mc_.scale_embed, s);
+        launch_embedding(ids, embed_, mc_.vocab, prev_embed_ + static_cast<size_t>(num_prev_ - 1) * H, H, 1, H, mc_.scale_embed, s);
         draft_first(num_history_, s);
     }
     CUDA_CHECK(cudaMemcpyAsync(st_ + 6, &history, sizeof(int), cudaMemcpyHostToDevice, s));
@@ -702,7 +702,7 @@ void Engine::prefill_rows(int n, int history, const int32_t* ids, const int32_t*
         }
     }
     if (has_eagle_) {
-        if (n > 1) launch_embedding(ids + 1, embed_, prev_embed_, H, n - 1, H, mc_.scale_embed, s);
+        if (n > 1) launch_embedding(ids + 1, embed_, mc_.vocab, prev_embed_, H, n - 1, H, mc_.scale_embed, s);
         copy_rows(prev_hidden_, H, norm_out_, H, n, H, s);
         CUDA_CHECK(cudaMemcpyAsync(eagle_pos_, pos, static_cast<size_t>(n) * 4, cudaMemcpyDeviceToDevice, s));
         num_prev_ = n;
@@ -945,12 +945,12 @@ void Engine::draft_levels(int32_t* tree_ids, int32_t* tree_pos, const int32_t* c
     }
     for (int d = 1; d < ec_.num_iter; ++d) {
         if (ec_.use_input_norm) {
-            launch_embedding_gather(tree_.fr_id, embed_, e_emb_, H, k, H, mc_.scale_embed, h_src, H, tree_.fr_src, hid_dst,
+            launch_embedding_gather(tree_.fr_id, embed_, mc_.vocab, e_emb_, H, k, H, mc_.scale_embed, h_src, H, tree_.fr_src, hid_dst,
                                     hid_ld, s);
             launch_rms_norm(e_emb_, H, in_norm1_, e_in_, ein_ld(), k, H, mc_.eps, s);
             launch_rms_norm(e_hid_, H, in_norm2_, ein_hidden(), ein_ld(), k, H, mc_.eps, s);
         } else {
-            launch_embedding_gather(tree_.fr_id, embed_, e_in_, ein_ld(), k, H, mc_.scale_embed, h_src, H, tree_.fr_src, hid_dst,
+            launch_embedding_gather(tree_.fr_id, embed_, mc_.vocab, e_in_, ein_ld(), k, H, mc_.scale_embed, h_src, H, tree_.fr_src, hid_dst,
                                     hid_ld, s);
         }
         h_src = e_h_;
@@ -983,7 +983,7 @@ void Engine::draft(int32_t* tree_ids, int32_t* tree_pos, const int32_t* cache_le
     const int H = mc_.hidden;
     if (first_draft_) {
         // the root token's embedding is the last "next token" input of the prompt rows
-        launch_embedding(tree_ids, embed_, prev_embed_ + static_cast<size_t>(num_prev_ - 1) * H, H, 1, H,
+        launch_embedding(tree_ids, embed_, mc_.vocab, prev_embed_ + static_cast<size_t>(num_prev_ - 1) * H, H, 1, H,
                          mc_.scale_embed, s);
         draft_first(num_history_, s);
     } else {
@@ -1101,7 +1101,7 @@ void Engine::enqueue_step(bool first, cudaStream_t s) {
     const bool capturing = (cap == cudaStreamCaptureStatusActive);
     launch_kernel(state_sync_kernel, dim3(1), dim3(1), 0, s, st_, static_cast<const int32_t*>(nullptr), t_ids_, 1);
     if (first) {
-        launch_embedding(t_ids_, embed_, prev_embed_ + static_cast<size_t>(num_prev_ - 1) * H, H, 1, H, mc_.scale_embed, s);
+        launch_embedding(t_ids_, embed_, mc_.vocab, prev_embed_ + static_cast<size_t>(num_prev_ - 1) * H, H, 1, H, mc_.scale_embed, s);
         draft_first(num_history_, s);
     } else {
         draft_catchup(s);
@@ -1120,7 +1120,7 @@ void Engine::enqueue_step(bool first, cudaStream_t s) {
     ForwardPlans& fp = target_plans(T);
     const int V = mc_.vocab;
     // target forward; the LM-head plan is cached because its output buffer is engine-owned
-    launch_embedding(t_ids_, embed_, x_, H, T, H, mc_.scale_embed, s);
+    launch_embedding(t_ids_, embed_, mc_.vocab, x_, H, T, H, mc_.scale_embed, s);
     sparse_prepare(c, s);
     const bf16* pending = nullptr;
     for (int l = 0; l < mc_.layers; ++l) {
