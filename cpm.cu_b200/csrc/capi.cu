@@ -477,6 +477,20 @@ int cpmcu_debug_decode_graphs(const int32_t* shapes, int n, int32_t* acts) {
     });
 }
 
+int cpmcu_debug_launch_order(const int32_t* holds, int n, int32_t* ended) {
+    return guarded([&] {
+        CPM_REQUIRE(holds != nullptr && ended != nullptr && n >= 0, "debug_launch_order: bad arguments");
+        LaunchOrder order;
+        for (int i = 0; i < n; ++i) {
+            ended[i] = 0;
+            while (order.ended(ended[i] + 1)) ++ended[i];
+            order.launched();
+            if (holds[i] != 0) order.held();
+        }
+        return 0;
+    });
+}
+
 int cpmcu_linear_swiglu_bf16(const void* x, const void* w, void* out, int rows, int inter, int K, int grid_limit) {
     return guarded([&] {
         Runtime& rt = runtime();
@@ -1018,7 +1032,7 @@ int cpmcu_grouped_linear(const void* x, const void* w, int n, int N, int N_s, in
         const bf16* src = static_cast<const bf16*>(w);
         for (int i = 0; i < n; ++i) retile_weight_rows(src + static_cast<size_t>(i) * N * K, N, K, static_cast<bf16*>(t.p) + i * one, K, 0, 0, 0, s);
         if (N_s > 0) retile_weight_rows(src + static_cast<size_t>(n) * N * K, N_s, K, static_cast<bf16*>(t.p) + n * one, K, 0, 0, 0, s);
-        launch_moe_gemm(make_grouped_plan(static_cast<const bf16*>(t.p), n, N, N_s, K, static_cast<const bf16*>(x), static_cast<bf16*>(y), ldy, rows), s);
+        launch_grouped(make_grouped_plan(static_cast<const bf16*>(t.p), n, N, N_s, K, static_cast<const bf16*>(x), static_cast<bf16*>(y), ldy, rows), s);
         sync_and_check("grouped_linear");
         return 0;
     });
@@ -1114,15 +1128,15 @@ int cpmcu_layer_mixture(const cpmcu_layer_spec* spec, float* x32, void* xh, cons
                                                single ? 1 : rows * sp.top, x, ld, static_cast<bf16*>(act.p), ld_act, rows, tile, m.b);
         MoeGemmPlan p2 = make_moe_down_plan(sp, static_cast<const bf16*>(dn.p), static_cast<const bf16*>(act.p), slots, ld_act, width,
                                             static_cast<bf16*>(y.p), ld, rows, tile, m.b);
-        launch_moe_route(sp, x32, static_cast<const bf16*>(router), correction, m.b, rows, ld, tile, single, s);
+        const long routed = launch_moe_route(sp, x32, static_cast<const bf16*>(router), correction, m.b, rows, ld, tile, single, s);
         if (!single) launch_moe_gather<bf16>(sp, x, static_cast<bf16*>(mx.p), m.b, rows, ld, s);
-        launch_moe_gemm(p1, s);
-        launch_moe_gemm(p2, s);
+        launch_moe_gemm(p1, s, routed);
+        launch_moe_gemm(p2, s, routed);
         MoeMix mix;
         mix.y = y.p; mix.expert = m.b.expert; mix.weight = m.b.weight; mix.rank = m.b.rank; mix.offset = m.b.offset; mix.id_weight = m.b.id_weight;
         mix.top = sp.top; mix.experts = sp.experts;
         mix.shared_row0 = sp.shared_ff > 0 ? rows * sp.top : -1;
-        mix.early = single ? 1 : 0;
+        mix.routed = routed;
         launch_out_norm<bf16>(x32, static_cast<bf16*>(xh), nullptr, mix, mult, static_cast<const bf16*>(w), rows, width, ld, eps, s);
         sync_and_check("layer_mixture");
         return 0;
@@ -1176,12 +1190,12 @@ int cpmcu_bench_experts(const cpmcu_layer_spec* spec, int width, int rows, int c
                                                        ld_act, width, static_cast<bf16*>(y.p), ld, rows, tile, m.b));
                 }
             }
-            for (int c = 0; c < 3; ++c) launch_moe_gemm(plans[c % copies], s);
+            for (int c = 0; c < 3; ++c) launch_moe_gemm(plans[c % copies], s, 0);
             cudaEvent_t e0, e1;
             CUDA_CHECK(cudaEventCreate(&e0));
             CUDA_CHECK(cudaEventCreate(&e1));
             CUDA_CHECK(cudaEventRecord(e0, s));
-            for (int i = 0; i < iters; ++i) launch_moe_gemm(plans[i % copies], s);
+            for (int i = 0; i < iters; ++i) launch_moe_gemm(plans[i % copies], s, 0);
             CUDA_CHECK(cudaEventRecord(e1, s));
             CUDA_CHECK(cudaStreamSynchronize(s));
             float ms = 0.f;

@@ -11,6 +11,8 @@
 #include <utility>
 #include <vector>
 
+#include "launch_order.h"
+
 typedef __nv_bfloat16 bf16;
 
 #define CUDA_CHECK(expr)                                                                            \
@@ -77,6 +79,7 @@ struct Runtime {
     int num_sms = 148;
     int device = 0;
     long launches = 0;  // kernels launched (or captured) so far by this library
+    LaunchOrder order;
     bool pdl = true;  // launch kernels with programmatic stream serialization (prologue overlap)
     // Optional per-launch timing (eager runs only): event pairs per kernel class.
     bool profile = false;
@@ -97,7 +100,8 @@ int read_and_clear_error();  // synchronises the stream
 
 // Kernel launch with programmatic dependent launch enabled: the grid may start
 // while its predecessor in the stream drains; every kernel here executes
-// griddepcontrol.wait before touching global memory, which restores the order.
+// griddepcontrol.wait before it touches memory that a launch before it may have
+// written, which restores the order.  The exceptions are listed at grid_dep_trigger().
 template <typename... KArgs, typename... Args>
 void launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
     cudaLaunchConfig_t cfg = {};
@@ -112,6 +116,7 @@ void launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
     cfg.numAttrs = runtime().pdl ? 1 : 0;
     CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...));
     runtime().launches++;
+    runtime().order.launched();
 }
 
 // The same for a kernel that runs as thread-block clusters of `cluster` CTAs (grid.x a multiple of it).
@@ -134,6 +139,7 @@ void launch_kernel_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size
     cfg.numAttrs = runtime().pdl ? 2 : 1;
     CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...));
     runtime().launches++;
+    runtime().order.launched();
 }
 
 // Clusters of `cluster` CTAs of this kernel that the device runs at once (0 when the query fails).  The SMs
@@ -159,9 +165,19 @@ int max_active_clusters(void (*kernel)(KArgs...), dim3 block, size_t smem, int c
     return n;
 }
 
-// Device side of the above.  Every kernel lets its successor start launching at once
-// (the successor can only set up and read constant data until its own wait returns) and
-// waits for its predecessor before it touches anything a previous kernel may have written.
+// Device side of the above.  A kernel lets its successor start launching at once (the successor can only set up and read constant
+// data until its own wait returns) and waits for its predecessor before it touches anything a previous kernel may have written,
+// but for these:
+//   hold the successor back until their own wait is over   moe_route_one_kernel, the experts' gate/up products (moe.cu, one_row.cu), one_row_kernel with
+//                                                           HOLD, scan_step_kernel (hold)
+//   use what older launches wrote before they wait          the experts' down products (the router's choice), one_row_kernel (ahead),
+//                                                           out_norm_kernel (early), qkv_norm_append_kernel (BESIDE), attn_combine_kernel (beside)
+// What the latter use was written by launches that have ended before they start; their launchers ask LaunchOrder for that, and where it is not
+// so they wait as all others do, or the launch is refused (down products).  A launch that begins so still ends after its predecessor: some CTA
+// of it, or every thread at its end, waits.  Such data is read past the first-level cache (__ldcg): the writes of a grid that has ended are in L2,
+// whereas that a first-level cache holds nothing older is promised to those who wait themselves.  That an L2 read suffices is how the
+// hardware behaves, not something the programming guide states.
+// The token shifts and recurrent states that kernels fetch before their wait are those of the pass before, which the host has waited for.
 __device__ __forceinline__ void grid_dep_trigger() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
@@ -266,7 +282,7 @@ struct SideRow {
     int table_ld = 0, col0 = 0, vocab = 0;
 };
 // M == 1, bf16 weights; with `rope` the product is q, k and v, which are rotated and appended; with `side` the side input's gate
-// hold: the next launch starts only after this one's wait (a plain product)
+// hold: the next launch starts only after this one's wait (a plain product; LaunchOrder)
 void launch_linear_one_row(const LinearPlan& plan, cudaStream_t stream, const RopeRow* rope = nullptr, const SideRow* side = nullptr, bool hold = false);
 bool linear_one_row_fits(int N, int K, int sms);   // whether that is the faster way for one row of N outputs
 // Same contract with 4-bit weights, w = (q - 8) * scale, K % 256 == 0 and N % 128 == 0.  `wq` holds one
@@ -379,7 +395,7 @@ bool biased_attn_fits(int hq, int hkv, int dk, int dv);
 AttnPlan make_biased_attn_plan(const bf16* q, int q_ld_tokens, const bf16* k_cache, const bf16* v_cache, int budget, int tq,
                                int hq, int hkv, int dk, int dv, int out_cols, int splits, float scale, int exact_window,
                                float bias_exp, bf16* out, int out_ld, float* ws_o, float* ws_ml);
-// One key split after the other, and the merge of several: in one call, or with other work between.  The merge alone runs beside its predecessor,
-// which starts it after its own wait, i.e. behind the splits.
+// One key split after the other, and the merge of several: in one call, or with other work between.  The merge alone runs beside its predecessor
+// where launch `splits_at` (LaunchOrder::issued right after the splits) has ended before it starts.
 enum AttnPart { ATTN_ALL, ATTN_SPLITS, ATTN_MERGE };
-void launch_tree_attention(const AttnPlan& p, cudaStream_t s, AttnPart part = ATTN_ALL);
+void launch_tree_attention(const AttnPlan& p, cudaStream_t s, AttnPart part = ATTN_ALL, long splits_at = 0);

@@ -219,11 +219,11 @@ private:
     void layered_mixture(int layer, LayeredPlans& lp, cudaStream_t s);
     // attention of lx_ and / or the recurrence of its mixes; the outputs lie side by side in lattn_
     template <typename T>
-    void layered_queries(int layer, LayeredPlans& lp, const int32_t* kv_len, int kv_off, bool beside, cudaStream_t s);
+    void layered_queries(int layer, LayeredPlans& lp, const int32_t* kv_len, int kv_off, long written_by, cudaStream_t s);
     template <typename T>
-    void layered_attention(int layer, LayeredPlans& lp, const int32_t* kv_len, int kv_off, AttnPart part, cudaStream_t s);
+    void layered_attention(int layer, LayeredPlans& lp, const int32_t* kv_len, int kv_off, AttnPart part, long splits_at, cudaStream_t s);
     template <typename T>
-    bool layered_rec_products(int layer, LayeredPlans& lp, bool hold, cudaStream_t s);   // whether they hold their successor back
+    void layered_rec_products(int layer, LayeredPlans& lp, bool hold, cudaStream_t s);   // hold: where they can, they hold their successor back
     template <typename T>
     void layered_recurrence(int layer, LayeredPlans& lp, const int32_t* kv_len, int kv_off, bool hold, cudaStream_t s);
     template <typename T>

@@ -521,11 +521,11 @@ void Engine::layered_mixture(int i, LayeredPlans& lp, cudaStream_t s) {
     const int rows = lp.rows, L = ld(), W = mc_.hidden;
     const bool single = rows == 1;
     const int tile = mc_.fp32 ? kF32Rows : lp.layers[i].gate_up.tile;
-    launch_moe_route(sp, x32_, w.router, w.correction, moe_, rows, L, tile, single, s);
+    const long routed = launch_moe_route(sp, x32_, w.router, w.correction, moe_, rows, L, tile, single, s);
     if (!single) launch_moe_gather<T>(sp, static_cast<const T*>(lx_), static_cast<T*>(moe_x_), moe_, rows, L, s);
     if constexpr (sizeof(T) == 2) {
-        launch_moe_gemm(lp.layers[i].gate_up, s);
-        launch_moe_gemm(lp.layers[i].down, s);
+        launch_moe_gemm(lp.layers[i].gate_up, s, routed);
+        launch_moe_gemm(lp.layers[i].down, s, routed);
     } else {
         const float* x = static_cast<const float*>(lx_);
         float *gu = static_cast<float*>(moe_gu_), *act = static_cast<float*>(moe_act_), *y = static_cast<float*>(moe_y_);
@@ -547,7 +547,7 @@ void Engine::layered_mixture(int i, LayeredPlans& lp, cudaStream_t s) {
     mix.expert = moe_.expert; mix.weight = moe_.weight; mix.rank = moe_.rank; mix.offset = moe_.offset; mix.id_weight = moe_.id_weight;
     mix.top = sp.top; mix.experts = sp.experts;
     mix.shared_row0 = sp.shared_ff > 0 ? rows * sp.top : -1;
-    mix.early = single && sizeof(T) == 2 ? 1 : 0;
+    mix.routed = routed;
     launch_out_norm<T>(x32_, static_cast<T*>(lx_), nullptr, mix, mc_.scale_residual, w.norm2, rows, W, L, mc_.eps, s);
 }
 
@@ -558,7 +558,7 @@ void Engine::run_product(const LayeredProduct& p, int rows, cudaStream_t s) {
 }
 
 template <typename T>
-void Engine::layered_queries(int i, LayeredPlans& lp, const int32_t* kv_len, int kv_off, bool beside, cudaStream_t s) {
+void Engine::layered_queries(int i, LayeredPlans& lp, const int32_t* kv_len, int kv_off, long written_by, cudaStream_t s) {
     const LayerSpec& sp = mc_.specs[i];
     const LayeredWeights& w = lw_[i];
     LayeredPlans::Layer& l = lp.layers[i];
@@ -573,12 +573,12 @@ void Engine::layered_queries(int i, LayeredPlans& lp, const int32_t* kv_len, int
     a.k_cache = sp.kv_from >= 0 ? nullptr : w.k;
     a.v_cache = sp.kv_from >= 0 ? nullptr : w.v;
     a.kv_len = kv_len; a.kv_off = kv_off; a.cache_rows = budget_; a.error = runtime().d_error;
-    a.beside = beside ? 1 : 0;
+    a.written_by = written_by;
     launch_qkv_norm_append<T>(a, rows, s);
 }
 
 template <typename T>
-void Engine::layered_attention(int i, LayeredPlans& lp, const int32_t* kv_len, int kv_off, AttnPart part, cudaStream_t s) {
+void Engine::layered_attention(int i, LayeredPlans& lp, const int32_t* kv_len, int kv_off, AttnPart part, long splits_at, cudaStream_t s) {
     const LayerSpec& sp = mc_.specs[i];
     const LayeredWeights& w = lw_[i];
     LayeredPlans::Layer& l = lp.layers[i];
@@ -586,7 +586,7 @@ void Engine::layered_attention(int i, LayeredPlans& lp, const int32_t* kv_len, i
     if (l.tensor_attn) {
         l.attn.kv_len = kv_len;
         l.attn.kv_len_add = kv_off + rows;
-        launch_tree_attention(l.attn, s, part);
+        launch_tree_attention(l.attn, s, part, splits_at);
     } else if (part != ATTN_MERGE) {
         PlainAttnArgs pa;
         pa.q = lq_; pa.k_cache = w.k; pa.v_cache = w.v; pa.out = lattn_;
@@ -600,22 +600,20 @@ void Engine::layered_attention(int i, LayeredPlans& lp, const int32_t* kv_len, i
 }
 
 template <typename T>
-bool Engine::layered_rec_products(int i, LayeredPlans& lp, bool hold, cudaStream_t s) {
+void Engine::layered_rec_products(int i, LayeredPlans& lp, bool hold, cudaStream_t s) {
     LayeredPlans::Layer& l = lp.layers[i];
     if (sizeof(T) == 2 && mc_.specs[i].rec == REC_TIME_MIX) {
-        launch_moe_gemm(l.mixes, s, hold);
-        return hold;
+        launch_grouped(l.mixes, s, hold);
+        return;
     }
     for (const LayeredProduct& p : l.rec) {
-        hold = hold && p.plan.one_row;
-        if (hold) {
+        if (hold && p.plan.one_row) {
             ProfileScope prof(KC_LINEAR, s);
             launch_linear_one_row(p.plan, s, nullptr, nullptr, true);
         } else {
             run_product<T>(p, lp.rows, s);
         }
     }
-    return hold;
 }
 
 template <typename T>
@@ -701,20 +699,23 @@ bool Engine::layered_tanh_layer(int i, LayeredPlans& lp, const int32_t* ids, con
     if (both && sizeof(T) == 2 && rows == 1 && scan_step_fits(sp.rec_dim, sp.rec_vdim, sp.rec == REC_TIME_MIX)) {
         // Two chains of one token's row: its queries and keys are normalised beside the recurrence's product, the splits of its attention are
         // merged beside the recurrence's step.  Each of the two pairs is one launch that starts its successor after its own wait and a
-        // successor that waits at its end.  1405 + 24 tokens of nine layers of 3072, six of them of this kind: 29.6 ms one after the other, 28.95
+        // successor that waits at its end (LaunchOrder).  1405 + 24 tokens of nine layers of 3072, six of them of this kind: 29.6 ms one after the other, 28.95
         // so; with the product beside the norms instead it starts its weights later and took 29.1.
         const bool merge = l.tensor_attn && l.attn.splits > 1;
+        const LaunchOrder& order = runtime().order;
         run_product<T>(l.qkv, rows, s);
-        const bool held = layered_rec_products<T>(i, lp, true, s);
-        layered_queries<T>(i, lp, kv_len, kv_off, held, s);
-        layered_attention<T>(i, lp, kv_len, kv_off, ATTN_SPLITS, s);
+        const long qkv_at = order.issued;
+        layered_rec_products<T>(i, lp, true, s);
+        layered_queries<T>(i, lp, kv_len, kv_off, qkv_at, s);
+        layered_attention<T>(i, lp, kv_len, kv_off, ATTN_SPLITS, 0, s);
+        const long splits_at = order.issued;
         layered_recurrence<T>(i, lp, kv_len, kv_off, merge, s);
-        layered_attention<T>(i, lp, kv_len, kv_off, ATTN_MERGE, s);
+        layered_attention<T>(i, lp, kv_len, kv_off, ATTN_MERGE, splits_at, s);
     } else {
         if (sp.heads > 0) {
             run_product<T>(l.qkv, rows, s);
-            layered_queries<T>(i, lp, kv_len, kv_off, false, s);
-            layered_attention<T>(i, lp, kv_len, kv_off, ATTN_ALL, s);
+            layered_queries<T>(i, lp, kv_len, kv_off, 0, s);
+            layered_attention<T>(i, lp, kv_len, kv_off, ATTN_ALL, 0, s);
         }
         if (sp.rec != REC_NONE) {
             layered_rec_products<T>(i, lp, false, s);
@@ -776,8 +777,8 @@ void Engine::layered_forward(int rows, const int32_t* ids, const int32_t* kv_len
             ready = layered_tanh_layer<T>(li, lp, ids, kv_len, kv_off, s);
         } else {
             run_product<T>(lp.layers[i].qkv, rows, s);
-            layered_queries<T>(static_cast<int>(i), lp, kv_len, kv_off, false, s);
-            layered_attention<T>(static_cast<int>(i), lp, kv_len, kv_off, ATTN_ALL, s);
+            layered_queries<T>(static_cast<int>(i), lp, kv_len, kv_off, 0, s);
+            layered_attention<T>(static_cast<int>(i), lp, kv_len, kv_off, ATTN_ALL, 0, s);
             run_product<T>(lp.layers[i].o, rows, s);
             launch_out_norm<T>(x32_, static_cast<T*>(lx_), static_cast<const T*>(ldelta_), MoeMix(), mc_.scale_residual, w.norm1, rows, W, L, mc_.eps, s);
             if (sp.experts + sp.identity > 0) layered_mixture<T>(static_cast<int>(i), lp, s);

@@ -82,7 +82,7 @@ struct QkvNormArgs {
     const int32_t* kv_len;
     int kv_off, cache_rows;
     int* error;
-    int beside = 0;          // the predecessor leaves qkv alone and has started this launch after its own wait: run beside it
+    long written_by = 0;     // the launch that wrote qkv (LaunchOrder): where it has ended before this one starts, this one runs beside its predecessor (bf16)
 };
 template <typename T>
 void launch_qkv_norm_append(const QkvNormArgs& a, int rows, cudaStream_t s);
@@ -98,7 +98,8 @@ struct MoeMix {
     const float* id_weight = nullptr;// [rows]: weight of the input itself (identity experts)
     int top = 0, experts = 0;
     int shared_row0 = -1;            // >= 0: y rows from here are the shared expert's
-    int early = 0;                   // the router had finished before this launch could start (one bf16 row: gate/up and down hold it back)
+    long routed = 0;                 // the router's launch (LaunchOrder): where it has ended before this one starts, one row reads its choice early
+    int early = 0;                   // set by the launcher
 };
 template <typename T>
 void launch_out_norm(float* x32, T* xh, const T* delta, const MoeMix& mix, float mult, const bf16* w, int rows, int width, int ld,
@@ -242,7 +243,8 @@ struct MoeBuffers {
 // keep_groups groups, weights = the chosen scores over their sum, times router_scale.  The last CTA lays the rows of every
 // expert out one after the other and cuts them into groups of at most `tile` rows.
 // `direct`: a single row feeds every expert, its input is not copied (x row 0 in every entry).
-void launch_moe_route(const LayerSpec& sp, const float* x32, const bf16* w, const float* correction, const MoeBuffers& b, int rows,
+// Returns its number (LaunchOrder).
+long launch_moe_route(const LayerSpec& sp, const float* x32, const bf16* w, const float* correction, const MoeBuffers& b, int rows,
                       int ld, int tile, bool direct, cudaStream_t s);
 size_t moe_ticket_ints(int max_rows);
 // Rows per group for `rows` tokens (16 .. 256) and the most groups that can come out.
@@ -281,8 +283,13 @@ MoeGemmPlan make_moe_gate_up_plan(const LayerSpec& sp, const bf16* w, const bf16
 // down: y[row][width]; act rows of ld_act columns
 MoeGemmPlan make_moe_down_plan(const LayerSpec& sp, const bf16* w, const bf16* act, int act_rows, int ld_act, int width, bf16* y,
                                int ld_y, int rows, int tile, const MoeBuffers& b);
-void launch_moe_gemm(const MoeGemmPlan& p, cudaStream_t s, bool hold = false);   // hold: one row, no router; as launch_linear_one_row's
-void launch_moe_one_row(const MoeGemmPlan& p, cudaStream_t s, bool hold = false);   // rows == 1 (one_row.cu)
+// routed: the router's launch (LaunchOrder), 0: its choice lay ready before.  The experts' gate/up products hold their successor back; down products read
+// the choice at once and are refused where the router may still be running.  Right behind a router before which everything has ended, the shared
+// expert's part of one row's gate/up product runs beside it.
+void launch_moe_gemm(const MoeGemmPlan& p, cudaStream_t s, long routed);
+// n products over one input (make_grouped_plan), no router.  hold: the next launch starts only after this one's wait (one row)
+void launch_grouped(const MoeGemmPlan& p, cudaStream_t s, bool hold = false);
+void launch_moe_one_row(const MoeGemmPlan& p, cudaStream_t s, bool hold, bool ahead);   // rows == 1 (one_row.cu)
 // elements of the two weight buffers (tile-major), and where an expert's (index `experts`: the shared expert's) part begins
 size_t moe_gate_up_elems(const LayerSpec& sp, int K);
 size_t moe_down_elems(const LayerSpec& sp, int width);

@@ -32,7 +32,7 @@ __global__ void embed_rows_kernel(const int32_t* __restrict__ ids, const bf16* _
     }
 }
 
-// One CTA per token row.
+// FRESH: past the first-level cache
 template <int VEC, bool FRESH, typename T>
 __device__ __forceinline__ void load_row(const T* p, float* f) {
     if constexpr (FRESH && VEC == 8 && sizeof(T) == 2) {
@@ -46,8 +46,8 @@ __device__ __forceinline__ void load_row(const T* p, float* f) {
     }
 }
 
-// BESIDE: the launch before the predecessor wrote the row, which is read past the first-level cache; the wait for the predecessor comes at the end,
-// so that whatever waits for this launch has waited for both.
+// One CTA per token row.  BESIDE: the row's writer has ended before this launch starts, and the wait for the predecessor comes at the end, so
+// that whatever waits for this launch has waited for both.
 template <typename T, int VEC, bool BESIDE>
 __global__ void qkv_norm_append_kernel(const QkvNormArgs a) {
     grid_dep_trigger();
@@ -331,7 +331,7 @@ void launch_qkv_norm_append(const QkvNormArgs& a, int rows, cudaStream_t s) {
     const bool v8 = a.dim % 8 == 0 && a.vdim % 8 == 0 && a.ld % 8 == 0 && (a.rot_dims / 2) % 8 == 0;
     auto run = [&](auto kernel) { launch_kernel(kernel, dim3(rows), dim3(256), 0, s, a); };
     if constexpr (sizeof(T) == 2) {
-        if (a.beside != 0) {
+        if (runtime().order.ended(a.written_by)) {
             if (v8) run(qkv_norm_append_kernel<T, 8, true>); else run(qkv_norm_append_kernel<T, 1, true>);
             return;
         }
@@ -340,9 +340,11 @@ void launch_qkv_norm_append(const QkvNormArgs& a, int rows, cudaStream_t s) {
 }
 
 template <typename T>
-void launch_out_norm(float* x32, T* xh, const T* delta, const MoeMix& mix, float mult, const bf16* w, int rows, int width, int ld,
+void launch_out_norm(float* x32, T* xh, const T* delta, const MoeMix& mix_, float mult, const bf16* w, int rows, int width, int ld,
                      float eps, cudaStream_t s) {
     ProfileScope prof(KC_ROW, s);
+    MoeMix mix = mix_;
+    mix.early = runtime().order.ended(mix.routed) ? 1 : 0;
     CPM_REQUIRE(ld % 64 == 0 && ld <= 512 * 8 * 4, "layered model: width above 16384 is not supported");
     CPM_REQUIRE(mix.top <= kMoeMaxTop, "mixture of experts: too many experts per token");
     const int vecs = ld / 8;

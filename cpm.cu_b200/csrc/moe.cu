@@ -311,7 +311,7 @@ moe_route_one_kernel(const RouteArgs a) {
         wv[j] = c < a.ld ? __ldg(reinterpret_cast<const uint2*>(w + c)) : make_uint2(0u, 0u);
     }
     grid_dep_wait();
-    grid_dep_trigger();   // not before the row exists: the shared expert's product starts on it (one_row.cu)
+    grid_dep_trigger();   // not before the row exists (LaunchOrder::held): the shared expert's product starts on it (one_row.cu)
     float acc = 0.f;
     auto add = [&](const uint2& wp, const float4& x) {
         const bf16* b = reinterpret_cast<const bf16*>(&wp);
@@ -857,7 +857,7 @@ int moe_max_entries(const LayerSpec& sp, int rows, int tile) {
     return static_cast<int>(std::min<long long>(slots, slots / tile + sp.experts));
 }
 
-void launch_moe_route(const LayerSpec& sp, const float* x32, const bf16* w, const float* correction, const MoeBuffers& b, int rows,
+long launch_moe_route(const LayerSpec& sp, const float* x32, const bf16* w, const float* correction, const MoeBuffers& b, int rows,
                       int ld, int tile, bool direct, cudaStream_t s) {
     ProfileScope prof(KC_ROUTE, s);
     RouteArgs a;
@@ -873,7 +873,8 @@ void launch_moe_route(const LayerSpec& sp, const float* x32, const bf16* w, cons
     if (rows == 1) {
         const size_t smem = (2 * a.outputs + 2 * a.groups) * sizeof(float);   // at most 16 KB
         launch_kernel(moe_route_one_kernel, dim3(ceil_div(a.outputs, RT_WARPS)), dim3(RT_WARPS * 32), smem, s, a);
-        return;
+        runtime().order.held();
+        return runtime().order.issued;
     }
     auto run = [&](auto we) {
         constexpr int WE = decltype(we)::value;
@@ -891,6 +892,7 @@ void launch_moe_route(const LayerSpec& sp, const float* x32, const bf16* w, cons
     else if (a.outputs > 16) run(std::integral_constant<int, 4>());
     else if (a.outputs > 8) run(std::integral_constant<int, 2>());
     else run(std::integral_constant<int, 1>());
+    return runtime().order.issued;
 }
 
 template <typename T>
@@ -967,12 +969,9 @@ MoeGemmPlan make_moe_down_plan(const LayerSpec& sp, const bf16* w, const bf16* a
     return p;
 }
 
-void launch_moe_gemm(const MoeGemmPlan& p, cudaStream_t s, bool hold) {
-    ProfileScope prof(p.uniform > 0 ? KC_LINEAR : KC_MOE, s);
-    if (p.rows == 1) {   // 4 of 30 experts of width 4096, ff 2048, and a shared one: 45.8 + 28.9 us as tiles, see one_row.cu
-        launch_moe_one_row(p, s, hold);
-        return;
-    }
+namespace {
+
+void launch_tiles(const MoeGemmPlan& p, cudaStream_t s) {
     GemmArgs a;
     a.n_tiles = p.n_tiles; a.kblocks = p.kblocks; a.N = p.N;
     a.n_tiles_s = p.n_tiles_s; a.kblocks_s = p.kblocks_s; a.N_s = p.N_s;
@@ -1012,4 +1011,24 @@ void launch_moe_gemm(const MoeGemmPlan& p, cudaStream_t s, bool hold) {
         case 256 * 2 + 1: launch_gemm<256, true>(p, a, grid, s); break;
         default: throw std::invalid_argument("cpmcu_b200: bad row group size");
     }
+}
+
+}  // namespace
+
+void launch_moe_gemm(const MoeGemmPlan& p, cudaStream_t s, long routed) {
+    ProfileScope prof(KC_MOE, s);
+    LaunchOrder& order = runtime().order;
+    CPM_REQUIRE(p.swiglu || routed == 0 || order.ended(routed), "mixture of experts: the router may still run when the down product starts");
+    // 4 of 30 experts of width 4096, ff 2048, and a shared one: 45.8 + 28.9 us as tiles, see one_row.cu
+    if (p.rows == 1) launch_moe_one_row(p, s, false, p.swiglu && routed == order.issued && order.ended(routed - 1));
+    else launch_tiles(p, s);
+    if (p.swiglu) order.held();
+}
+
+void launch_grouped(const MoeGemmPlan& p, cudaStream_t s, bool hold) {
+    ProfileScope prof(KC_LINEAR, s);
+    CPM_REQUIRE(p.uniform > 0 && (!hold || p.rows == 1), "grouped product: bad plan");
+    if (p.rows == 1) launch_moe_one_row(p, s, hold, false);
+    else launch_tiles(p, s);
+    if (hold) runtime().order.held();
 }

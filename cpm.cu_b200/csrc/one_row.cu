@@ -31,7 +31,7 @@ struct OneRowArgs {
     const int4* entries;             // router's choice: {expert, input row, output row, 1}
     const int32_t* n_entries;
     int uniform;                     // > 0: matrix i has row i of x and y
-    int ahead;                       // !EARLY: the shared matrix's CTAs run beside the router
+    int ahead;                       // !EARLY: the shared matrix's CTAs run beside the router (LaunchOrder)
     float gate_limit, gate_alpha;
     RopeRow rope;                    // ROPE
     SideRow side;                    // SIDE
@@ -51,9 +51,9 @@ __device__ __forceinline__ f32x2 widen(uint32_t two) { return pair(__uint_as_flo
 // SIDE: the output is gated into the token's side input.
 enum Epilogue { PLAIN, GATED, ROPE, SIDE };
 // Rotation and append as a launch of their own cost 1.7 us a layer (8 layers of 2048: 418 us a pass, 410 with them here).
-// EARLY: the router's choice may be read before the wait for the predecessor.  Without it the predecessor is the router: it starts this launch
-// only when the row it reads exists (its own wait is over), so the shared matrix's CTAs compute and store beside it, with no wait.  The other
-// CTAs of the launch wait, and so this launch still ends after the router.  The router is 8 us of latency on five CTAs: 32 tokens of six layers
+// EARLY: the router's choice may be read before the wait for the predecessor.  Without it (gate/up) the launch lets its successor start after its own
+// wait, and right behind a router that starts it only when the row exists, the shared matrix's CTAs compute and store beside it, with no wait
+// (ahead).  The other CTAs of the launch wait, and so it still ends after the router.  The router is 8 us of latency on five CTAs: 32 tokens of six layers
 // of 4096 with a shared expert of 4096 took 24.7 ms, now 22.5.
 // HOLD: the successor starts only after this launch's wait; it may then run beside this launch on what was there before it.
 template <int R, Epilogue EPI, bool EARLY, bool HOLD>
@@ -257,12 +257,13 @@ void launch_linear_one_row(const LinearPlan& p, cudaStream_t s, const RopeRow* r
         launch<GATED, true>(R, a, a.ctas, s);
     } else if (hold) {
         launch<PLAIN, true, true>(R, a, a.ctas, s);
+        runtime().order.held();
     } else {
         launch<PLAIN, true>(R, a, a.ctas, s);
     }
 }
 
-void launch_moe_one_row(const MoeGemmPlan& p, cudaStream_t s, bool hold) {
+void launch_moe_one_row(const MoeGemmPlan& p, cudaStream_t s, bool hold, bool ahead) {
     OneRowArgs a = {};
     a.w = p.w; a.x = p.x; a.xs = p.xs; a.y = p.y;
     a.N = p.N; a.kblocks = p.kblocks; a.N_s = p.N_s; a.kblocks_s = p.kblocks_s;
@@ -275,9 +276,7 @@ void launch_moe_one_row(const MoeGemmPlan& p, cudaStream_t s, bool hold) {
     a.ctas = ceil_div(p.N, R / per);
     a.ctas_s = p.n_tiles_s > 0 ? ceil_div(p.N_s, R / per) : 0;
     const int grid = a.ctas_s + p.max_entries * a.ctas;
-    a.ahead = p.max_entries > 0;   // some CTA waits for the router
-    // the router's choice: gate/up waits for it and lets its successor start only then, so down may read it at once
-    CPM_REQUIRE(!hold || p.uniform > 0, "one row: the router's products have an order of their own");
+    a.ahead = ahead && p.max_entries > 0;   // some CTA waits for the router
     if (hold) launch<PLAIN, true, true>(R, a, grid, s);
     else if (p.swiglu) launch<GATED, false>(R, a, grid, s);
     else launch<PLAIN, true>(R, a, grid, s);

@@ -670,6 +670,7 @@ void launch_scan_step(const ScanStepArgs& a, cudaStream_t s) {
     const size_t smem = sizeof(float) * (3 * p.kp + p.cols + std::max(groups * p.cols, a.rank + STEP_THREADS));
     if (time_mix) launch_kernel(scan_step_kernel<T, true>, grid, dim3(STEP_THREADS), smem, s, p);
     else launch_kernel(scan_step_kernel<T, false>, grid, dim3(STEP_THREADS), smem, s, p);
+    if (a.hold != 0) runtime().order.held();
 }
 template void launch_scan_step<bf16>(const ScanStepArgs&, cudaStream_t);
 template void launch_scan_step<float>(const ScanStepArgs&, cudaStream_t);

@@ -552,7 +552,7 @@ __global__ void attn_combine_kernel(const float* __restrict__ ws_o, const float*
                                     int rows, int hq, float scale_log2, bf16* __restrict__ out, int out_ld, int out_cols,
                                     int sink, float out_scale, int beside) {
     grid_dep_trigger();
-    if (beside == 0) grid_dep_wait();   // else at the end (ATTN_MERGE): the partial results are there, their producer is two launches back
+    if (beside == 0) grid_dep_wait();   // else at the end: the splits have ended before this launch starts (LaunchOrder)
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (row >= rows) return;
@@ -675,7 +675,7 @@ AttnPlan make_biased_attn_plan(const bf16* q, int q_ld_tokens, const bf16* k_cac
 
 namespace {
 template <int DK, int DV, bool BIASED>
-void launch_attn(const AttnPlan& p, const AttnArgs& a, AttnPart part, cudaStream_t s) {
+void launch_attn(const AttnPlan& p, const AttnArgs& a, AttnPart part, long splits_at, cudaStream_t s) {
     static bool configured = false;
     if (!configured) {
         CUDA_CHECK(cudaFuncSetAttribute(tree_attn_kernel<DK, DV, BIASED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -687,15 +687,14 @@ void launch_attn(const AttnPlan& p, const AttnArgs& a, AttnPart part, cudaStream
                       s, p.tm_q, p.tm_k, p.tm_v, a);
     }
     if (p.splits > 1 && part != ATTN_SPLITS) {
-        const int rows = p.tq * p.hq;
+        const int rows = p.tq * p.hq, beside = part == ATTN_MERGE && runtime().order.ended(splits_at) ? 1 : 0;
         launch_kernel(attn_combine_kernel<DV>, dim3(ceil_div(rows, 4)), dim3(128), 0, s, p.ws_o, p.ws_ml, p.splits, rows, p.hq,
-                      BIASED && p.bias_exp > 0.f ? 1.f : a.scale_log2, p.out, p.out_ld, p.out_cols, p.sink, p.out_scale,
-                      part == ATTN_MERGE ? 1 : 0);
+                      BIASED && p.bias_exp > 0.f ? 1.f : a.scale_log2, p.out, p.out_ld, p.out_cols, p.sink, p.out_scale, beside);
     }
 }
 }  // namespace
 
-void launch_tree_attention(const AttnPlan& p, cudaStream_t s, AttnPart part) {
+void launch_tree_attention(const AttnPlan& p, cudaStream_t s, AttnPart part, long splits_at) {
     if (part == ATTN_MERGE && p.splits == 1) return;
     ProfileScope prof(KC_ATTENTION, s);
     AttnArgs a;
@@ -754,9 +753,9 @@ void launch_tree_attention(const AttnPlan& p, cudaStream_t s, AttnPart part) {
         launch_pair_attention(p, a, s);
         return;
     }
-    if (!p.biased) launch_attn<128, 128, false>(p, a, part, s);
-    else if (p.d == 128 && p.dv == 128) launch_attn<128, 128, true>(p, a, part, s);
-    else if (p.d == 128) launch_attn<128, 64, true>(p, a, part, s);
-    else if (p.dv == 128) launch_attn<64, 128, true>(p, a, part, s);
-    else launch_attn<64, 64, true>(p, a, part, s);
+    if (!p.biased) launch_attn<128, 128, false>(p, a, part, splits_at, s);
+    else if (p.d == 128 && p.dv == 128) launch_attn<128, 128, true>(p, a, part, splits_at, s);
+    else if (p.d == 128) launch_attn<128, 64, true>(p, a, part, splits_at, s);
+    else if (p.dv == 128) launch_attn<64, 128, true>(p, a, part, splits_at, s);
+    else launch_attn<64, 64, true>(p, a, part, splits_at, s);
 }
