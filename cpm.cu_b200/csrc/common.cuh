@@ -282,8 +282,7 @@ struct SideRow {
     int table_ld = 0, col0 = 0, vocab = 0;
 };
 // M == 1, bf16 weights; with `rope` the product is q, k and v, which are rotated and appended; with `side` the side input's gate
-// hold: the next launch starts only after this one's wait (a plain product; LaunchOrder)
-void launch_linear_one_row(const LinearPlan& plan, cudaStream_t stream, const RopeRow* rope = nullptr, const SideRow* side = nullptr, bool hold = false);
+void launch_linear_one_row(const LinearPlan& plan, cudaStream_t stream, const RopeRow* rope = nullptr, const SideRow* side = nullptr);
 bool linear_one_row_fits(int N, int K, int sms);   // whether that is the faster way for one row of N outputs
 // Same contract with 4-bit weights, w = (q - 8) * scale, K % 256 == 0 and N % 128 == 0.  `wq` holds one
 // contiguous 16896-byte block per (128-feature tile, 256-k unit), tile-major: [4 k-blocks][2 halves]

@@ -223,7 +223,7 @@ private:
     template <typename T>
     void layered_attention(int layer, LayeredPlans& lp, const int32_t* kv_len, int kv_off, AttnPart part, long splits_at, cudaStream_t s);
     template <typename T>
-    void layered_rec_products(int layer, LayeredPlans& lp, bool hold, cudaStream_t s);   // hold: where they can, they hold their successor back
+    void layered_rec_products(int layer, LayeredPlans& lp, bool hold, cudaStream_t s);   // hold: one bf16 row of a time mix, whose product is to hold its successor back
     template <typename T>
     void layered_recurrence(int layer, LayeredPlans& lp, const int32_t* kv_len, int kv_off, bool hold, cudaStream_t s);
     template <typename T>

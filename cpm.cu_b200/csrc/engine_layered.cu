@@ -606,14 +606,7 @@ void Engine::layered_rec_products(int i, LayeredPlans& lp, bool hold, cudaStream
         launch_grouped(l.mixes, s, hold);
         return;
     }
-    for (const LayeredProduct& p : l.rec) {
-        if (hold && p.plan.one_row) {
-            ProfileScope prof(KC_LINEAR, s);
-            launch_linear_one_row(p.plan, s, nullptr, nullptr, true);
-        } else {
-            run_product<T>(p, lp.rows, s);
-        }
-    }
+    for (const LayeredProduct& p : l.rec) run_product<T>(p, lp.rows, s);
 }
 
 template <typename T>
@@ -695,8 +688,7 @@ bool Engine::layered_tanh_layer(int i, LayeredPlans& lp, const int32_t* ids, con
     LayeredPlans::Layer& l = lp.layers[i];
     const int rows = lp.rows, L = ld(), W = mc_.hidden, layers = static_cast<int>(lw_.size());
     T *x = static_cast<T*>(lx_), *delta = static_cast<T*>(ldelta_);
-    const bool both = sp.heads > 0 && sp.rec != REC_NONE;
-    if (both && sizeof(T) == 2 && rows == 1 && scan_step_fits(sp.rec_dim, sp.rec_vdim, sp.rec == REC_TIME_MIX)) {
+    if (sp.heads > 0 && sp.rec == REC_TIME_MIX && sizeof(T) == 2 && rows == 1 && scan_step_fits(sp.rec_dim, sp.rec_vdim, true)) {
         // Two chains of one token's row: its queries and keys are normalised beside the recurrence's product, the splits of its attention are
         // merged beside the recurrence's step.  Each of the two pairs is one launch that starts its successor after its own wait and a
         // successor that waits at its end (LaunchOrder).  1405 + 24 tokens of nine layers of 3072, six of them of this kind: 29.6 ms one after the other, 28.95

@@ -236,7 +236,7 @@ void launch(int R, const OneRowArgs& a, int grid, cudaStream_t s) {
 
 }  // namespace
 
-void launch_linear_one_row(const LinearPlan& p, cudaStream_t s, const RopeRow* rope, const SideRow* side, bool hold) {
+void launch_linear_one_row(const LinearPlan& p, cudaStream_t s, const RopeRow* rope, const SideRow* side) {
     OneRowArgs a = {};
     a.w = p.w; a.x = p.x; a.y = p.y; a.bias = p.bias;
     a.N = p.N; a.kblocks = p.K / BLOCK_COLS;
@@ -255,9 +255,6 @@ void launch_linear_one_row(const LinearPlan& p, cudaStream_t s, const RopeRow* r
         launch<SIDE, true>(R, a, a.ctas, s);
     } else if (p.swiglu) {
         launch<GATED, true>(R, a, a.ctas, s);
-    } else if (hold) {
-        launch<PLAIN, true, true>(R, a, a.ctas, s);
-        runtime().order.held();
     } else {
         launch<PLAIN, true>(R, a, a.ctas, s);
     }
