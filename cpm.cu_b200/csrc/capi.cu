@@ -988,36 +988,30 @@ int cpmcu_layer_side_step(float* x32, const void* delta, const void* w, const vo
         }
         DynTanh post;
         post.w = static_cast<const bf16*>(w); post.b = static_cast<const bf16*>(b); post.alpha = alpha;
-        const bf16 *tab = static_cast<const bf16*>(table), *nw = static_cast<const bf16*>(norm), *gw = static_cast<const bf16*>(g.p), *pw = static_cast<const bf16*>(p.p);
         const size_t es = fp32 ? 4 : 2;
         DeviceBuf x(ld * es), z(dp * es), sg(dp * es), y(ld * es), ws(linear_workspace_bytes(16, runtime().num_sms)), tickets(2 * sizeof(int) * (ceil_div(std::max(width, dim), 128) + 1));
         CUDA_CHECK(cudaMemsetAsync(z.p, 0, dp * es, s));
         CUDA_CHECK(cudaMemsetAsync(sg.p, 0, dp * es, s));
         CUDA_CHECK(cudaMemsetAsync(y.p, 0, ld * es, s));
         CUDA_CHECK(cudaMemsetAsync(tickets.p, 0, 2 * sizeof(int) * (ceil_div(std::max(width, dim), 128) + 1), s));
-        if (fp32) {
-            float *xf = static_cast<float*>(x.p), *zf = static_cast<float*>(z.p), *sf = static_cast<float*>(sg.p), *yf = static_cast<float*>(y.p);
-            launch_tanh_residual<float>(x32, static_cast<const float*>(delta), post, DynTanh(), xf, 1, ld, s);
-            launch_linear_f32(xf, ld, gw, 0, zf, dp, 1, dim, ld, nullptr, nullptr, 0, false, s);
-            launch_side_gate<float>(zf, dp, id, tab, layers * dim, layer * dim, dim, vocab, sf, 1, s);
-            launch_linear_f32(sf, dp, pw, 0, yf, ld, 1, width, dp, nullptr, nullptr, 0, false, s);
-            launch_side_add<float>(x32, yf, nw, DynTanh(), xf, TokenShift(), 1, width, ld, eps, s);
-        } else {
-            bf16 *xh = static_cast<bf16*>(x.p), *zh = static_cast<bf16*>(z.p), *sh = static_cast<bf16*>(sg.p), *yh = static_cast<bf16*>(y.p);
-            launch_tanh_residual<bf16>(x32, static_cast<const bf16*>(delta), post, DynTanh(), xh, 1, ld, s);
-            LinearPlan gp = make_linear_plan(xh, 1, gw, 1, dim, ld, zh, dp, nullptr, static_cast<float*>(ws.p), static_cast<int*>(tickets.p), runtime().num_sms);
-            if (gp.one_row) {
-                SideRow side;
-                side.ids = id; side.table = tab; side.table_ld = layers * dim; side.col0 = layer * dim; side.vocab = vocab;
-                gp.y = sh;
-                launch_linear_one_row(gp, s, nullptr, &side);
-            } else {
-                launch_linear(gp, s);
-                launch_side_gate<bf16>(zh, dp, id, tab, layers * dim, layer * dim, dim, vocab, sh, 1, s);
+        auto product = [&](void* in, const DeviceBuf& wt, int K, int N, void* out, int ldy) {
+            LayeredProduct q;
+            q.x = in; q.w = static_cast<const bf16*>(wt.p); q.N = N; q.K = K; q.y = out; q.ldy = ldy;
+            if (!fp32) {
+                q.plan = make_linear_plan(static_cast<const bf16*>(in), 1, q.w, 1, N, K, static_cast<bf16*>(out), ldy, nullptr, static_cast<float*>(ws.p),
+                                          static_cast<int*>(tickets.p), runtime().num_sms);
             }
-            launch_linear(make_linear_plan(sh, 1, pw, 1, width, dp, yh, ld, nullptr, static_cast<float*>(ws.p), static_cast<int*>(tickets.p), runtime().num_sms), s);
-            launch_side_add<bf16>(x32, yh, nw, DynTanh(), xh, TokenShift(), 1, width, ld, eps, s);
-        }
+            return q;
+        };
+        SideInput a;
+        a.x32 = x32; a.delta = delta;
+        a.post = post;
+        a.gate = product(x.p, g, ld, dim, z.p, dp); a.proj = product(sg.p, p, dp, width, y.p, ld);
+        a.norm = static_cast<const bf16*>(norm);
+        a.ids = id; a.table = static_cast<const bf16*>(table); a.table_ld = layers * dim; a.col0 = layer * dim; a.vocab = vocab;
+        a.rows = 1; a.width = width; a.ld = ld; a.eps = eps;
+        if (fp32) launch_side_input<float>(a, s);
+        else launch_side_input<bf16>(a, s);
         sync_and_check("layer_side_step");
         return 0;
     });

@@ -89,15 +89,6 @@ struct LayeredWeights {
     // token side input
     bf16 *side_gate = nullptr, *side_proj = nullptr, *side_norm = nullptr;
 };
-// y[rows][ldy] = x[rows][K] w^T, N columns
-struct LayeredProduct {
-    const void* x = nullptr;
-    const bf16* w = nullptr;
-    int N = 0, K = 0;
-    void* y = nullptr;
-    int ldy = 0;
-    LinearPlan plan;   // bf16
-};
 struct LayeredPlans {
     struct Layer {
         LayeredProduct qkv, o;
@@ -233,8 +224,6 @@ private:
     template <typename T>
     bool layered_tanh_layer(int layer, LayeredPlans& lp, const int32_t* ids, const int32_t* kv_len, int kv_off, cudaStream_t s);
     TokenShift token_shift(int layer, int rows, const int32_t* kv_len, int kv_off) const;
-    template <typename T>
-    void run_product(const LayeredProduct& p, int rows, cudaStream_t s);
     bool has_recurrence() const;
     void layered_check_errors(const char* where);
     // columns of a row of the recurrence's projections

@@ -552,12 +552,6 @@ void Engine::layered_mixture(int i, LayeredPlans& lp, cudaStream_t s) {
 }
 
 template <typename T>
-void Engine::run_product(const LayeredProduct& p, int rows, cudaStream_t s) {
-    if constexpr (sizeof(T) == 2) launch_linear(p.plan, s);
-    else launch_linear_f32(static_cast<const float*>(p.x), p.K, p.w, 0, static_cast<float*>(p.y), p.ldy, rows, p.N, p.K, nullptr, nullptr, 0, false, s);
-}
-
-template <typename T>
 void Engine::layered_queries(int i, LayeredPlans& lp, const int32_t* kv_len, int kv_off, long written_by, cudaStream_t s) {
     const LayerSpec& sp = mc_.specs[i];
     const LayeredWeights& w = lw_[i];
@@ -606,7 +600,7 @@ void Engine::layered_rec_products(int i, LayeredPlans& lp, bool hold, cudaStream
         launch_grouped(l.mixes, s, hold);
         return;
     }
-    for (const LayeredProduct& p : l.rec) run_product<T>(p, lp.rows, s);
+    for (const LayeredProduct& p : l.rec) launch_product<T>(p, lp.rows, s);
 }
 
 template <typename T>
@@ -664,10 +658,10 @@ void Engine::layered_dense(int i, LayeredPlans& lp, cudaStream_t s) {
     if (l.ff_fused) {
         launch_linear(l.ff_gate_up.plan, s);
     } else {
-        run_product<T>(l.ff_gate_up, lp.rows, s);
+        launch_product<T>(l.ff_gate_up, lp.rows, s);
         launch_clamped_gate<T>(static_cast<const T*>(lgu_), 2 * ff, static_cast<T*>(lact_), ff, lp.rows, ff, sp.ff_limit, sp.ff_alpha, sizeof(T) == 2, s);
     }
-    run_product<T>(l.ff_down, lp.rows, s);
+    launch_product<T>(l.ff_down, lp.rows, s);
 }
 
 TokenShift Engine::token_shift(int i, int rows, const int32_t* kv_len, int kv_off) const {
@@ -695,7 +689,7 @@ bool Engine::layered_tanh_layer(int i, LayeredPlans& lp, const int32_t* ids, con
         // so; with the product beside the norms instead it starts its weights later and took 29.1.
         const bool merge = l.tensor_attn && l.attn.splits > 1;
         const LaunchOrder& order = runtime().order;
-        run_product<T>(l.qkv, rows, s);
+        launch_product<T>(l.qkv, rows, s);
         const long qkv_at = order.issued;
         layered_rec_products<T>(i, lp, true, s);
         layered_queries<T>(i, lp, kv_len, kv_off, qkv_at, s);
@@ -705,7 +699,7 @@ bool Engine::layered_tanh_layer(int i, LayeredPlans& lp, const int32_t* ids, con
         layered_attention<T>(i, lp, kv_len, kv_off, ATTN_MERGE, splits_at, s);
     } else {
         if (sp.heads > 0) {
-            run_product<T>(l.qkv, rows, s);
+            launch_product<T>(l.qkv, rows, s);
             layered_queries<T>(i, lp, kv_len, kv_off, 0, s);
             layered_attention<T>(i, lp, kv_len, kv_off, ATTN_ALL, 0, s);
         }
@@ -714,7 +708,7 @@ bool Engine::layered_tanh_layer(int i, LayeredPlans& lp, const int32_t* ids, con
             layered_recurrence<T>(i, lp, kv_len, kv_off, false, s);
         }
     }
-    run_product<T>(l.o, rows, s);
+    launch_product<T>(l.o, rows, s);
     // a row's mixes need the row before it, which only a single row has at hand at a layer's end
     const bool next = i + 1 < layers && mc_.side_dim > 0 && (rows == 1 || mc_.specs[i + 1].rec != REC_TIME_MIX);
     const DynTanh next_norm = next ? lw_[i + 1].tanh1 : DynTanh();
@@ -724,28 +718,18 @@ bool Engine::layered_tanh_layer(int i, LayeredPlans& lp, const int32_t* ids, con
         layered_dense<T>(i, lp, s);
     }
     const DynTanh& last = sp.ff > 0 ? w.tanh2b : w.tanh1b;
-    launch_tanh_residual<T>(x32_, delta, last, DynTanh(), x, rows, L, s);
-    if (mc_.side_dim == 0) return false;
-    bool gated = false;
-    if constexpr (sizeof(T) == 2) {
-        // A single row: residual sum, two products and the sum with norm and mixes are four launches of 1.3 to 3 us that start beside one
-        // another's ends.  One cluster of 16 CTAs with four dependent phases took 15.5 us a layer of width 3072 (24 tokens of
-        // nine layers 31.2 -> 29.8 ms; four layers of 4096 14.0 -> 13.2 ms over 40 tokens, of 2048 8.9 -> 8.6, of 512 7.2 and 7.3).
-        if (rows == 1 && l.side_gate.plan.one_row) {   // gated where the product ends
-            LinearPlan gate = l.side_gate.plan;
-            gate.y = static_cast<bf16*>(lsg_);
-            SideRow side;
-            side.ids = ids; side.table = side_embed_; side.table_ld = layers * mc_.side_dim; side.col0 = i * mc_.side_dim; side.vocab = mc_.vocab;
-            ProfileScope prof(KC_LINEAR, s);
-            launch_linear_one_row(gate, s, nullptr, &side);
-            gated = true;
-        }
+    if (mc_.side_dim == 0) {
+        launch_tanh_residual<T>(x32_, delta, last, DynTanh(), x, rows, L, s);
+        return false;
     }
-    if (!gated) run_product<T>(l.side_gate, rows, s);
-    if (!gated) launch_side_gate<T>(static_cast<const T*>(lside_), pad64(mc_.side_dim), ids, side_embed_, layers * mc_.side_dim, i * mc_.side_dim, mc_.side_dim,
-                        mc_.vocab, static_cast<T*>(lsg_), rows, s);
-    run_product<T>(l.side_proj, rows, s);
-    launch_side_add<T>(x32_, delta, w.side_norm, next_norm, x, next_shift, rows, W, L, mc_.eps, s);
+    SideInput side;
+    side.x32 = x32_; side.delta = ldelta_;
+    side.post = last;
+    side.gate = l.side_gate; side.proj = l.side_proj; side.norm = w.side_norm;
+    side.ids = ids; side.table = side_embed_; side.table_ld = layers * mc_.side_dim; side.col0 = i * mc_.side_dim; side.vocab = mc_.vocab;
+    side.next = next_norm; side.h = lx_; side.shift = next_shift;
+    side.rows = rows; side.width = W; side.ld = L; side.eps = mc_.eps;
+    launch_side_input<T>(side, s);
     return next;
 }
 
@@ -768,10 +752,10 @@ void Engine::layered_forward(int rows, const int32_t* ids, const int32_t* kv_len
             if (!ready) launch_tanh_norm<T>(x32_, nullptr, w.tanh1, static_cast<T*>(lx_), token_shift(li, rows, kv_len, kv_off), rows, L, s);
             ready = layered_tanh_layer<T>(li, lp, ids, kv_len, kv_off, s);
         } else {
-            run_product<T>(lp.layers[i].qkv, rows, s);
+            launch_product<T>(lp.layers[i].qkv, rows, s);
             layered_queries<T>(static_cast<int>(i), lp, kv_len, kv_off, 0, s);
             layered_attention<T>(static_cast<int>(i), lp, kv_len, kv_off, ATTN_ALL, 0, s);
-            run_product<T>(lp.layers[i].o, rows, s);
+            launch_product<T>(lp.layers[i].o, rows, s);
             launch_out_norm<T>(x32_, static_cast<T*>(lx_), static_cast<const T*>(ldelta_), MoeMix(), mc_.scale_residual, w.norm1, rows, W, L, mc_.eps, s);
             if (sp.experts + sp.identity > 0) layered_mixture<T>(static_cast<int>(i), lp, s);
         }

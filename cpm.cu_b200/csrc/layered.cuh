@@ -125,20 +125,41 @@ struct TokenShift {
 template <typename T>
 void launch_tanh_norm(const float* x32, const int32_t* rows_idx, const DynTanh& n, T* h, const TokenShift& shift, int rows, int ld,
                       cudaStream_t s);
+// y[rows][ldy] = x[rows][K] w^T, N columns
+struct LayeredProduct {
+    const void* x = nullptr;
+    const bf16* w = nullptr;
+    int N = 0, K = 0;
+    void* y = nullptr;
+    int ldy = 0;
+    LinearPlan plan;   // bf16
+};
 // x32 += post(delta); out = next(x32) in T, or x32 itself where next has no weights
 template <typename T>
 void launch_tanh_residual(float* x32, const T* delta, const DynTanh& post, const DynTanh& next, T* out, int rows, int ld, cudaStream_t s);
 // act = clamped gate of gu (two blocks of ff columns, or interleaved in groups of 64: see launch_silu_gate)
 template <typename T>
 void launch_clamped_gate(const T* gu, int ld_gu, T* act, int ld_act, int rows, int ff, float limit, float alpha, bool interleaved, cudaStream_t s);
-// Token side input: g[r] = gelu_tanh(z[r]) * table[ids[r]][col0 ..], dim columns, zero up to ld
+// End of a layer with a token side input: x32 += post(delta), gate.x = x32 in T; gate.y = gate.x W_gate^T, proj.x = gelu_tanh(gate.y) *
+// table[ids][col0 ..] (dim columns, zero up to gate.ldy), proj.y = proj.x W_proj^T, x32 += rms(proj.y) * norm; with `next`, h = next(x32) in T and, for a
+// single row, its mixes.
+struct SideInput {
+    float* x32 = nullptr;
+    const void* delta = nullptr;
+    DynTanh post;
+    LayeredProduct gate, proj;
+    const bf16* norm = nullptr;
+    const int32_t* ids = nullptr;
+    const bf16* table = nullptr;
+    int table_ld = 0, col0 = 0, vocab = 0;
+    DynTanh next;
+    void* h = nullptr;
+    TokenShift shift;
+    int rows = 0, width = 0, ld = 0;
+    float eps = 0.f;
+};
 template <typename T>
-void launch_side_gate(const T* z, int ld, const int32_t* ids, const bf16* table, int table_ld, int col0, int dim, int vocab, T* g, int rows,
-                      cudaStream_t s);
-// x32 += rms(y) * w; with `next`, h = next(x32) in T and, for a single row, its mixes
-template <typename T>
-void launch_side_add(float* x32, const T* y, const bf16* w, const DynTanh& next, T* h, const TokenShift& shift, int rows, int width, int ld,
-                     float eps, cudaStream_t s);
+void launch_side_input(const SideInput& a, cudaStream_t s);
 // dst [cols][rows] = src [rows][cols], host or device memory
 void upload_transposed(const void* src, int rows, int cols, bf16* dst, cudaStream_t s);
 // Decays of a time-mix layer: out[r][c] = exp(-exp(sum_k w2[k][c] tanh(x[r][k]) + w0[c])), c < channels; x: `rank` columns of
@@ -218,6 +239,11 @@ void launch_plain_attention(const PlainAttnArgs& a, cudaStream_t s);
 constexpr int kF32Rows = 64;
 void launch_linear_f32(const float* x, int ldx, const bf16* w, size_t w_stride, float* y, int ldy, int M, int N, int K,
                        const int4* entries, const int32_t* n_entries, int max_entries, bool x_at_y, cudaStream_t s);
+template <typename T>
+void launch_product(const LayeredProduct& p, int rows, cudaStream_t s) {
+    if constexpr (sizeof(T) == 2) launch_linear(p.plan, s);
+    else launch_linear_f32(static_cast<const float*>(p.x), p.K, p.w, 0, static_cast<float*>(p.y), p.ldy, rows, p.N, p.K, nullptr, nullptr, 0, false, s);
+}
 // act[r][c] = silu(gu[r][c]) * gu[r][ff + c], IEEE exponential and division
 void launch_silu_f32(const float* gu, int ld_gu, float* act, int ld_act, int rows, int ff, cudaStream_t s);
 

@@ -342,21 +342,41 @@ void launch_clamped_gate(const T* gu, int ld_gu, T* act, int ld_act, int rows, i
 }
 
 template <typename T>
-void launch_side_gate(const T* z, int ld, const int32_t* ids, const bf16* table, int table_ld, int col0, int dim, int vocab, T* g, int rows,
-                      cudaStream_t s) {
+void launch_side_input(const SideInput& a, cudaStream_t s) {
+    T *x = static_cast<T*>(const_cast<void*>(a.gate.x)), *g = static_cast<T*>(const_cast<void*>(a.proj.x));
+    launch_tanh_residual<T>(a.x32, static_cast<const T*>(a.delta), a.post, DynTanh(), x, a.rows, a.ld, s);
+    bool gated = false;
+    if constexpr (sizeof(T) == 2) {
+        // A single row: residual sum, two products and the sum with norm and mixes are four launches of 1.3 to 3 us that start beside one
+        // another's ends.  One cluster of 16 CTAs with four dependent phases took 15.5 us a layer of width 3072 (24 tokens of
+        // nine layers 31.2 -> 29.8 ms; four layers of 4096 14.0 -> 13.2 ms over 40 tokens, of 2048 8.9 -> 8.6, of 512 7.2 and 7.3).
+        if (a.rows == 1 && a.gate.plan.one_row) {   // gated where the product ends; proj.x is zero beyond it
+            LinearPlan gate = a.gate.plan;
+            gate.y = g;
+            SideRow side;
+            side.ids = a.ids; side.table = a.table; side.table_ld = a.table_ld; side.col0 = a.col0; side.vocab = a.vocab;
+            ProfileScope prof(KC_LINEAR, s);
+            launch_linear_one_row(gate, s, nullptr, &side);
+            gated = true;
+        }
+    }
+    if (!gated) {
+        launch_product<T>(a.gate, a.rows, s);
+        ProfileScope prof(KC_ROW, s);
+        launch_kernel(side_gate_kernel<T>, dim3(a.rows), dim3(64), 0, s, static_cast<const T*>(a.gate.y), a.gate.ldy, a.ids, a.table, a.table_ld, a.col0,
+                      a.gate.N, a.vocab, g);
+    }
+    launch_product<T>(a.proj, a.rows, s);
     ProfileScope prof(KC_ROW, s);
-    launch_kernel(side_gate_kernel<T>, dim3(rows), dim3(64), 0, s, z, ld, ids, table, table_ld, col0, dim, vocab, g);
-}
-
-template <typename T>
-void launch_side_add(float* x32, const T* y, const bf16* w, const DynTanh& next, T* h, const TokenShift& shift, int rows, int width, int ld,
-                     float eps, cudaStream_t s) {
-    ProfileScope prof(KC_ROW, s);
-    CPM_REQUIRE(ld % 64 == 0 && ld <= 512 * 8 * 4 && (shift.mu == nullptr || rows == 1), "side_add: bad arguments");
-    const int vecs = ld / 8;
+    CPM_REQUIRE(a.ld % 64 == 0 && a.ld <= 512 * 8 * 4 && (a.shift.mu == nullptr || a.rows == 1), "side input: bad arguments");
+    const int vecs = a.ld / 8;
     const int threads = vecs >= 512 ? 512 : (vecs + 31) / 32 * 32;
-    if (vecs <= 512) launch_kernel(side_add_kernel<T, 1>, dim3(rows), dim3(threads), 0, s, x32, y, w, next, h, shift, width, ld, eps);
-    else launch_kernel(side_add_kernel<T, 4>, dim3(rows), dim3(threads), 0, s, x32, y, w, next, h, shift, width, ld, eps);
+    auto add = [&](auto kernel) {
+        launch_kernel(kernel, dim3(a.rows), dim3(threads), 0, s, a.x32, static_cast<const T*>(a.proj.y), a.norm, a.next, static_cast<T*>(a.h), a.shift,
+                      a.width, a.ld, a.eps);
+    };
+    if (vecs <= 512) add(side_add_kernel<T, 1>);
+    else add(side_add_kernel<T, 4>);
 }
 
 template <typename T>
@@ -396,9 +416,7 @@ void launch_norm_gate(const float* o, int ld_o, int groups, int group, const bf1
     template void launch_tanh_norm<T>(const float*, const int32_t*, const DynTanh&, T*, const TokenShift&, int, int, cudaStream_t);         \
     template void launch_tanh_residual<T>(float*, const T*, const DynTanh&, const DynTanh&, T*, int, int, cudaStream_t);                    \
     template void launch_clamped_gate<T>(const T*, int, T*, int, int, int, float, float, bool, cudaStream_t);                               \
-    template void launch_side_gate<T>(const T*, int, const int32_t*, const bf16*, int, int, int, int, T*, int, cudaStream_t);               \
-    template void launch_side_add<T>(float*, const T*, const bf16*, const DynTanh&, T*, const TokenShift&, int, int, int, float,            \
-                                     cudaStream_t);                                                                                         \
+    template void launch_side_input<T>(const SideInput&, cudaStream_t);                                                                    \
     template void launch_decay<T>(const T*, int, const bf16*, const bf16*, int, int, float*, int, int, cudaStream_t);                       \
     template void launch_norm_gate<T>(const float*, int, int, int, const bf16*, const T*, int, bool, float, float, T*, int, int, cudaStream_t);
 CPM_INSTANTIATE(bf16)
