@@ -817,13 +817,16 @@ moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
     if (threadIdx.x == 0 && *abort_flag) atomicOr(a.error, ERR_GEMM_TIMEOUT);
 }
 
+// jobs: pairs of tiles, at most
 template <int MT, bool SWIGLU>
-void launch_pair(const MoeGemmPlan& p, const GemmArgs& a, int grid, cudaStream_t s) {
-    static bool configured = false;
-    if (!configured) {
+void launch_pair(const MoeGemmPlan& p, const GemmArgs& a, long long jobs, cudaStream_t s) {
+    static int pairs = 0;   // that the device holds at once
+    if (pairs == 0) {
         CUDA_CHECK(cudaFuncSetAttribute(moe_gemm_pair_kernel<MT, SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<MT>::SMEM_BYTES));
-        configured = true;
+        const int held = max_active_clusters(moe_gemm_pair_kernel<MT, SWIGLU>, dim3(NUM_THREADS), PairCfg<MT>::SMEM_BYTES, 2);
+        pairs = held > 0 ? held : runtime().num_sms / 2;
     }
+    const int grid = 2 * static_cast<int>(std::max<long long>(1, std::min<long long>(jobs, pairs)));
     launch_kernel_cluster(moe_gemm_pair_kernel<MT, SWIGLU>, dim3(grid), dim3(NUM_THREADS), PairCfg<MT>::SMEM_BYTES, s, 2, p.tm_w, p.tm_x, p.tm_xs, a);
 }
 
@@ -989,12 +992,12 @@ void launch_tiles(const MoeGemmPlan& p, cudaStream_t s) {
     if (p.tile >= 128 && p.n_tiles % 2 == 0) {
         a.n_tiles /= 2;
         a.n_tiles_s = ceil_div(a.n_tiles_s, 2);   // the shared matrix is the last one: an odd tile's partner reads zeros beyond the map
-        const int pairs = 2 * static_cast<int>(std::max<long long>(1, std::min<long long>(most / 2, runtime().num_sms / 2)));
+        const long long jobs = static_cast<long long>(a.groups_s) * a.n_tiles_s + static_cast<long long>(p.max_entries) * a.n_tiles;
         switch (p.tile * 2 + p.swiglu) {
-            case 128 * 2: launch_pair<128, false>(p, a, pairs, s); break;
-            case 128 * 2 + 1: launch_pair<128, true>(p, a, pairs, s); break;
-            case 256 * 2: launch_pair<256, false>(p, a, pairs, s); break;
-            default: launch_pair<256, true>(p, a, pairs, s); break;
+            case 128 * 2: launch_pair<128, false>(p, a, jobs, s); break;
+            case 128 * 2 + 1: launch_pair<128, true>(p, a, jobs, s); break;
+            case 256 * 2: launch_pair<256, false>(p, a, jobs, s); break;
+            default: launch_pair<256, true>(p, a, jobs, s); break;
         }
         return;
     }
