@@ -656,6 +656,18 @@ struct PairCfg {
     static_assert(SMEM_BYTES <= 232448, "shared memory budget");
 };
 
+// Columns of a pair's product for a group of `rows` rows (one that is not full costs little more than its rows).  An MMA of 256 weight rows on two
+// CTAs takes columns in steps of 32, 16 of each CTA's rows.
+__host__ __device__ constexpr int pair_columns(int rows, int tile) { return rows >= tile ? tile : (rows + 31) / 32 * 32; }
+constexpr bool pair_columns_fit(int tile) {
+    for (int r = 1; r <= tile; ++r) {
+        const int n = pair_columns(r, tile);
+        if (n < r || n > tile || n % 32 != 0 || n - r >= 32) return false;
+    }
+    return true;
+}
+static_assert(pair_columns_fit(128) && pair_columns_fit(256), "columns of the pairs' products");
+
 template <int MT, bool SWIGLU>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
@@ -702,8 +714,8 @@ moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     const int shared_tiles = a.groups_s * a.n_tiles_s;
-    // columns of the product (a group that is not full costs only its rows) and the boxes of rows that each CTA fetches
-    auto columns = [](const TileJob& j) { return min(MT, (j.rows + 15) & ~15); };
+    // columns of the product and the boxes of rows that each CTA fetches
+    auto columns = [](const TileJob& j) { return pair_columns(j.rows, MT); };
     auto boxes_of = [&](const TileJob& j) { return (columns(j) / 2 + XBOX - 1) / XBOX; };
     auto load_w = [&](int s, const TileJob& j, int kb) {
         if (rank == 0) ptx::mbar_arrive_expect_tx(&full[s], 2 * (W_TILE_BYTES + boxes_of(j) * XBOX_BYTES));

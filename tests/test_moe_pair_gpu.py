@@ -1,5 +1,5 @@
 """Grouped products on pairs of CTAs (moe.cu: groups of 128 or 256 rows, an even number of 128-feature tiles per matrix) at the row counts
-where the halves of a group change (columns are rounded up to 16, each CTA fetches half of them in boxes of 64), with an odd tile of
+where the halves of a group change (columns are rounded up to 32, each CTA fetches half of them in boxes of 64), with an odd tile of
 the extra matrix, and beside them matrices of an odd number of tiles (single CTAs); against 64 bits.
 
 Sums of fp32 products in some order are within 8 K ulp of 2^-24 of the sum of magnitudes, the bf16 store adds half a step."""
