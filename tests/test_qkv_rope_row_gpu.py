@@ -32,19 +32,25 @@ def test_qkv_rope_row(hq, hkv, K, pos):
     ref = torch.cat([lo * angle.cos() - hi * angle.sin(), hi * angle.cos() + lo * angle.sin()], dim=-1)
     room = 2.0 ** -8 * ref.abs() + 1e-6 * (lo.abs() + hi.abs()).repeat(1, 2)
 
-    def run(valid, cache_rows):
+    def run(valid, cache_rows, kc, vc):
         q = torch.full((hq * 128,), float("nan"), dtype=torch.bfloat16, device="cuda")
-        kc, vc = (torch.zeros(rows, hkv, 128, dtype=torch.bfloat16, device="cuda") for _ in range(2))
         C.call("cpmcu_qkv_rope_row", ptr(x), ptr(w), K, hq, hkv, ptr(inv_freq), ptr(p), ptr(n), -3, ptr(valid), cache_rows, ptr(q), ptr(kc), ptr(vc))
         assert bool(((q.double().view(hq, 128) - ref[:hq]).abs() <= room[:hq]).all())
-        return kc, vc
+
+    def caches():
+        return [torch.zeros(rows, hkv, 128, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
 
     for valid in (None, torch.tensor([1], dtype=torch.int32, device="cuda")):
-        kc, vc = run(valid, at + 1)
+        kc, vc = caches()
+        run(valid, at + 1, kc, vc)
         assert bool(((kc[at].double() - ref[hq:]).abs() <= room[hq:]).all()) and torch.equal(vc[at].double(), before[hq + hkv:])
         kc[at] = vc[at] = 0
         assert float(kc.abs().max()) == 0.0 and float(vc.abs().max()) == 0.0
-    kc, vc = run(torch.tensor([0], dtype=torch.int32, device="cuda"), rows)
+    kc, vc = caches()
+    run(torch.tensor([0], dtype=torch.int32, device="cuda"), rows, kc, vc)
     assert float(kc.abs().max()) == 0.0 and float(vc.abs().max()) == 0.0
-    with pytest.raises(RuntimeError, match="8"):   # beyond the cache: nothing is stored, the error word says so
-        run(None, at)
+    # beyond the cache: the error word says so, and nothing is stored (the caches hold 64 rows, so a stray row would lie in them)
+    kc, vc = caches()
+    with pytest.raises(RuntimeError, match="error flags 8 "):
+        run(None, at, kc, vc)
+    assert float(kc.abs().max()) == 0.0 and float(vc.abs().max()) == 0.0
