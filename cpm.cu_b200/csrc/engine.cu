@@ -728,8 +728,9 @@ void Engine::decode(int n, int padded_len, const int32_t* ids, const int32_t* po
     decode_rows(n, ids, pos, cache_length, mask, logits_out);
 }
 
-// A token that the host has goes along with a launch, and the logits go straight to the caller's buffer: no copy from pinned memory and no
-// repeated copy of the logits on the caller's stream, whose launches and waits took 17 to 27 us of a pass (2 layers of 256: 97 us -> 68,
+// A token that the host has goes along with a launch, and the logits go to a buffer of the caller's: from the head itself in a plain pass of a
+// Llama-format model, from the engine's buffer in a replayed one, from `work` in a layered model.  What is saved are the copy from pinned memory
+// and the clone of the logits on the caller's stream, whose launches and waits took 17 to 27 us of a pass (2 layers of 256: 97 us -> 68,
 // 8 layers of 2048 405 -> 381).
 void Engine::decode_token(int token, int position, void* work, void* logits_out, bool cuda_graph) {
     CPM_REQUIRE(storage_ready_, "decode before init_storage");
