@@ -547,7 +547,8 @@ tree_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 // Merge split partials: out = sum_s 2^((m_s - M) c) O_s / sum_s 2^((m_s - M) c) l_s.
 // One warp per (token, head) row; lane s first owns split s's (max, sum) pair, then
 // every lane accumulates four output columns with independent loads in flight.
-template <int DV>
+// B: splits whose partial outputs are in flight at once
+template <int DV, int B>
 __global__ void attn_combine_kernel(const float* __restrict__ ws_o, const float* __restrict__ ws_ml, int nsplit,
                                     int rows, int hq, float scale_log2, bf16* __restrict__ out, int out_ld, int out_cols,
                                     int sink, float out_scale, int beside) {
@@ -556,10 +557,7 @@ __global__ void attn_combine_kernel(const float* __restrict__ ws_o, const float*
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (row >= rows) return;
-    // the partial outputs of as many splits as a launch commonly has are requested before the (max, sum) pairs they are weighted
-    // with: all loads are in flight together.  Twelve at a time, two round trips: a token of eight layers of 2048 384 us (382 now), of six of
-    // 4096 with experts 589 (583), a step of 32 layers of 4096 4.801 ms (4.791)
-    constexpr int B = 24;
+    // the first B splits' partial outputs are requested before the (max, sum) pairs they are weighted with: all loads are in flight together
     constexpr int CPL = DV / 32;   // output columns per lane
     using Vec = typename std::conditional<CPL == 4, float4, float2>::type;
     auto zero = []() { Vec z; memset(&z, 0, sizeof(z)); return z; };
@@ -688,8 +686,15 @@ void launch_attn(const AttnPlan& p, const AttnArgs& a, AttnPart part, long split
     }
     if (p.splits > 1 && part != ATTN_SPLITS) {
         const int rows = p.tq * p.hq, beside = part == ATTN_MERGE && runtime().order.ended(splits_at) ? 1 : 0;
-        launch_kernel(attn_combine_kernel<DV>, dim3(ceil_div(rows, 4)), dim3(128), 0, s, p.ws_o, p.ws_ml, p.splits, rows, p.hq,
-                      BIASED && p.bias_exp > 0.f ? 1.f : a.scale_log2, p.out, p.out_ld, p.out_cols, p.sink, p.out_scale, beside);
+        auto merge = [&](auto kernel) {
+            launch_kernel(kernel, dim3(ceil_div(rows, 4)), dim3(128), 0, s, p.ws_o, p.ws_ml, p.splits, rows, p.hq,
+                          BIASED && p.bias_exp > 0.f ? 1.f : a.scale_log2, p.out, p.out_ld, p.out_cols, p.sink, p.out_scale, beside);
+        };
+        // 24 at once where 12 would take a second round trip, and where rows are many; a few rows of a few splits only pay for the longer list.
+        // Attention and merge, back to back, us, 12 / 24 at once: 60 rows x 16/4 heads, 18 splits 16.0 / 14.3, 4 splits 11.8 / 12.3, 8 splits 12.1 / 12.4;
+        // 1 row x 32/2, 18 splits 10.6 / 9.9, 4 splits 9.2 / 9.4; 33 rows x 32/2, 4 splits 11.9 / 12.3; 60 rows x 32/2, 4 splits 12.4 / 12.1, 12 splits 24.3 / 23.6
+        if (p.splits > 12 || rows > 8 * runtime().num_sms) merge(attn_combine_kernel<DV, 24>);
+        else merge(attn_combine_kernel<DV, 12>);
     }
 }
 }  // namespace
