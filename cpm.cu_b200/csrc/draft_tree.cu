@@ -62,9 +62,10 @@ __device__ uint32_t warp_select(uint32_t* keys, int n, int k, int lane) {
 // threshold's lp (tau) and no more (k candidates of one segment above it would have raised it), so the candidates above it (got, in order)
 // stay, and the places behind them go to the lowest indices at it: from a segment's own logits where it may hide some, and each such
 // segment has one at least, else from its candidates.  k passes over the row by one warp took 4.3 ms a level at 73448 entries, which two
-// levels of a 64-token request met; ten rows with their best entries in one segment 9.7 ms, now 55 us (45 without any).
-__device__ __noinline__ int2 entries_at_threshold(const bf16* x, int vocab, const float4* rst, const unsigned long long* mycand, int nseg, int k, uint32_t got,
-                                                  uint32_t tau, float mx, float ls, int lane) {
+// levels of a 64-token request met, and 9.7 ms for ten rows with their best entries in one segment.  Now a level of ten such rows takes 33 us
+// by itself (without overlap; the mean of six levels), 21.2 us where nothing is hidden (32768 entries 21.1 and 15.4, 4096 14.7 and 13.3).
+__device__ __forceinline__ int2 entries_at_threshold(const bf16* x, int vocab, const float4* rst, const unsigned long long* mycand, int nseg, int k,
+                                                     uint32_t got, uint32_t tau, float mx, float ls, int lane) {
     int my_idx = 0;
     auto lp_of = [&](bf16 v) { return __float2bfloat16(__bfloat162float(v) - mx - ls); };
     int have = __popc(__ballot_sync(0xffffffffu, lane < k && (got >> 16) > tau));
@@ -112,8 +113,9 @@ __device__ __noinline__ int2 entries_at_threshold(const bf16* x, int vocab, cons
 // candidate still reaches the answer's threshold lp (all k of its candidates compete in the top bucket); the last
 // CTA detects that and looks for such a row's entries at the threshold in those segments' logits.  With 36 segments and k = 10 this
 // needs ten of a row's best entries inside one segment; the small vocabularies of the tests take the path routinely.
-// Three CTAs per SM: the full vocabulary's 360 are one wave (with two per SM the six levels of a step took 1.432 ms with their passes, now 1.411).
-__global__ void __launch_bounds__(SCAN_THREADS, 3) draft_level_kernel(DraftTreeState st, const bf16* __restrict__ logits, int ld, int vocab, int nseg,
+// 40 registers, three CTAs per SM: the full vocabulary's 360 are one wave.  The search for hidden entries in the loop over rows, as a call or in place, made
+// levels without any slower (32768 entries 15.4 -> 16.6 us, 73448 21.4 -> 21.9; draft half of a step over 32768 1.082 -> 1.086 ms, 1.078 now).
+__global__ void draft_level_kernel(DraftTreeState st, const bf16* __restrict__ logits, int ld, int vocab, int nseg,
                                    float4* __restrict__ stats, unsigned long long* __restrict__ cand,
                                    unsigned* __restrict__ ticket, int level, const int32_t* __restrict__ last_row_ptr,
                                    int group_rows) {
@@ -233,6 +235,7 @@ __global__ void __launch_bounds__(SCAN_THREADS, 3) draft_level_kernel(DraftTreeS
     __shared__ int s_pos[32 * 32];
     __shared__ uint32_t s_ckey[32 * 32];
     __shared__ int s_sel[32];
+    __shared__ float2 s_stat[32];
     __shared__ uint64_t s_oldmask[32];
     const int per_row = nseg * k;
     constexpr int NW = SCAN_THREADS / 32;
@@ -242,6 +245,7 @@ __global__ void __launch_bounds__(SCAN_THREADS, 3) draft_level_kernel(DraftTreeS
         // one coalesced pass brings the group's candidate lists on chip
         for (int i = threadIdx.x; i < gn * per_row; i += SCAN_THREADS) sh_keys[i] = cand[static_cast<size_t>(g0) * per_row + i];
         __syncthreads();
+        uint32_t crowded = 0u;
         for (int rr = warp; rr < gn; rr += NW) {
             const int r = g0 + rr;
             unsigned long long* mycand = sh_keys + static_cast<size_t>(rr) * per_row;
@@ -286,11 +290,12 @@ __global__ void __launch_bounds__(SCAN_THREADS, 3) draft_level_kernel(DraftTreeS
             }
             bf16 my_lp = __float2bfloat16(0.f);
             int my_idx = 0;
-            if (__any_sync(0xffffffffu, saturated)) {
-                const int2 at = entries_at_threshold(logits + static_cast<size_t>(r + row0) * ld, vocab, rst, mycand, nseg, k, got, tau, mx, ls, lane);
-                my_idx = at.x;
-                my_lp = __ushort_as_bfloat16(static_cast<unsigned short>(at.y));
-            } else if (got) {
+            if (__any_sync(0xffffffffu, saturated)) {   // below, out of the common rows' way
+                crowded |= 1u << (rr / NW);   // at most two rows a warp
+                if (lane < k) mysel[lane] = got;
+                if (lane == 0) s_stat[rr] = make_float2(mx, ls);
+            }
+            if (got) {
                 const unsigned long long c = mycand[0xFFFF - (got & 0xFFFFu)];
                 my_idx = key_index(c);
                 my_lp = __float2bfloat16(__bfloat162float(bf16_from_orderable(static_cast<uint32_t>(c >> 32))) - mx - ls);
@@ -298,6 +303,20 @@ __global__ void __launch_bounds__(SCAN_THREADS, 3) draft_level_kernel(DraftTreeS
             if (lane < k) {
                 s_val[r * k + lane] = my_lp;
                 s_pos[r * k + lane] = my_idx;
+            }
+        }
+        // after the loop: as a call inside it, the rows that need nothing of the kind paid for it
+        __syncwarp();
+        for (int rr = warp; crowded != 0u; rr += NW, crowded >>= 1) {
+            if ((crowded & 1u) == 0u) continue;
+            const int r = g0 + rr;
+            const uint32_t got = lane < k ? sel_keys[static_cast<size_t>(rr) * per_row + lane] : 0u;
+            const float2 ms = s_stat[rr];
+            const int2 at = entries_at_threshold(logits + static_cast<size_t>(r + row0) * ld, vocab, stats + static_cast<size_t>(r) * nseg,
+                                                 sh_keys + static_cast<size_t>(rr) * per_row, nseg, k, got, __shfl_sync(0xffffffffu, got, k - 1) >> 16, ms.x, ms.y, lane);
+            if (lane < k) {
+                s_val[r * k + lane] = __ushort_as_bfloat16(static_cast<unsigned short>(at.y));
+                s_pos[r * k + lane] = at.x;
             }
         }
         __syncthreads();
