@@ -8,8 +8,8 @@
 // layout keeps the R rows of a k-block together), the eight warps take k-blocks in turn, and only sums of one CTA
 // meet.  A warp keeps eight 16-byte loads per lane in flight, the first of them before the wait for the predecessor.  About
 // 20 instructions per 16 bytes leave three quarters of the issue slots free at the HBM rate.
-// Back to back, weights from HBM, tensor-core tiles / this: 2048 x 2048 7.0 / 3.5 us, 2048 x 8192 11.0 / 8.1, 4096 x 16384 22.8 / 21.2,
-// 11008 x 4096 gated 39.8 / 28.8, 73448 x 4096 88 / 84 (7.2 TB/s); 512 x 256 3.7 / 3.5.
+// Back to back, weights from HBM, tensor-core tiles / this: 2048 x 2048 7.0 / 2.6 us, 2048 x 8192 11.0 / 7.4, 4096 x 16384 22.8 / 19.9,
+// 73448 x 4096 88 / 83 (7.2 TB/s); 512 x 256 3.7 / 3.3.
 #include "common.cuh"
 #include "layered.cuh"
 #include "row_ops.cuh"
@@ -128,9 +128,15 @@ one_row_kernel(const OneRowArgs a) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int kb = kb0 + u * ONE_WARPS;
-            const uint4* px = reinterpret_cast<const uint4*>(x + kb * BLOCK_COLS);
-            if (ahead) xv[u] = kb < kblocks ? __ldcg(px) : make_uint4(0u, 0u, 0u, 0u);   // the first-level cache has not been waited for
-            else xv[u] = kb < kblocks ? *px : make_uint4(0u, 0u, 0u, 0u);
+            // the choice of the load only where there is one: in every kernel, even as a constant, it cost products of long rows
+            // (4096 x 16384 21.1 us instead of 19.9, 512 x 16384 10.7 and 9.6, 4096 x 4096 6.26 and 6.06)
+            if constexpr (EARLY) {
+                xv[u] = kb < kblocks ? *reinterpret_cast<const uint4*>(x + kb * BLOCK_COLS) : make_uint4(0u, 0u, 0u, 0u);
+            } else {
+                const uint4* px = reinterpret_cast<const uint4*>(x + kb * BLOCK_COLS);
+                if (ahead) xv[u] = kb < kblocks ? __ldcg(px) : make_uint4(0u, 0u, 0u, 0u);   // the first-level cache has not been waited for
+                else xv[u] = kb < kblocks ? *px : make_uint4(0u, 0u, 0u, 0u);
+            }
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
