@@ -157,6 +157,7 @@ struct Raw8 {
 // Without experts, with them, or with them for one row.  Many rows are bound by memory and hide one another's round trips (4096 rows of 2048 with
 // the loads of one row: 45 -> 48.5 us, without experts 18 -> 21); one row is a chain of round trips: the router's choice and the
 // stream are asked for before the wait (MoeMix::early), then eight experts' pieces at once.  A token of six layers of 4096 580 -> 571 us.
+// Rows wider than 4096 (four pieces a thread) keep the form of many rows; one row of them has not been measured.
 enum Mixture { NO_MIX, MIX_ROWS, MIX_ONE };
 template <typename T, int VPT, Mixture MIX>
 __global__ void __launch_bounds__(512)
