@@ -103,6 +103,7 @@ _SIGNATURES = {
     "cpmcu_silu_gate": (_c_int, [_c_void_p, _c_void_p, _c_int, _c_int]),
     "cpmcu_linear_swiglu_bf16": (_c_int, [_c_void_p] * 3 + [_c_int] * 4),
     "cpmcu_debug_decode_graphs": (_c_int, [_c_void_p, _c_int, _c_void_p]),
+    "cpmcu_debug_moe_pairs": (_c_int, [_c_int] * 5),
     "cpmcu_debug_launch_order": (_c_int, [_c_void_p, _c_int, _c_void_p]),
     "cpmcu_debug_linear_schedule": (_c_int, [_c_int] * 4 + [_c_void_p, _c_int]),
     "cpmcu_argmax": (_c_int, [_c_void_p, _c_int, _c_int, _c_void_p]),

@@ -477,6 +477,13 @@ int cpmcu_debug_decode_graphs(const int32_t* shapes, int n, int32_t* acts) {
     });
 }
 
+int cpmcu_debug_moe_pairs(int tile, int n_tiles, int kblocks, int tiles, int sms) {
+    return guarded([&] {
+        CPM_REQUIRE(tile >= 1 && n_tiles >= 1 && kblocks >= 1 && tiles >= 1 && sms >= 1, "debug_moe_pairs: bad arguments");
+        return moe_gemm_on_pairs(tile, n_tiles, kblocks, tiles, sms) ? 1 : 0;
+    });
+}
+
 int cpmcu_debug_launch_order(const int32_t* holds, int n, int32_t* ended) {
     return guarded([&] {
         CPM_REQUIRE(holds != nullptr && ended != nullptr && n >= 0, "debug_launch_order: bad arguments");

@@ -313,6 +313,8 @@ MoeGemmPlan make_moe_down_plan(const LayerSpec& sp, const bf16* w, const bf16* a
 // the choice at once and are refused where the router may still be running.  Right behind a router before which everything has ended, the shared
 // expert's part of one row's gate/up product runs beside it.
 void launch_moe_gemm(const MoeGemmPlan& p, cudaStream_t s, long routed);
+// Whether a launch with groups of `tile` rows runs on pairs of CTAs: n_tiles tiles of 128 weight rows and kblocks blocks of 64 columns a matrix, `tiles` in all at most
+bool moe_gemm_on_pairs(int tile, int n_tiles, int kblocks, long long tiles, int sms);
 // n products over one input (make_grouped_plan), no router.  hold: the next launch starts only after this one's wait (one row)
 void launch_grouped(const MoeGemmPlan& p, cudaStream_t s, bool hold = false);
 void launch_moe_one_row(const MoeGemmPlan& p, cudaStream_t s, bool hold, bool ahead);   // rows == 1 (one_row.cu)

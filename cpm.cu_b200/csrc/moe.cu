@@ -984,8 +984,6 @@ MoeGemmPlan make_moe_down_plan(const LayerSpec& sp, const bf16* w, const bf16* a
     return p;
 }
 
-namespace {
-
 // Where pairs of CTAs are the faster way: with groups of 256 rows from some forty k-blocks a CTA on, of 128 rows from 256 on (their operands are a
 // smaller load), and not with fewer than 16 k-blocks a tile, whatever the number of tiles: a pair starts and ends its tiles 0.5 to 1 us later.
 // Groups of 64 rows and fewer leave a pair as much weight to fetch as two CTAs, and halves of 32 rows to multiply them with.
@@ -993,10 +991,12 @@ namespace {
 // 4 x 2048 x 2048 at 160 rows 20.5 / 22.0 and at 256 rows 24.1 / 22.5, at 520 rows 36.9 / 34.7; 3 experts of 1408 in width 2048, down, at 512 rows 12.5 / 13.4,
 // at 1024 rows 19.0 / 17.3; 4 x 3072 x 3072 at 129 rows 28.7 / 27.6, at 1024 rows 76 / 67.  Groups of 128: 4 x 3072 x 3072 26.6 / 27.7, 62 experts of
 // 640 in width 2048 at 1024 rows 64.4 / 65.0 and 31.5 / 34.7, 60 of 1024 at 1024 rows 111 / 108.5 and 58.3 / 59.0.
-bool pairs_pay(int tile, int kblocks, long long tiles) {
-    const long long per_cta = kblocks * ((tiles + runtime().num_sms - 1) / runtime().num_sms);
-    return kblocks >= 16 && ((tile == 256 && per_cta > 32) || (tile == 128 && per_cta > 256));
+bool moe_gemm_on_pairs(int tile, int n_tiles, int kblocks, long long tiles, int sms) {
+    const long long per_cta = kblocks * ((tiles + sms - 1) / sms);
+    return n_tiles % 2 == 0 && kblocks >= 16 && ((tile == 256 && per_cta > 32) || (tile == 128 && per_cta > 256));
 }
+
+namespace {
 
 void launch_tiles(const MoeGemmPlan& p, cudaStream_t s) {
     GemmArgs a;
@@ -1012,7 +1012,7 @@ void launch_tiles(const MoeGemmPlan& p, cudaStream_t s) {
     a.error = runtime().d_error;
     const long long most = static_cast<long long>(a.groups_s) * a.n_tiles_s + static_cast<long long>(p.max_entries) * p.n_tiles;
     const int grid = static_cast<int>(std::max<long long>(1, std::min<long long>(most, runtime().num_sms)));
-    if (p.n_tiles % 2 == 0 && pairs_pay(p.tile, p.kblocks, most)) {
+    if (moe_gemm_on_pairs(p.tile, p.n_tiles, p.kblocks, most, runtime().num_sms)) {
         a.n_tiles /= 2;
         a.n_tiles_s = ceil_div(a.n_tiles_s, 2);   // the shared matrix is the last one: an odd tile's partner reads zeros beyond the map
         const long long jobs = static_cast<long long>(a.groups_s) * a.n_tiles_s + static_cast<long long>(p.max_entries) * a.n_tiles;

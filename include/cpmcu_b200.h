@@ -265,6 +265,10 @@ int cpmcu_debug_linear_schedule(int M, int N, int K, int grid_limit, int32_t* ou
  * that tell shapes apart) on a Llama-format model: acts (HOST int32[n]) = 0 launched kernel by kernel, 1 captured first, 2 replayed. */
 int cpmcu_debug_decode_graphs(const int32_t* shapes, int n, int32_t* acts);
 
+/* Host only, no GPU needed: 1 where a grouped product runs on pairs of CTAs, with row groups of `tile`, n_tiles tiles of 128 weight rows and
+ * kblocks blocks of 64 columns a matrix, `tiles` tiles x groups in all, on a GPU of `sms` SMs; 0 where it runs on single CTAs. */
+int cpmcu_debug_moe_pairs(int tile, int n_tiles, int kblocks, int tiles, int sms);
+
 /* Host only, no GPU needed: of n launches, of which those with holds[i] != 0 let their successor start only after their own wait for
  * their predecessor and the others at once, ended (HOST int32[n]) = how many have surely ended when launch i starts (0 <= ended[i] <= i). */
 int cpmcu_debug_launch_order(const int32_t* holds, int n, int32_t* ended);
