@@ -113,10 +113,11 @@ void launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = runtime().pdl ? 1 : 0;
+    Runtime& rt = runtime();
+    cfg.numAttrs = rt.pdl ? 1 : 0;
     CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...));
-    runtime().launches++;
-    runtime().order.launched();
+    rt.launches++;
+    rt.order.launched();
 }
 
 // The same for a kernel that runs as thread-block clusters of `cluster` CTAs (grid.x a multiple of it).
@@ -136,10 +137,11 @@ void launch_kernel_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = runtime().pdl ? 2 : 1;
+    Runtime& rt = runtime();
+    cfg.numAttrs = rt.pdl ? 2 : 1;
     CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...));
-    runtime().launches++;
-    runtime().order.launched();
+    rt.launches++;
+    rt.order.launched();
 }
 
 // Clusters of `cluster` CTAs of this kernel that the device runs at once (0 when the query fails).  The SMs
